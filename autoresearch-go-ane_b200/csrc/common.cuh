@@ -20,6 +20,7 @@ enum DeviceStatus : int {
   DEV_MBAR_TIMEOUT_PRODUCER = 101,
   DEV_MBAR_TIMEOUT_MMA = 102,
   DEV_MBAR_TIMEOUT_EPILOGUE = 103,
+  DEV_GRID_TIMEOUT = 104,
   DEV_BAD_INDEX = 110,
 };
 

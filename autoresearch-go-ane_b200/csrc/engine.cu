@@ -266,7 +266,14 @@ class EngineT final : public EngineBase {
   bool x3_ = false;      // fp32 engine whose GEMMs run as three bf16 tensor-core products (ANE_DTYPE_BF16X3)
   SplitScratch split_;   // its operand halves (one stream at a time: no side stream in this mode)
   bool decoding_ = false;  // forward() runs one KV-cached decode step
-  std::vector<T*> kcache_, vcache_;  // [B, S_, KV*hd] per layer, allocated by the first decode
+  std::vector<T*> kcache_, vcache_;  // [B, S_, KV*hd] per layer (one block each for all layers), allocated by the first decode
+  // scratch of the persistent decode kernel (bf16 engines)
+  float* dec_x_ = nullptr;
+  bf16 *dec_q_ = nullptr, *dec_att_ = nullptr, *dec_gate_ = nullptr;
+  unsigned long long* dec_best_ = nullptr;
+  double* dec_psum_ = nullptr;
+  unsigned* dec_bar_ = nullptr;
+  uint8_t* dec_words_ = nullptr;
   int32_t* d_argmax_ = nullptr;
   double* d_dec_u_ = nullptr;  // uniform draws of a sampling decode, [n_new][n_seq]
   uint16_t *d_dec_tok_ = nullptr, *d_dec_out_ = nullptr;
@@ -1812,9 +1819,23 @@ int EngineT<T>::decode(const uint16_t* prompts, uint32_t n_seq, uint32_t prompt_
   if (kcache_.empty()) {
     kcache_.assign(L_, nullptr);
     vcache_.assign(L_, nullptr);
+    T *kc = nullptr, *vc = nullptr;
+    const size_t per_layer = (size_t)B_ * S_ * KVD_;
+    if ((rc = dalloc(&kc, per_layer * L_)) != 0 || (rc = dalloc(&vc, per_layer * L_)) != 0) {
+      kcache_.clear();
+      return rc;
+    }
     for (int l = 0; l < L_; ++l) {
-      if ((rc = dalloc(&kcache_[l], (size_t)B_ * S_ * KVD_)) != 0) return rc;
-      if ((rc = dalloc(&vcache_[l], (size_t)B_ * S_ * KVD_)) != 0) return rc;
+      kcache_[l] = kc + per_layer * l;
+      vcache_[l] = vc + per_layer * l;
+    }
+    if constexpr (!kIsF32) {
+      const size_t rows = std::min(B_, 32);  // the persistent kernel takes up to 32 sequences at a time
+      if ((rc = dalloc(&dec_x_, rows * D_)) != 0 || (rc = dalloc(&dec_q_, rows * QD_)) != 0 || (rc = dalloc(&dec_att_, rows * QD_)) != 0 ||
+          (rc = dalloc(&dec_gate_, rows * Hd_)) != 0 || (rc = dalloc(&dec_best_, 3 * rows)) != 0 ||
+          (rc = dalloc(&dec_psum_, rows * gemm_num_sms())) != 0 || (rc = dalloc(&dec_bar_, 1)) != 0 ||
+          (rc = dalloc(&dec_words_, decode_words_bytes(D_, Hd_, H_, KV_, hd_))) != 0)
+        return rc;
     }
     if ((rc = dalloc(&d_argmax_, B_)) != 0) return rc;
     if ((rc = dalloc(&d_dec_tok_, B_)) != 0) return rc;
@@ -1846,8 +1867,38 @@ int EngineT<T>::decode(const uint16_t* prompts, uint32_t n_seq, uint32_t prompt_
     return 0;
   };
   if ((rc = next_token(P, 0)) != 0) return rc;
+  bool done = false;
+  if constexpr (!kIsF32) {
+    if (decode_steps_supported(D_, Hd_, H_, KV_, hd_, V_, std::min(B, 32))) {
+      wait_all_buckets();
+      for (int b0 = 0; b0 < B; b0 += 32) {
+        DecodeArgs a;
+        a.w = Sh_; a.p = P_;
+        a.off_qkv = s_qkv_[0].off; a.off_wo = s_wo_[0].off; a.off_w13 = s_w13_[0].off; a.off_w2 = s_w2_[0].off;
+        a.layer_stride = L_ > 1 ? s_qkv_[1].off - s_qkv_[0].off : 0;
+        a.off_embed = a.off_embed_f32 = s_embed_.off;
+        a.off_rms_att = s_rms_att_[0].off; a.off_rms_ffn = s_rms_ffn_[0].off; a.off_rms_final = s_rms_final_.off;
+        a.rms_stride = L_ > 1 ? s_rms_att_[1].off - s_rms_att_[0].off : 0;
+        a.cosb = rope_cos_; a.sinb = rope_sin_;
+        a.kcache = kcache_[0] + (size_t)b0 * S_ * KVD_; a.vcache = vcache_[0] + (size_t)b0 * S_ * KVD_;
+        a.kv_layer = (size_t)B_ * S_ * KVD_;
+        a.x = dec_x_; a.q = dec_q_; a.att = dec_att_; a.gate = dec_gate_;
+        a.logits = logits_; a.best = dec_best_; a.psum = dec_psum_;
+        a.u = d_dec_u_ + b0; a.u_stride = B;
+        a.tok = d_dec_tok_ + b0; a.out = d_dec_out_ + (size_t)b0 * n_new;
+        a.bar = dec_bar_; a.status = d_status_;
+        a.temperature = sampling ? temperature : 0.f;
+        a.B = std::min(32, B - b0); a.D = D_; a.Hd = Hd_; a.L = L_; a.H = H_; a.KV = KV_; a.hd = hd_; a.V = V_; a.S = S_;
+        a.prompt = P; a.n_new = (int)n_new;
+        count_launch();
+        if (decode_steps(a, dec_words_, gemm_num_sms(), stream_) != 0)
+          return fail(ANE_ERR_KERNEL, "storiesane decode: persistent kernel launch failed");
+      }
+      done = true;
+    }
+  }
   decoding_ = true;
-  for (int step = 1; step < (int)n_new; ++step) {
+  for (int step = 1; step < (int)n_new && !done; ++step) {
     const int pos = P + step - 1;  // position of the token generated in the previous step
     if ((rc = forward(d_dec_tok_, B, 1, pos)) != 0) {
       decoding_ = false;

@@ -98,6 +98,35 @@ template <typename T>
 void attention_decode_simt(const T* qkv, const T* kcache, const T* vcache, T* out, int B, int max_seq, int pos, int H,
                            int KV, int hd, float scale, cudaStream_t s);
 
+// All steps of a generation after the first token in one persistent kernel (decode.cu): bf16 weights, llama-style
+// architecture, up to 32 sequences.  `w` / `p` are the flat bf16 and fp32 parameter buffers with element offsets of
+// layer 0's tensors; layers follow at layer_stride (matrices) and rms_stride (norm weights).
+struct DecodeArgs {
+  const bf16* w;
+  const float* p;
+  size_t off_qkv, off_wo, off_w13, off_w2, layer_stride, off_embed, off_embed_f32;
+  size_t off_rms_att, off_rms_ffn, rms_stride, off_rms_final;
+  const float *cosb, *sinb;      // rotation tables [positions, hd / 2]
+  bf16 *kcache, *vcache;         // [L][B, S, KV * hd] with kv_layer elements per layer
+  size_t kv_layer;
+  float* x;                      // scratch: residual stream [B, D]
+  bf16 *q, *att, *gate;          // scratch: [B, H * hd], [B, H * hd], [B, Hd]
+  float* logits;                 // scratch [B, V], written when sampling
+  unsigned long long* best;      // scratch [3][B]
+  double* psum;                  // scratch [CTAs][B]
+  const double* u;               // draws [n_new][u_stride]
+  uint16_t *tok, *out;           // tok [B]: the first token in; out [B][n_new], columns 1.. are written
+  unsigned* bar;
+  int* status;
+  float temperature;             // <= 1e-6: argmax
+  int B, D, Hd, L, H, KV, hd, V, S, prompt, n_new, u_stride;
+  int umax, group, stage_bytes;  // set by decode_steps
+  uint2 *w_x0, *w_x1, *w_qkv, *w_att, *w_gate;
+};
+bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int batch);
+size_t decode_words_bytes(int D, int Hd, int H, int KV, int hd);  // size of `words`, scratch for exchanges between SMs
+int decode_steps(DecodeArgs a, void* words, int sms, cudaStream_t s);
+
 // Tensor-core causal attention (bf16 operands, head_dim 64 only; see attention_tc.cu).
 bool attention_tc_supported(int hd);
 // `out_lo` (optional, [M, H*64] like `out`) receives bf16(O - bf16(O)): given to the backward as well, it makes
