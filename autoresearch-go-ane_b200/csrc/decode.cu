@@ -7,8 +7,9 @@
 // one CTA per SM stays resident and walks through the five phases of a layer (q|k|v, attention, Wo, W1|W3, W2).  What
 // bounds it is the latency of a phase: how fast one SM's results reach all others, and the chain of instructions
 // between reading activations and publishing results.  So:
-//   * Weights never change: each warp requests its share of the NEXT phase's weights (cp.async) before it waits
-//     for that phase's activations, so the weight stream runs under the exchange.
+//   * Weights never change, and the 8 weight rows of a unit are one contiguous piece of 16 K bytes: one thread streams
+//     them into a ring of shared-memory slots with bulk copies, as far ahead as the ring reaches, across phases and steps.
+//     (Measured with all SMs reading: 30 B/clk per SM through per-lane loads or cp.async, 70 through bulk copies.)
 //   * Up to 8 sequences (R8 = 1): results are exchanged as 8-byte words {value, epoch}, written and read with single
 //     64-bit accesses.  A reader polls the words it needs; there is no barrier, no fence and no second round trip (a
 //     grid barrier with its stores and loads takes 1.8 us on this GPU, a flagged word about 0.6).  A word is not
@@ -22,8 +23,8 @@
 // SMs.  tcgen05 tiles start at 64 rows of A and would leave most of the tile empty.  Inside a CTA the sixteen warps split
 // the contraction in 32-wide chunks (a warp's A fragments then stay in registers for all units of the CTA) and their
 // partial sums meet in shared memory.  The order of k inside a chunk is free as long as both operands agree, so every
-// lane requests 16 contiguous bytes of a weight row (k = 8 (lane % 4) ..) and uses them as the fragments of two MMAs: no
-// ldmatrix, and nobody else ever reads its slot.
+// lane reads 16 contiguous bytes of a weight row (k = 8 (lane % 4) ..) and uses them as the fragments of two MMAs: no
+// ldmatrix.
 #include <algorithm>
 
 #include "common.cuh"
@@ -42,17 +43,25 @@ struct Part {
   static constexpr int kVecs = kTile * (R8 == 4 ? 2 : 1);
 };
 
-// 16 bytes of a weight row into this lane's slot of the ring (zeros instead when `in` is false); past L1
-__device__ __forceinline__ void request_weight(uint32_t slot, const bf16* p, bool in) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(slot), "l"(p), "r"(in ? 16 : 0) : "memory");
+// `bytes` of global memory into shared memory, counted on the barrier
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
-__device__ __forceinline__ void requests_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void requests_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+// Values that other SMs wrote earlier in this kernel: L2 only.  Predicated in one instruction, so that a run of them is
+// in flight together.
+__device__ __forceinline__ uint4 ld_l2_if(const void* p, bool take) {
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+      "@p ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((uint32_t)take) : "memory");
+  return v;
 }
-// Values that other SMs wrote earlier in this kernel: L2 only.
-__device__ __forceinline__ uint4 ld_l2(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
+__device__ __forceinline__ float4 ldf_l2_if(const float* p, bool take) {
+  const uint4 v = ld_l2_if(p, take);
+  return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
@@ -69,6 +78,13 @@ __device__ __forceinline__ float sigmoid(float x) {
 __device__ __forceinline__ void mma16816(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Rows 0-7 only: the accumulators of rows 8-15 are not kept.
+__device__ __forceinline__ void mma16816_top(float& c0, float& c1, uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  [[maybe_unused]] float x, y;
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %5}, {%7, %8}, {%0, %1, %9, %9};"
+               : "+f"(c0), "+f"(c1), "=f"(x), "=f"(y) : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 // ---- exchange of results between SMs (R8 = 1) -----------------------------------------------------------------------
@@ -117,8 +133,8 @@ struct GridBarrier {
       asm volatile("fence.acq_rel.gpu;\n\tred.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
       unsigned seen;
       long long t0 = 0;
-  #pragma unroll 1
-    for (unsigned n = 0;; ++n) {
+#pragma unroll 1
+      for (unsigned n = 0;; ++n) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
         if ((int)(seen - target) >= 0 || wait.expired(n, t0)) break;
       }
@@ -130,198 +146,193 @@ struct GridBarrier {
 
 // ---- products -------------------------------------------------------------------------------------------------------
 enum Kind { kQkv = 0, kWo = 1, kW13 = 2, kW2 = 3, kHead = 4 };
-// One product's share of this CTA (in shared memory): `nu` units of 8 weight rows.
+// One product's share of this CTA (in shared memory): `nu` units of 8 weight rows, the first at row `row`, the others in
+// alternating steps of inc[0] and inc[1] rows (the grid is a multiple of 4, so W1|W3 blocks keep their phase).
 struct Prod {
   size_t off, layer_stride;
-  int K, nu, u0, kind;
-  __device__ __forceinline__ int row0(int i) const {
-    if (kind == kHead) return (u0 + i) * 8;  // a contiguous range of the vocabulary
-    if (kind != kW13) return ((int)blockIdx.x + i * (int)gridDim.x) * 8;
-    // W1 and W3 lie in blocks of 32 rows; units 2j and 2j+1 are matching rows of the two
-    const int p = (int)blockIdx.x + (i >> 1) * (int)gridDim.x;
-    return (p >> 2) * 64 + (p & 3) * 8 + (i & 1) * 32;
-  }
+  int K, nu, row, inc[2], u0, kind, per;  // per: units of a group
+  __device__ __forceinline__ int row0(int i) const { return row + (i >> 1) * (inc[0] + inc[1]) + (i & 1) * inc[0]; }
 };
-__device__ __forceinline__ void make_prod(Prod& d, int kind, size_t off, size_t layer_stride, int K, int n_units) {
+__device__ __forceinline__ void make_prod(Prod& d, int kind, size_t off, size_t layer_stride, int K, int n_units, int per) {
   const int g = (int)gridDim.x, b = (int)blockIdx.x;
   d.off = off;
   d.layer_stride = layer_stride;
   d.K = K;
   d.kind = kind;
+  d.per = per;
   d.u0 = 0;
-  if (kind == kHead) {
+  if (kind == kHead) {  // a contiguous range of the vocabulary
     d.u0 = (int)((long long)n_units * b / g);
     d.nu = (int)((long long)n_units * (b + 1) / g) - d.u0;
-  } else if (kind == kW13) {
+    d.row = d.u0 * 8;
+    d.inc[0] = d.inc[1] = 8;
+  } else if (kind == kW13) {  // W1 and W3 lie in blocks of 32 rows; units 2j and 2j+1 are matching rows of the two
     const int pairs = n_units / 2;
     d.nu = b < pairs ? 2 * ((pairs - b + g - 1) / g) : 0;
+    d.row = (b >> 2) * 64 + (b & 3) * 8;
+    d.inc[0] = 32;
+    d.inc[1] = 16 * g - 32;
   } else {
     d.nu = b < n_units ? (n_units - b + g - 1) / g : 0;
+    d.row = b * 8;
+    d.inc[0] = d.inc[1] = 8 * g;
   }
 }
 
-// A warp's walk over the weights of units [first, first + n) of a product.  Eight 16-byte vectors per lane are in
-// flight, each in a shared-memory slot of its lane (registers would be spilled while activations are staged, and a
-// spill waits for its load): four units of up to two 32-wide chunks, or two units of up to four chunks (longer
-// contractions block by block).
-constexpr int kSlots = 8;
-constexpr int kRingBytes = kWarps * kSlots * 512;
-struct Walk {
-  uint32_t ring;       // this lane's first slot
-  const bf16* base;    // weights + this lane's column
-  int K, k0, nc;       // this lane's first column, this warp's chunks
-  int unit, end, blk;  // next to request
-  template <int NCB>
-  __device__ __forceinline__ void request(const Prod& p, int slot) {
-    if (unit < end) {  // warp-uniform
-      const int lane = threadIdx.x & 31;
-      const bf16* q = base + (size_t)(p.row0(unit) + (lane >> 2)) * K + blk * 128;
-      const int k = k0 + blk * 128, left = nc - blk * 4;
-#pragma unroll
-      for (int c = 0; c < NCB; ++c) {
-        const bool in = k + c * 32 < K;
-        if (c < left) request_weight(ring + (uint32_t)(slot + c) * 512u, in ? q + c * 32 : q, in);
-      }
-      if (NCB == 2 || ++blk * 4 >= nc) {
-        blk = 0;
-        ++unit;
-      }
-    }
-    requests_commit();  // one group per block, empty or not
-  }
-  __device__ __forceinline__ void start(const Prod& p, const bf16* w, int first, int n) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    K = p.K;
-    const int chunks = (K + 31) >> 5, per = (chunks + kWarps - 1) / kWarps, c0 = min(warp * per, chunks);
-    nc = min(per, chunks - c0);
-    k0 = c0 * 32 + (lane & 3) * 8;
-    base = w + k0;
-    unit = first;
-    end = nc > 0 ? first + n : 0;
-    blk = 0;
-    if (nc <= 2) {
+// The weights of the whole generation in the order they are used, in groups of up to kUnits units of one product, each
+// group in one slot of the ring.  One lane of the last warp, which has little to do in the epilogues, issues; a slot is
+// free again after the CTA barrier behind its MMAs.
+template <int R8>
+struct Ring {
+  static constexpr int kUnits = R8 == 4 ? 2 : 4;  // per group; even, because W1|W3 units come in pairs
+  static constexpr int kSlots = R8 == 4 ? 4 : 3;
+};
+__device__ __forceinline__ const float* norm_gains(const DecodeArgs& a, int kind, int layer) {
+  if (kind == kWo || kind == kW2) return nullptr;
+  return a.p + (kind == kHead ? a.off_rms_final : (kind == kQkv ? a.off_rms_att : a.off_rms_ffn) + (size_t)layer * a.rms_stride);
+}
+template <int R8>
+struct Feed {
+  uint32_t bar, slot;  // shared-memory addresses of the first barrier and slot
+  int slot_bytes, issued, used;
+  int step, idx, g0;   // next group
+  __device__ __forceinline__ void issue(const DecodeArgs& a, const Prod* prods) {
 #pragma unroll 1
-      for (int i = 0; i < kSlots; i += 2) request<2>(p, i);
-    } else {
+    while (issued - used < Ring<R8>::kSlots && step < a.n_new) {
+      const int layer = idx >> 2;
+      const Prod& p = prods[layer == a.L ? kHead : idx & 3];
+      const int n = min(p.per, p.nu - g0);
+      if (n > 0) {
+        const int at = issued % Ring<R8>::kSlots;
+        const uint32_t bytes = (uint32_t)p.K * 16u, b = bar + 8u * at;
+        const bf16* w = a.w + p.off + (size_t)layer * p.layer_stride;
+        const float* gains = g0 == 0 ? norm_gains(a, p.kind, layer) : nullptr;  // travel with the first group, at the slot's end
+        mbar_expect_tx(b, bytes * n + (gains ? a.D * 4u : 0u));
+        if (gains) bulk_copy(slot + (uint32_t)((at + 1) * slot_bytes - a.D * 4), gains, a.D * 4u, b);
 #pragma unroll 1
-      for (int i = 0; i < kSlots; i += 4) request<4>(p, i);
+        for (int u = 0; u < n; ++u) bulk_copy(slot + (uint32_t)(at * slot_bytes) + bytes * u, w + (size_t)p.row0(g0 + u) * p.K, bytes, b);
+        ++issued;
+        g0 += n;
+      }
+      if (g0 >= p.nu) {
+        g0 = 0;
+        if (++idx > 4 * a.L) {
+          idx = 0;
+          ++step;
+        }
+      }
     }
   }
 };
 
-// Where a warp's A fragments come from: normalised rows staged in shared memory (read once per product when two chunks
-// or fewer), or, for Wo and W2 (no norm, and mostly one unit per CTA), straight from the exchanged bf16 rows.
-template <int R8>
-struct StagedRows {
-  const uint4* stage;
-  template <int NCB>
-  __device__ __forceinline__ void read(uint4 (&f)[NCB][R8], const Walk& w, int first) const {
-    const uint4* st = stage + (size_t)((w.k0 >> 5) + first) * R8 * 32 + (threadIdx.x & 31);
-#pragma unroll
-    for (int c = 0; c < NCB; ++c)
-#pragma unroll
-      for (int r = 0; r < R8; ++r)
-        if (c < w.nc - first) f[c][r] = st[(c * R8 + r) * 32];
-  }
+// A warp's part of a contraction: chunks [c0, c0 + nc) of 32 columns.
+struct Share {
+  int K, c0, nc;
 };
-template <int R8>
-struct PlainRows {
+__device__ __forceinline__ Share make_share(int K) {
+  const int warp = threadIdx.x >> 5, chunks = (K + 31) >> 5, per = (chunks + kWarps - 1) / kWarps;
+  Share s;
+  s.K = K;
+  s.c0 = min(warp * per, chunks);
+  s.nc = min(per, chunks - s.c0);
+  return s;
+}
+
+// Where a warp's A fragments come from: normalised rows staged in shared memory, or, for Wo and W2 (no norm, and
+// mostly one unit per CTA), straight from the exchanged bf16 rows.
+struct Source {
+  const uint4* stage;  // nullptr: rows / words
   const bf16* rows;
-  int B;
-  template <int NCB>
-  __device__ __forceinline__ void read(uint4 (&f)[NCB][R8], const Walk& w, int first) const {
-    const int g = (threadIdx.x & 31) >> 2;
-#pragma unroll
-    for (int c = 0; c < NCB; ++c) {
-      const int k = w.k0 + (first + c) * 32;
-      const bool in = c < w.nc - first && k < w.K;
-#pragma unroll
-      for (int r = 0; r < R8; ++r) {
-        const bool ok = in && r * 8 + g < B;
-        f[c][r] = ok ? ld_l2(rows + (size_t)(r * 8 + g) * w.K + k) : make_uint4(0, 0, 0, 0);
-      }
-    }
-  }
-};
-struct WordRows {  // R8 = 1; words {two values, epoch}
-  const uint2* words;
+  const uint2* words;  // R8 = 1: {two values, epoch}
   int B;
   uint32_t epoch;
-  Wait wait;
-  template <int NCB>
-  __device__ __forceinline__ void read(uint4 (&f)[NCB][1], const Walk& w, int first) const {
-    const int g = (threadIdx.x & 31) >> 2;
+};
+template <int R8>
+__device__ __forceinline__ void read_a(uint4 (&f)[4][R8], const Source& s, const Share& w, int first, const Wait& wait) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, left = w.nc - first;
+  if (s.stage != nullptr) {
+    const uint4* st = s.stage + (size_t)(w.c0 + first) * R8 * 32 + lane;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int r = 0; r < R8; ++r)
+        if (c < left) f[c][r] = st[(c * R8 + r) * 32];
+    return;
+  }
+  const int k = (w.c0 + first) * 32 + (lane & 3) * 8;
+  if constexpr (R8 == 1) {
+    const uint2* p = s.words + ((size_t)(g < s.B ? g : 0) * w.K + k) / 2;
     long long t0 = 0;
 #pragma unroll 1
     for (unsigned n = 0;; ++n) {
       bool ok = true;
 #pragma unroll
-      for (int c = 0; c < NCB; ++c) {
-        const int k = w.k0 + (first + c) * 32;
-        uint4 x = make_uint4(0, epoch, 0, epoch), y = x;
-        if (c < w.nc - first && k < w.K && g < B) {
-          const uint2* p = words + ((size_t)g * w.K + k) / 2;
-          x = get_words(p);
-          y = get_words(p + 2);
+      for (int c = 0; c < 4; ++c) {
+        uint4 x = make_uint4(0, s.epoch, 0, s.epoch), y = x;
+        if (c < left && k + c * 32 < w.K && g < s.B) {
+          x = get_words(p + c * 16);
+          y = get_words(p + c * 16 + 2);
         }
-        ok = ok && x.y == epoch && x.w == epoch && y.y == epoch && y.w == epoch;
+        ok = ok && x.y == s.epoch && x.w == s.epoch && y.y == s.epoch && y.w == s.epoch;
         f[c][0] = make_uint4(x.x, x.z, y.x, y.z);
       }
       if (__all_sync(0xffffffffu, ok) || wait.expired(n, t0)) return;
     }
-  }
-};
-
-// Partial sums of the n units the walk was started on: this warp's chunks.
-template <int R8, int NCB, class Rows>
-__device__ __forceinline__ void run_units(const Prod& p, Walk& w, int n, float2* part, const Rows& rows) {
-  constexpr int T = (R8 + 1) / 2, BLOCKS = kSlots / NCB;
-  using P = Part<R8>;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float2* d = part + (size_t)warp * P::kVecs + (lane & 3) * P::kPitch + (lane >> 2);
-  float acc[T][4] = {};
-  constexpr int NA = NCB == 4 && R8 == 4 ? 2 : NCB;  // chunks whose A fragments are held together (registers)
-  uint4 a[NA][R8];
-  if (NCB == 2) rows.template read<NA>(a, w, 0);  // all chunks of this warp: the same for every unit
-  int unit = 0, blk = 0, slot = 0;
-#pragma unroll 1
-  while (unit < n) {
-    if (NCB == 4) rows.template read<NA>(a, w, blk * 4);
-    requests_wait<BLOCKS - 1>();
-    const int left = w.nc - blk * 4;
+  } else {
 #pragma unroll
-    for (int c = 0; c < NCB; ++c) {
-      if (NA < NCB && c == NA) rows.template read<NA>(a, w, blk * 4 + NA);
-      if (c < left) {
-        uint4 b;
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "r"(w.ring + (uint32_t)(slot + c) * 512u) : "memory");
+    for (int r = 0; r < R8; ++r) {
+      const bool live = r * 8 + g < s.B;
+      const bf16* p = s.rows + (size_t)(live ? r * 8 + g : 0) * w.K + k;
 #pragma unroll
-        for (int t = 0; t < T; ++t) {
-          const uint4 lo = a[c % NA][2 * t], hi = R8 > 1 ? a[c % NA][R8 > 1 ? 2 * t + 1 : 0] : make_uint4(0, 0, 0, 0);
-          mma16816(acc[t], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-          mma16816(acc[t], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
-        }
-      }
-    }
-    w.request<NCB>(p, slot);
-    slot = (slot + NCB) & (kSlots - 1);
-    if (NCB == 2 || ++blk * 4 >= w.nc) {
-      blk = 0;
-#pragma unroll
-      for (int t = 0; t < T; ++t) {
-        d[t * P::kTile] = make_float2(acc[t][0], acc[t][1]);
-        if (R8 > 1) d[t * P::kTile + 8] = make_float2(acc[t][2], acc[t][3]);
-        acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-      }
-      d += kWarps * P::kVecs;
-      ++unit;
+      for (int c = 0; c < 4; ++c) f[c][r] = ld_l2_if(p + c * 32, live && c < left && k + c * 32 < w.K);
     }
   }
 }
-template <int R8, class Rows>
-__device__ __forceinline__ void run_product(const Prod& p, Walk& w, int n, float2* part, const Rows& rows) {
-  if (w.nc <= 2) run_units<R8, 2>(p, w, n, part, rows);
-  else run_units<R8, 4>(p, w, n, part, rows);
+
+// Partial sums of the n units in a slot (rows of K bf16): this warp's chunks.
+template <int R8>
+__device__ __forceinline__ void run_units(const Share& w, int n, const uint8_t* slot, float2* part, const Source& src, uint4 (&a)[4][R8], bool read, const Wait& wait) {
+  constexpr int T = (R8 + 1) / 2;
+  using P = Part<R8>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2* d = part + (size_t)warp * P::kVecs + (lane & 3) * P::kPitch + (lane >> 2);
+  const int k0 = w.c0 * 32 + (lane & 3) * 8;
+  const uint4* wp = reinterpret_cast<const uint4*>(slot) + ((lane >> 2) * w.K + k0) / 8;
+  float acc[T][4] = {};
+#pragma unroll 1
+  for (; n > 0; --n) {
+#pragma unroll 1
+    for (int blk = 0; blk == 0 || blk < w.nc; blk += 4) {
+      if (read) read_a<R8>(a, src, w, blk, wait);
+      read = w.nc > 4;  // four chunks or fewer: the same fragments for every unit
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (blk + c < w.nc) {
+          uint4 b = make_uint4(0, 0, 0, 0);
+          if (k0 + (blk + c) * 32 < w.K) b = wp[(blk + c) * 4];
+#pragma unroll
+          for (int t = 0; t < T; ++t) {
+            const uint4 lo = a[c][2 * t], hi = R8 > 1 ? a[c][R8 > 1 ? 2 * t + 1 : 0] : make_uint4(0, 0, 0, 0);
+            if constexpr (R8 == 1) {
+              mma16816_top(acc[t][0], acc[t][1], lo.x, lo.y, b.x, b.y);
+              mma16816_top(acc[t][0], acc[t][1], lo.z, lo.w, b.z, b.w);
+            } else {
+              mma16816(acc[t], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+              mma16816(acc[t], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+            }
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      d[t * P::kTile] = make_float2(acc[t][0], acc[t][1]);
+      if (R8 > 1) d[t * P::kTile + 8] = make_float2(acc[t][2], acc[t][3]);
+      acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+    }
+    d += kWarps * P::kVecs;
+    wp += w.K;
+  }
 }
 
 // Sum over the warps of column pair (2c, 2c + 1) of row b.
@@ -348,296 +359,249 @@ __device__ __forceinline__ int frag_at(int r, int k) {
   return ((((k >> 5) * R8 + (r >> 3)) * 32 + (r & 7) * 4 + ((k & 31) >> 3)) << 4) + (k & 7) * 2;
 }
 
-// A warp holds one row in segments of 768 columns, 24 values per lane: plain fp32 as six float4, words as twelve pairs.
-constexpr int kSeg = 768;
-struct RowSeg {
-  float v[24];
+// Which rows a warp normalises: up to 8 sequences share the warps (16 / B per row), more take a warp each, 17 and more
+// two rows a warp.
+struct RowShare {
+  int row, sub, per_row;
 };
-// plain: values 4 i .. 4 i + 3 are columns k0 + 4 (lane + 32 i)
-__device__ __forceinline__ void read_plain(RowSeg& x, const float* row, int k0, int K) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    const int k = k0 + 4 * (lane + 32 * i);
-    const float4 f = k < K ? __ldcg(reinterpret_cast<const float4*>(row + k0 + 4 * lane) + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    x.v[4 * i] = f.x; x.v[4 * i + 1] = f.y; x.v[4 * i + 2] = f.z; x.v[4 * i + 3] = f.w;
-  }
-}
-// words: values 2 i, 2 i + 1 are columns k0 + 2 (lane + 32 i)
-__device__ __forceinline__ void read_words(RowSeg& x, const uint2* row, int k0, int K, uint32_t epoch, const Wait& wait) {
-  const int lane = threadIdx.x & 31;
-  long long t0 = 0;
+// Normalised rows, bf16(x * rms^-1 * gain), rounded like the training forward's.  row(r) = plain fp32 values; words:
+// {value, epoch} pairs instead (R8 = 1).  A warp's part of a row stays in registers between the sum of squares and the
+// conversion for dim <= 768; wider rows go through in segments and are read twice.  gains(): the norm's weights in
+// shared memory, waited for when they are needed.
+template <int R8, class Row, class Gains>
+__device__ __forceinline__ void stage_norm(int K, int B, Row row, const uint2* words, uint32_t epoch, Gains gains, uint8_t* stage,
+                                           float* s_sq, const RowShare& sh, const Wait& wait) {
+  constexpr int V = R8 == 1 ? 3 : 6;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int stride = sh.per_row * 128, seg = stride * V, nseg = (K + seg - 1) / seg;
 #pragma unroll 1
-  for (unsigned n = 0;; ++n) {
-    bool ok = true;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const int k = k0 + 2 * (lane + 32 * i);
-      uint4 u = make_uint4(0, epoch, 0, epoch);
-      if (k < K) u = get_words(row + k0 + 2 * lane + 64 * i);
-      ok = ok && u.y == epoch && u.w == epoch;
-      x.v[2 * i] = __uint_as_float(u.x);
-      x.v[2 * i + 1] = __uint_as_float(u.z);
-    }
-    if (__all_sync(0xffffffffu, ok) || wait.expired(n, t0)) return;
-  }
-}
-// the norm's weights of the same columns
-template <bool WORDS>
-__device__ __forceinline__ void read_gains(RowSeg& g, const float* __restrict__ wn, int k0, int K) {
-  const int lane = threadIdx.x & 31;
-  if constexpr (WORDS) {
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const float2 f = k0 + 2 * (lane + 32 * i) < K ? __ldg(reinterpret_cast<const float2*>(wn + k0 + 2 * lane) + 32 * i) : make_float2(0.f, 0.f);
-      g.v[2 * i] = f.x; g.v[2 * i + 1] = f.y;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const float4 f = k0 + 4 * (lane + 32 * i) < K ? __ldg(reinterpret_cast<const float4*>(wn + k0 + 4 * lane) + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      g.v[4 * i] = f.x; g.v[4 * i + 1] = f.y; g.v[4 * i + 2] = f.z; g.v[4 * i + 3] = f.w;
-    }
-  }
-}
-template <int R8, bool WORDS>
-__device__ __forceinline__ void put_seg(const RowSeg& x, float rms, const RowSeg& g, int r, int k0, int K, uint8_t* stage) {
-  const int lane = threadIdx.x & 31;
-  if constexpr (WORDS) {
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const int k = k0 + 2 * (lane + 32 * i);
-      if (k < K) *reinterpret_cast<uint32_t*>(stage + frag_at<R8>(r, k)) = pack2(x.v[2 * i] * rms * g.v[2 * i], x.v[2 * i + 1] * rms * g.v[2 * i + 1]);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const int k = k0 + 4 * (lane + 32 * i);
-      if (k < K)
-        *reinterpret_cast<uint2*>(stage + frag_at<R8>(r, k)) =
-            make_uint2(pack2(x.v[4 * i] * rms * g.v[4 * i], x.v[4 * i + 1] * rms * g.v[4 * i + 1]),
-                       pack2(x.v[4 * i + 2] * rms * g.v[4 * i + 2], x.v[4 * i + 3] * rms * g.v[4 * i + 3]));
-    }
-  }
-}
-// Normalised rows, bf16(x * rms^-1 * w), rounded like the training forward's: warp w takes rows w and w + 16.
-template <int R8, bool WORDS, class Row>
-__device__ __forceinline__ void stage_norm(int K, int B, Row row, uint32_t epoch, const float* __restrict__ wn, uint8_t* stage, const Wait& wait) {
-  const int warp = threadIdx.x >> 5;
-  RowSeg x, gain;
-  auto read = [&](int r, int k0) {
-    if constexpr (WORDS) read_words(x, row(r), k0, K, epoch, wait);
-    else read_plain(x, row(r), k0, K);
-  };
-  auto squares = [&] {
-    float q[4] = {};
-#pragma unroll
-    for (int e = 0; e < 24; ++e) q[e & 3] += x.v[e] * x.v[e];
-    return (q[0] + q[1]) + (q[2] + q[3]);
-  };
-  if (warp >= B) return;
-  const bool one = K <= kSeg;
-  if (one) read_gains<WORDS>(gain, wn, 0, K);  // travels together with the row
+  for (int r = sh.row; r < (R8 == 4 ? B : 16); r += 16) {
+    const bool has = r < B;
+    const float* px = row(has ? r : 0);
+    const uint2* pw = words + (size_t)(has ? r : 0) * K;
+    float sq = 0.f, rms = 0.f;
 #pragma unroll 1
-  for (int r = warp; r < B; r += kWarps) {
-    float sq = 0.f;
+    for (int it = 0; it < (nseg == 1 ? 1 : 2 * nseg); ++it) {
+      const int k0 = (it < nseg ? it : it - nseg) * seg + (sh.sub * 32 + lane) * 4;
+      float4 x[V];
+#pragma unroll
+      for (int i = 0; i < V; ++i) x[i] = ldf_l2_if(px + k0 + i * stride, has && k0 + i * stride < K && (R8 > 1 || words == nullptr));
+      if (R8 == 1 && words != nullptr) {
+        long long t0 = 0;
 #pragma unroll 1
-    for (int k0 = 0; k0 < K; k0 += kSeg) {
-      read(r, k0);
-      sq += squares();
-    }
-    const float rms = 1.0f / sqrtf(warp_sum(sq) / (float)K + 1e-5f);
-#pragma unroll 1
-    for (int k0 = 0; k0 < K; k0 += kSeg) {
-      if (!one) {  // wider rows are read again
-        read_gains<WORDS>(gain, wn, k0, K);
-        read(r, k0);
+        for (unsigned n = 0;; ++n) {
+          bool ok = true;
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            if (!has || k0 + i * stride >= K) continue;
+            const uint4 a = get_words(pw + k0 + i * stride), b = get_words(pw + k0 + i * stride + 2);
+            ok = ok && a.y == epoch && a.w == epoch && b.y == epoch && b.w == epoch;
+            x[i] = make_float4(__uint_as_float(a.x), __uint_as_float(a.z), __uint_as_float(b.x), __uint_as_float(b.z));
+          }
+          if (__all_sync(0xffffffffu, ok) || wait.expired(n, t0)) break;
+        }
       }
-      put_seg<R8, WORDS>(x, rms, gain, r, k0, K, stage);
+      if (it < nseg) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) sq += (x[i].x * x[i].x + x[i].y * x[i].y) + (x[i].z * x[i].z + x[i].w * x[i].w);
+      }
+      if (it == nseg - 1) {
+        sq = warp_sum(sq);
+        if (R8 == 1) {  // the row's other warps
+          if (lane == 0) s_sq[warp] = sq;
+          __syncthreads();
+          sq = 0.f;
+#pragma unroll 1
+          for (int i = 0; i < sh.per_row; ++i) sq += s_sq[warp - sh.sub + i];
+        }
+        rms = 1.0f / sqrtf(sq / (float)K + 1e-5f);
+      }
+      if (it >= nseg || nseg == 1) {
+        const float* gp = gains();
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          if (!has || k0 + i * stride >= K) continue;
+          const float4 g = *reinterpret_cast<const float4*>(gp + k0 + i * stride);
+          *reinterpret_cast<uint2*>(stage + frag_at<R8>(r, k0 + i * stride)) =
+              make_uint2(pack2(x[i].x * rms * g.x, x[i].y * rms * g.y), pack2(x[i].z * rms * g.z, x[i].w * rms * g.w));
+        }
+      }
     }
   }
 }
 
 // ---- attention ------------------------------------------------------------------------------------------------------
-// One new token per sequence over cache positions 0..pos.  A work item is one sequence and G query heads of one KV head;
-// its keys are dealt to groups of `lpk` lanes (8 dimensions of the head each), every group keeps its own running
-// maximum, sum and P*V, and they are merged at the end.  Scores in the log2 domain.  With flagged words (R8 = 1) q and
-// the new key and value come from the words, the older ones from the cache.
-template <int R8, int G>
+// One new token per sequence over cache positions 0..pos.  A work item is one sequence and the (up to 8) query heads
+// of one KV head, which are the rows of the MMAs; every warp takes 16 keys at a time and keeps a running maximum, sum and
+// P*V, merged at the end.  No operand is transposed or staged:
+//   scores  B[k = dim, n = key]: lane (g, c) reads 16 bytes of key g at dims 8c.. and 32 + 8c.., two MMAs each (the
+//           order of k is free as long as q is read the same way);
+//   P * V   B[k = key, n]: lane (g, c) reads dims 8g.. of keys 2c, 2c + 1, 2c + 8, 2c + 9; MMA j takes element j of each, so
+//           its column n stands for dim 8n + j.  P enters as bf16 hi + lo, two MMAs, so that it keeps 16 bits.
+// hd <= 64 is one panel of 64 dims (what lies past hd reads as zero), up to 128 two.  With flagged words (R8 = 1) q and the
+// new key and value come from the words, the older ones from the cache.
+template <int R8, int PANELS>
 __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16* kc, const bf16* vc, int pos, float* sm, uint32_t epoch, const Wait& wait) {
-  constexpr int U = R8 == 1 ? 2 : 4;  // keys per group in flight
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int lpk = a.hd <= 8 ? 1 : a.hd <= 16 ? 2 : a.hd <= 32 ? 4 : a.hd <= 64 ? 8 : 16;
-  const int per_warp = 32 / lpk, groups = per_warp * kWarps;
-  const int sub = lane & (lpk - 1), gid = warp * per_warp + lane / lpk;
-  const bool act = sub * 8 < a.hd;
-  const int d0 = act ? sub * 8 : 0;
-  const int kvd = a.KV * a.hd, qd = a.H * a.hd, rep = a.H / a.KV, hgroups = a.H / G;
-  const float sc = 1.4426950408889634f / sqrtf((float)a.hd);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
+  const int kvd = a.KV * a.hd, qd = a.H * a.hd, rep = a.H / a.KV, G = a.group, hgroups = a.H / G;
+  const float sc = 1.4426950408889634f / sqrtf((float)a.hd);  // scores in the log2 domain
 #pragma unroll 1
   for (int item = blockIdx.x; item < a.B * hgroups; item += gridDim.x) {
     const int b = item / hgroups, h0 = (item - b * hgroups) * G, kvh = h0 / rep;
-    const bf16* kb = kc + (size_t)b * a.S * kvd + (size_t)kvh * a.hd + d0;
-    const bf16* vb = vc + (size_t)b * a.S * kvd + (size_t)kvh * a.hd + d0;
-    uint4 kr[U], vr[U], kn = make_uint4(0, 0, 0, 0), vn = kn;
-    auto fetch = [&](int j0) {
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int j = min(j0 + u * groups, pos);  // clamped: a repeated key gets no weight below
-        kr[u] = ld_l2(kb + (size_t)j * kvd);
-        vr[u] = ld_l2(vb + (size_t)j * kvd);
-      }
-    };
-    fetch(gid);  // cached keys do not depend on this step (R8 = 1: the newest is replaced below)
-    float q[G][8];
-    auto set_q = [&](int g, uint4 u) {
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = unpack2(w[e]);
-        q[g][2 * e] = act ? f.x * sc : 0.f;
-        q[g][2 * e + 1] = act ? f.y * sc : 0.f;
-      }
-    };
+    const bf16* kb = kc + (size_t)b * a.S * kvd + (size_t)kvh * a.hd;
+    const bf16* vb = vc + (size_t)b * a.S * kvd + (size_t)kvh * a.hd;
+    const uint2* wk = nullptr;  // words of the new key
+    uint4 q[PANELS][2];
     if constexpr (R8 == 1) {
       const uint2* row = a.w_qkv + (size_t)b * ((qd + 2 * kvd) / 2);
+      wk = row + (qd + kvh * a.hd) / 2;
+      // every word of this item: q rows, key and value (the last two are read again below, from L2 as well)
       long long t0 = 0;
-  #pragma unroll 1
-    for (unsigned n = 0;; ++n) {
+#pragma unroll 1
+      for (unsigned n = 0;; ++n) {
         bool ok = true;
-        auto four = [&](int col) {
-          const uint4 x = get_words(row + (col >> 1)), y = get_words(row + (col >> 1) + 2);
-          ok = ok && x.y == epoch && x.w == epoch && y.y == epoch && y.w == epoch;
-          return make_uint4(x.x, x.z, y.x, y.z);
-        };
 #pragma unroll
-        for (int g = 0; g < G; ++g) set_q(g, four((h0 + g) * a.hd + d0));
-        kn = four(qd + kvh * a.hd + d0);
-        vn = four(qd + kvd + kvh * a.hd + d0);
+        for (int i = 0; i < 2 * PANELS; ++i) {
+          const int d = i * 32 + c * 8;
+          q[i >> 1][i & 1] = make_uint4(0, 0, 0, 0);
+          if (d < a.hd) {
+            const uint4 k0 = get_words(wk + d / 2), k1 = get_words(wk + d / 2 + 2), v0 = get_words(wk + (kvd + d) / 2), v1 = get_words(wk + (kvd + d) / 2 + 2);
+            ok = ok && k0.y == epoch && k0.w == epoch && k1.y == epoch && k1.w == epoch && v0.y == epoch && v0.w == epoch && v1.y == epoch && v1.w == epoch;
+            if (g < G) {
+              const uint2* p = row + ((h0 + g) * a.hd + d) / 2;
+              const uint4 x = get_words(p), y = get_words(p + 2);
+              ok = ok && x.y == epoch && x.w == epoch && y.y == epoch && y.w == epoch;
+              q[i >> 1][i & 1] = make_uint4(x.x, x.z, y.x, y.z);
+            }
+          }
+        }
         if (__all_sync(0xffffffffu, ok) || wait.expired(n, t0)) break;
       }
     } else {
 #pragma unroll
-      for (int g = 0; g < G; ++g) set_q(g, ld_l2(a.q + (size_t)b * qd + (size_t)(h0 + g) * a.hd + d0));
+      for (int i = 0; i < 2 * PANELS; ++i) {
+        const int d = i * 32 + c * 8;
+        q[i >> 1][i & 1] = ld_l2_if(a.q + (size_t)b * qd + (size_t)(h0 + g) * a.hd + d, g < G && d < a.hd);
+      }
     }
-    float m[G], l[G], acc[G][8];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      m[g] = -INFINITY;
-      l[g] = 0.f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[g][e] = 0.f;
-    }
+    // 16 bytes of a key's or value's dims d..d+7 from the cache (R8 = 1: all but the newest, which put_new() adds)
+    const int cached = R8 == 1 ? pos : pos + 1;
+    auto fetch = [&](const bf16* base, int j, int d) { return ld_l2_if(base + (size_t)j * kvd + d, d < a.hd && j < cached); };
+    auto put_new = [&](uint4& v, int off, int j, int d) {
+      if (R8 == 1 && j == pos && d < a.hd) {
+        const uint4 x = get_words(wk + (off + d) / 2), y = get_words(wk + (off + d) / 2 + 2);
+        v = make_uint4(x.x, x.z, y.x, y.z);
+      }
+    };
+    float m = -INFINITY, l = 0.f, acc[PANELS][8][2] = {};
 #pragma unroll 1
-    for (int j0 = gid; __any_sync(0xffffffffu, j0 <= pos); j0 += groups * U) {
-      if (j0 != gid) fetch(j0);
-      if constexpr (R8 == 1) {
+    for (int j0 = warp * 16; j0 <= pos; j0 += kWarps * 16) {
+      uint4 kr[2][2 * PANELS], vr[4][PANELS];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (j0 + u * groups >= pos) {
-            kr[u] = kn;
-            vr[u] = vn;
-          }
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int i = 0; i < 2 * PANELS; ++i) kr[t][i] = fetch(kb, j0 + t * 8 + g, i * 32 + c * 8);
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int p = 0; p < PANELS; ++p) vr[t][p] = fetch(vb, j0 + 2 * c + (t & 1) + (t >> 1) * 8, p * 64 + g * 8);
+      if (R8 == 1 && j0 + 16 > pos) {  // this warp holds the newest key
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int i = 0; i < 2 * PANELS; ++i) put_new(kr[t][i], 0, j0 + t * 8 + g, i * 32 + c * 8);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+          for (int p = 0; p < PANELS; ++p) put_new(vr[t][p], kvd, j0 + 2 * c + (t & 1) + (t >> 1) * 8, p * 64 + g * 8);
       }
-      float s[U][G];
+      float s[2][2] = {}, mn = m;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint32_t w[4] = {kr[u].x, kr[u].y, kr[u].z, kr[u].w};
+      for (int t = 0; t < 2; ++t) {
 #pragma unroll
-        for (int g = 0; g < G; ++g) s[u][g] = 0.f;
+        for (int i = 0; i < 2 * PANELS; ++i) {
+          const uint4 k = kr[t][i], x = q[i >> 1][i & 1];
+          mma16816_top(s[t][0], s[t][1], x.x, x.y, k.x, k.y);
+          mma16816_top(s[t][0], s[t][1], x.z, x.w, k.z, k.w);
+        }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = unpack2(w[e]);
-#pragma unroll
-          for (int g = 0; g < G; ++g) s[u][g] += q[g][2 * e] * f.x + q[g][2 * e + 1] * f.y;
+        for (int e = 0; e < 2; ++e) {
+          s[t][e] = j0 + t * 8 + 2 * c + e <= pos ? s[t][e] * sc : -INFINITY;
+          mn = fmaxf(mn, s[t][e]);
         }
       }
-#pragma unroll 1
-      for (int o = lpk >> 1; o > 0; o >>= 1) {
+      mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+      mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2));  // finite: key j0 is visible
+      const float corr = exp2f(m - mn);
+      m = mn;
+      l *= corr;
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+      for (int p = 0; p < PANELS; ++p)
 #pragma unroll
-          for (int g = 0; g < G; ++g) s[u][g] += __shfl_xor_sync(0xffffffffu, s[u][g], o);
+        for (int j = 0; j < 8; ++j) {
+          acc[p][j][0] *= corr;
+          acc[p][j][1] *= corr;
+        }
+      uint32_t hi[2], lo[2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const float x = exp2f(s[t][0] - mn), y = exp2f(s[t][1] - mn);
+        l += x + y;
+        hi[t] = pack2(x, y);
+        const float2 f = unpack2(hi[t]);
+        lo[t] = pack2(x - f.x, y - f.y);
       }
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        float mn = m[g];
+      for (int p = 0; p < PANELS; ++p) {
+        const uint32_t v[4][4] = {{vr[0][p].x, vr[0][p].y, vr[0][p].z, vr[0][p].w}, {vr[1][p].x, vr[1][p].y, vr[1][p].z, vr[1][p].w},
+                                  {vr[2][p].x, vr[2][p].y, vr[2][p].z, vr[2][p].w}, {vr[3][p].x, vr[3][p].y, vr[3][p].z, vr[3][p].w}};
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (j0 + u * groups > pos) s[u][g] = -INFINITY;
-          mn = fmaxf(mn, s[u][g]);
-        }
-        const float base = mn == -INFINITY ? 0.f : mn;  // a group without keys so far
-        const float corr = exp2f(m[g] - base);
-        m[g] = mn;
-        l[g] *= corr;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[g][e] *= corr;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          s[u][g] = exp2f(s[u][g] - base);
-          l[g] += s[u][g];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint32_t w[4] = {vr[u].x, vr[u].y, vr[u].z, vr[u].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = unpack2(w[e]);
-#pragma unroll
-          for (int g = 0; g < G; ++g) {
-            acc[g][2 * e] = fmaf(s[u][g], f.x, acc[g][2 * e]);
-            acc[g][2 * e + 1] = fmaf(s[u][g], f.y, acc[g][2 * e + 1]);
-          }
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;  // element j of two keys
+          const uint32_t b0 = __byte_perm(v[0][j >> 1], v[1][j >> 1], sel), b1 = __byte_perm(v[2][j >> 1], v[3][j >> 1], sel);
+          mma16816_top(acc[p][j][0], acc[p][j][1], hi[0], hi[1], b0, b1);
+          mma16816_top(acc[p][j][0], acc[p][j][1], lo[0], lo[1], b0, b1);
         }
       }
     }
-    // groups of a warp, then the warps
-#pragma unroll 1
-    for (int o = lpk; o < 32; o <<= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    const int pitch = PANELS * 64 + 2;  // per warp and head: P*V, maximum, sum
+    float* mine = sm + (warp * 8 + g) * pitch;
+    __syncthreads();                    // the previous item's merge has been read
+    if (g < G) {
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const float mo = __shfl_xor_sync(0xffffffffu, m[g], o), lo = __shfl_xor_sync(0xffffffffu, l[g], o);
-        const float mn = fmaxf(m[g], mo), base = mn == -INFINITY ? 0.f : mn;
-        const float f = exp2f(m[g] - base), fo = exp2f(mo - base);
-        m[g] = mn;
-        l[g] = l[g] * f + lo * fo;
+      for (int p = 0; p < PANELS; ++p)
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[g][e] = acc[g][e] * f + __shfl_xor_sync(0xffffffffu, acc[g][e], o) * fo;
-      }
-    }
-    float* s_ml = sm;                    // [G][kWarps][2]
-    float* s_acc = sm + G * kWarps * 2;  // [G][kWarps][hd]
-    __syncthreads();                     // the previous item's merge has been read
-    if (lane < lpk && act) {
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        if (sub == 0) {
-          s_ml[(g * kWarps + warp) * 2] = m[g];
-          s_ml[(g * kWarps + warp) * 2 + 1] = l[g];
+        for (int j = 0; j < 8; ++j) {  // columns 2c, 2c + 1 of MMA j
+          mine[p * 64 + 16 * c + j] = acc[p][j][0];
+          mine[p * 64 + 16 * c + 8 + j] = acc[p][j][1];
         }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) s_acc[(g * kWarps + warp) * a.hd + d0 + e] = acc[g][e];
+      if (c == 0) {
+        mine[PANELS * 64] = m;
+        mine[PANELS * 64 + 1] = l;
       }
     }
     __syncthreads();
+    const int used = min(kWarps, pos / 16 + 1);  // warps that had keys
 #pragma unroll 1
     for (int i = threadIdx.x; i < G * a.hd / 2; i += kThreads) {
-      const int g = 2 * i / a.hd, d = 2 * i - g * a.hd;
+      const int h = (2 * i) / a.hd, d = 2 * i - h * a.hd;
+      const float* from = sm + h * pitch;
       float mx = -INFINITY;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, s_ml[(g * kWarps + w) * 2]);
+#pragma unroll 4
+      for (int w = 0; w < used; ++w) mx = fmaxf(mx, from[w * 8 * pitch + PANELS * 64]);
       float ls = 0.f, o0 = 0.f, o1 = 0.f;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        const float f = exp2f(s_ml[(g * kWarps + w) * 2] - mx);  // warps without a key: exp2(-inf) = 0
-        ls += s_ml[(g * kWarps + w) * 2 + 1] * f;
-        o0 += s_acc[(g * kWarps + w) * a.hd + d] * f;
-        o1 += s_acc[(g * kWarps + w) * a.hd + d + 1] * f;
+#pragma unroll 4
+      for (int w = 0; w < used; ++w) {
+        const float* x = from + w * 8 * pitch;
+        const float f = exp2f(x[PANELS * 64] - mx);
+        ls += x[PANELS * 64 + 1] * f;
+        o0 += x[d] * f;
+        o1 += x[d + 1] * f;
       }
       const uint32_t v = pack2(o0 / ls, o1 / ls);
-      const size_t at = (size_t)b * (qd / 2) + (size_t)((h0 + g) * a.hd + d) / 2;
+      const size_t at = (size_t)b * (qd / 2) + (size_t)((h0 + h) * a.hd + d) / 2;
       if constexpr (R8 == 1) put_word(a.w_att + at, v, epoch);
       else __stcg(reinterpret_cast<unsigned*>(a.att) + at, v);
     }
@@ -658,32 +622,54 @@ template <int R8>
 __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_constant__ DecodeArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_tok[32], s_abort;
+  __shared__ float s_sq[2 * kWarps], s_cos[64], s_sin[64];
+  __shared__ __align__(8) uint64_t s_full[Ring<R8>::kSlots];
   __shared__ unsigned long long s_best[32];
   __shared__ double s_before[32], s_target[32];
   __shared__ Prod s_prod[5];
   constexpr int BP = 8 * R8, J = kThreads / BP;  // a thread's row of the batch is fixed: threadIdx.x % BP
   constexpr bool kWords = R8 == 1;
   uint8_t* stage = smem;
-  float2* part = reinterpret_cast<float2*>(smem + a.stage_bytes + kRingBytes);  // staged rows | ring of weights | partial sums
+  float2* part = reinterpret_cast<float2*>(smem + a.stage_bytes + Ring<R8>::kSlots * a.slot_bytes);  // staged rows | ring of weights | partial sums
   const int row = threadIdx.x & (BP - 1), j0 = threadIdx.x / BP;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int D = a.D, QD = a.H * a.hd, KVD = a.KV * a.hd;
   const bool sampling = a.temperature > 1e-6f, live = row < a.B;
   if (threadIdx.x == 0) {
+    constexpr int units = Ring<R8>::kUnits;
     s_abort = 0;
-    make_prod(s_prod[kQkv], kQkv, a.off_qkv, a.layer_stride, D, (QD + 2 * KVD) / 8);
-    make_prod(s_prod[kWo], kWo, a.off_wo, a.layer_stride, QD, D / 8);
-    make_prod(s_prod[kW13], kW13, a.off_w13, a.layer_stride, D, 2 * a.Hd / 8);
-    make_prod(s_prod[kW2], kW2, a.off_w2, a.layer_stride, a.Hd, D / 8);
-    make_prod(s_prod[kHead], kHead, a.off_embed, 0, D, a.V / 8);
+    make_prod(s_prod[kQkv], kQkv, a.off_qkv, a.layer_stride, D, (QD + 2 * KVD) / 8, units);
+    make_prod(s_prod[kWo], kWo, a.off_wo, a.layer_stride, QD, D / 8, units);
+    make_prod(s_prod[kW13], kW13, a.off_w13, a.layer_stride, D, 2 * a.Hd / 8, units);
+    make_prod(s_prod[kW2], kW2, a.off_w2, a.layer_stride, a.Hd, D / 8, min(units, a.slot_bytes / (16 * a.Hd)));
+    make_prod(s_prod[kHead], kHead, a.off_embed, 0, D, a.V / 8, units);
   }
   for (int i = threadIdx.x * 16; i < a.stage_bytes; i += kThreads * 16) *reinterpret_cast<uint4*>(stage + i) = make_uint4(0, 0, 0, 0);
   __syncthreads();
   const Wait wait{a.status, &s_abort};
   GridBarrier bar{a.bar, 0u, wait};
-  Walk w;
-  w.ring = smem_u32(smem) + (uint32_t)a.stage_bytes + (uint32_t)((warp * kSlots * 32 + lane) * 16);
-  w.start(s_prod[kQkv], a.w + a.off_qkv, 0, min(a.umax, s_prod[kQkv].nu));
+  RowShare share;
+  share.per_row = a.B >= 16 ? 1 : kWarps / a.B;
+  share.row = warp / share.per_row;
+  share.sub = warp - share.row * share.per_row;
+  constexpr int kFeeder = kThreads - 32;
+  Feed<R8> feed{smem_u32(s_full), smem_u32(smem) + (uint32_t)a.stage_bytes, a.slot_bytes, 0, 0, 1, 0, 0};
+  if (threadIdx.x == kFeeder) {
+    for (int i = 0; i < Ring<R8>::kSlots; ++i) mbar_init(feed.bar + 8u * i, 1);
+    fence_mbar_init();
+    feed.issue(a, s_prod);
+  }
+  __syncthreads();
+  int group = 0;  // groups consumed
+  auto group_ready = [&] {
+    if (!mbar_wait(feed.bar + 8u * (group % Ring<R8>::kSlots), (uint32_t)(group / Ring<R8>::kSlots) & 1u, a.status, DEV_GRID_TIMEOUT)) s_abort = 1;
+  };
+  // every way out before the end: no copy may still be on its way into this CTA's shared memory
+  auto leave = [&] {
+    if (threadIdx.x == kFeeder)
+      for (int i = feed.used; i < feed.issued; ++i)
+        mbar_wait(feed.bar + 8u * (i % Ring<R8>::kSlots), (uint32_t)(i / Ring<R8>::kSlots) & 1u, nullptr, 0);
+  };
 
 #pragma unroll 1
   for (int step = 1; step < a.n_new; ++step) {
@@ -703,6 +689,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
       if (blockIdx.x == 0) __stcg(a.best + ((step + 1) % 3) * a.B + threadIdx.x, 0ull);
     }
     if (threadIdx.x < 32) s_best[threadIdx.x] = 0;
+    if ((int)threadIdx.x < a.hd / 2) {
+      s_cos[threadIdx.x] = a.cosb[pos * (a.hd / 2) + threadIdx.x];
+      s_sin[threadIdx.x] = a.sinb[pos * (a.hd / 2) + threadIdx.x];
+    }
     __syncthreads();
     float bv = -INFINITY;
     int bi = -1;
@@ -712,44 +702,47 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
       const int l = idx >> 2, kind = l == a.L ? kHead : idx & 3;
       const Prod& p = s_prod[kind];
       const uint32_t epoch = (uint32_t)(step * a.L + l + 1);
-      auto start_next = [&] {  // also across the end of the step: weights do not change
-        const int next = idx == 4 * a.L ? 0 : idx + 1;
-        const Prod& q = s_prod[next == 4 * a.L ? kHead : next & 3];
-        if (step + 1 < a.n_new || idx < 4 * a.L)
-          w.start(q, a.w + q.off + (size_t)(next >> 2) * q.layer_stride, 0, min(a.umax, q.nu));
+      const bool direct = kind == kWo || kind == kW2;
+      Source src{nullptr, nullptr, nullptr, a.B, epoch};
+      float2 old = make_float2(0.f, 0.f);  // residual of this thread's first pair
+      const float* xrow = kind == kWo && l == 0 ? a.p + a.off_embed_f32 + (size_t)s_tok[live ? row : 0] * D : a.x + (size_t)row * D;
+      const uint2* wrow = (kind == kWo ? a.w_x0 : a.w_x1) + (size_t)row * D;
+      auto residual = [&](int col) {
+        if (!kWords || (kind == kWo && l == 0)) return __ldcg(reinterpret_cast<const float2*>(xrow + col));
+        const uint4 o = get_words(wrow + col);  // complete: this CTA has staged it
+        return make_float2(__uint_as_float(o.x), __uint_as_float(o.z));
       };
-      if (p.nu == 0) {
-        start_next();
+      if (direct) {
+        if (kWords) __syncthreads();  // the partial sums of the phase before have been read
+        src.rows = kind == kWo ? a.att : a.gate;
+        src.words = kind == kWo ? a.w_att : a.w_gate;
+        if (live && j0 < p.nu * 4) old = residual(p.row0(j0 >> 2) + 2 * (j0 & 3));
       } else {
-        const bool direct = kind == kWo || kind == kW2;
-        if (!direct) {
-          // x before this layer (after W2 of the one below; the embedding row for layer 0), or after Wo for W1|W3
-          const bool embed = kind == kQkv && l == 0;
-          const float* wn = a.p + (kind == kHead ? a.off_rms_final : (kind == kQkv ? a.off_rms_att : a.off_rms_ffn) + (size_t)l * a.rms_stride);
-          if (kWords && !embed) {
-            const uint2* x = kind == kW13 ? a.w_x1 : a.w_x0;
-            stage_norm<R8, true>(D, a.B, [&](int r) { return x + (size_t)r * D; }, kind == kW13 ? epoch : epoch - 1, wn, stage, wait);
-          } else {
-            stage_norm<R8, false>(D, a.B, [&](int r) { return embed ? a.p + a.off_embed_f32 + (size_t)s_tok[r] * D : a.x + (size_t)r * D; },
-                                  0u, wn, stage, wait);
-          }
-          __syncthreads();
-        } else if (kWords) {
-          __syncthreads();  // the partial sums of the phase before have been read
-        }
+        // x before this layer (after W2 of the one below; the embedding row for layer 0), or after Wo for W1|W3
+        const bool embed = kind == kQkv && l == 0;
+        const uint2* words = !kWords || embed ? nullptr : kind == kW13 ? a.w_x1 : a.w_x0;
+        auto gains = [&] {
+          group_ready();
+          return reinterpret_cast<const float*>(smem + a.stage_bytes + (group % Ring<R8>::kSlots + 1) * a.slot_bytes - D * 4);
+        };
+        stage_norm<R8>(D, a.B, [&](int r) { return embed ? a.p + a.off_embed_f32 + (size_t)s_tok[r] * D : a.x + (size_t)r * D; }, words,
+                       kind == kW13 ? epoch : epoch - 1, gains, stage, s_sq, share, wait);
+        __syncthreads();
+        src.stage = reinterpret_cast<const uint4*>(stage);
+      }
+      {
+        const Share mine = make_share(p.K);
+        uint4 frag[4][R8];
 #pragma unroll 1
-        for (int g0 = 0; g0 < p.nu; g0 += a.umax) {
-          const int n = min(a.umax, p.nu - g0);
-          if (!direct) {
-            run_product<R8>(p, w, n, part, StagedRows<R8>{reinterpret_cast<const uint4*>(stage)});
-          } else if constexpr (kWords) {
-            run_product<R8>(p, w, n, part, WordRows{kind == kWo ? a.w_att : a.w_gate, a.B, epoch, wait});
-          } else {
-            run_product<R8>(p, w, n, part, PlainRows<R8>{kind == kWo ? a.att : a.gate, a.B});
-          }
-          if (g0 + n < p.nu) w.start(p, a.w + p.off + (size_t)l * p.layer_stride, g0 + n, min(a.umax, p.nu - g0 - n));
-          else start_next();
+        for (int g0 = 0; g0 < p.nu; g0 += p.per, ++group) {
+          const int n = min(p.per, p.nu - g0);
+          group_ready();
+          run_units<R8>(mine, n, smem + a.stage_bytes + (group % Ring<R8>::kSlots) * a.slot_bytes, part, src, frag, g0 == 0, wait);
           __syncthreads();
+          if (threadIdx.x == kFeeder) {  // the slot is free: refill it
+            ++feed.used;
+            feed.issue(a, s_prod);
+          }
           if (live) {
             if (kind == kW13) {
 #pragma unroll 1
@@ -757,7 +750,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
                 const int u = (i >> 2) * 2, c = i & 3;
                 const float2 h1 = pair_sum<R8>(part, u, row, c), h3 = pair_sum<R8>(part, u + 1, row, c);
                 const uint32_t g = pack2(h1.x * h3.x * sigmoid(h1.x), h1.y * h3.y * sigmoid(h1.y));
-                const int pair = (int)blockIdx.x + ((g0 + u) >> 1) * (int)gridDim.x;
+                const int pair = (int)blockIdx.x + ((g0 + u) >> 1) * (int)gridDim.x;  // columns 8 pair .. of the gate
                 const size_t at = (size_t)row * (a.Hd / 2) + pair * 4 + c;
                 if (kWords) put_word(a.w_gate + at, g, epoch);
                 else __stcg(reinterpret_cast<unsigned*>(a.gate) + at, g);
@@ -770,8 +763,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
                 float x = s.x, y = s.y;
                 if (kind == kQkv) {
                   if (col < QD + KVD) {
-                    const int r = pos * (a.hd / 2) + (col % a.hd) / 2;
-                    const float c = a.cosb[r], sn = a.sinb[r];
+                    const int r = (col - (int)__umulhi((unsigned)col, a.hd_magic) * a.hd) >> 1;
+                    const float c = s_cos[r], sn = s_sin[r];
                     const float t = x * c - y * sn;
                     y = y * c + x * sn;
                     x = t;
@@ -789,15 +782,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
                   if (sampling) __stcg(reinterpret_cast<float2*>(a.logits + (size_t)row * a.V + col), s);
                 } else {  // x += product; every element is updated by one thread
                   const size_t at = (size_t)row * D + col;
-                  float2 old;
-                  if (kind == kWo && l == 0) {
-                    old = __ldg(reinterpret_cast<const float2*>(a.p + a.off_embed_f32 + (size_t)s_tok[row] * D + col));
-                  } else if (kWords) {
-                    const uint4 o = get_words((kind == kWo ? a.w_x0 : a.w_x1) + at);  // complete: this CTA has staged it
-                    old = make_float2(__uint_as_float(o.x), __uint_as_float(o.z));
-                  } else {
-                    old = __ldcg(reinterpret_cast<const float2*>(a.x + at));
-                  }
+                  if (g0 > 0 || i != j0) old = residual(col);
                   x += old.x;
                   y += old.y;
                   if (kWords) {
@@ -814,25 +799,29 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
           if (g0 + n < p.nu) __syncthreads();
         }
       }
-      if (kWords) {
-        if (s_abort) return;
-      } else if (kind != kHead && !bar.sync()) {
+      if (kWords ? s_abort != 0 : kind != kHead && !bar.sync()) {
+        leave();
         return;
       }
       if (kind == kQkv) {
         const size_t cl = (size_t)l * a.kv_layer;
         float* sm = reinterpret_cast<float*>(part);
-        if (a.group == 3) attention_phase<R8, 3>(a, a.kcache + cl, a.vcache + cl, pos, sm, epoch, wait);
-        else if (a.group == 2) attention_phase<R8, 2>(a, a.kcache + cl, a.vcache + cl, pos, sm, epoch, wait);
-        else attention_phase<R8, 1>(a, a.kcache + cl, a.vcache + cl, pos, sm, epoch, wait);
-        if (!kWords && !bar.sync()) return;
+        if (a.hd <= 64) attention_phase<R8, 1>(a, a.kcache + cl, a.vcache + cl, pos, sm, epoch, wait);
+        else attention_phase<R8, 2>(a, a.kcache + cl, a.vcache + cl, pos, sm, epoch, wait);
+        if (!kWords && !bar.sync()) {
+          leave();
+          return;
+        }
       }
     }
     // ---- the best logit of every row
     if (bi >= 0) atomicMax(&s_best[row], pack_best(bv, bi));
     __syncthreads();
     if ((int)threadIdx.x < a.B && s_best[threadIdx.x] != 0) atomicMax(best + threadIdx.x, s_best[threadIdx.x]);
-    if (!bar.sync()) return;
+    if (!bar.sync()) {
+      leave();
+      return;
+    }
     if (!sampling) continue;
     // ---- temperature sampling (ane/train_full.go:318-342): this CTA's vocabulary range of every row in double, the
     // ranges' sums in order, and the CTA whose range holds the target walks it
@@ -848,7 +837,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
       s = warp_sum_d(s);
       if (lane == 0) __stcg(a.psum + (size_t)blockIdx.x * a.B + b, s);
     }
-    if (!bar.sync()) return;
+    if (!bar.sync()) {
+      leave();
+      return;
+    }
     double* s_sums = reinterpret_cast<double*>(part);  // [gridDim.x][B]
 #pragma unroll 1
     for (int i = threadIdx.x; i < (int)gridDim.x * a.B; i += kThreads) s_sums[i] = __ldcg(a.psum + i);
@@ -905,7 +897,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
         a.out[(size_t)b * a.n_new + step] = (uint16_t)pick;
       }
     }
-    if (!bar.sync()) return;
+    if (!bar.sync()) {
+      leave();
+      return;
+    }
   }
   if (!sampling && a.n_new > 1 && blockIdx.x == 0 && (int)threadIdx.x < a.B) {
     const unsigned long long k = __ldcg(a.best + ((a.n_new - 1) % 3) * a.B + threadIdx.x);
@@ -914,23 +909,25 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
 }
 
 size_t stage_bytes(int r8, int D) { return (size_t)((D + 31) / 32) * r8 * 512; }
-size_t unit_bytes(int r8) { return sizeof(float2) * kWarps * (size_t)(r8 == 1 ? Part<1>::kVecs : r8 == 2 ? Part<2>::kVecs : Part<4>::kVecs); }
-constexpr size_t kSmemLimit = 222 * 1024;  // beside the static arrays
-
-// Units per group: as many as shared memory holds beside the staged activations (a power of two, 2..32; W1|W3 units
-// come in pairs).
-int decode_umax(int r8, int D) {
-  for (int u = 32; u >= 2; u >>= 1)
-    if (stage_bytes(r8, D) + kRingBytes + u * unit_bytes(r8) <= kSmemLimit) return u;
-  return 0;
+// units of a group, or one W2 unit, and the norm's gains
+size_t slot_bytes(int r8, int D, int Hd) { return std::max((size_t)16 * Hd, (size_t)16 * (r8 == 4 ? Ring<4>::kUnits : Ring<2>::kUnits) * D + 4 * D); }
+size_t tail_bytes(int r8, int hd, int ctas, int B) {  // partial sums; the attention merge and the sampler's sums use the same memory
+  const size_t unit = sizeof(float2) * kWarps * (size_t)(r8 == 1 ? Part<1>::kVecs : r8 == 2 ? Part<2>::kVecs : Part<4>::kVecs);
+  return std::max(unit * (r8 == 4 ? Ring<4>::kUnits : Ring<2>::kUnits),
+                  std::max(sizeof(float) * (size_t)(kWarps * 8 * (2 + (hd <= 64 ? 64 : 128))), sizeof(double) * (size_t)ctas * B));
 }
+size_t smem_bytes(int r8, int D, int Hd, int hd, int ctas, int B) {
+  return stage_bytes(r8, D) + (r8 == 4 ? Ring<4>::kSlots : Ring<2>::kSlots) * slot_bytes(r8, D, Hd) + tail_bytes(r8, hd, ctas, B);
+}
+constexpr size_t kSmemLimit = 224 * 1024;  // beside the static arrays
+
 int row_groups(int batch) { return batch <= 8 ? 1 : batch <= 16 ? 2 : 4; }
 
 }  // namespace
 
 bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int batch) {
-  return batch >= 1 && batch <= 32 && hd % 8 == 0 && hd <= 128 && D % 8 == 0 && Hd % 32 == 0 && V % 8 == 0 && H % KV == 0 &&
-         decode_umax(row_groups(batch), D) > 0;
+  return batch >= 1 && batch <= 32 && hd % 8 == 0 && hd <= 128 && D % 8 == 0 && H * hd == D && Hd % 32 == 0 && V % 8 == 0 && H % KV == 0 &&
+         (H + 2 * KV) * hd >= 32 && smem_bytes(row_groups(batch), D, Hd, hd, 148, batch) <= kSmemLimit;
 }
 size_t decode_words_bytes(int D, int Hd, int H, int KV, int hd) {  // exchange buffers of up to 8 sequences
   return sizeof(uint2) * 8 * ((size_t)2 * D + (size_t)(H + 2 * KV) * hd / 2 + (size_t)H * hd / 2 + (size_t)Hd / 2);
@@ -939,31 +936,21 @@ size_t decode_words_bytes(int D, int Hd, int H, int KV, int hd) {  // exchange b
 int decode_steps(DecodeArgs a, void* words, int sms, cudaStream_t s) {
   if (a.n_new < 2) return 0;
   const int r8 = row_groups(a.B), qd = a.H * a.hd, qkv = (a.H + 2 * a.KV) * a.hd;
-  a.umax = decode_umax(r8, a.D);
-  if (a.umax == 0) return -2;
   a.stage_bytes = (int)stage_bytes(r8, a.D);
+  a.slot_bytes = (int)slot_bytes(r8, a.D, a.Hd);
   // The exchange of flagged words needs every CTA to own units of q|k|v and of W1|W3; more CTAs than that would idle anyway.
-  const int ctas = std::min(sms, std::min(qkv / 8, a.Hd / 8));
-  // Query heads per attention item: heads that share keys read them once, as long as the items still fill half of the
-  // SMs; a single sequence takes one head per CTA.
+  // A multiple of 4: see Prod.
+  const int ctas = std::min(std::min(sms, 148), std::min(qkv / 8, a.Hd / 8)) & ~3;
   const int rep = a.H / a.KV;
-  a.group = 1;
-  for (int g = 3; g > 1; --g)
-    if (rep % g == 0 && a.B * (a.H / g) * 2 >= ctas) {
-      a.group = g;
-      break;
-    }
+  a.group = rep <= 8 ? rep : 1;  // query heads per attention item: rows of one fragment
+  a.hd_magic = 0xffffffffu / (unsigned)a.hd + 1u;  // col / hd = umulhi(col, hd_magic) for col < 2^16
   uint2* p = reinterpret_cast<uint2*>(words);
   a.w_x0 = p; p += (size_t)8 * a.D;
   a.w_x1 = p; p += (size_t)8 * a.D;
   a.w_qkv = p; p += (size_t)8 * qkv / 2;
   a.w_att = p; p += (size_t)8 * qd / 2;
   a.w_gate = p;
-  // the attention merge and the sampler's sums use the partial sums' memory
-  size_t tail = a.umax * unit_bytes(r8);
-  tail = std::max(tail, sizeof(float) * (size_t)(3 * kWarps * (2 + a.hd)));
-  tail = std::max(tail, sizeof(double) * (size_t)ctas * a.B);
-  const size_t bytes = a.stage_bytes + kRingBytes + tail;
+  const size_t bytes = smem_bytes(r8, a.D, a.Hd, a.hd, ctas, a.B);
   auto kern = r8 == 1 ? decode_steps_kernel<1> : r8 == 2 ? decode_steps_kernel<2> : decode_steps_kernel<4>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return -3;
   if (cudaMemsetAsync(a.bar, 0, sizeof(unsigned), s) != cudaSuccess ||

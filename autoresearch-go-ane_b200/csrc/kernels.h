@@ -120,7 +120,8 @@ struct DecodeArgs {
   int* status;
   float temperature;             // <= 1e-6: argmax
   int B, D, Hd, L, H, KV, hd, V, S, prompt, n_new, u_stride;
-  int umax, group, stage_bytes;  // set by decode_steps
+  int group, stage_bytes, slot_bytes;  // set by decode_steps
+  unsigned hd_magic;
   uint2 *w_x0, *w_x1, *w_qkv, *w_att, *w_gate;
 };
 bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int batch);
