@@ -150,16 +150,15 @@ enum Kind { kQkv = 0, kWo = 1, kW13 = 2, kW2 = 3, kHead = 4 };
 // alternating steps of inc[0] and inc[1] rows (the grid is a multiple of 4, so W1|W3 blocks keep their phase).
 struct Prod {
   size_t off, layer_stride;
-  int K, nu, row, inc[2], u0, kind, per;  // per: units of a group
+  int K, nu, row, inc[2], u0, kind;
   __device__ __forceinline__ int row0(int i) const { return row + (i >> 1) * (inc[0] + inc[1]) + (i & 1) * inc[0]; }
 };
-__device__ __forceinline__ void make_prod(Prod& d, int kind, size_t off, size_t layer_stride, int K, int n_units, int per) {
+__device__ __forceinline__ void make_prod(Prod& d, int kind, size_t off, size_t layer_stride, int K, int n_units) {
   const int g = (int)gridDim.x, b = (int)blockIdx.x;
   d.off = off;
   d.layer_stride = layer_stride;
   d.K = K;
   d.kind = kind;
-  d.per = per;
   d.u0 = 0;
   if (kind == kHead) {  // a contiguous range of the vocabulary
     d.u0 = (int)((long long)n_units * b / g);
@@ -201,7 +200,7 @@ struct Feed {
     while (issued - used < Ring<R8>::kSlots && step < a.n_new) {
       const int layer = idx >> 2;
       const Prod& p = prods[layer == a.L ? kHead : idx & 3];
-      const int n = min(p.per, p.nu - g0);
+      const int n = min(Ring<R8>::kUnits, p.nu - g0);
       if (n > 0) {
         const int at = issued % Ring<R8>::kSlots;
         const uint32_t bytes = (uint32_t)p.K * 16u, b = bar + 8u * at;
@@ -366,10 +365,10 @@ struct RowShare {
 };
 // Normalised rows, bf16(x * rms^-1 * gain), rounded like the training forward's.  row(r) = plain fp32 values; words:
 // {value, epoch} pairs instead (R8 = 1).  A warp's part of a row stays in registers between the sum of squares and the
-// conversion for dim <= 768; wider rows go through in segments and are read twice.  gains(): the norm's weights in
-// shared memory, waited for when they are needed.
-template <int R8, class Row, class Gains>
-__device__ __forceinline__ void stage_norm(int K, int B, Row row, const uint2* words, uint32_t epoch, Gains gains, uint8_t* stage,
+// conversion for dim <= 768; wider rows go through in segments and are read twice.  gains: the norm's weights in
+// shared memory.
+template <int R8, class Row>
+__device__ __forceinline__ void stage_norm(int K, int B, Row row, const uint2* words, uint32_t epoch, const float* gains, uint8_t* stage,
                                            float* s_sq, const RowShare& sh, const Wait& wait) {
   constexpr int V = R8 == 1 ? 3 : 6;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -417,11 +416,10 @@ __device__ __forceinline__ void stage_norm(int K, int B, Row row, const uint2* w
         rms = 1.0f / sqrtf(sq / (float)K + 1e-5f);
       }
       if (it >= nseg || nseg == 1) {
-        const float* gp = gains();
 #pragma unroll
         for (int i = 0; i < V; ++i) {
           if (!has || k0 + i * stride >= K) continue;
-          const float4 g = *reinterpret_cast<const float4*>(gp + k0 + i * stride);
+          const float4 g = *reinterpret_cast<const float4*>(gains + k0 + i * stride);
           *reinterpret_cast<uint2*>(stage + frag_at<R8>(r, k0 + i * stride)) =
               make_uint2(pack2(x[i].x * rms * g.x, x[i].y * rms * g.y), pack2(x[i].z * rms * g.z, x[i].w * rms * g.w));
         }
@@ -636,13 +634,12 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
   const int D = a.D, QD = a.H * a.hd, KVD = a.KV * a.hd;
   const bool sampling = a.temperature > 1e-6f, live = row < a.B;
   if (threadIdx.x == 0) {
-    constexpr int units = Ring<R8>::kUnits;
     s_abort = 0;
-    make_prod(s_prod[kQkv], kQkv, a.off_qkv, a.layer_stride, D, (QD + 2 * KVD) / 8, units);
-    make_prod(s_prod[kWo], kWo, a.off_wo, a.layer_stride, QD, D / 8, units);
-    make_prod(s_prod[kW13], kW13, a.off_w13, a.layer_stride, D, 2 * a.Hd / 8, units);
-    make_prod(s_prod[kW2], kW2, a.off_w2, a.layer_stride, a.Hd, D / 8, min(units, a.slot_bytes / (16 * a.Hd)));
-    make_prod(s_prod[kHead], kHead, a.off_embed, 0, D, a.V / 8, units);
+    make_prod(s_prod[kQkv], kQkv, a.off_qkv, a.layer_stride, D, (QD + 2 * KVD) / 8);
+    make_prod(s_prod[kWo], kWo, a.off_wo, a.layer_stride, QD, D / 8);
+    make_prod(s_prod[kW13], kW13, a.off_w13, a.layer_stride, D, 2 * a.Hd / 8);
+    make_prod(s_prod[kW2], kW2, a.off_w2, a.layer_stride, a.Hd, D / 8);
+    make_prod(s_prod[kHead], kHead, a.off_embed, 0, D, a.V / 8);
   }
   for (int i = threadIdx.x * 16; i < a.stage_bytes; i += kThreads * 16) *reinterpret_cast<uint4*>(stage + i) = make_uint4(0, 0, 0, 0);
   __syncthreads();
@@ -721,10 +718,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
         // x before this layer (after W2 of the one below; the embedding row for layer 0), or after Wo for W1|W3
         const bool embed = kind == kQkv && l == 0;
         const uint2* words = !kWords || embed ? nullptr : kind == kW13 ? a.w_x1 : a.w_x0;
-        auto gains = [&] {
-          group_ready();
-          return reinterpret_cast<const float*>(smem + a.stage_bytes + (group % Ring<R8>::kSlots + 1) * a.slot_bytes - D * 4);
-        };
+        group_ready();
+        const float* gains = reinterpret_cast<const float*>(smem + a.stage_bytes + (group % Ring<R8>::kSlots + 1) * a.slot_bytes - D * 4);
         stage_norm<R8>(D, a.B, [&](int r) { return embed ? a.p + a.off_embed_f32 + (size_t)s_tok[r] * D : a.x + (size_t)r * D; }, words,
                        kind == kW13 ? epoch : epoch - 1, gains, stage, s_sq, share, wait);
         __syncthreads();
@@ -734,8 +729,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
         const Share mine = make_share(p.K);
         uint4 frag[4][R8];
 #pragma unroll 1
-        for (int g0 = 0; g0 < p.nu; g0 += p.per, ++group) {
-          const int n = min(p.per, p.nu - g0);
+        for (int g0 = 0; g0 < p.nu; g0 += Ring<R8>::kUnits, ++group) {
+          const int n = min(Ring<R8>::kUnits, p.nu - g0);
           group_ready();
           run_units<R8>(mine, n, smem + a.stage_bytes + (group % Ring<R8>::kSlots) * a.slot_bytes, part, src, frag, g0 == 0, wait);
           __syncthreads();
@@ -909,15 +904,18 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
 }
 
 size_t stage_bytes(int r8, int D) { return (size_t)((D + 31) / 32) * r8 * 512; }
-// units of a group, or one W2 unit, and the norm's gains
-size_t slot_bytes(int r8, int D, int Hd) { return std::max((size_t)16 * Hd, (size_t)16 * (r8 == 4 ? Ring<4>::kUnits : Ring<2>::kUnits) * D + 4 * D); }
+// a group's units with the norm's gains behind them, or the W2 units of a CTA (mostly one)
+size_t slot_bytes(int r8, int D, int Hd, int ctas) {
+  const int units = r8 == 4 ? Ring<4>::kUnits : Ring<2>::kUnits, w2 = std::min(units, (D / 8 + ctas - 1) / ctas);
+  return std::max((size_t)16 * w2 * Hd, (size_t)16 * units * D + 4 * D);
+}
 size_t tail_bytes(int r8, int hd, int ctas, int B) {  // partial sums; the attention merge and the sampler's sums use the same memory
   const size_t unit = sizeof(float2) * kWarps * (size_t)(r8 == 1 ? Part<1>::kVecs : r8 == 2 ? Part<2>::kVecs : Part<4>::kVecs);
   return std::max(unit * (r8 == 4 ? Ring<4>::kUnits : Ring<2>::kUnits),
                   std::max(sizeof(float) * (size_t)(kWarps * 8 * (2 + (hd <= 64 ? 64 : 128))), sizeof(double) * (size_t)ctas * B));
 }
 size_t smem_bytes(int r8, int D, int Hd, int hd, int ctas, int B) {
-  return stage_bytes(r8, D) + (r8 == 4 ? Ring<4>::kSlots : Ring<2>::kSlots) * slot_bytes(r8, D, Hd) + tail_bytes(r8, hd, ctas, B);
+  return stage_bytes(r8, D) + (r8 == 4 ? Ring<4>::kSlots : Ring<2>::kSlots) * slot_bytes(r8, D, Hd, ctas) + tail_bytes(r8, hd, ctas, B);
 }
 constexpr size_t kSmemLimit = 224 * 1024;  // beside the static arrays
 
@@ -925,9 +923,14 @@ int row_groups(int batch) { return batch <= 8 ? 1 : batch <= 16 ? 2 : 4; }
 
 }  // namespace
 
-bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int batch) {
+// The exchange of flagged words needs every CTA to own units of q|k|v and of W1|W3; more CTAs than that would idle anyway.
+// A multiple of 4: see Prod.
+static int decode_ctas(int sms, int Hd, int H, int KV, int hd) { return std::min(std::min(sms, 148), std::min((H + 2 * KV) * hd / 8, Hd / 8)) & ~3; }
+
+bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int batch, int sms) {
+  const int ctas = decode_ctas(sms, Hd, H, KV, hd);
   return batch >= 1 && batch <= 32 && hd % 8 == 0 && hd <= 128 && D % 8 == 0 && H * hd == D && Hd % 32 == 0 && V % 8 == 0 && H % KV == 0 &&
-         (H + 2 * KV) * hd >= 32 && smem_bytes(row_groups(batch), D, Hd, hd, 148, batch) <= kSmemLimit;
+         ctas > 0 && smem_bytes(row_groups(batch), D, Hd, hd, ctas, batch) <= kSmemLimit;
 }
 size_t decode_words_bytes(int D, int Hd, int H, int KV, int hd) {  // exchange buffers of up to 8 sequences
   return sizeof(uint2) * 8 * ((size_t)2 * D + (size_t)(H + 2 * KV) * hd / 2 + (size_t)H * hd / 2 + (size_t)Hd / 2);
@@ -937,10 +940,8 @@ int decode_steps(DecodeArgs a, void* words, int sms, cudaStream_t s) {
   if (a.n_new < 2) return 0;
   const int r8 = row_groups(a.B), qd = a.H * a.hd, qkv = (a.H + 2 * a.KV) * a.hd;
   a.stage_bytes = (int)stage_bytes(r8, a.D);
-  a.slot_bytes = (int)slot_bytes(r8, a.D, a.Hd);
-  // The exchange of flagged words needs every CTA to own units of q|k|v and of W1|W3; more CTAs than that would idle anyway.
-  // A multiple of 4: see Prod.
-  const int ctas = std::min(std::min(sms, 148), std::min(qkv / 8, a.Hd / 8)) & ~3;
+  const int ctas = decode_ctas(sms, a.Hd, a.H, a.KV, a.hd);
+  a.slot_bytes = (int)slot_bytes(r8, a.D, a.Hd, ctas);
   const int rep = a.H / a.KV;
   a.group = rep <= 8 ? rep : 1;  // query heads per attention item: rows of one fragment
   a.hd_magic = 0xffffffffu / (unsigned)a.hd + 1u;  // col / hd = umulhi(col, hd_magic) for col < 2^16

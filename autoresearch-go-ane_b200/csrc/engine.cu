@@ -1869,7 +1869,7 @@ int EngineT<T>::decode(const uint16_t* prompts, uint32_t n_seq, uint32_t prompt_
   if ((rc = next_token(P, 0)) != 0) return rc;
   bool done = false;
   if constexpr (!kIsF32) {
-    if (decode_steps_supported(D_, Hd_, H_, KV_, hd_, V_, std::min(B, 32))) {
+    if (decode_steps_supported(D_, Hd_, H_, KV_, hd_, V_, std::min(B, 32), gemm_num_sms())) {
       wait_all_buckets();
       for (int b0 = 0; b0 < B; b0 += 32) {
         DecodeArgs a;

@@ -124,7 +124,7 @@ struct DecodeArgs {
   unsigned hd_magic;
   uint2 *w_x0, *w_x1, *w_qkv, *w_att, *w_gate;
 };
-bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int batch);
+bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int batch, int sms);
 size_t decode_words_bytes(int D, int Hd, int H, int KV, int hd);  // size of `words`, scratch for exchanges between SMs
 int decode_steps(DecodeArgs a, void* words, int sms, cudaStream_t s);
 
