@@ -9,78 +9,437 @@
 
 namespace ane {
 
-static constexpr int kAttWarps = 4;
 static constexpr int kMaxHdPerLane = 4;  // head_dim <= 128
 
-// One warp per query row (b, h, t).  Dynamic smem: kAttWarps * hd floats (query vectors).
-template <typename T, typename TO>
-__global__ void attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out,
-                                              float* __restrict__ lse, int B, int seq, int H, int KV, int hd,
-                                              float scale) {
-  extern __shared__ float s_q[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long wid = (long long)blockIdx.x * kAttWarps + warp;
-  const long long total = (long long)B * H * seq;
-  if (wid >= total) return;
-  const int t = (int)(wid % seq);
-  const int h = (int)((wid / seq) % H);
-  const int b = (int)(wid / ((long long)seq * H));
-  const int kvh = h / (H / KV);
+// ------------------------------------------------------------------------------------------------
+// Training attention in fp32 on the FMA units.  A block of 128 threads keeps 32 rows of one head resident in shared
+// memory (queries in the forward and dQ kernels, keys in the dK/dV kernel) and streams tiles of 64 rows of the other
+// side.  Thread (ty, tx) owns a 4 x 4 piece of every score tile (resident rows 4 ty .., streamed rows tx + 16 j) and, in
+// the products with the tile, 4 resident rows x HDP / 16 columns.  All operands stay row-major with a pitch of HDP + 4
+// floats, so score operands are read as float4 along the head dimension without bank conflicts, 64 FMAs for eight
+// 16-byte reads; probabilities pass through shared memory transposed, [streamed row][resident row], one float4 per
+// streamed row.  32 resident rows (not 64 or 128) because the fp32 modes run with few sequences: 2 x 12 heads x 256
+// make 192 blocks.  One warp per query with scalar loads and global atomics, which this replaces, took 709 us for
+// the backward of 2 x 12 heads x 256 x 64.
+// ------------------------------------------------------------------------------------------------
+namespace {
+
+constexpr int kRes = 32, kStr = 64, kSimtThreads = 128;
+constexpr int kPPitch = kRes + 4;  // floats of one streamed row of the probability tile
+
+template <int HDP>
+struct Simt {
+  static constexpr int kPitch = HDP + 4;
+  static constexpr int kResFloats = kRes * kPitch, kStrFloats = kStr * kPitch, kProbFloats = kStr * kPPitch;
+  static constexpr size_t kFwdSmem = sizeof(float) * (kResFloats + 2 * kStrFloats + kProbFloats);
+  static constexpr size_t kDqSmem = sizeof(float) * (2 * kResFloats + 2 * kStrFloats + kProbFloats);
+  static constexpr size_t kDkvSmem = sizeof(float) * (2 * kResFloats + 2 * kStrFloats + 2 * kProbFloats + 3 * kStr);
+};
+
+template <typename T>
+__device__ __forceinline__ float4 load4(const T* p) {
+  if constexpr (sizeof(T) == 4) {
+    return *reinterpret_cast<const float4*>(p);
+  } else {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+}
+
+// ROWS x hd values (row pitch ld) into shared memory as fp32; rows >= valid and columns >= hd become zero.
+template <int HDP, int ROWS, typename T>
+__device__ __forceinline__ void load_rows(float* dst, const T* src, int ld, int valid, int hd) {
+  constexpr int PER = ROWS * (HDP / 4) / kSimtThreads;
+  float4 v[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = threadIdx.x + i * kSimtThreads, r = e / (HDP / 4), c = (e - r * (HDP / 4)) * 4;
+    v[i] = (r < valid && c < hd) ? load4<T>(src + (size_t)r * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = threadIdx.x + i * kSimtThreads, r = e / (HDP / 4), c = (e - r * (HDP / 4)) * 4;
+    *reinterpret_cast<float4*>(dst + r * Simt<HDP>::kPitch + c) = v[i];
+  }
+}
+
+// s[i][j] = <resident row 4 ty + i, streamed row tx + 16 j>
+template <int HDP>
+__device__ __forceinline__ void scores(float (&s)[4][4], const float* res, const float* str, int ty, int tx) {
+  constexpr int P = Simt<HDP>::kPitch;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 4
+  for (int d = 0; d < HDP; d += 4) {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(res + (4 * ty + i) * P + d);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(str + (tx + 16 * j) * P + d);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        s[i][j] = fmaf(a[i].x, b[j].x, fmaf(a[i].y, b[j].y, fmaf(a[i].z, b[j].z, fmaf(a[i].w, b[j].w, s[i][j]))));
+  }
+}
+
+// Columns of thread tx: float4 / float2 groups where the width allows, else every 16th.
+template <int HDP>
+__device__ __forceinline__ int col_of(int tx, int c) {
+  if (HDP == 48) return tx + 16 * c;
+  if (HDP == 32) return 2 * tx + c;
+  if (c < 4) return 4 * tx + c;
+  return HDP == 96 ? 64 + 2 * tx + (c - 4) : 64 + 4 * tx + (c - 4);
+}
+template <int HDP>
+__device__ __forceinline__ void load_cols(float (&v)[HDP / 16], const float* row, int tx) {
+  if constexpr (HDP == 48) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[c] = row[tx + 16 * c];
+  } else if constexpr (HDP == 32) {
+    const float2 a = *reinterpret_cast<const float2*>(row + 2 * tx);
+    v[0] = a.x; v[1] = a.y;
+  } else {
+    const float4 a = *reinterpret_cast<const float4*>(row + 4 * tx);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    if constexpr (HDP == 96) {
+      const float2 b = *reinterpret_cast<const float2*>(row + 64 + 2 * tx);
+      v[4] = b.x; v[5] = b.y;
+    } else if constexpr (HDP == 128) {
+      const float4 b = *reinterpret_cast<const float4*>(row + 64 + 4 * tx);
+      v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+  }
+}
+// acc[i][c] += sum_n prob[n][4 ty + i] * str[n][col c]
+template <int HDP>
+__device__ __forceinline__ void accumulate(float (&acc)[4][HDP / 16], const float* prob, const float* str, int ty, int tx) {
+#pragma unroll 4
+  for (int n = 0; n < kStr; ++n) {
+    const float4 p = *reinterpret_cast<const float4*>(prob + n * kPPitch + 4 * ty);
+    float v[HDP / 16];
+    load_cols<HDP>(v, str + n * Simt<HDP>::kPitch, tx);
+#pragma unroll
+    for (int c = 0; c < HDP / 16; ++c) {
+      acc[0][c] = fmaf(p.x, v[c], acc[0][c]);
+      acc[1][c] = fmaf(p.y, v[c], acc[1][c]);
+      acc[2][c] = fmaf(p.z, v[c], acc[2][c]);
+      acc[3][c] = fmaf(p.w, v[c], acc[3][c]);
+    }
+  }
+}
+__device__ __forceinline__ void put_probs(float* prob, const float (&s)[4][4], int ty, int tx) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    *reinterpret_cast<float4*>(prob + (tx + 16 * j) * kPPitch + 4 * ty) = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
+}
+__device__ __forceinline__ float row_max(float v) {  // over the 16 threads of a row
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ __forceinline__ float row_sum(float v) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <int HDP>
+__device__ __forceinline__ void zero(float (&a)[4][HDP / 16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int c = 0; c < HDP / 16; ++c) a[i][c] = 0.f;
+}
+
+// Forward: grid (B * H, query tiles), the longest rows first.
+template <int HDP, typename T, typename TO>
+__global__ void __launch_bounds__(kSimtThreads)
+attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, float* __restrict__ lse, int seq, int H, int KV, int hd, float scale) {
+  extern __shared__ __align__(16) float simt_smem[];
+  float* Qs = simt_smem;
+  float* Ks = Qs + Simt<HDP>::kResFloats;
+  float* Vs = Ks + Simt<HDP>::kStrFloats;
+  float* Ps = Vs + Simt<HDP>::kStrFloats;
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int b = blockIdx.x / H, h = blockIdx.x - b * H, kvh = h / (H / KV);
+  const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRes;
   const int ld = (H + 2 * KV) * hd;
   const size_t row0 = (size_t)b * seq;
-  float* q = s_q + warp * hd;
-  const T* qp = qkv + (row0 + t) * ld + (size_t)h * hd;
-  for (int d = lane; d < hd; d += 32) q[d] = to_f<T>(qp[d]);
-  __syncwarp();
-  const T* kbase = qkv + row0 * ld + (size_t)(H + kvh) * hd;
-  const T* vbase = qkv + row0 * ld + (size_t)(H + KV + kvh) * hd;
-  float m_run = -INFINITY, l_run = 0.f;
-  float acc[kMaxHdPerLane] = {0.f, 0.f, 0.f, 0.f};
-  for (int j0 = 0; j0 <= t; j0 += 32) {
-    const int j = j0 + lane;
-    float s = -INFINITY;
-    if (j <= t) {
-      const T* kp = kbase + (size_t)j * ld;
-      float dot = 0.f;
-      for (int d = 0; d < hd; ++d) dot += q[d] * to_f<T>(kp[d]);
-      s = dot * scale;
+  const T* kb = qkv + row0 * ld + (size_t)(H + kvh) * hd;
+  const T* vb = qkv + row0 * ld + (size_t)(H + KV + kvh) * hd;
+  load_rows<HDP, kRes>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
+  float m[4], l[4], acc[4][HDP / 16];
+  zero<HDP>(acc);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+  }
+  const int last = min(q0 + kRes, seq) - 1;
+  for (int k0 = 0; k0 <= last; k0 += kStr) {
+    __syncthreads();
+    load_rows<HDP, kStr>(Ks, kb + (size_t)k0 * ld, ld, seq - k0, hd);
+    load_rows<HDP, kStr>(Vs, vb + (size_t)k0 * ld, ld, seq - k0, hd);
+    __syncthreads();
+    float s[4][4];
+    scores<HDP>(s, Qs, Ks, ty, tx);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = q0 + 4 * ty + i;
+      float mx = m[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] = k0 + tx + 16 * j <= row ? s[i][j] * scale : -INFINITY;
+        mx = fmaxf(mx, s[i][j]);
+      }
+      mx = row_max(mx);  // finite from the first tile on: every row sees key 0
+      const float corr = expf(m[i] - mx);
+      m[i] = mx;
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] = expf(s[i][j] - mx);
+        sum += s[i][j];
+      }
+      l[i] = l[i] * corr + sum;  // this thread's part of the sum
+#pragma unroll
+      for (int c = 0; c < HDP / 16; ++c) acc[i][c] *= corr;
     }
-    const float m_new = fmaxf(m_run, warp_max(s));
-    const float corr = __expf(m_run - m_new);  // exp(-inf) = 0 on the first chunk
-    const float p = (j <= t) ? __expf(s - m_new) : 0.f;
-    l_run = l_run * corr + warp_sum(p);
+    put_probs(Ps, s, ty, tx);
+    __syncthreads();
+    accumulate<HDP>(acc, Ps, Vs, ty, tx);
+  }
 #pragma unroll
-    for (int c = 0; c < kMaxHdPerLane; ++c) acc[c] *= corr;
-    const int lim = min(32, t - j0 + 1);
-    for (int jj = 0; jj < lim; ++jj) {
-      const float pj = __shfl_sync(0xffffffffu, p, jj);
-      const T* vp = vbase + (size_t)(j0 + jj) * ld;
+  for (int i = 0; i < 4; ++i) {
+    const int row = q0 + 4 * ty + i;
+    const float sum = row_sum(l[i]);
+    if (row >= seq) continue;
+    const float inv = 1.0f / sum;
+    TO* op = out + (row0 + row) * (size_t)(H * hd) + (size_t)h * hd;
 #pragma unroll
-      for (int c = 0; c < kMaxHdPerLane; ++c) {
-        const int d = lane + 32 * c;
-        if (d < hd) acc[c] += pj * to_f<T>(vp[d]);
+    for (int c = 0; c < HDP / 16; ++c) {
+      const int d = col_of<HDP>(tx, c);
+      if (d < hd) op[d] = from_f<TO>(acc[i][c] * inv);
+    }
+    if (tx == 0 && lse) lse[((size_t)b * H + h) * seq + row] = m[i] + logf(sum);
+  }
+}
+
+// Backward, first kernel: row statistics for this scale (maximum, 1 / sum, delta = sum_j P dP; the forward's own do not
+// serve, its scale may differ) in one sweep over the keys, dQ in a second.
+template <int HDP, typename T, typename TD>
+__global__ void __launch_bounds__(kSimtThreads)
+attention_dq_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_out, float* __restrict__ dqkv, float* __restrict__ stats, int rows, int seq,
+                         int H, int KV, int hd, float scale) {
+  extern __shared__ __align__(16) float simt_smem[];
+  float* Qs = simt_smem;
+  float* dOs = Qs + Simt<HDP>::kResFloats;
+  float* Ks = dOs + Simt<HDP>::kResFloats;
+  float* Vs = Ks + Simt<HDP>::kStrFloats;
+  float* Ps = Vs + Simt<HDP>::kStrFloats;
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int b = blockIdx.x / H, h = blockIdx.x - b * H, kvh = h / (H / KV);
+  const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRes;
+  const int ld = (H + 2 * KV) * hd;
+  const size_t row0 = (size_t)b * seq;
+  const T* kb = qkv + row0 * ld + (size_t)(H + kvh) * hd;
+  const T* vb = qkv + row0 * ld + (size_t)(H + KV + kvh) * hd;
+  load_rows<HDP, kRes>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
+  load_rows<HDP, kRes>(dOs, d_out + (row0 + q0) * (size_t)(H * hd) + (size_t)h * hd, H * hd, seq - q0, hd);
+  const int last = min(q0 + kRes, seq) - 1;
+  float m[4], l[4], dl[4], acc[4][HDP / 16];
+  zero<HDP>(acc);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = dl[i] = 0.f;
+  }
+  float s[4][4], dp[4][4];
+  for (int k0 = 0; k0 <= last; k0 += kStr) {
+    __syncthreads();
+    load_rows<HDP, kStr>(Ks, kb + (size_t)k0 * ld, ld, seq - k0, hd);
+    load_rows<HDP, kStr>(Vs, vb + (size_t)k0 * ld, ld, seq - k0, hd);
+    __syncthreads();
+    scores<HDP>(s, Qs, Ks, ty, tx);
+    scores<HDP>(dp, dOs, Vs, ty, tx);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = q0 + 4 * ty + i;
+      float mx = m[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] = k0 + tx + 16 * j <= row ? s[i][j] * scale : -INFINITY;
+        mx = fmaxf(mx, s[i][j]);
+      }
+      mx = row_max(mx);
+      const float corr = expf(m[i] - mx);
+      m[i] = mx;
+      l[i] *= corr;
+      dl[i] *= corr;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = expf(s[i][j] - mx);
+        l[i] += p;
+        dl[i] += p * dp[i][j];
       }
     }
-    m_run = m_new;
   }
-  const float inv = 1.0f / l_run;
-  TO* op = out + (row0 + t) * (size_t)(H * hd) + (size_t)h * hd;
 #pragma unroll
-  for (int c = 0; c < kMaxHdPerLane; ++c) {
-    const int d = lane + 32 * c;
-    if (d < hd) op[d] = from_f<TO>(acc[c] * inv);
+  for (int i = 0; i < 4; ++i) {
+    l[i] = 1.0f / row_sum(l[i]);
+    dl[i] = row_sum(dl[i]) * l[i];
+    const int row = q0 + 4 * ty + i;
+    if (tx == 0 && row < seq) {
+      float* st = stats + ((size_t)b * H + h) * seq + row;
+      st[0] = m[i];
+      st[(size_t)rows] = l[i];
+      st[(size_t)2 * rows] = dl[i];
+    }
   }
-  if (lane == 0 && lse) lse[((size_t)b * H + h) * seq + t] = m_run + logf(l_run);
+  for (int k0 = 0; k0 <= last; k0 += kStr) {
+    if (last >= kStr) {  // more than one tile: the first sweep ended on another one
+      __syncthreads();
+      load_rows<HDP, kStr>(Ks, kb + (size_t)k0 * ld, ld, seq - k0, hd);
+      load_rows<HDP, kStr>(Vs, vb + (size_t)k0 * ld, ld, seq - k0, hd);
+      __syncthreads();
+      scores<HDP>(s, Qs, Ks, ty, tx);
+      scores<HDP>(dp, dOs, Vs, ty, tx);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = q0 + 4 * ty + i;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        // one tile: s holds the scaled and masked scores of the first sweep
+        const float sc = last >= kStr ? (k0 + tx + 16 * j <= row ? s[i][j] * scale : -INFINITY) : s[i][j];
+        const float p = expf(sc - m[i]) * l[i];
+        s[i][j] = p * (dp[i][j] - dl[i]) * scale;
+      }
+    }
+    put_probs(Ps, s, ty, tx);
+    __syncthreads();
+    accumulate<HDP>(acc, Ps, Ks, ty, tx);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = q0 + 4 * ty + i;
+    if (row >= seq) continue;
+    float* op = dqkv + (row0 + row) * ld + (size_t)h * hd;
+#pragma unroll
+    for (int c = 0; c < HDP / 16; ++c) {
+      const int d = col_of<HDP>(tx, c);
+      if (d < hd) op[d] = acc[i][c];
+    }
+  }
 }
+
+// Backward, second kernel: dK and dV of 32 keys over the queries of every head that shares them; no atomics.
+template <int HDP, typename T, typename TD>
+__global__ void __launch_bounds__(kSimtThreads)
+attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_out, float* __restrict__ dqkv, const float* __restrict__ stats, int rows,
+                          int seq, int H, int KV, int hd, float scale) {
+  extern __shared__ __align__(16) float simt_smem[];
+  float* Ks = simt_smem;
+  float* Vs = Ks + Simt<HDP>::kResFloats;
+  float* Qs = Vs + Simt<HDP>::kResFloats;
+  float* dOs = Qs + Simt<HDP>::kStrFloats;
+  float* Ps = dOs + Simt<HDP>::kStrFloats;
+  float* Ds = Ps + Simt<HDP>::kProbFloats;
+  float* st = Ds + Simt<HDP>::kProbFloats;  // maximum, 1 / sum, delta of the 64 queries
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int b = blockIdx.x / KV, kvh = blockIdx.x - b * KV, group = H / KV;
+  const int k0 = (int)blockIdx.y * kRes;
+  const int ld = (H + 2 * KV) * hd;
+  const size_t row0 = (size_t)b * seq;
+  load_rows<HDP, kRes>(Ks, qkv + (row0 + k0) * ld + (size_t)(H + kvh) * hd, ld, seq - k0, hd);
+  load_rows<HDP, kRes>(Vs, qkv + (row0 + k0) * ld + (size_t)(H + KV + kvh) * hd, ld, seq - k0, hd);
+  float dk[4][HDP / 16], dv[4][HDP / 16];
+  zero<HDP>(dk);
+  zero<HDP>(dv);
+  for (int h = kvh * group; h < (kvh + 1) * group; ++h) {
+    for (int q0 = k0 / kStr * kStr; q0 < seq; q0 += kStr) {
+      __syncthreads();
+      load_rows<HDP, kStr>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
+      load_rows<HDP, kStr>(dOs, d_out + (row0 + q0) * (size_t)(H * hd) + (size_t)h * hd, H * hd, seq - q0, hd);
+      for (int i = threadIdx.x; i < 3 * kStr; i += kSimtThreads) {
+        const int q = q0 + (i & (kStr - 1));
+        st[i] = q < seq ? stats[(size_t)(i / kStr) * rows + ((size_t)b * H + h) * seq + q] : 0.f;
+      }
+      __syncthreads();
+      float s[4][4], dp[4][4];
+      scores<HDP>(s, Ks, Qs, ty, tx);
+      scores<HDP>(dp, Vs, dOs, ty, tx);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int q = tx + 16 * j;
+        const float mq = st[q], lq = st[kStr + q], dq = st[2 * kStr + q];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const bool see = k0 + 4 * ty + i <= q0 + q && q0 + q < seq;
+          const float p = see ? expf(s[i][j] * scale - mq) * lq : 0.f;
+          s[i][j] = p;
+          dp[i][j] = p * (dp[i][j] - dq) * scale;
+        }
+      }
+      put_probs(Ps, s, ty, tx);
+      put_probs(Ds, dp, ty, tx);
+      __syncthreads();
+      accumulate<HDP>(dv, Ps, dOs, ty, tx);
+      accumulate<HDP>(dk, Ds, Qs, ty, tx);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = k0 + 4 * ty + i;
+    if (row >= seq) continue;
+    float* kp = dqkv + (row0 + row) * ld + (size_t)(H + kvh) * hd;
+    float* vp = dqkv + (row0 + row) * ld + (size_t)(H + KV + kvh) * hd;
+#pragma unroll
+    for (int c = 0; c < HDP / 16; ++c) {
+      const int d = col_of<HDP>(tx, c);
+      if (d < hd) {
+        kp[d] = dk[i][c];
+        vp[d] = dv[i][c];
+      }
+    }
+  }
+}
+
+template <int HDP, typename T, typename TO>
+void forward_hdp(const T* qkv, TO* out, float* lse, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
+  auto kern = attention_forward_simt_kernel<HDP, T, TO>;
+  static unsigned long long done = 0;
+  smem_opt_in(kern, Simt<HDP>::kFwdSmem, done);
+  kern<<<dim3(B * H, (seq + kRes - 1) / kRes), kSimtThreads, Simt<HDP>::kFwdSmem, s>>>(qkv, out, lse, seq, H, KV, hd, scale);
+}
+template <int HDP, typename T, typename TD>
+void backward_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
+  auto dq = attention_dq_simt_kernel<HDP, T, TD>;
+  auto dkv = attention_dkv_simt_kernel<HDP, T, TD>;
+  static unsigned long long done_q = 0, done_k = 0;
+  smem_opt_in(dq, Simt<HDP>::kDqSmem, done_q);
+  smem_opt_in(dkv, Simt<HDP>::kDkvSmem, done_k);
+  const int tiles = (seq + kRes - 1) / kRes, rows = B * H * seq;
+  dq<<<dim3(B * H, tiles), kSimtThreads, Simt<HDP>::kDqSmem, s>>>(qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
+  dkv<<<dim3(B * KV, tiles), kSimtThreads, Simt<HDP>::kDkvSmem, s>>>(qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
+}
+
+}  // namespace
 
 template <typename T, typename TO>
 void attention_forward_simt(const T* qkv, TO* out, float* lse, int B, int seq, int H, int KV, int hd, float scale,
                             cudaStream_t s) {
-  const long long total = (long long)B * H * seq;
-  if (total <= 0) return;
-  const unsigned blocks = (unsigned)((total + kAttWarps - 1) / kAttWarps);
-  attention_forward_simt_kernel<T, TO><<<blocks, kAttWarps * 32, kAttWarps * hd * sizeof(float), s>>>(qkv, out, lse, B, seq,
-                                                                                                   H, KV, hd, scale);
+  if (B <= 0 || seq <= 0) return;
+  if (hd <= 32) forward_hdp<32>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
+  else if (hd <= 48) forward_hdp<48>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
+  else if (hd <= 64) forward_hdp<64>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
+  else if (hd <= 96) forward_hdp<96>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
+  else forward_hdp<128>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
 }
 template void attention_forward_simt<float, float>(const float*, float*, float*, int, int, int, int, int, float,
                                                    cudaStream_t);
@@ -89,115 +448,22 @@ template void attention_forward_simt<bf16, bf16>(const bf16*, bf16*, float*, int
 template void attention_forward_simt<float, bf16>(const float*, bf16*, float*, int, int, int, int, int, float,
                                                   cudaStream_t);
 
-// Backward: one warp per query row.  Dynamic smem per warp: 2*hd (q, dO) + 2*seq (scores, dP) floats.
-// dq/dk/dv accumulate into a zero-initialised fp32 [M, (H+2KV)*hd] buffer with atomics.
 template <typename T, typename TD>
-__global__ void attention_backward_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_out,
-                                               float* __restrict__ dqkv, int B, int seq, int H, int KV, int hd,
-                                               float scale) {
-  extern __shared__ float s_mem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long wid = (long long)blockIdx.x * kAttWarps + warp;
-  const long long total = (long long)B * H * seq;
-  if (wid >= total) return;
-  const int t = (int)(wid % seq);
-  const int h = (int)((wid / seq) % H);
-  const int b = (int)(wid / ((long long)seq * H));
-  const int kvh = h / (H / KV);
-  const int ld = (H + 2 * KV) * hd;
-  const size_t row0 = (size_t)b * seq;
-  float* base = s_mem + (size_t)warp * (2 * hd + 2 * seq);
-  float* q = base;
-  float* dO = base + hd;
-  float* sc = base + 2 * hd;
-  float* dP = sc + seq;
-  const T* qp = qkv + (row0 + t) * ld + (size_t)h * hd;
-  const TD* dop = d_out + (row0 + t) * (size_t)(H * hd) + (size_t)h * hd;
-  for (int d = lane; d < hd; d += 32) {
-    q[d] = to_f<T>(qp[d]);
-    dO[d] = to_f<TD>(dop[d]);
-  }
-  __syncwarp();
-  const T* kbase = qkv + row0 * ld + (size_t)(H + kvh) * hd;
-  const T* vbase = qkv + row0 * ld + (size_t)(H + KV + kvh) * hd;
-  float mx = -INFINITY;
-  for (int j = lane; j <= t; j += 32) {
-    const T* kp = kbase + (size_t)j * ld;
-    const T* vp = vbase + (size_t)j * ld;
-    float dot = 0.f, dp = 0.f;
-    for (int d = 0; d < hd; ++d) {
-      dot += q[d] * to_f<T>(kp[d]);
-      dp += dO[d] * to_f<T>(vp[d]);
-    }
-    sc[j] = dot * scale;
-    dP[j] = dp;
-    mx = fmaxf(mx, dot * scale);
-  }
-  mx = warp_max(mx);
-  float tot = 0.f;
-  for (int j = lane; j <= t; j += 32) {
-    const float e = expf(sc[j] - mx);
-    sc[j] = e;
-    tot += e;
-  }
-  tot = warp_sum(tot);
-  const float inv = 1.0f / tot;
-  float ds_sum = 0.f;
-  for (int j = lane; j <= t; j += 32) {
-    const float p = sc[j] * inv;
-    sc[j] = p;
-    ds_sum += p * dP[j];
-  }
-  ds_sum = warp_sum(ds_sum);
-  __syncwarp();
-  float dq_acc[kMaxHdPerLane] = {0.f, 0.f, 0.f, 0.f};
-  float* dkb = dqkv + row0 * ld + (size_t)(H + kvh) * hd;
-  float* dvb = dqkv + row0 * ld + (size_t)(H + KV + kvh) * hd;
-  for (int j = 0; j <= t; ++j) {
-    const float p = sc[j];
-    const float ds = p * (dP[j] - ds_sum) * scale;
-    const T* kp = kbase + (size_t)j * ld;
-#pragma unroll
-    for (int c = 0; c < kMaxHdPerLane; ++c) {
-      const int d = lane + 32 * c;
-      if (d < hd) {
-        dq_acc[c] += ds * to_f<T>(kp[d]);
-        atomicAdd(dkb + (size_t)j * ld + d, ds * q[d]);
-        atomicAdd(dvb + (size_t)j * ld + d, p * dO[d]);
-      }
-    }
-  }
-  float* dqp = dqkv + (row0 + t) * ld + (size_t)h * hd;
-#pragma unroll
-  for (int c = 0; c < kMaxHdPerLane; ++c) {
-    const int d = lane + 32 * c;
-    if (d < hd) dqp[d] = dq_acc[c];  // each (row, head) is owned by exactly one warp
-  }
-}
-
-template <typename T, typename TD>
-void attention_backward_simt(const T* qkv, const TD* d_out, float* dqkv_f32, int B, int seq, int H, int KV, int hd,
+void attention_backward_simt(const T* qkv, const TD* d_out, float* dqkv_f32, float* stats, int B, int seq, int H, int KV, int hd,
                              float scale, cudaStream_t s) {
-  const long long total = (long long)B * H * seq;
-  if (total <= 0) return;
-  const unsigned blocks = (unsigned)((total + kAttWarps - 1) / kAttWarps);
-  const size_t smem = sizeof(float) * (size_t)kAttWarps * (2 * hd + 2 * seq);
-  static bool attr_done = false;  // one flag per template instantiation
-  if (!attr_done && smem > 48 * 1024) {
-    cudaFuncSetAttribute(attention_backward_simt_kernel<T, TD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         200 * 1024);
-    attr_done = true;
-  }
-  attention_backward_simt_kernel<T, TD><<<blocks, kAttWarps * 32, smem, s>>>(qkv, d_out, dqkv_f32, B, seq, H, KV, hd,
-                                                                         scale);
+  if (B <= 0 || seq <= 0) return;
+  if (hd <= 32) backward_hdp<32>(qkv, d_out, dqkv_f32, stats, B, seq, H, KV, hd, scale, s);
+  else if (hd <= 48) backward_hdp<48>(qkv, d_out, dqkv_f32, stats, B, seq, H, KV, hd, scale, s);
+  else if (hd <= 64) backward_hdp<64>(qkv, d_out, dqkv_f32, stats, B, seq, H, KV, hd, scale, s);
+  else if (hd <= 96) backward_hdp<96>(qkv, d_out, dqkv_f32, stats, B, seq, H, KV, hd, scale, s);
+  else backward_hdp<128>(qkv, d_out, dqkv_f32, stats, B, seq, H, KV, hd, scale, s);
 }
-template void attention_backward_simt<float, float>(const float*, const float*, float*, int, int, int, int, int, float,
+template void attention_backward_simt<float, float>(const float*, const float*, float*, float*, int, int, int, int, int, float,
                                                     cudaStream_t);
-template void attention_backward_simt<bf16, bf16>(const bf16*, const bf16*, float*, int, int, int, int, int, float,
+template void attention_backward_simt<bf16, bf16>(const bf16*, const bf16*, float*, float*, int, int, int, int, int, float,
                                                   cudaStream_t);
-template void attention_backward_simt<float, bf16>(const float*, const bf16*, float*, int, int, int, int, int, float,
+template void attention_backward_simt<float, bf16>(const float*, const bf16*, float*, float*, int, int, int, int, int, float,
                                                    cudaStream_t);
-
 
 // ------------------------------------------------------------------------------------------------
 // KV cache for decoding: caches are [B, max_seq, KV*hd].

@@ -1,5 +1,5 @@
 // Causal flash-style attention on tensor cores (bf16 operands, fp32 softmax and accumulation),
-// head_dim 64, GQA-aware.  Probabilities are never written to memory: the forward keeps a running
+// head_dim 32, 48 or 64, GQA-aware.  Probabilities are never written to memory: the forward keeps a running
 // (max, sum) per query row, the backward recomputes each score tile from Q, K and the saved
 // log-sum-exp.  Key/value (forward, dQ) or query/dO (dK/dV) tiles stream through a two-stage
 // cp.async ring so loads overlap the MMAs.
@@ -20,11 +20,20 @@ namespace ane {
 
 namespace {
 
-constexpr int HD = 64;
 constexpr int KT = 64;           // streamed tile (keys in fwd/dQ, queries in dK/dV)
-constexpr int BR = 128;          // resident tile rows per block (8 warps x 16 rows)
-constexpr int LDS = HD + 8;      // padded smem row (144 B: 16-B aligned rows, conflict-free ldmatrix)
-constexpr int ATT_THREADS = 256;
+// Tile of one kernel instance: head size HD, NW warps of 16 resident rows each.  Eight warps share every streamed tile
+// among 128 rows; four make twice as many blocks, which is faster while 128-row blocks leave SMs idle (see rows_per_block).
+template <int HD_, int NW_>
+struct Tile {
+  static constexpr int HD = HD_;
+  static constexpr int BR = 16 * NW_;       // resident tile rows per block
+  static constexpr int LDS = HD_ + 8;       // padded smem row (16-B aligned rows; pitches of 80, 112 and 144 B: conflict-free ldmatrix)
+  static constexpr int THREADS = 32 * NW_;
+  static constexpr int NT = HD_ / 8;        // 8-column accumulator tiles of the head
+  static constexpr size_t kFwdSmem = (size_t)(BR + 4 * KT) * LDS * sizeof(bf16);
+  static constexpr size_t kDqSmem = (size_t)(2 * BR + 4 * KT) * LDS * sizeof(bf16);
+  static constexpr size_t kDkvSmem = (size_t)(2 * BR + 4 * KT) * LDS * sizeof(bf16) + 4 * KT * sizeof(float);
+};
 constexpr float kLog2e = 1.4426950408889634f;
 
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const bf16* p) {
@@ -60,35 +69,38 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Asynchronously copies an [nrows x 64] bf16 tile (row pitch ld) into padded smem; rows >= rows_valid
+// Asynchronously copies an [nrows x HD] bf16 tile (row pitch ld) into padded smem; rows >= rows_valid
 // are zero-filled.  rows_valid >= 1.
+template <class C>
 __device__ __forceinline__ void load_tile_async(bf16* dst, const bf16* src, int ld, int nrows, int rows_valid) {
-  for (int i = threadIdx.x; i < nrows * (HD / 8); i += ATT_THREADS) {
-    const int r = i >> 3, c = (i & 7) * 8;
+  for (int i = threadIdx.x; i < nrows * C::NT; i += C::THREADS) {
+    const int r = i / C::NT, c = (i - r * C::NT) * 8;
     const bool ok = r < rows_valid;
-    cp_async_16(dst + r * LDS + c, src + (size_t)(ok ? r : 0) * ld + c, ok);
+    cp_async_16(dst + r * C::LDS + c, src + (size_t)(ok ? r : 0) * ld + c, ok);
   }
 }
 
 // acc (16 x 64) += A(16 rows of a_tile from a_row0; K = HD) * B^T, with B stored [n][k] in b_tile (64 rows).
+template <class C>
 __device__ __forceinline__ void gemm_a_smem_b_nk(float (&acc)[8][4], const bf16* a_tile, int a_row0, const bf16* b_tile,
                                                  int lane) {
 #pragma unroll
-  for (int kk = 0; kk < HD / 16; ++kk) {
+  for (int kk = 0; kk < C::HD / 16; ++kk) {
     uint32_t a[4];
-    ldsm_x4(a, a_tile + (a_row0 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDS + kk * 16 + (lane >> 4) * 8);
+    ldsm_x4(a, a_tile + (a_row0 + (lane & 7) + ((lane >> 3) & 1) * 8) * C::LDS + kk * 16 + (lane >> 4) * 8);
 #pragma unroll
     for (int np = 0; np < 4; ++np) {
       uint32_t b[4];
-      ldsm_x4(b, b_tile + (np * 16 + (lane & 7) + (lane >> 4) * 8) * LDS + kk * 16 + ((lane >> 3) & 1) * 8);
+      ldsm_x4(b, b_tile + (np * 16 + (lane & 7) + (lane >> 4) * 8) * C::LDS + kk * 16 + ((lane >> 3) & 1) * 8);
       mma_bf16(acc[2 * np], a, b[0], b[1]);
       mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
     }
   }
 }
 
-// acc (16 x 64) += P (16 x 64 in registers, accumulator layout, rounded to bf16) * B, with B stored [k][n] (64 rows).
-__device__ __forceinline__ void gemm_a_regs_b_kn(float (&acc)[8][4], const float (&p)[8][4], const bf16* b_tile,
+// acc (16 x HD) += P (16 x 64 in registers, accumulator layout, rounded to bf16) * B, with B stored [k][n] (64 rows).
+template <class C>
+__device__ __forceinline__ void gemm_a_regs_b_kn(float (&acc)[C::NT][4], const float (&p)[8][4], const bf16* b_tile,
                                                  int lane) {
 #pragma unroll
   for (int kk = 0; kk < KT / 16; ++kk) {
@@ -98,9 +110,9 @@ __device__ __forceinline__ void gemm_a_regs_b_kn(float (&acc)[8][4], const float
     a[2] = pack_bf16(p[2 * kk + 1][0], p[2 * kk + 1][1]);
     a[3] = pack_bf16(p[2 * kk + 1][2], p[2 * kk + 1][3]);
 #pragma unroll
-    for (int np = 0; np < HD / 16; ++np) {
+    for (int np = 0; np < C::HD / 16; ++np) {
       uint32_t b[4];
-      ldsm_x4_t(b, b_tile + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDS + np * 16 + (lane >> 4) * 8);
+      ldsm_x4_t(b, b_tile + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * C::LDS + np * 16 + (lane >> 4) * 8);
       mma_bf16(acc[2 * np], a, b[0], b[1]);
       mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
     }
@@ -115,17 +127,19 @@ __device__ __forceinline__ float quad_sum(float v) {
   v += __shfl_xor_sync(0xffffffffu, v, 1);
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
-__device__ __forceinline__ void zero_acc(float (&a)[8][4]) {
+template <int N>
+__device__ __forceinline__ void zero_acc(float (&a)[N][4]) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) a[i][e] = 0.f;
 }
 
-// Writes one accumulator (16 rows x 64 cols per warp) as bf16 into a packed gradient row, optionally
+// Writes one accumulator (16 rows x HD cols per warp) as bf16 into a packed gradient row, optionally
 // undoing the pair rotation first (each thread holds whole (even, odd) pairs).
+template <class C>
 __device__ __forceinline__ void store_grad_bf16(bf16* base, int ld, int row_lo, int T, size_t row0,
-                                                const float (&acc)[8][4], const float* cosb, const float* sinb,
+                                                const float (&acc)[C::NT][4], const float* cosb, const float* sinb,
                                                 int g, int t4) {
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -133,11 +147,11 @@ __device__ __forceinline__ void store_grad_bf16(bf16* base, int ld, int row_lo, 
     if (row >= T) continue;
     bf16* p = base + (row0 + row) * ld;
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
+    for (int nt = 0; nt < C::NT; ++nt) {
       float e = acc[nt][2 * r], o = acc[nt][2 * r + 1];
       if (cosb) {
         const int pair = nt * 4 + t4;
-        const float c = cosb[row * (HD / 2) + pair], s = sinb[row * (HD / 2) + pair];
+        const float c = cosb[row * (C::HD / 2) + pair], s = sinb[row * (C::HD / 2) + pair];
         const float e2 = e * c + o * s, o2 = o * c - e * s;
         e = e2;
         o = o2;
@@ -148,11 +162,13 @@ __device__ __forceinline__ void store_grad_bf16(bf16* base, int ld, int row_lo, 
 }
 
 // ------------------------------------------------------------------------------------------------
-// Forward: grid (query tiles of 128, B*H); 8 warps x 16 query rows; key/value tiles of 64 streamed.
+// Forward: grid (query tiles of BR, B*H); 16 query rows per warp; key/value tiles of 64 streamed.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(ATT_THREADS)
+template <class C>
+__global__ void __launch_bounds__(C::THREADS)
 attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf16* __restrict__ out_lo,
                         float* __restrict__ lse, int T, int H, int KV, float scale) {
+  constexpr int HD = C::HD, BR = C::BR, LDS = C::LDS;
   extern __shared__ __align__(16) uint8_t att_smem[];
   bf16* Qs = reinterpret_cast<bf16*>(att_smem);   // [BR][LDS]
   bf16* Ks = Qs + BR * LDS;                       // [2][KT][LDS]
@@ -167,11 +183,11 @@ attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf
   const int n_kv = q_last / KT + 1;
   const bf16* kbase = qkv + row0 * ld + (size_t)(H + kvh) * HD;
   const bf16* vbase = qkv + row0 * ld + (size_t)(H + KV + kvh) * HD;
-  load_tile_async(Qs, qkv + (row0 + q0) * ld + (size_t)h * HD, ld, BR, min(BR, T - q0));
-  load_tile_async(Ks, kbase, ld, KT, min(KT, T));
-  load_tile_async(Vs, vbase, ld, KT, min(KT, T));
+  load_tile_async<C>(Qs, qkv + (row0 + q0) * ld + (size_t)h * HD, ld, BR, min(BR, T - q0));
+  load_tile_async<C>(Ks, kbase, ld, KT, min(KT, T));
+  load_tile_async<C>(Vs, vbase, ld, KT, min(KT, T));
   cp_async_commit();
-  float o[8][4];
+  float o[C::NT][4];
   zero_acc(o);
   float m_i[2] = {-INFINITY, -INFINITY}, l_i[2] = {0.f, 0.f};
   const float sl2 = scale * kLog2e;
@@ -180,8 +196,8 @@ attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf
     const int k0 = j * KT;
     if (j + 1 < n_kv) {
       const int kn = k0 + KT;
-      load_tile_async(Ks + ((j + 1) & 1) * KT * LDS, kbase + (size_t)kn * ld, ld, KT, min(KT, T - kn));
-      load_tile_async(Vs + ((j + 1) & 1) * KT * LDS, vbase + (size_t)kn * ld, ld, KT, min(KT, T - kn));
+      load_tile_async<C>(Ks + ((j + 1) & 1) * KT * LDS, kbase + (size_t)kn * ld, ld, KT, min(KT, T - kn));
+      load_tile_async<C>(Vs + ((j + 1) & 1) * KT * LDS, vbase + (size_t)kn * ld, ld, KT, min(KT, T - kn));
       cp_async_commit();
       cp_async_wait<1>();
     } else {
@@ -193,7 +209,7 @@ attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf
       const bf16* Vc = Vs + (j & 1) * KT * LDS;
       float s[8][4];
       zero_acc(s);
-      gemm_a_smem_b_nk(s, Qs, warp * 16, Kc, lane);
+      gemm_a_smem_b_nk<C>(s, Qs, warp * 16, Kc, lane);
       float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
@@ -227,10 +243,10 @@ attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf
 #pragma unroll
       for (int r = 0; r < 2; ++r) l_i[r] = l_i[r] * corr[r] + rs[r];
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+      for (int nt = 0; nt < C::NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[nt][e] *= corr[e >> 1];
-      gemm_a_regs_b_kn(o, s, Vc, lane);
+      gemm_a_regs_b_kn<C>(o, s, Vc, lane);
     }
     __syncthreads();
   }
@@ -242,7 +258,7 @@ attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf
       const float inv = 1.0f / l_i[r];
       bf16* op = out + (row0 + row) * (size_t)(H * HD) + (size_t)h * HD;
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
+      for (int nt = 0; nt < C::NT; ++nt) {
         const float ox = o[nt][2 * r] * inv, oy = o[nt][2 * r + 1] * inv;
         const __nv_bfloat162 hi = __floats2bfloat162_rn(ox, oy);
         *reinterpret_cast<__nv_bfloat162*>(op + nt * 8 + 2 * t4) = hi;
@@ -257,7 +273,7 @@ attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf
 
 // delta[b,h,t] = sum_d dO * O  (one warp per (token, head))
 __global__ void attention_delta_kernel(const bf16* __restrict__ d_out, const bf16* __restrict__ out,
-                                       const bf16* __restrict__ out_lo, float* __restrict__ delta, int B, int T, int H) {
+                                       const bf16* __restrict__ out_lo, float* __restrict__ delta, int B, int T, int H, int HD) {
   const long long wid = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (wid >= (long long)B * T * H) return;
@@ -265,24 +281,29 @@ __global__ void attention_delta_kernel(const bf16* __restrict__ d_out, const bf1
   const long long m = wid / H;
   const int b = (int)(m / T), t = (int)(m - (long long)b * T);
   const size_t off = (size_t)m * (H * HD) + (size_t)h * HD + 2 * lane;
+  float v = 0.f;
+  if (2 * lane < HD) {
   const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(d_out + off);
   const __nv_bfloat162 c = *reinterpret_cast<const __nv_bfloat162*>(out + off);
-  float v = __bfloat162float(a.x) * __bfloat162float(c.x) + __bfloat162float(a.y) * __bfloat162float(c.y);
+  v = __bfloat162float(a.x) * __bfloat162float(c.x) + __bfloat162float(a.y) * __bfloat162float(c.y);
   if (out_lo) {
     const __nv_bfloat162 d = *reinterpret_cast<const __nv_bfloat162*>(out_lo + off);
     v += __bfloat162float(a.x) * __bfloat162float(d.x) + __bfloat162float(a.y) * __bfloat162float(d.y);
+  }
   }
   v = warp_sum(v);
   if (lane == 0) delta[((size_t)b * H + h) * T + t] = v;
 }
 
 // ------------------------------------------------------------------------------------------------
-// Backward, dQ: grid (query tiles of 128, B*H); key/value tiles streamed.
+// Backward, dQ: grid (query tiles of BR, B*H); key/value tiles streamed.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(ATT_THREADS)
+template <class C>
+__global__ void __launch_bounds__(C::THREADS)
 attention_bwd_dq_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ d_out, const float* __restrict__ lse,
                            const float* __restrict__ delta, bf16* __restrict__ dqkv, const float* __restrict__ cosb,
                            const float* __restrict__ sinb, int T, int H, int KV, float scale) {
+  constexpr int HD = C::HD, BR = C::BR, LDS = C::LDS;
   extern __shared__ __align__(16) uint8_t att_smem[];
   bf16* Qs = reinterpret_cast<bf16*>(att_smem);   // [BR][LDS]
   bf16* dOs = Qs + BR * LDS;                      // [BR][LDS]
@@ -298,10 +319,10 @@ attention_bwd_dq_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
   const int n_kv = (q0 + q_valid - 1) / KT + 1;
   const bf16* kbase = qkv + row0 * ld + (size_t)(H + kvh) * HD;
   const bf16* vbase = qkv + row0 * ld + (size_t)(H + KV + kvh) * HD;
-  load_tile_async(Qs, qkv + (row0 + q0) * ld + (size_t)h * HD, ld, BR, q_valid);
-  load_tile_async(dOs, d_out + (row0 + q0) * (size_t)(H * HD) + (size_t)h * HD, H * HD, BR, q_valid);
-  load_tile_async(Ks, kbase, ld, KT, min(KT, T));
-  load_tile_async(Vs, vbase, ld, KT, min(KT, T));
+  load_tile_async<C>(Qs, qkv + (row0 + q0) * ld + (size_t)h * HD, ld, BR, q_valid);
+  load_tile_async<C>(dOs, d_out + (row0 + q0) * (size_t)(H * HD) + (size_t)h * HD, H * HD, BR, q_valid);
+  load_tile_async<C>(Ks, kbase, ld, KT, min(KT, T));
+  load_tile_async<C>(Vs, vbase, ld, KT, min(KT, T));
   cp_async_commit();
   const int r_lo = q0 + warp * 16;
   float lse_r[2], del_r[2];
@@ -312,15 +333,15 @@ attention_bwd_dq_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
     lse_r[r] = ok ? lse[((size_t)b * H + h) * T + row] * kLog2e : 0.f;
     del_r[r] = ok ? delta[((size_t)b * H + h) * T + row] : 0.f;
   }
-  float dq[8][4];
+  float dq[C::NT][4];
   zero_acc(dq);
   const float sl2 = scale * kLog2e;
   for (int j = 0; j < n_kv; ++j) {
     const int k0 = j * KT;
     if (j + 1 < n_kv) {
       const int kn = k0 + KT;
-      load_tile_async(Ks + ((j + 1) & 1) * KT * LDS, kbase + (size_t)kn * ld, ld, KT, min(KT, T - kn));
-      load_tile_async(Vs + ((j + 1) & 1) * KT * LDS, vbase + (size_t)kn * ld, ld, KT, min(KT, T - kn));
+      load_tile_async<C>(Ks + ((j + 1) & 1) * KT * LDS, kbase + (size_t)kn * ld, ld, KT, min(KT, T - kn));
+      load_tile_async<C>(Vs + ((j + 1) & 1) * KT * LDS, vbase + (size_t)kn * ld, ld, KT, min(KT, T - kn));
       cp_async_commit();
       cp_async_wait<1>();
     } else {
@@ -333,8 +354,8 @@ attention_bwd_dq_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
       float s[8][4], dp[8][4];
       zero_acc(s);
       zero_acc(dp);
-      gemm_a_smem_b_nk(s, Qs, warp * 16, Kc, lane);
-      gemm_a_smem_b_nk(dp, dOs, warp * 16, Vc, lane);
+      gemm_a_smem_b_nk<C>(s, Qs, warp * 16, Kc, lane);
+      gemm_a_smem_b_nk<C>(dp, dOs, warp * 16, Vc, lane);
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
@@ -345,22 +366,24 @@ attention_bwd_dq_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
           if (col <= row && row < T) p = exp2f(s[nt][e] * sl2 - lse_r[e >> 1]);
           s[nt][e] = p * (dp[nt][e] - del_r[e >> 1]) * scale;  // dS
         }
-      gemm_a_regs_b_kn(dq, s, Kc, lane);
+      gemm_a_regs_b_kn<C>(dq, s, Kc, lane);
     }
     __syncthreads();
   }
-  store_grad_bf16(dqkv + (size_t)h * HD, ld, r_lo, T, row0, dq, cosb, sinb, g, t4);
+  store_grad_bf16<C>(dqkv + (size_t)h * HD, ld, r_lo, T, row0, dq, cosb, sinb, g, t4);
 }
 
 // ------------------------------------------------------------------------------------------------
-// Backward, dK/dV: grid (key tiles of 128, B*KV); 8 warps x 16 key rows; streams the query/dO tiles
+// Backward, dK/dV: grid (key tiles of BR, B*KV); 16 key rows per warp; streams the query/dO tiles
 // of every query head that shares this KV head, so no atomics are needed.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(ATT_THREADS, 2)
+template <class C>
+__global__ void __launch_bounds__(C::THREADS, C::THREADS == 128 ? 3 : 2)
 attention_bwd_dkv_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ d_out,
                             const float* __restrict__ lse, const float* __restrict__ delta, bf16* __restrict__ dqkv,
                             const float* __restrict__ cosb, const float* __restrict__ sinb, int T, int H, int KV,
                             float scale) {
+  constexpr int HD = C::HD, BR = C::BR, LDS = C::LDS;
   extern __shared__ __align__(16) uint8_t att_smem[];
   bf16* Ks = reinterpret_cast<bf16*>(att_smem);   // [BR][LDS]
   bf16* Vs = Ks + BR * LDS;                       // [BR][LDS]
@@ -385,8 +408,8 @@ attention_bwd_dkv_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict
     const int q0 = (i0 + it % per_head) * KT;
     const int q_valid = min(KT, T - q0);
     const int bufi = it & 1;
-    load_tile_async(Qs + bufi * KT * LDS, qkv + (row0 + q0) * ld + (size_t)hq * HD, ld, KT, q_valid);
-    load_tile_async(dOs + bufi * KT * LDS, d_out + (row0 + q0) * (size_t)(H * HD) + (size_t)hq * HD, H * HD, KT,
+    load_tile_async<C>(Qs + bufi * KT * LDS, qkv + (row0 + q0) * ld + (size_t)hq * HD, ld, KT, q_valid);
+    load_tile_async<C>(dOs + bufi * KT * LDS, d_out + (row0 + q0) * (size_t)(H * HD) + (size_t)hq * HD, H * HD, KT,
                     q_valid);
     if (threadIdx.x < KT) {
       const int row = q0 + threadIdx.x;
@@ -395,11 +418,11 @@ attention_bwd_dkv_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict
       del_s[bufi * KT + threadIdx.x] = ok ? delta[((size_t)b * H + hq) * T + row] : 0.f;
     }
   };
-  load_tile_async(Ks, qkv + (row0 + k0) * ld + (size_t)(H + kvh) * HD, ld, BR, k_valid);
-  load_tile_async(Vs, qkv + (row0 + k0) * ld + (size_t)(H + KV + kvh) * HD, ld, BR, k_valid);
+  load_tile_async<C>(Ks, qkv + (row0 + k0) * ld + (size_t)(H + kvh) * HD, ld, BR, k_valid);
+  load_tile_async<C>(Vs, qkv + (row0 + k0) * ld + (size_t)(H + KV + kvh) * HD, ld, BR, k_valid);
   issue(0);
   cp_async_commit();
-  float dk[8][4], dv[8][4];
+  float dk[C::NT][4], dv[C::NT][4];
   zero_acc(dk);
   zero_acc(dv);
   const float sl2 = scale * kLog2e;
@@ -422,8 +445,8 @@ attention_bwd_dkv_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict
       float st[8][4], dpt[8][4];
       zero_acc(st);
       zero_acc(dpt);
-      gemm_a_smem_b_nk(st, Ks, warp * 16, Qc, lane);     // S^T  = K  Q^T
-      gemm_a_smem_b_nk(dpt, Vs, warp * 16, dOc, lane);   // dP^T = V dO^T
+      gemm_a_smem_b_nk<C>(st, Ks, warp * 16, Qc, lane);     // S^T  = K  Q^T
+      gemm_a_smem_b_nk<C>(dpt, Vs, warp * 16, dOc, lane);   // dP^T = V dO^T
       // st becomes P^T in place; after dV it becomes dS^T in place, so only two 16x64 temporaries live.
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
@@ -436,7 +459,7 @@ attention_bwd_dkv_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict
           if (krow <= qrow && qrow < T) p = exp2f(st[nt][e] * sl2 - lse_c[qc]);
           st[nt][e] = p;
         }
-      gemm_a_regs_b_kn(dv, st, dOc, lane);   // dV += P^T dO
+      gemm_a_regs_b_kn<C>(dv, st, dOc, lane);   // dV += P^T dO
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
@@ -444,66 +467,83 @@ attention_bwd_dkv_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict
           const int qc = nt * 8 + 2 * t4 + (e & 1);
           st[nt][e] = st[nt][e] * (dpt[nt][e] - del_c[qc]) * scale;   // dS^T
         }
-      gemm_a_regs_b_kn(dk, st, Qc, lane);    // dK += dS^T Q
+      gemm_a_regs_b_kn<C>(dk, st, Qc, lane);    // dK += dS^T Q
     }
     __syncthreads();
   }
-  store_grad_bf16(dqkv + (size_t)(H + kvh) * HD, ld, kr_lo, T, row0, dk, cosb, sinb, g, t4);
-  store_grad_bf16(dqkv + (size_t)(H + KV + kvh) * HD, ld, kr_lo, T, row0, dv, nullptr, nullptr, g, t4);
+  store_grad_bf16<C>(dqkv + (size_t)(H + kvh) * HD, ld, kr_lo, T, row0, dk, cosb, sinb, g, t4);
+  store_grad_bf16<C>(dqkv + (size_t)(H + KV + kvh) * HD, ld, kr_lo, T, row0, dv, nullptr, nullptr, g, t4);
 }
 
-constexpr size_t kFwdSmem = (size_t)(BR + 4 * KT) * LDS * sizeof(bf16);
-constexpr size_t kDqSmem = (size_t)(2 * BR + 4 * KT) * LDS * sizeof(bf16);
-constexpr size_t kDkvSmem = (size_t)(2 * BR + 4 * KT) * LDS * sizeof(bf16) + 4 * KT * sizeof(float);
-
-bool g_attr_done = false;
-bool ensure_attrs() {
-  if (g_attr_done) return true;
-  if (cudaFuncSetAttribute(attention_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(attention_bwd_dq_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDqSmem) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(attention_bwd_dkv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDkvSmem) !=
-          cudaSuccess)
-    return false;
-  g_attr_done = true;
+template <class C>
+bool launch_forward(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B, int seq, int H, int KV, float scale, cudaStream_t s) {
+  static unsigned long long done = 0;
+  if (!smem_opt_in(attention_fwd_tc_kernel<C>, C::kFwdSmem, done)) return false;
+  dim3 grid((seq + C::BR - 1) / C::BR, B * H);
+  attention_fwd_tc_kernel<C><<<grid, C::THREADS, C::kFwdSmem, s>>>(qkv, out, out_lo, lse, seq, H, KV, scale);
   return true;
+}
+template <class CQ, class CK>
+bool launch_backward(const bf16* qkv, const bf16* d_out, const float* lse, const float* delta, bf16* dqkv, const float* cosb, const float* sinb,
+                     int B, int seq, int H, int KV, float scale, cudaStream_t s) {
+  static unsigned long long done_q = 0, done_k = 0;
+  if (!smem_opt_in(attention_bwd_dq_tc_kernel<CQ>, CQ::kDqSmem, done_q) || !smem_opt_in(attention_bwd_dkv_tc_kernel<CK>, CK::kDkvSmem, done_k))
+    return false;
+  dim3 gq((seq + CQ::BR - 1) / CQ::BR, B * H);
+  attention_bwd_dq_tc_kernel<CQ><<<gq, CQ::THREADS, CQ::kDqSmem, s>>>(qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV, scale);
+  dim3 gk((seq + CK::BR - 1) / CK::BR, B * KV);
+  attention_bwd_dkv_tc_kernel<CK><<<gk, CK::THREADS, CK::kDkvSmem, s>>>(qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV, scale);
+  return true;
+}
+
+// 64-row blocks while 128-row ones would not fill the two blocks per SM that fit.
+bool small_blocks(int units, int seq) { return (long long)units * ((seq + 127) / 128) < 2 * 148; }
+
+template <int HD>
+bool forward_hd(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B, int seq, int H, int KV, float scale, cudaStream_t s) {
+  return small_blocks(B * H, seq) ? launch_forward<Tile<HD, 4>>(qkv, out, out_lo, lse, B, seq, H, KV, scale, s)
+                                  : launch_forward<Tile<HD, 8>>(qkv, out, out_lo, lse, B, seq, H, KV, scale, s);
+}
+template <int HD>
+bool backward_hd(const bf16* qkv, const bf16* d_out, const float* lse, const float* delta, bf16* dqkv, const float* cosb, const float* sinb, int B,
+                 int seq, int H, int KV, float scale, cudaStream_t s) {
+  if (small_blocks(B * KV, seq))
+    return launch_backward<Tile<HD, 4>, Tile<HD, 4>>(qkv, d_out, lse, delta, dqkv, cosb, sinb, B, seq, H, KV, scale, s);
+  return launch_backward<Tile<HD, 8>, Tile<HD, 8>>(qkv, d_out, lse, delta, dqkv, cosb, sinb, B, seq, H, KV, scale, s);
 }
 
 }  // namespace
 
-bool attention_tc_supported(int hd) { return hd == HD; }
+bool attention_tc_supported(int hd) { return hd == 32 || hd == 48 || hd == 64; }
 
-void attention_forward_tc(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B, int seq, int H, int KV, float scale,
+void attention_forward_tc(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B, int seq, int H, int KV, int hd, float scale,
                           int* d_status, cudaStream_t s) {
-  if (B <= 0 || seq <= 0 || !ensure_attrs()) return;
+  if (B <= 0 || seq <= 0) return;
   static const bool legacy = getenv("ANE_B200_ATT_LEGACY") != nullptr;
-  if (!legacy && attention_tcgen05_supported(HD, seq) &&
+  if (!legacy && attention_tcgen05_supported(hd, seq) &&
       attention_forward_tcgen05(qkv, out, out_lo, lse, B, seq, H, KV, scale, d_status, s) == 0)
     return;
-  dim3 grid((seq + BR - 1) / BR, B * H);
-  attention_fwd_tc_kernel<<<grid, ATT_THREADS, kFwdSmem, s>>>(qkv, out, out_lo, lse, seq, H, KV, scale);
+  if (hd == 64) forward_hd<64>(qkv, out, out_lo, lse, B, seq, H, KV, scale, s);
+  else if (hd == 48) forward_hd<48>(qkv, out, out_lo, lse, B, seq, H, KV, scale, s);
+  else forward_hd<32>(qkv, out, out_lo, lse, B, seq, H, KV, scale, s);
 }
 
 int attention_backward_tc(const bf16* qkv, const bf16* out, const bf16* out_lo, const bf16* d_out, const float* lse, float* delta,
                           bf16* dqkv, const float* cosb, const float* sinb, const float* rope_chunks, int B, int seq, int H,
-                          int KV, float scale, int* d_status, cudaStream_t s) {
-  if (B <= 0 || seq <= 0 || !ensure_attrs()) return 0;
+                          int KV, int hd, float scale, int* d_status, cudaStream_t s) {
+  if (B <= 0 || seq <= 0) return 0;
   // ANE_B200_ATT_LEGACY=1 keeps the mma.sync kernels (A/B measurements).
   static const bool legacy = getenv("ANE_B200_ATT_LEGACY") != nullptr;
-  if (!legacy && attention_tcgen05_supported(HD, seq)) {
+  if (!legacy && attention_tcgen05_supported(hd, seq)) {
     const int n = attention_backward_tcgen05(qkv, out, out_lo, d_out, lse, delta, dqkv, cosb, sinb, rope_chunks, B, seq, H, KV, scale,
                                              d_status, s);
     if (n > 0) return n;
   }
   const long long warps = (long long)B * seq * H;
-  attention_delta_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(d_out, out, out_lo, delta, B, seq, H);
-  dim3 gq((seq + BR - 1) / BR, B * H);
-  attention_bwd_dq_tc_kernel<<<gq, ATT_THREADS, kDqSmem, s>>>(qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV,
-                                                               scale);
-  dim3 gk((seq + BR - 1) / BR, B * KV);
-  attention_bwd_dkv_tc_kernel<<<gk, ATT_THREADS, kDkvSmem, s>>>(qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV,
-                                                                 scale);
+  attention_delta_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(d_out, out, out_lo, delta, B, seq, H, hd);
+  if (hd == 64) backward_hd<64>(qkv, d_out, lse, delta, dqkv, cosb, sinb, B, seq, H, KV, scale, s);
+  else if (hd == 48) backward_hd<48>(qkv, d_out, lse, delta, dqkv, cosb, sinb, B, seq, H, KV, scale, s);
+  else backward_hd<32>(qkv, d_out, lse, delta, dqkv, cosb, sinb, B, seq, H, KV, scale, s);
   return 3;
 }
 

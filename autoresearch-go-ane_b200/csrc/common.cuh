@@ -283,6 +283,18 @@ __device__ __forceinline__ bf16 from_f<bf16>(float v) { return __float2bfloat16_
 // Launches `kernel` with programmatic stream serialization (unless ANE_B200_PDL=0): every kernel
 // launched this way calls pdl_wait() before its first dependent memory access.
 bool pdl_enabled();
+
+// Shared-memory opt-in above 48 KB, once per kernel instance and device (`done`: one bit per device).
+template <class K>
+inline bool smem_opt_in(K kernel, size_t bytes, unsigned long long& done) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done & bit) return true;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+  done |= bit;
+  return true;
+}
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               Args&&... args) {

@@ -284,6 +284,7 @@ class EngineT final : public EngineBase {
   bool att_split_ = false;
   bf16 *qkvh_ = nullptr, *qkvl_ = nullptr, *dqkv_raw_ = nullptr;
   float* att_lse_b_ = nullptr;
+  float* att_stats_ = nullptr;  // row statistics of the SIMT attention backward
   float lr_ = 0, embed_lr_ = 0, scalar_lr_ = 0, lambda_lr_ = 0;
   int ce_rows_ = 0;
   // ---- parameters
@@ -592,6 +593,7 @@ int EngineT<T>::alloc_buffers() {
     A(qkvh_, (size_t)M_ * QKVD_); A(qkvl_, (size_t)M_ * QKVD_); A(dqkv_raw_, (size_t)M_ * QKVD_);
     A(att_lse_b_, (size_t)B_ * H_ * S_);
   }
+  if (!att_tc_) A(att_stats_, (size_t)3 * B_ * H_ * S_);
   A(logits_, (size_t)ce_rows_ * V_);
   if (head_fused_) {
     A(ce_stats_, (size_t)2 * ((V_ + 255) / 256) * M_); A(ce_lse2_, M_); A(ce_coef_, M_);
@@ -898,7 +900,7 @@ int EngineT<T>::forward(const uint16_t* d_tok, int B, int Tl, int pos0) {
         attention_forward_simt<float, T>((const float*)a.qkv, a.att, a.lse, B, Tl, H_, KV_, hd_, att_scale, stream_);
     } else if constexpr (!kIsF32) {
       if (att_tc_)
-        attention_forward_tc((const bf16*)a.qkv, a.att, (bf16*)a.att_lo, a.lse, B, Tl, H_, KV_, att_scale, d_status_, stream_);
+        attention_forward_tc((const bf16*)a.qkv, a.att, (bf16*)a.att_lo, a.lse, B, Tl, H_, KV_, hd_, att_scale, d_status_, stream_);
       else
         attention_forward_simt<T, T>((const T*)a.qkv, a.att, a.lse, B, Tl, H_, KV_, hd_, att_scale, stream_);
     }
@@ -1233,24 +1235,22 @@ int EngineT<T>::backward_layers(int B) {
         }
       }
       if (!done) {
-        cudaMemsetAsync(dqkv_f32, 0, sizeof(float) * (size_t)M * QKVD_, stream_);
-        count_launch();
-        attention_backward_simt<float, T>((const float*)a.qkv, datt_, dqkv_f32, B, S_, H_, KV_, hd_, att_scale_bwd, stream_);
+        count_launch(2);
+        attention_backward_simt<float, T>((const float*)a.qkv, datt_, dqkv_f32, att_stats_, B, S_, H_, KV_, hd_, att_scale_bwd, stream_);
       }
     } else if constexpr (!kIsF32) {
       if (att_tc_) {
         // Tensor-core path: the kernels undo the rotation and emit bf16 operands directly.
         count_launch(attention_backward_tc((const bf16*)a.qkv, a.att, (const bf16*)a.att_lo, datt_, a.lse, att_delta_, dqkv_[pb], rope_cos_, rope_sin_, rope_chunks_, B, S_,
-                                           H_, KV_, att_scale_bwd, d_status_, stream_));
+                                           H_, KV_, hd_, att_scale_bwd, d_status_, stream_));
         dqkv_ready = true;
         if (o_.debug_taps) {
           count_launch();
           to_f32_kernel<T><<<ew_grid((uint64_t)M * QKVD_), 256, 0, stream_>>>(dqkv_[pb], a.t_dqkv, (uint64_t)M * QKVD_);
         }
       } else {
-        cudaMemsetAsync(dqkv_f32, 0, sizeof(float) * (size_t)M * QKVD_, stream_);
-        count_launch();
-        attention_backward_simt<T, T>((const T*)a.qkv, datt_, dqkv_f32, B, S_, H_, KV_, hd_, att_scale_bwd, stream_);
+        count_launch(2);
+        attention_backward_simt<T, T>((const T*)a.qkv, datt_, dqkv_f32, att_stats_, B, S_, H_, KV_, hd_, att_scale_bwd, stream_);
       }
     }
     if (!dqkv_ready) {

@@ -81,9 +81,9 @@ void swiglu_backward(const T* dgate, const T* h13, T* dh13, int M, int Hd, cudaS
 template <typename T, typename TO>
 void attention_forward_simt(const T* qkv, TO* out, float* lse, int B, int seq, int H, int KV, int hd, float scale,
                             cudaStream_t s);
-// dq,dk,dv accumulate into fp32 [M, (H+2KV)*hd] (must be zeroed by the caller).
+// Writes every element of dq,dk,dv (fp32 [M, (H+2KV)*hd]); stats: scratch of 3*B*H*seq floats.
 template <typename T, typename TD>
-void attention_backward_simt(const T* qkv, const TD* d_out, float* dqkv_f32, int B, int seq, int H, int KV, int hd,
+void attention_backward_simt(const T* qkv, const TD* d_out, float* dqkv_f32, float* stats, int B, int seq, int H, int KV, int hd,
                              float scale, cudaStream_t s);
 
 // KV cache (decode): caches are [B, max_seq, KV*hd]; qkv rows are packed q|k|v as above.
@@ -128,12 +128,12 @@ bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int bat
 size_t decode_words_bytes(int D, int Hd, int H, int KV, int hd);  // size of `words`, scratch for exchanges between SMs
 int decode_steps(DecodeArgs a, void* words, int sms, cudaStream_t s);
 
-// Tensor-core causal attention (bf16 operands, head_dim 64 only; see attention_tc.cu).
+// Tensor-core causal attention (bf16 operands; head_dim 32, 48 or 64; see attention_tc.cu).
 bool attention_tc_supported(int hd);
 // `out_lo` (optional, [M, H*64] like `out`) receives bf16(O - bf16(O)): given to the backward as well, it makes
 // delta = rowsum(dO * O) as accurate as an fp32 O would (with bf16 O alone that rounding is the largest
 // error of dQ).
-void attention_forward_tc(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B, int seq, int H, int KV, float scale,
+void attention_forward_tc(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B, int seq, int H, int KV, int hd, float scale,
                           int* d_status, cudaStream_t s);
 int attention_forward_tcgen05(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B, int seq, int H, int KV,
                               float scale, int* d_status, cudaStream_t s);
@@ -145,7 +145,7 @@ int attention_forward_tcgen05(const bf16* qkv, bf16* out, bf16* out_lo, float* l
 // `rope_chunks` (optional): the tables as attention_rope_chunk_tables() lays them out, for the seq-256 backward.
 int attention_backward_tc(const bf16* qkv, const bf16* out, const bf16* out_lo, const bf16* d_out, const float* lse, float* delta,
                           bf16* dqkv, const float* cosb, const float* sinb, const float* rope_chunks, int B, int seq, int H,
-                          int KV, float scale, int* d_status, cudaStream_t s);
+                          int KV, int hd, float scale, int* d_status, cudaStream_t s);
 void attention_rope_chunk_tables(const float* cosb, const float* sinb, float* out, int seq, cudaStream_t s);
 bool attention_tcgen05_supported(int hd, int seq);
 // Backward for q|k|v kept in fp32 and given as bf16 (hi, lo) pairs: scores at split precision, own row

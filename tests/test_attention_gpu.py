@@ -1,0 +1,50 @@
+"""Attention kernels at the edges of their tiles, against the oracle: the fp32 kernels (32 resident rows, streamed tiles of
+64, head sizes padded to 32 / 48 / 64 / 96 / 128) and the mma.sync kernels (head sizes 32, 48 and 64; 64- or 128-row blocks)."""
+import numpy as np
+import pytest
+
+import ane
+from oracle import oracle as O
+from parity_utils import compare_grads, make_pair, oracle_batch_accumulate
+from test_parity_gpu import BWD_TAPS, F32_TOL, FWD_TAPS, batch_tokens, tap_errors
+
+pytestmark = pytest.mark.gpu
+
+
+def _step(dtype, arch, quirks, hd, heads, kv, seq, batch, std):
+    cfg = dict(dim=hd * heads, hidden=64, heads=heads, kv_heads=kv, layers=2, vocab=96, seq=seq)
+    m, e = make_pair(ane, cfg, arch=arch, quirks=quirks, dtype=dtype, batch=batch, std=std,
+                     hyper=dict(accum_steps=1000, grad_clip=1.0))
+    inp, tgt = batch_tokens(cfg, batch, 7, invalid=False)
+    r = e.step_tokens(inp, tgt)
+    assert r.device_status == 0
+    return cfg, m, e, inp, tgt
+
+
+@pytest.mark.parametrize("arch,hd,heads,kv,seq", [
+    (O.ARCH_L, 8, 2, 1, 31), (O.ARCH_L, 32, 2, 2, 33), (O.ARCH_L, 48, 2, 1, 64), (O.ARCH_L, 64, 1, 1, 65), (O.ARCH_L, 72, 2, 1, 97),
+    (O.ARCH_L, 128, 2, 1, 130), (O.ARCH_N, 48, 2, 2, 129), (O.ARCH_N, 104, 1, 1, 63)])
+def test_fp32_tiles(arch, hd, heads, kv, seq):
+    cfg, m, e, inp, tgt = _step(ane.DTYPE_F32, arch, int(arch == O.ARCH_N), hd, heads, kv, seq, 2, 0.1)
+    oracle_batch_accumulate(m, inp, tgt, seq)
+    errs = tap_errors(m, e, cfg, 2, FWD_TAPS + BWD_TAPS)
+    assert max(errs.values()) < F32_TOL, max(errs.items(), key=lambda kv: kv[1])
+    rep = []
+    assert compare_grads(m, e, rep) < F32_TOL, rep
+    e.close()
+
+
+@pytest.mark.parametrize("hd,heads,kv,seq,batch", [(32, 2, 1, 63, 2), (48, 2, 2, 65, 2), (48, 4, 2, 200, 2), (48, 2, 2, 257, 50),
+                                                   (64, 2, 1, 100, 2), (64, 4, 4, 129, 40)])
+def test_bf16_tiles(hd, heads, kv, seq, batch):
+    """q, k, v and d att are rounded to bf16 (2^-9 each) before products that cancel: dq / dk within 2e-2 as the
+    kernels for head size 64 (test_bf16_attention_multi_tile_sequences), everything forward within 1e-2."""
+    cfg, m, e, inp, tgt = _step(ane.DTYPE_BF16, O.ARCH_L, 0, hd, heads, kv, seq, batch, 0.05)
+    m.accumulate(np.ascontiguousarray(inp[-1]), np.ascontiguousarray(tgt[-1]))  # the oracle's taps are its last sequence's
+    for layer in range(cfg["layers"]):
+        for tap, tol in ((O.TAP_Q, 1e-2), (O.TAP_ATT, 1e-2), (O.TAP_DQ, 2e-2), (O.TAP_DK, 2e-2), (O.TAP_DV, 2e-2)):
+            want = m.tap(tap, layer).astype(np.float64)
+            got = e.tap(tap, layer).reshape(batch, want.shape[0], seq)[-1].astype(np.float64)
+            err = np.linalg.norm(got - want) / np.linalg.norm(want)
+            assert err < tol, (layer, tap, err)
+    e.close()
