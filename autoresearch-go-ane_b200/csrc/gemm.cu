@@ -698,7 +698,243 @@ int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t
 }
 
 // ------------------------------------------------------------------------------------------
-// fp32 SIMT GEMM (parity mode).  64x64x16 tiles, 256 threads, 4x4 micro-tiles.
+// fp32 GEMM on the FMA units (the fp32 mode).  Tiles of 16 TM x 16 TN, 256 threads with TM x TN accumulators each,
+// a three-stage cp.async ring of 16-deep slices, two blocks per SM.
+//   * Operands stay in the order they have in memory: K-major rows [m][k] with a pitch of 20 floats, MN-major slices
+//     [k][m].  Either way four k of a thread's TM (TN) rows are TM (TN) conflict-free 16-byte reads, 4 TM TN FMAs for
+//     TM + TN reads, so the FMA pipe is the limit (148 SMs x 128 FMA/clk: 72 TFLOP/s at 1.9 GHz).
+//   * Few tiles (N = 288: 48 of 128 x 96) leave SMs idle, so the contraction is split over the blocks of a cluster;
+//     their partial tiles meet in distributed shared memory, each block finishing a share of the rows: no workspace,
+//     no atomics, always the same order of additions.
+// The 64 x 64 kernel below (4 x 4 accumulators, scalar loads) took 327 us for 2048 x 288 x 288 with N tiles of 64.
+// ------------------------------------------------------------------------------------------
+static constexpr int F32_BK = 16, F32_STAGES = 3, F32_KPITCH = F32_BK + 4;
+
+__device__ __forceinline__ void f32_copy16(uint32_t dst, const float* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+// One 16-deep slice of an operand's R rows: K-major [row][k] or MN-major [k][row].
+template <int R, bool MN>
+__device__ __forceinline__ void f32_load(uint32_t dst, const float* p, int row0, int rows, int k0, int k_end, int ld) {
+  constexpr int CHUNKS = R * F32_BK / 4;
+#pragma unroll
+  for (int i = 0; i < (CHUNKS + 255) / 256; ++i) {
+    const int c = threadIdx.x + i * 256;
+    if (CHUNKS % 256 != 0 && c >= CHUNKS) break;
+    if constexpr (MN) {
+      const int k = c / (R / 4), r = (c - k * (R / 4)) * 4;
+      const bool in = k0 + k < k_end && row0 + r < rows;
+      f32_copy16(dst + (k * R + r) * 4, in ? p + (size_t)(k0 + k) * ld + row0 + r : p, in);
+    } else {
+      const int r = c >> 2, k = (c & 3) * 4;
+      const bool in = k0 + k < k_end && row0 + r < rows;
+      f32_copy16(dst + (r * F32_KPITCH + k) * 4, in ? p + (size_t)(row0 + r) * ld + k0 + k : p, in);
+    }
+  }
+}
+// f[i][q]: element k = 4 kk + q of this thread's row i
+template <int T, bool MN>
+__device__ __forceinline__ void f32_frag(float (&f)[T][4], const float* s, int kk, int t) {
+  if constexpr (MN) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float* row = s + (4 * kk + q) * (16 * T);
+      const float4 a = *reinterpret_cast<const float4*>(row + 4 * t);
+      f[0][q] = a.x; f[1][q] = a.y; f[2][q] = a.z; f[3][q] = a.w;
+      if constexpr (T == 8) {
+        const float4 b = *reinterpret_cast<const float4*>(row + 64 + 4 * t);
+        f[4][q] = b.x; f[5][q] = b.y; f[6][q] = b.z; f[7][q] = b.w;
+      } else {
+        const float2 b = *reinterpret_cast<const float2*>(row + 64 + 2 * t);
+        f[4][q] = b.x; f[5][q] = b.y;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < T; ++i) {
+      const float4 a = *reinterpret_cast<const float4*>(s + (t + 16 * i) * F32_KPITCH + 4 * kk);
+      f[i][0] = a.x; f[i][1] = a.y; f[i][2] = a.z; f[i][3] = a.w;
+    }
+  }
+}
+template <int T, bool MN>
+__device__ __forceinline__ int f32_row(int t, int i) {  // tile row (column) of accumulator index i
+  if (!MN) return t + 16 * i;
+  if (i < 4) return 4 * t + i;
+  return T == 8 ? 64 + 4 * t + (i - 4) : 64 + 2 * t + (i - 4);
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+struct F32Args {
+  const float *A, *B;
+  float* C;
+  int M, N, K, lda, ldb, ldc, out, ldres, split, tiles_m;
+  float alpha;
+  const float *res1, *s1, *res2, *s2;
+};
+
+template <int TM, int TN, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(const F32Args a) {
+  constexpr int BM = 16 * TM, BN = 16 * TN, A_FL = BM * F32_KPITCH, B_FL = BN * F32_KPITCH, CP = BN + 4;
+  extern __shared__ __align__(16) float f32_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);
+  const int tile = blockIdx.x / a.split, rank = blockIdx.x - tile * a.split;
+  const int m0 = (tile % a.tiles_m) * BM, n0 = (tile / a.tiles_m) * BN;
+  const int slices = (a.K + F32_BK - 1) / F32_BK, per = (slices + a.split - 1) / a.split;
+  const int k_begin = rank * per * F32_BK, k_end = min(a.K, k_begin + per * F32_BK);
+  const int n_it = k_end > k_begin ? (k_end - k_begin + F32_BK - 1) / F32_BK : 0;
+  const uint32_t sa = smem_u32(f32_smem), sb = sa + F32_STAGES * A_FL * 4;
+  auto request = [&](int it) {
+    if (it < n_it) {
+      const int st = it % F32_STAGES, k0 = k_begin + it * F32_BK;
+      f32_load<BM, A_MN>(sa + st * A_FL * 4, a.A, m0, a.M, k0, k_end, a.lda);
+      f32_load<BN, B_MN>(sb + st * B_FL * 4, a.B, n0, a.N, k0, k_end, a.ldb);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+  request(0);
+  request(1);
+  for (int it = 0; it < n_it; ++it) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    request(it + 2);  // its slot was read in iteration it - 1
+    const float* As = f32_smem + (it % F32_STAGES) * A_FL;
+    const float* Bs = f32_smem + F32_STAGES * A_FL + (it % F32_STAGES) * B_FL;
+#pragma unroll
+    for (int kk = 0; kk < F32_BK / 4; ++kk) {
+      float fb[TN][4], fa[TM][4];
+      f32_frag<TN, B_MN>(fb, Bs, kk, tx);
+      f32_frag<TM, A_MN>(fa, As, kk, ty);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(fa[i][q], fb[j][q], acc[i][j]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) f32_smem[f32_row<TM, A_MN>(ty, i) * CP + f32_row<TN, B_MN>(tx, j)] = acc[i][j];
+  if (a.split > 1) cluster_sync_all();
+  else __syncthreads();
+  float a1 = 0.f, a2 = 0.f;
+  if (a.res1) a1 = a.s1 ? *a.s1 : 1.f;
+  if (a.res2) a2 = a.s2 ? *a.s2 : 1.f;
+  const int r0 = BM * rank / a.split, r1 = BM * (rank + 1) / a.split;
+  for (int e = threadIdx.x; e < (r1 - r0) * (BN / 4); e += 256) {
+    const int r = r0 + e / (BN / 4), c = (e % (BN / 4)) * 4, m = m0 + r, n = n0 + c;
+    if (m >= a.M || n >= a.N) continue;
+    const uint32_t at = sa + (uint32_t)(r * CP + c) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (a.split > 1) {
+      for (int p = 0; p < a.split; ++p) {
+        const float4 t = ld_cluster4(map_to_cta(at, p));
+        v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+      }
+    } else {
+      v = *reinterpret_cast<const float4*>(f32_smem + r * CP + c);
+    }
+    v.x *= a.alpha; v.y *= a.alpha; v.z *= a.alpha; v.w *= a.alpha;
+    float4* cp = reinterpret_cast<float4*>(a.C + (size_t)m * a.ldc + n);
+    if (a.out == GEMM_OUT_ACCUM) {
+      const float4 t = *cp;
+      v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+    } else {
+      if (a.res1) {
+        const float4 t = *reinterpret_cast<const float4*>(a.res1 + (size_t)m * a.ldres + n);
+        v.x += a1 * t.x; v.y += a1 * t.y; v.z += a1 * t.z; v.w += a1 * t.w;
+      }
+      if (a.res2) {
+        const float4 t = *reinterpret_cast<const float4*>(a.res2 + (size_t)m * a.ldres + n);
+        v.x += a2 * t.x; v.y += a2 * t.y; v.z += a2 * t.z; v.w += a2 * t.w;
+      }
+    }
+    *cp = v;
+  }
+  if (a.split > 1) cluster_sync_all();  // the peers have read this block's partial sums
+}
+
+template <int TM, int TN, bool A_MN, bool B_MN>
+static cudaError_t launch_f32_tile(const F32Args& a, int tiles, cudaStream_t stream) {
+  auto kern = gemm_f32_tile_kernel<TM, TN, A_MN, B_MN>;
+  constexpr size_t ring = sizeof(float) * F32_STAGES * (16 * TM + 16 * TN) * F32_KPITCH, out = sizeof(float) * 16 * TM * (16 * TN + 4);
+  constexpr size_t bytes = ring > out ? ring : out;
+  static unsigned long long done = 0;
+  if (!smem_opt_in(kern, bytes, done)) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * a.split));
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)a.split;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = a.split > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, a);
+}
+template <int TM, int TN>
+static cudaError_t launch_f32_layout(const F32Args& a, bool a_mn, bool b_mn, int tiles, cudaStream_t stream) {
+  if (!a_mn && !b_mn) return launch_f32_tile<TM, TN, false, false>(a, tiles, stream);
+  if (!a_mn) return launch_f32_tile<TM, TN, false, true>(a, tiles, stream);
+  if (b_mn) return launch_f32_tile<TM, TN, true, true>(a, tiles, stream);
+  return launch_f32_tile<TM, TN, true, false>(a, tiles, stream);
+}
+
+// Tile and split: the fewest slice-times of the busiest SM (two blocks share one), counting padding and a start and
+// end of about four slices per block; 96-wide tiles read more operands per FMA and must win by their padding.
+static cudaError_t launch_f32(const GemmDesc& d, cudaStream_t stream) {
+  const int slots = 2 * gemm_num_sms(), slices = (d.K + F32_BK - 1) / F32_BK;
+  double best = 0;
+  int bm = 8, bn = 8, split = 1;
+  for (int tm : {8, 6})
+    for (int tn : {8, 6})
+      for (int sp : {1, 2, 4, 8}) {
+        if (sp > 1 && sp * 2 > slices) continue;
+        const long tiles = (long)((d.M + 16 * tm - 1) / (16 * tm)) * ((d.N + 16 * tn - 1) / (16 * tn));
+        const long waves = (tiles * sp + slots - 1) / slots;
+        const double pen = tm + tn == 16 ? 1.0 : tm + tn == 14 ? 1.05 : 1.1;
+        const double cost = (double)waves * (((slices + sp - 1) / sp) + 4 + (sp > 1 ? 2 : 0)) * tm * tn * pen;
+        if (best == 0 || cost < best) {
+          best = cost;
+          bm = tm;
+          bn = tn;
+          split = sp;
+        }
+      }
+  F32Args a{reinterpret_cast<const float*>(d.A), reinterpret_cast<const float*>(d.B), reinterpret_cast<float*>(d.C), d.M, d.N, d.K, d.lda, d.ldb,
+            d.ldc, d.out, d.ldres, split, (d.M + 16 * bm - 1) / (16 * bm), d.alpha, d.res1, d.s1, d.res2, d.s2};
+  const int tiles = a.tiles_m * ((d.N + 16 * bn - 1) / (16 * bn));
+  if (bm == 8 && bn == 8) return launch_f32_layout<8, 8>(a, d.a_mn, d.b_mn, tiles, stream);
+  if (bm == 8) return launch_f32_layout<8, 6>(a, d.a_mn, d.b_mn, tiles, stream);
+  if (bn == 8) return launch_f32_layout<6, 8>(a, d.a_mn, d.b_mn, tiles, stream);
+  return launch_f32_layout<6, 6>(a, d.a_mn, d.b_mn, tiles, stream);
+}
+// What the 16-byte copies of the tiled kernel need.
+static bool f32_aligned(const GemmDesc& d) {
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  return al(d.A) && al(d.B) && al(d.C) && al(d.res1) && al(d.res2) && d.lda % 4 == 0 && d.ldb % 4 == 0 && d.ldc % 4 == 0 && d.N % 4 == 0 &&
+         (!(d.res1 || d.res2) || d.ldres % 4 == 0) && (d.a_mn ? d.M % 4 == 0 : d.K % 4 == 0) && (d.b_mn || d.K % 4 == 0);
+}
+
+// ------------------------------------------------------------------------------------------
+// The same for operands that are not 16-byte aligned: 64x64x16 tiles, 256 threads, 4x4 micro-tiles.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N,
@@ -773,6 +1009,14 @@ int gemm_f32(const GemmDesc& d, cudaStream_t stream) {
   if (d.out == GEMM_OUT_BF16) {
     g_gemm_err = "fp32 GEMM cannot write bf16";
     return -2;
+  }
+  if (f32_aligned(d)) {
+    const cudaError_t e = launch_f32(d, stream);
+    if (e != cudaSuccess) {
+      g_gemm_err = std::string("gemm_f32 launch: ") + cudaGetErrorString(e);
+      return -4;
+    }
+    return 0;
   }
   dim3 grid((d.N + 63) / 64, (d.M + 63) / 64);
   gemm_f32_kernel<<<grid, 256, 0, stream>>>(

@@ -150,6 +150,22 @@ def test_split_precision_gemm_carries_fp32_operands_through_the_tensor_cores():
     assert rel_l2(got, C0 + At.astype(np.float64).T @ B.astype(np.float64)) < 2e-5
 
 
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 1), (1, 0)])
+@pytest.mark.parametrize("m,n,k", [(128, 96, 16), (4, 4, 4), (100, 92, 60), (288, 96, 2048), (97 * 4, 132, 1000), (2048, 288, 288), (20000, 128, 36)])
+def test_fp32_tiles_and_cluster_splits(a_mn, b_mn, m, n, k):
+    """96- and 128-wide tiles, one block and clusters of 2, 4 and 8 along the contraction, ragged edges, a residual and
+    accumulation.  Any order of k fp32 additions of N(0, 1) products is within sqrt(k) 2^-23 < 1e-5 (rel-L2)."""
+    rng = np.random.default_rng(m + n + k)
+    A = rng.standard_normal((m, k)).astype(np.float32)
+    B = rng.standard_normal((k, n)).astype(np.float32)
+    C = rng.standard_normal((m, n)).astype(np.float32)
+    a = np.ascontiguousarray(A.T) if a_mn else A
+    b = B if b_mn else np.ascontiguousarray(B.T)
+    want = A.astype(np.float64) @ B.astype(np.float64) + C
+    assert rel_l2(_gemm(ane.DTYPE_F32, a, b, np.zeros_like(C), m, n, k, a_mn, b_mn, 1, res=C), want) < 1e-5
+    assert rel_l2(_gemm(ane.DTYPE_F32, a, b, C, m, n, k, a_mn, b_mn, 2), want) < 1e-5
+
+
 @pytest.mark.parametrize("dtype", [ane.DTYPE_BF16, ane.DTYPE_F32, ane.DTYPE_BF16X3])
 @pytest.mark.parametrize("oc,ic,seq", [(96, 64, 40), (256, 136, 300), (768, 256, 128)])
 def test_linear_forward_dx_dw_match_oracle(dtype, oc, ic, seq):
