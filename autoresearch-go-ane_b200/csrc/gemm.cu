@@ -6,6 +6,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <string>
@@ -166,6 +167,15 @@ static int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
     }
     return 0;
   }
+  if constexpr (GemmCfg<BN, MT>::SPLIT) {  // split_k = -(CTAs per tile)
+    cudaError_t e = launch_pdl_cluster(kern, dim3((unsigned)(base_tiles * -split_k)), dim3(threads), smem_bytes, stream, (unsigned)-split_k, ta, tb,
+                                       tc, td, epi, d.M, d.N, d.K, split_k, d_status, (const GemmGroup*)nullptr);
+    if (e != cudaSuccess) {
+      g_gemm_err = std::string("gemm_tc split launch: ") + cudaGetErrorString(e);
+      return -4;
+    }
+    return 0;
+  }
   int grid;
   if (split_k > 0) {
     const int tiles = base_tiles * split_k;
@@ -191,11 +201,12 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
                         int* d_status, cudaStream_t stream) {
   EpiParams epi{d.alpha, d.res1, d.s1, d.res2, d.s2, d.ldres, reinterpret_cast<bf16*>(d.aux), d.ldaux,
                 d.rope_cos, d.rope_sin, d.rope_seq, d.rope_pos0, d.rope_cols, d.tgt, d.tgt_out, d.tgt_row0,
-                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0};
+                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, d.seg_kb};
+  const int whole = GemmCfg<BN, MT>::SPLIT ? split_k : 1;  // schedule of the epilogues that need whole tiles
   CUtensorMap tc;
   if (d.out == GEMM_OUT_BF16) {
     if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false)) return -2;
-    return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16>(ta, tb, tc, tc, epi, d, 1, d_status, stream);
+    return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
   }
   if (d.out == GEMM_OUT_BF16_TGT) {
     if constexpr (!A_MN && !B_MN) {
@@ -204,7 +215,7 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
         return -2;
       }
       if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false)) return -2;
-      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16_TGT>(ta, tb, tc, tc, epi, d, 1, d_status, stream);
+      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16_TGT>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
     } else {
       g_gemm_err = "the target-logit epilogue takes K-major operands only";
       return -2;
@@ -213,7 +224,7 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   if (d.out == GEMM_OUT_BF16_ROPE) {
     if constexpr (!A_MN && !B_MN) {
       if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false)) return -2;
-      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16_ROPE>(ta, tb, tc, tc, epi, d, 1, d_status, stream);
+      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16_ROPE>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
     } else {
       g_gemm_err = "the rotary epilogue takes K-major operands only";
       return -2;
@@ -225,7 +236,7 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
       if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false) ||
           !make_tmap(&td, d.aux, d.N / 2, d.M, d.ldaux, 64, 32, false))
         return -2;
-      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16_SWIGLU>(ta, tb, tc, td, epi, d, 1, d_status, stream);
+      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16_SWIGLU>(ta, tb, tc, td, epi, d, whole, d_status, stream);
     } else {
       g_gemm_err = "the SwiGLU epilogue takes K-major operands only";
       return -2;
@@ -236,7 +247,7 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
       CUtensorMap td;  // gate [M, N], same pieces as C
       if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false) || !make_tmap(&td, d.aux, d.N, d.M, d.ldaux, 64, 32, false))
         return -2;
-      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16_RELU2>(ta, tb, tc, td, epi, d, 1, d_status, stream);
+      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16_RELU2>(ta, tb, tc, td, epi, d, whole, d_status, stream);
     } else {
       g_gemm_err = "the ReLU^2 epilogue takes K-major operands only";
       return -2;
@@ -245,32 +256,32 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   if (d.out == GEMM_OUT_CE_STATS || d.out == GEMM_OUT_CE_GRAD) {
     if constexpr (!A_MN && !B_MN && BN == 256 && (MT == 1 || MT == GEMM_MT_PAIR)) {
       if (d.out == GEMM_OUT_CE_STATS)  // no output tensor: the A map stands in for the unused descriptors
-        return launch_tc<BN, MT, A_MN, B_MN, EPI_CE_STATS>(ta, tb, ta, ta, epi, d, 1, d_status, stream);
+        return launch_tc<BN, MT, A_MN, B_MN, EPI_CE_STATS>(ta, tb, ta, ta, epi, d, whole, d_status, stream);
       if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false)) return -2;
-      return launch_tc<BN, MT, A_MN, B_MN, EPI_CE_GRAD>(ta, tb, tc, tc, epi, d, 1, d_status, stream);
+      return launch_tc<BN, MT, A_MN, B_MN, EPI_CE_GRAD>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
     } else {
       g_gemm_err = "the classifier-head epilogues take K-major operands on 256-column tiles";
       return -2;
     }
   }
   if (d.out == GEMM_OUT_DSWIGLU) {
-    if constexpr (!A_MN && B_MN && BN == 256 && (MT == 1 || MT == GEMM_MT_PAIR)) {
+    if constexpr (!A_MN && B_MN && ((BN == 256 && (MT == 1 || MT == GEMM_MT_PAIR)) || MT == GEMM_MT_SPLIT)) {
       CUtensorMap td;  // h13 in, d h13 out: [M, 2N] bf16, pieces of 32 rows x 64 columns
       if (!make_tmap(&tc, d.C, 2 * (uint64_t)d.N, d.M, d.ldc, 64, 32, false) ||
           !make_tmap(&td, d.aux, 2 * (uint64_t)d.N, d.M, d.ldaux, 64, 32, false))
         return -2;
-      return launch_tc<BN, MT, A_MN, B_MN, EPI_DSWIGLU>(ta, tb, tc, td, epi, d, 1, d_status, stream);
+      return launch_tc<BN, MT, A_MN, B_MN, EPI_DSWIGLU>(ta, tb, tc, td, epi, d, whole, d_status, stream);
     } else {
       g_gemm_err = "the SwiGLU-backward epilogue takes the dX form (A K-major, B MN-major) on 256-column tiles";
       return -2;
     }
   }
   if (d.out == GEMM_OUT_DRELU2) {
-    if constexpr (!A_MN && B_MN && BN == 256 && (MT == 1 || MT == GEMM_MT_PAIR)) {
+    if constexpr (!A_MN && B_MN && ((BN == 256 && (MT == 1 || MT == GEMM_MT_PAIR)) || MT == GEMM_MT_SPLIT)) {
       CUtensorMap td;  // h in, d h out: [M, N] bf16, pieces of 32 rows x 64 columns
       if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false) || !make_tmap(&td, d.aux, d.N, d.M, d.ldaux, 64, 32, false))
         return -2;
-      return launch_tc<BN, MT, A_MN, B_MN, EPI_DRELU2>(ta, tb, tc, td, epi, d, 1, d_status, stream);
+      return launch_tc<BN, MT, A_MN, B_MN, EPI_DRELU2>(ta, tb, tc, td, epi, d, whole, d_status, stream);
     } else {
       g_gemm_err = "the ReLU^2-backward epilogue takes the dX form (A K-major, B MN-major) on 256-column tiles";
       return -2;
@@ -284,13 +295,13 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
       if (d.res1 != nullptr && d.res2 == nullptr && !no_tma_res) {
         CUtensorMap td;
         if (!make_tmap(&td, d.res1, d.N, d.M, d.ldres, 32, 32, true)) return -2;
-        return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_F32_TMARES>(ta, tb, tc, td, epi, d, 1, d_status, stream);
+        return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_F32_TMARES>(ta, tb, tc, td, epi, d, whole, d_status, stream);
       }
     }
-    return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_F32>(ta, tb, tc, tc, epi, d, 1, d_status, stream);
+    return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_F32>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
   }
-  if constexpr (GemmCfg<BN, MT>::PAIR) {
-    g_gemm_err = "CTA-pair tiles are built for the non-accumulating epilogues";
+  if constexpr (GemmCfg<BN, MT>::PAIR || GemmCfg<BN, MT>::SPLIT) {
+    g_gemm_err = "cluster tiles are built for the non-accumulating epilogues";
     return -2;
   } else {
     return launch_tc<BN, MT, A_MN, B_MN, EPI_REDUCE_F32>(ta, tb, tc, tc, epi, d, split_k, d_status, stream);
@@ -301,17 +312,18 @@ template <int BN, int MT>
 static int dispatch_layout(const GemmDesc& d, int split_k, int* d_status, cudaStream_t stream) {
   CUtensorMap ta, tb;
   bool ok;
-  if (!d.a_mn) ok = make_tmap(&ta, d.A, d.K, d.M, d.lda, GEMM_BK, GEMM_BM);
-  else         ok = make_tmap(&ta, d.A, d.M, d.K, d.lda, 64, GEMM_BK);
+  const int k_extent = d.seg_kb > 0 ? 2 * d.seg_kb * GEMM_BK : d.K;  // (hi | lo) operands: both halves
+  if (!d.a_mn) ok = make_tmap(&ta, d.A, k_extent, d.M, d.lda, GEMM_BK, GEMM_BM);
+  else         ok = make_tmap(&ta, d.A, d.M, k_extent, d.lda, 64, GEMM_BK);
   if (!ok) return -2;
   // K-major B: one box per CTA and stage (a CTA of a pair loads half of the tile's rows)
-  if (!d.b_mn) ok = make_tmap(&tb, d.B, d.K, d.N, d.ldb, GEMM_BK, GemmCfg<BN, MT>::PAIR ? BN / 2 : BN);
-  else         ok = make_tmap(&tb, d.B, d.N, d.K, d.ldb, 64, GEMM_BK);
+  if (!d.b_mn) ok = make_tmap(&tb, d.B, k_extent, d.N, d.ldb, GEMM_BK, GemmCfg<BN, MT>::PAIR ? BN / 2 : BN);
+  else         ok = make_tmap(&tb, d.B, d.N, k_extent, d.ldb, 64, GEMM_BK);
   if (!ok) return -2;
-  if constexpr (GemmCfg<BN, MT>::PAIR) {  // forward and dX forms only (A K-major)
+  if constexpr (GemmCfg<BN, MT>::PAIR || GemmCfg<BN, MT>::SPLIT) {  // forward and dX forms only (A K-major)
     if (!d.a_mn && !d.b_mn) return dispatch_epi<BN, MT, false, false>(ta, tb, d, split_k, d_status, stream);
     if (!d.a_mn && d.b_mn) return dispatch_epi<BN, MT, false, true>(ta, tb, d, split_k, d_status, stream);
-    g_gemm_err = "CTA-pair tiles: unsupported operand layout";
+    g_gemm_err = "cluster tiles: unsupported operand layout";
     return -2;
   } else {
   if (!d.a_mn && !d.b_mn) return dispatch_epi<BN, MT, false, false>(ta, tb, d, split_k, d_status, stream);
@@ -435,6 +447,45 @@ static GemmPlan plan_gemm(const GemmDesc& d, int sms) {
   return p;
 }
 
+// Clusters of `size` CTAs of the split kernels that the device holds at once (one CTA per SM).
+static int resident_clusters(int size) {
+  static int known[4] = {0, 0, 0, 0};
+  const int at = size == 8 ? 3 : size == 4 ? 2 : 1;
+  if (known[at] == 0) {
+    using Cfg = GemmCfg<128, GEMM_MT_SPLIT>;
+    auto kern = gemm_tc_kernel<128, GEMM_MT_SPLIT, false, false, EPI_STORE_F32>;
+    const int bytes = (int)Cfg::smem_bytes(false);
+    int n = 0;
+    cudaLaunchConfig_t q = {};
+    q.gridDim = dim3((unsigned)(size * 148));
+    q.blockDim = dim3(GEMM_THREADS);
+    q.dynamicSmemBytes = bytes;
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeClusterDimension;
+    a[0].val.clusterDim.x = (unsigned)size;
+    a[0].val.clusterDim.y = 1;
+    a[0].val.clusterDim.z = 1;
+    q.attrs = a;
+    q.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &q) != cudaSuccess || n <= 0)
+      n = gemm_num_sms() / size;
+    cudaGetLastError();
+    known[at] = std::min(n, gemm_num_sms() / size);
+  }
+  return known[at];
+}
+// How many CTAs share a 128 x 128 tile (0: none): as many as stay resident together with at least two k-blocks each.
+static int cluster_split(const GemmDesc& d) {
+  static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_CLUSTER_SPLIT"); return e && e[0] == '0'; }();  // A/B measurements
+  if (off || d.a_mn || d.out == GEMM_OUT_ACCUM || d.out == GEMM_OUT_CE_STATS || d.out == GEMM_OUT_CE_GRAD || d.out == GEMM_OUT_BF16_TGT) return 0;
+  const long tiles = (long)((d.M + 127) / 128) * ((d.N + 127) / 128);
+  const int kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;
+  for (int s : {8, 4, 2})
+    if (kblocks >= 2 * s && tiles <= resident_clusters(s)) return s;
+  return 0;
+}
+
 int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return 0;
   if (d.out == GEMM_OUT_F32 && (d.res1 || d.res2) && (d.ldres % 4 != 0 ||
@@ -464,6 +515,7 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
                    "output 16-byte aligned with pitches % 8 == 0";
       return -2;
     }
+    if (const int s = cluster_split(d)) return dispatch_layout<128, GEMM_MT_SPLIT>(d, -s, d_status, stream);
     // 256-column tiles: CTA pairs when they fill their waves (the step's shape), else one CTA per tile
     const int pairs = gemm_num_sms() / 2;
     const long tiles = (long)((d.M + 255) / 256) * ((d.N + 255) / 256);
@@ -488,6 +540,7 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
     if (!no_pair && d.M >= 256 && eff >= 0.8) return dispatch_layout<256, GEMM_MT_PAIR>(d, 1, d_status, stream);
     return dispatch_layout<256, 1>(d, 1, d_status, stream);
   }
+  if (const int s = cluster_split(d)) return dispatch_layout<128, GEMM_MT_SPLIT>(d, -s, d_status, stream);
   GemmPlan p = plan_gemm(d, gemm_num_sms());
   if (d.out == GEMM_OUT_BF16_SWIGLU && p.bn == 192) p.bn = 256;  // gate rows pair up two 64-column pieces
   // CTA-pair tiles (256 x 256 per two SMs, half of the B tile per CTA): measured faster than both single-CTA
@@ -617,84 +670,112 @@ size_t gemm_group_slot_bytes() { return sizeof(GemmGroup); }
 // ------------------------------------------------------------------------------------------
 // Split-precision GEMM: fp32 operands as bf16 (hi, lo) pairs, three tensor-core products.
 // ------------------------------------------------------------------------------------------
-// src [rows, cols] fp32 with row pitch ld  ->  hi, lo [rows, ldo] bf16 (ldo >= cols, a multiple of 8)
-__global__ void split_rows_kernel(const float* __restrict__ src, bf16* __restrict__ hi, bf16* __restrict__ lo, int rows,
-                                  int cols, long long ld, int ldo) {
-  const long long total = (long long)rows * cols;
+// Both operands of a product in one launch (blockIdx.y), four values per thread and step.  Operand [rows, cols] fp32
+// with row pitch ld; its halves lie behind one another along the contraction: for a K-major operand (k = cols)
+// [rows][hi (kp) | lo (kp)], for an MN-major one (k = rows) [hi (kp rows) | lo (kp rows)][cols rounded up to 8].  kp =
+// k rounded up to a whole k-block; what lies past k is zero.
+struct SplitOperand {
+  const float* src;
+  bf16* dst;
+  long long ld;
+  int rows, cols, kp, pitch, k_major, vec;  // vec: float4 reads are aligned
+};
+__global__ void split_operands_kernel(const SplitOperand a, const SplitOperand b) {
+  const SplitOperand& o = blockIdx.y == 0 ? a : b;
+  const int out_rows = o.k_major ? o.rows : o.kp, out_cols = o.k_major ? o.kp : o.pitch, per = out_cols / 4;
+  const size_t lo = o.k_major ? (size_t)o.kp : (size_t)o.kp * o.pitch;
+  const long long total = (long long)out_rows * per;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(i / cols), c = (int)(i - (long long)r * cols);
-    const float x = src[(size_t)r * ld + c];
-    const bf16 h = __float2bfloat16_rn(x);
-    hi[(size_t)r * ldo + c] = h;
-    lo[(size_t)r * ldo + c] = __float2bfloat16_rn(x - __bfloat162float(h));
+    const int r = (int)(i / per), c = (int)(i - (long long)r * per) * 4;
+    float x[4] = {0.f, 0.f, 0.f, 0.f};
+    if (r < o.rows) {
+      const float* p = o.src + (size_t)r * o.ld + c;
+      if (o.vec && c + 4 <= o.cols) {
+        const float4 v = *reinterpret_cast<const float4*>(p);
+        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (c + e < o.cols) x[e] = p[e];
+      }
+    }
+    uint2 h, l;
+    uint32_t* hp = &h.x;
+    uint32_t* lp = &l.x;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const __nv_bfloat162 v = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
+      const __nv_bfloat162 w = __floats2bfloat162_rn(x[2 * e] - __bfloat162float(v.x), x[2 * e + 1] - __bfloat162float(v.y));
+      hp[e] = *reinterpret_cast<const uint32_t*>(&v);
+      lp[e] = *reinterpret_cast<const uint32_t*>(&w);
+    }
+    bf16* q = o.dst + (size_t)r * o.pitch + c;
+    *reinterpret_cast<uint2*>(q) = h;
+    *reinterpret_cast<uint2*>(q + lo) = l;
   }
 }
 
 void SplitScratch::release() {
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < 2; ++i) {
     if (buf[i]) cudaFree(buf[i]);
     buf[i] = nullptr;
     cap[i] = 0;
   }
 }
 
+// The three products run as one: its contraction is three passes of kp over (hi, hi), (hi, lo) and (lo, hi), so the
+// accumulators stay in tensor memory between them.  (Three launches, the second and third adding to C in memory, and
+// two scalar conversion launches before them took 9.8 us each for 512 token rows.)
 int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t stream) {
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return 0;
   if (d.out != GEMM_OUT_F32 && d.out != GEMM_OUT_ACCUM) {
     g_gemm_err = "split-precision GEMM writes fp32 (store or accumulate) only";
     return -2;
   }
-  // stored shapes of the operands
-  const int a_rows = d.a_mn ? d.K : d.M, a_cols = d.a_mn ? d.M : d.K;
-  const int b_rows = d.b_mn ? d.K : d.N, b_cols = d.b_mn ? d.N : d.K;
-  const int lda = (a_cols + 7) / 8 * 8, ldb = (b_cols + 7) / 8 * 8;
-  const size_t need[4] = {(size_t)a_rows * lda * 2, (size_t)a_rows * lda * 2, (size_t)b_rows * ldb * 2, (size_t)b_rows * ldb * 2};
-  for (int i = 0; i < 4; ++i) {
-    if (sc->cap[i] >= need[i]) continue;
-    // the previous, smaller buffer may still be read by GEMMs in flight on this stream
-    if (sc->buf[i]) {
-      cudaStreamSynchronize(stream);
-      cudaFree(sc->buf[i]);
-      sc->buf[i] = nullptr;
-      sc->cap[i] = 0;
+  const int kp = (d.K + GEMM_BK - 1) / GEMM_BK * GEMM_BK;
+  SplitOperand o[2];
+  for (int i = 0; i < 2; ++i) {
+    const bool mn = i == 0 ? d.a_mn : d.b_mn;
+    const int outer = i == 0 ? d.M : d.N;
+    o[i].src = reinterpret_cast<const float*>(i == 0 ? d.A : d.B);
+    o[i].ld = i == 0 ? d.lda : d.ldb;
+    o[i].rows = mn ? d.K : outer;
+    o[i].cols = mn ? outer : d.K;
+    o[i].kp = kp;
+    o[i].k_major = mn ? 0 : 1;
+    o[i].pitch = mn ? (outer + 7) / 8 * 8 : 2 * kp;
+    o[i].vec = o[i].ld % 4 == 0 && (reinterpret_cast<uintptr_t>(o[i].src) & 15) == 0;
+    const size_t need = sizeof(bf16) * (size_t)(mn ? 2 * kp : outer) * o[i].pitch;
+    if (sc->cap[i] < need) {
+      // the previous, smaller buffer may still be read by GEMMs in flight on this stream
+      if (sc->buf[i]) {
+        cudaStreamSynchronize(stream);
+        cudaFree(sc->buf[i]);
+        sc->buf[i] = nullptr;
+        sc->cap[i] = 0;
+      }
+      const size_t bytes = need + need / 4 + 256;
+      if (cudaMalloc(&sc->buf[i], bytes) != cudaSuccess) {
+        g_gemm_err = "split-precision GEMM: out of memory for the operand halves";
+        return -3;
+      }
+      sc->cap[i] = bytes;
     }
-    const size_t bytes = need[i] + need[i] / 4 + 256;
-    if (cudaMalloc(&sc->buf[i], bytes) != cudaSuccess) {
-      g_gemm_err = "split-precision GEMM: out of memory for the operand halves";
-      return -3;
-    }
-    sc->cap[i] = bytes;
+    o[i].dst = reinterpret_cast<bf16*>(sc->buf[i]);
   }
-  bf16* ah = reinterpret_cast<bf16*>(sc->buf[0]);
-  bf16* al = reinterpret_cast<bf16*>(sc->buf[1]);
-  bf16* bh = reinterpret_cast<bf16*>(sc->buf[2]);
-  bf16* bl = reinterpret_cast<bf16*>(sc->buf[3]);
-  auto grid = [](long long n) {
-    long long g = (n + 255) / 256;
-    return (unsigned)(g > 148LL * 16 ? 148LL * 16 : (g < 1 ? 1 : g));
-  };
-  split_rows_kernel<<<grid((long long)a_rows * a_cols), 256, 0, stream>>>(reinterpret_cast<const float*>(d.A), ah, al, a_rows,
-                                                                          a_cols, d.lda, lda);
-  split_rows_kernel<<<grid((long long)b_rows * b_cols), 256, 0, stream>>>(reinterpret_cast<const float*>(d.B), bh, bl, b_rows,
-                                                                          b_cols, d.ldb, ldb);
+  const long long most = std::max((long long)(o[0].k_major ? o[0].rows : kp) * (o[0].k_major ? kp : o[0].pitch),
+                                  (long long)(o[1].k_major ? o[1].rows : kp) * (o[1].k_major ? kp : o[1].pitch));
+  const unsigned blocks = (unsigned)std::min<long long>(148 * 8, (most / 4 + 255) / 256);
+  split_operands_kernel<<<dim3(blocks, 2), 256, 0, stream>>>(o[0], o[1]);
   if (cudaGetLastError() != cudaSuccess) {
     g_gemm_err = "split-precision GEMM: operand split launch failed";
     return -4;
   }
-  GemmDesc g = d;  // the large term keeps the output kind (store with residuals, or accumulate)
-  g.A = ah; g.B = bh; g.lda = lda; g.ldb = ldb;
-  int rc = gemm_bf16(g, d_status, stream);
-  if (rc != 0) return rc;
-  GemmDesc c = g;  // the two cross terms accumulate on top
-  c.out = GEMM_OUT_ACCUM;
-  c.res1 = c.res2 = nullptr;
-  c.s1 = c.s2 = nullptr;
-  c.split_k = 0;
-  c.B = bl;
-  if ((rc = gemm_bf16(c, d_status, stream)) != 0) return rc;
-  c.A = al;
-  c.B = bh;
-  return gemm_bf16(c, d_status, stream);
+  GemmDesc g = d;
+  g.A = o[0].dst; g.B = o[1].dst; g.lda = o[0].pitch; g.ldb = o[1].pitch;
+  g.K = 3 * kp;
+  g.seg_kb = kp / GEMM_BK;
+  return gemm_bf16(g, d_status, stream);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -80,6 +80,7 @@ struct GemmDesc {
   int ce_rows = 0, ce_col0 = 0;
   bool ce_softcap = false;
   int split_k = 0;  // 0 => choose
+  int seg_kb = 0;   // > 0: operands hold bf16 (hi | lo) halves of seg_kb k-blocks of 64, K = 3 * 64 * seg_kb (see gemm_bf16x3)
 };
 
 // bf16 operands, tcgen05 tensor cores.  Returns 0 or a negative error code.
@@ -88,13 +89,13 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream);
 int gemm_f32(const GemmDesc& d, cudaStream_t stream);
 
 // fp32 operands at split precision on the tensor cores: A and B are each cut into a bf16 (hi, lo) pair
-// (hi = bf16(x), lo = bf16(x - hi): together ~16 significand bits) and the product is formed as the three
-// bf16 GEMMs Ah*Bh + Ah*Bl + Al*Bh accumulated in fp32 (the dropped Al*Bl term is ~2^-18 relative).  Output
-// kinds GEMM_OUT_F32 (with residuals) and GEMM_OUT_ACCUM.  The scratch holds the four operand halves and
-// grows on demand; one scratch serves one stream at a time.
+// (hi = bf16(x), lo = bf16(x - hi): together ~16 significand bits) and the product is formed as Ah*Bh + Ah*Bl + Al*Bh
+// with fp32 accumulation, one GEMM over a contraction of three passes (the dropped Al*Bl term is ~2^-18 relative).
+// Output kinds GEMM_OUT_F32 (with residuals) and GEMM_OUT_ACCUM.  The scratch holds both operands' halves and grows on
+// demand; one scratch serves one stream at a time.
 struct SplitScratch {
-  void* buf[4] = {nullptr, nullptr, nullptr, nullptr};  // A hi, A lo, B hi, B lo
-  size_t cap[4] = {0, 0, 0, 0};                         // bytes
+  void* buf[2] = {nullptr, nullptr};  // A, B
+  size_t cap[2] = {0, 0};             // bytes
   void release();
 };
 int gemm_bf16x3(const GemmDesc& d, SplitScratch* scratch, int* d_status, cudaStream_t stream);

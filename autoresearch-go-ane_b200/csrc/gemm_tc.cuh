@@ -43,12 +43,19 @@ static constexpr int GEMM_THREADS = 192;  // TMA warp, MMA warp, four epilogue w
 // accumulator set): the least fill per FLOP, for long K with few columns.
 static constexpr int GEMM_MT_PAIR = 4;
 static constexpr int GEMM_MT_PAIR2 = 5;
+// MT = GEMM_MT_SPLIT: a cluster of 2, 4 or 8 CTAs shares one 128 x BN tile along the contraction.  With few tiles (256
+// token rows: 12 tiles of 128 x 128 for N = 768) the k-blocks of a tile are a serial chain on one SM, 64 of them for
+// K = 4096; split, each CTA runs its share, parks its fp32 accumulators in its own shared memory (the pipeline stages
+// are free by then), and after one cluster barrier every CTA finishes its share of the tile's pieces, summing the
+// partial sums over distributed shared memory in rank order.  No workspace, no atomics; every epilogue kind works.
+static constexpr int GEMM_MT_SPLIT = 6;
 static constexpr uint32_t GEMM_TMARES_BYTES = 4 * 2 * 4096;
 static constexpr uint32_t GEMM_SMEM_LIMIT = 232448u;
 template <int BN, int MT>
 struct GemmCfg {
-  static constexpr bool PAIR = MT >= GEMM_MT_PAIR;
-  static constexpr int SUBS = MT == GEMM_MT_PAIR ? 1 : (MT == GEMM_MT_PAIR2 ? 2 : MT);  // 128-row sub-tiles per CTA
+  static constexpr bool PAIR = MT == GEMM_MT_PAIR || MT == GEMM_MT_PAIR2;
+  static constexpr bool SPLIT = MT == GEMM_MT_SPLIT;
+  static constexpr int SUBS = (MT == GEMM_MT_PAIR || SPLIT) ? 1 : (MT == GEMM_MT_PAIR2 ? 2 : MT);  // 128-row sub-tiles per CTA
   static constexpr int BM_TILE = (PAIR ? 2 : 1) * SUBS * GEMM_BM;       // rows of a scheduled tile
   static constexpr uint32_t A_BYTES = SUBS * GEMM_BM * GEMM_BK * 2;     // per CTA and stage
   // a CTA of a pair holds half of the tile's B rows, rounded up to whole 64-column chunks (an MN-major half of
@@ -75,7 +82,7 @@ struct GemmCfg {
   // `depth`: input pieces each epilogue warp keeps in flight; `ew`: epilogue warps
   __host__ __device__ static constexpr int stages(bool tma_res, bool room = false, int depth = 2, int ew = 4) {
     const uint32_t res = (uint32_t)(ew * depth) * 4096u;
-    const uint32_t avail = GEMM_SMEM_LIMIT - 1024u - staging_bytes(ew) - (((PAIR || room) && tma_res) ? res : 0u);
+    const uint32_t avail = GEMM_SMEM_LIMIT - 1024u - staging_bytes(ew) - (((PAIR || SPLIT || room) && tma_res) ? res : 0u);
     const int n = (int)(avail / (A_BYTES + B_BYTES));
     return n > 6 ? 6 : n;
   }
@@ -183,6 +190,7 @@ struct EpiParams {
   int ce_rows;           // row count of the statistics buffer
   int ce_col0;           // vocabulary column of this product's column 0
   int ce_softcap;        // z = 15 tanh(logit / 15) (ane/common.go:272-287)
+  int seg_kb;            // > 0: operands are (hi | lo) halves of seg_kb k-blocks each, three passes hi*hi, hi*lo, lo*hi
 };
 
 // Several accumulating products with one contraction length, run by one launch (the four weight gradients of a
@@ -198,6 +206,7 @@ struct alignas(64) GemmGroup {
 
 // Work scheduler shared by the three warp roles (each role walks the same sequence).
 //   split_k > 0 : classic persistent schedule, work item = (k split, tile), stride gridDim.x.
+//   split_k < 0 : one tile per cluster of -split_k CTAs, each with an equal share of the k-blocks.
 //   split_k == 0: stream-K.  The tiles x k-blocks units are dealt out in equal contiguous ranges, one per
 //                 CTA; a range is cut into segments at tile boundaries and every segment ends in a
 //                 reduce-add, so it needs an accumulating epilogue.  Removes the partial last wave.
@@ -219,7 +228,9 @@ struct GemmSched {
     tiles = g ? g->tile0[g->n] : tiles_m * tiles_n;
     kblocks = (K + GEMM_BK - 1) / GEMM_BK;
     split_k = split;
-    if (split_k > 0) {
+    if (split_k < 0) {
+      w = 0;
+    } else if (split_k > 0) {
       kb_per_split = (kblocks + split_k - 1) / split_k;
       total_work = tiles * split_k;
       w = bid;
@@ -231,6 +242,15 @@ struct GemmSched {
   }
   // Next non-empty segment: tile (tm, tn) and k-block range [kb0, kb1).
   __device__ __forceinline__ bool next(int& tm, int& tn, int& kb0, int& kb1) {
+    if (split_k < 0) {
+      if (w != 0) return false;
+      w = 1;
+      const int part = bid % -split_k;
+      kb0 = kblocks * part / -split_k;
+      kb1 = kblocks * (part + 1) / -split_k;
+      place(bid / -split_k, tm, tn);
+      return true;
+    }
     if (split_k > 0) {
       while (w < total_work) {
         const int split = w / tiles;
@@ -276,6 +296,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   using Cfg = GemmCfg<BN, MT>;
   // grouped launches exist for the accumulating weight-gradient form on single-CTA tiles only
   constexpr bool kGroup = A_MN && B_MN && EPI == EPI_REDUCE_F32 && MT < GEMM_MT_PAIR;
+  constexpr bool SPLIT = Cfg::SPLIT;
+  const int parts = SPLIT ? -split_k : 1;  // CTAs that share a tile
   const GemmGroup* grp = kGroup ? group : nullptr;
   int M = M0, N = N0;  // the epilogue of a grouped launch sets them per tile
   constexpr bool kTmaRes = (EPI == EPI_STORE_F32_TMARES || EPI == EPI_DSWIGLU || EPI == EPI_DRELU2);  // an input piece per output piece, by TMA
@@ -308,8 +330,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   // A pipeline wait that gave up earlier in this stream poisons the status word: later launches
   // return at once instead of each running into its own time-out.
-  // (a pair always runs through: its two CTAs must take the same path, and every wait below is bounded)
-  if (!PAIR && status != nullptr && *reinterpret_cast<volatile int*>(status) != DEV_OK) return;
+  // (a cluster always runs through: its CTAs must take the same path, and every wait below is bounded)
+  if (!PAIR && !SPLIT && status != nullptr && *reinterpret_cast<volatile int*>(status) != DEV_OK) return;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;  // 0 = the CTA that issues the MMAs
   const int sched_id = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int sched_n = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -371,6 +393,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
           const uint32_t sa = smem_a0 + stage * Cfg::A_BYTES;
           const uint32_t sb = smem_b0 + stage * Cfg::B_BYTES;
+          int ka = kb * BK, kb_ = ka;  // first k of this block in A and B
+          if (epi.seg_kb > 0) {
+            const int pass = kb / epi.seg_kb, in_pass = kb - pass * epi.seg_kb;
+            ka = (in_pass + (pass == 2 ? epi.seg_kb : 0)) * BK;
+            kb_ = (in_pass + (pass == 1 ? epi.seg_kb : 0)) * BK;
+          }
           if constexpr (PAIR) {
             // both CTAs' bytes complete on the leader's barrier, which expects the sum
             const uint32_t full = map_to_cta(smem_u32(&bar_full[stage]), 0);
@@ -381,19 +409,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               const int m0 = tm * BM + sub_row(i);
               const uint32_t sai = sa + i * (GEMM_BM * BK * 2);
               if constexpr (!A_MN) {
-                tma_load_2d_pair(sai, &tmA, full, kb * BK, m0);
+                tma_load_2d_pair(sai, &tmA, full, ka, m0);
               } else {
 #pragma unroll
                 for (int j = 0; j < GEMM_BM / 64; ++j)
-                  tma_load_2d_pair(sai + j * (64 * BK * 2), &tmA, full, m0 + j * 64, kb * BK);
+                  tma_load_2d_pair(sai + j * (64 * BK * 2), &tmA, full, m0 + j * 64, ka);
               }
             }
             if constexpr (!B_MN) {
-              tma_load_2d_pair(sb, &tmB, full, kb * BK, n0);  // box of BN/2 rows
+              tma_load_2d_pair(sb, &tmB, full, kb_, n0);  // box of BN/2 rows
             } else {
 #pragma unroll
               for (int j = 0; j < Cfg::B_ROWS / 64; ++j)  // the last chunk may reach past this CTA's half: unused columns
-                tma_load_2d_pair(sb + j * (64 * BK * 2), &tmB, full, n0 + j * 64, kb * BK);
+                tma_load_2d_pair(sb + j * (64 * BK * 2), &tmB, full, n0 + j * 64, kb_);
             }
           } else {
           const uint32_t full = smem_u32(&bar_full[stage]);
@@ -401,23 +429,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if constexpr (!A_MN) {
 #pragma unroll
             for (int i = 0; i < SUBS; ++i)
-              tma_load_2d(sa + i * (GEMM_BM * BK * 2), pA, full, kb * BK, tm * BM + i * GEMM_BM);
+              tma_load_2d(sa + i * (GEMM_BM * BK * 2), pA, full, ka, tm * BM + i * GEMM_BM);
           } else {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
-              tma_load_2d(sa + j * (64 * BK * 2), pA, full, tm * BM + j * 64, kb * BK);
+              tma_load_2d(sa + j * (64 * BK * 2), pA, full, tm * BM + j * 64, ka);
           }
           if constexpr (!B_MN) {
-            tma_load_2d(sb, pB, full, kb * BK, tn * BN);
+            tma_load_2d(sb, pB, full, kb_, tn * BN);
           } else {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(sb + j * (64 * BK * 2), pB, full, tn * BN + j * 64, kb * BK);
+              tma_load_2d(sb + j * (64 * BK * 2), pB, full, tn * BN + j * 64, kb_);
           }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
+    }
+    if constexpr (SPLIT) {
+      __syncwarp();
+      cluster_sync_all();  // the epilogue warps' exchange
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
@@ -474,6 +506,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         ++local;
       }
     }
+    if constexpr (SPLIT) {
+      __syncwarp();
+      cluster_sync_all();
+    }
   } else {
     // ------------------------------ epilogue warps ------------------------------
     const int lane_group = warp & 3;  // TMEM lanes [32*lane_group, 32*lane_group+32)
@@ -497,7 +533,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t res_base = smem_stage0 + Cfg::staging_bytes(EW) + (uint32_t)(warp - 2) * (uint32_t)(RD * 4096);
     // with eight warps, warps 2-5 take the first half of the tile's columns and warps 6-9 the second
     constexpr int CSPAN = BN / (EW / 4);
-    const int c_begin = ((warp - 2) >> 2) * CSPAN, c_end = c_begin + CSPAN;
+    // CTAs that share a tile take its pieces in turns (SwiGLU forward: pairs of pieces, which make one gate piece)
+    constexpr int CGRP = EPI == EPI_STORE_BF16_SWIGLU ? 2 * CW : CW;
+    const int part = SPLIT ? (int)blockIdx.x % parts : 0;
+    const int c_begin = ((warp - 2) >> 2) * CSPAN + part * CGRP, c_end = ((warp - 2) >> 2) * CSPAN + CSPAN;
+    auto c_next = [&](int c) { return (!SPLIT || (CGRP > CW && ((c / CW) & 1) == 0)) ? c + CW : c + CW + (parts - 1) * CGRP; };
     const uint8_t* res_ptr = smem_raw + (res_base - smem_u32(smem_raw));
     uint32_t res_uses = 0;  // pieces consumed so far (buffer = uses % RD, phase = (uses / RD) & 1)
     GemmSched sched;
@@ -519,7 +559,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       auto prefetch_first = [&](int m) {
         if constexpr (EPI == EPI_STORE_F32) {
           pre_ok = false;
-          if (epi.res1 && m < M && tn * BN + c_begin + 32 <= N) {
+          if (epi.res1 && m < M && c_begin < c_end && tn * BN + c_begin + 32 <= N) {
             const float4* rp = reinterpret_cast<const float4*>(epi.res1 + (size_t)m * epi.ldres + tn * BN + c_begin);
 #pragma unroll
             for (int q = 0; q < 8; ++q) pre[q] = rp[q];
@@ -546,13 +586,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       };
       if constexpr (kTmaRes) {  // first two pieces of sub-tile 0, while the MMAs still run
 #pragma unroll
-        for (int k = 0; k < RD; ++k) issue_res(tm * BM + sub_row(0) + lane_group * 32, tn * BN + c_begin + k * CW);
+        for (int k = 0; k < RD; ++k) issue_res(tm * BM + sub_row(0) + lane_group * 32, tn * BN + c_begin + k * CW * parts);
       }
-      if (!mbar_wait(smem_u32(&bar_tfull[buf]), tphase, status, DEV_MBAR_TIMEOUT_EPILOGUE)) {
+      const bool landed = mbar_wait(smem_u32(&bar_tfull[buf]), tphase, status, DEV_MBAR_TIMEOUT_EPILOGUE);
+      if (!SPLIT && !landed) {
         ok = false;
         break;
       }
       tc_fence_after();
+      if constexpr (SPLIT) {
+        // this CTA's partial sums as [column / 4][row] float4 over the pipeline stages, which the MMAs no longer need
+        const uint32_t mine = smem_base + (uint32_t)((lane_group * 32 + lane) * 16);
+#pragma unroll 1
+        for (int c = 0; c < BN; c += 32) {
+          float v[32];
+          __syncwarp();
+          tmem_ld_32x32(tmem_base + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)c, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(mine + (uint32_t)((c / 4 + q) * GEMM_BM * 16)), "f"(v[4 * q]),
+                         "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
+                         : "memory");
+        }
+        __syncwarp();
+        cluster_sync_all();
+      }
 #pragma unroll 1
       for (int sub = 0; sub < SUBS; ++sub) {
       const int m_warp = tm * BM + sub_row(sub) + lane_group * 32;
@@ -561,7 +620,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         prefetch_first(m);
         if constexpr (kTmaRes) {
 #pragma unroll
-          for (int k = 0; k < RD; ++k) issue_res(m_warp, tn * BN + c_begin + k * CW);
+          for (int k = 0; k < RD; ++k) issue_res(m_warp, tn * BN + c_begin + k * CW * parts);
         }
       }
       int tgt_col = -1;        // EPI_STORE_BF16_TGT: this row's target column
@@ -593,13 +652,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const uint32_t taddr = tmem_base + ((uint32_t)(lane_group * 32) << 16) +
                              (uint32_t)(buf * Cfg::ACC_COLS + sub * BN);
 #pragma unroll 1
-      for (int c = c_begin; c < c_end; c += CW) {
+      for (int c = c_begin; c < c_end; c = c_next(c)) {
         const int n0 = tn * BN + c;
         if (n0 >= N || m_warp >= M) break;  // warp-uniform
         float acc[CW];
         __syncwarp();
-        tmem_ld_32x32(taddr + (uint32_t)c, acc);
-        if constexpr (CW == 64) tmem_ld_32x32(taddr + (uint32_t)c + 32u, acc + 32);
+        if constexpr (SPLIT) {  // all CTAs' partial sums, in rank order
+          const uint32_t at = smem_base + (uint32_t)((c / 4 * GEMM_BM + lane_group * 32 + lane) * 16);
+#pragma unroll
+          for (int e = 0; e < CW; ++e) acc[e] = 0.f;
+#pragma unroll 1
+          for (int p = 0; p < parts; ++p) {
+            const uint32_t from = map_to_cta(at, (uint32_t)p);
+#pragma unroll
+            for (int q = 0; q < CW / 4; ++q) {
+              float4 t;
+              asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
+                           : "r"(from + (uint32_t)(q * GEMM_BM * 16)) : "memory");
+              acc[4 * q] += t.x; acc[4 * q + 1] += t.y; acc[4 * q + 2] += t.z; acc[4 * q + 3] += t.w;
+            }
+          }
+        } else {
+          tmem_ld_32x32(taddr + (uint32_t)c, acc);
+          if constexpr (CW == 64) tmem_ld_32x32(taddr + (uint32_t)c + 32u, acc + 32);
+        }
         float4 cur[8];
         bool cur_ok = false;
         if constexpr (EPI == EPI_STORE_F32) {
@@ -607,15 +683,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
           for (int q = 0; q < 8; ++q) cur[q] = pre[q];
           pre_ok = false;
-          const int nn = n0 + CW;
-          if (epi.res1 && m < M && c + CW < c_end && nn + 32 <= N) {
+          const int nn = tn * BN + c_next(c);
+          if (epi.res1 && m < M && c_next(c) < c_end && nn + 32 <= N) {
             const float4* rp = reinterpret_cast<const float4*>(epi.res1 + (size_t)m * epi.ldres + nn);
 #pragma unroll
             for (int q = 0; q < 8; ++q) pre[q] = rp[q];
             pre_ok = true;
           }
         }
-        tmem_ld_wait();
+        if constexpr (!SPLIT) tmem_ld_wait();
         if constexpr (EPI == EPI_CE_STATS) {
           constexpr float kL2e = 1.4426950408889634f;
           const int t = tgt_col - epi.ce_col0 - n0;
@@ -904,7 +980,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         __syncwarp();
         if constexpr (kTmaRes) {  // this residual buffer is free: fetch the piece after next
           ++res_uses;
-          issue_res(m_warp, n0 + RD * CW);
+          issue_res(m_warp, n0 + RD * CW * parts);
         }
         if (lane == 0) {
           const uint32_t src = stage_base + (uint32_t)sbuf * 4096u;
@@ -933,7 +1009,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();  // the peer has drained its accumulators and its last loads have landed
+  // the peer has drained its accumulators and its last loads have landed; all partial sums have been read
+  if constexpr (PAIR || SPLIT) cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
     if constexpr (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);

@@ -279,6 +279,26 @@ def test_relu2_backward_fused_into_the_dx_product(M, Hd, K):
         lib.ane_dev_free(p)
 
 
+@pytest.mark.parametrize("M,N,K,b_mn", [(1, 8, 256, 0), (37, 768, 768, 0), (128, 128, 1024, 1), (256, 768, 4096, 1), (129, 136, 520, 0),
+                                        (300, 2304, 768, 0), (512, 1000, 264, 1)])
+def test_tiles_shared_by_a_cluster(M, N, K, b_mn):
+    """Few 128 x 128 tiles: two, four or eight CTAs share one along the contraction and meet in distributed shared memory
+    (uneven shares of the k-blocks, ragged rows and columns, more CTAs than pieces), plain and with a TMA-fed residual."""
+    rng = np.random.default_rng(M + N + K)
+    A = _bf16_round(rng.standard_normal((M, K)).astype(np.float32) * 0.1)
+    B = _bf16_round(rng.standard_normal((K, N) if b_mn else (N, K)).astype(np.float32) * 0.1)
+    R = rng.standard_normal((M, N)).astype(np.float32)
+    want = A.astype(np.float64) @ (B if b_mn else B.T).astype(np.float64)
+    assert rel_l2(_gemm(ane.DTYPE_BF16, A, B, np.zeros((M, N), np.float32), M, N, K, 0, b_mn, 1), want) < 1e-5
+    assert rel_l2(_gemm(ane.DTYPE_BF16, A, B, np.zeros((M, N), np.float32), M, N, K, 0, b_mn, 1, res=R), want + R) < 1e-5
+
+
+@pytest.mark.parametrize("M,Hd,K", [(256, 2048, 768), (200, 320, 264), (100, 64, 512)])
+def test_activation_backward_on_tiles_shared_by_a_cluster(M, Hd, K):
+    test_swiglu_backward_fused_into_the_dx_product(M, Hd, K)
+    test_relu2_backward_fused_into_the_dx_product(M, Hd, K)
+
+
 def test_gemm_rejects_misaligned_pitch():
     A = np.zeros((16, 20), np.float32)  # 20 bf16 = 40 bytes per row: not a 16-byte multiple
     dA, dB, dC = _up_bf16(A), _up_bf16(A), _up(np.zeros((16, 16), np.float32))
