@@ -475,14 +475,18 @@ static int resident_clusters(int size) {
   }
   return known[at];
 }
-// How many CTAs share a 128 x 128 tile (0: none): as many as stay resident together with at least two k-blocks each.
+// How many CTAs share a 128 x 128 tile (0: none): as many as stay resident together with at least four k-blocks each (the
+// exchange costs about as much as four).  The bf16 epilogues without input pieces are short and have only two 64-column
+// pieces to share (SwiGLU forward: one pair), so there the exchange costs more than it saves for short K: excluded; measured
+// on the one-window step with the bf16 store / SwiGLU left out, 2552 -> 2535 / 2522 us.
 static int cluster_split(const GemmDesc& d) {
   static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_CLUSTER_SPLIT"); return e && e[0] == '0'; }();  // A/B measurements
-  if (off || d.a_mn || d.out == GEMM_OUT_ACCUM || d.out == GEMM_OUT_CE_STATS || d.out == GEMM_OUT_CE_GRAD || d.out == GEMM_OUT_BF16_TGT) return 0;
+  if (off || d.a_mn) return 0;
+  if (d.out != GEMM_OUT_F32 && d.out != GEMM_OUT_BF16_ROPE && d.out != GEMM_OUT_DSWIGLU && d.out != GEMM_OUT_DRELU2) return 0;
   const long tiles = (long)((d.M + 127) / 128) * ((d.N + 127) / 128);
   const int kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;
   for (int s : {8, 4, 2})
-    if (kblocks >= 2 * s && tiles <= resident_clusters(s)) return s;
+    if (kblocks >= 4 * s && tiles <= resident_clusters(s)) return s;
   return 0;
 }
 
