@@ -725,27 +725,25 @@ void dot_accumulate(const float* a, const float* b, uint64_t n, float alpha, flo
   dot_accumulate_kernel<<<grid, 256, 0, s>>>(a, b, n, alpha, out);
 }
 
-// The three passes of one residual's lambda gradients in one (ane/train_full.go:733-782):
-//   out_a += sum(d * a),  out_b += sum(d * b)  (products rounded to fp32, summed in double),  y += *alpha * d.
-// d is read once instead of three times: 5 instead of 7 tensor passes over HBM, one launch instead of three.
+// The three reductions / updates that both residuals of a layer contribute to the lambda gradients and the x0 gradient,
+// (ane/train_full.go:733-782; products rounded to fp32, summed in double) in one pass over seven tensors (one pass per residual read ten: 21 us each at 8192 x 768, at the memory's rate).
 __global__ void __launch_bounds__(256)
-lambda_grads_kernel(const float* __restrict__ d, const float* __restrict__ a, const float* __restrict__ b,
-                    float* __restrict__ y, const float* __restrict__ alpha, uint64_t n4, float* __restrict__ out_a,
-                    float* __restrict__ out_b) {
+lambda_grads_kernel(const float4* __restrict__ d1, const float4* __restrict__ a1, const float4* __restrict__ d2,
+                    const float4* __restrict__ a2, const float4* __restrict__ b, float4* __restrict__ y, int assign,
+                    const float* __restrict__ alpha, uint64_t n4, float* __restrict__ out_a, float* __restrict__ out_b) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const float al = *alpha;
   double sa = 0.0, sb = 0.0;
-  const float4* d4 = reinterpret_cast<const float4*>(d);
-  const float4* a4 = reinterpret_cast<const float4*>(a);
-  const float4* b4 = reinterpret_cast<const float4*>(b);
-  float4* y4 = reinterpret_cast<float4*>(y);
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
-    const float4 dv = d4[i], av = a4[i], bv = b4[i];
-    float4 yv = y4[i];
-    sa += (double)(dv.x * av.x) + (double)(dv.y * av.y) + (double)(dv.z * av.z) + (double)(dv.w * av.w);
-    sb += (double)(dv.x * bv.x) + (double)(dv.y * bv.y) + (double)(dv.z * bv.z) + (double)(dv.w * bv.w);
-    yv.x += al * dv.x; yv.y += al * dv.y; yv.z += al * dv.z; yv.w += al * dv.w;
-    y4[i] = yv;
+    const float4 u = d1[i], av = a1[i], v = d2[i], aw = a2[i], bv = b[i];
+    float4 yv = assign ? make_float4(0.f, 0.f, 0.f, 0.f) : y[i];
+    sa += (double)(u.x * av.x) + (double)(u.y * av.y) + (double)(u.z * av.z) + (double)(u.w * av.w);
+    sa += (double)(v.x * aw.x) + (double)(v.y * aw.y) + (double)(v.z * aw.z) + (double)(v.w * aw.w);
+    sb += (double)(u.x * bv.x) + (double)(u.y * bv.y) + (double)(u.z * bv.z) + (double)(u.w * bv.w);
+    sb += (double)(v.x * bv.x) + (double)(v.y * bv.y) + (double)(v.z * bv.z) + (double)(v.w * bv.w);
+    yv.x += al * u.x; yv.y += al * u.y; yv.z += al * u.z; yv.w += al * u.w;
+    yv.x += al * v.x; yv.y += al * v.y; yv.z += al * v.z; yv.w += al * v.w;
+    y[i] = yv;
   }
   sa = warp_sum_d(sa);
   sb = warp_sum_d(sb);
@@ -767,12 +765,14 @@ lambda_grads_kernel(const float* __restrict__ d, const float* __restrict__ a, co
   }
 }
 // n must be a multiple of 4 and the buffers 16-byte aligned (token-major activations are).
-void lambda_grads(const float* d, const float* a, const float* b, float* y, const float* alpha, uint64_t n, float* out_a,
-                  float* out_b, cudaStream_t s) {
+void lambda_grads(const float* d1, const float* a1, const float* d2, const float* a2, const float* b, float* y, bool assign,
+                  const float* alpha, uint64_t n, float* out_a, float* out_b, cudaStream_t s) {
   if (!n) return;
   int grid = grid_for(n / 4, 256);
   if (grid > 148 * 8) grid = 148 * 8;
-  lambda_grads_kernel<<<grid, 256, 0, s>>>(d, a, b, y, alpha, n / 4, out_a, out_b);
+  auto v = [](const float* p) { return reinterpret_cast<const float4*>(p); };
+  lambda_grads_kernel<<<grid, 256, 0, s>>>(v(d1), v(a1), v(d2), v(a2), v(b), reinterpret_cast<float4*>(y), assign ? 1 : 0, alpha, n / 4,
+                                           out_a, out_b);
 }
 
 __global__ void axpy_dev_kernel(float* __restrict__ y, const float* __restrict__ x, const float* __restrict__ alpha,

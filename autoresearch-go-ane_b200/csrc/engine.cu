@@ -832,7 +832,10 @@ int EngineT<T>::forward(const uint16_t* d_tok, int B, int Tl, int pos0) {
     const float* xl = isN_ ? P_ + s_x0l_.off + l : nullptr;
     if (l % bucket_layers_ == 0) wait_bucket(l / bucket_layers_);
     count_launch();
-    rmsnorm_forward<T>(xs_[l], w_att, a.xn, a.rstd1, M, D_, stream_);
+    // reference arch: both blocks of a layer add rl * (their input) + xl * x0; the norm that reads the input writes that sum
+    RmsBlend blend;
+    if (isN_) blend = RmsBlend{x0_, rl, xl, dxn_};
+    rmsnorm_forward<T>(xs_[l], w_att, a.xn, a.rstd1, M, D_, stream_, blend);
     // llama arch, bf16, head_dim 64: the rotation of q and k happens on the fp32 accumulators in the epilogue
     static const bool no_fuse_rope = getenv("ANE_B200_NO_FUSE_ROPE") != nullptr;  // A/B measurements
     const bool fused_rope = !kIsF32 && !qkv_f32_ && !isN_ && hd_ == 64 && !no_fuse_rope;
@@ -908,13 +911,12 @@ int EngineT<T>::forward(const uint16_t* d_tok, int B, int Tl, int pos0) {
       GemmDesc g;  // x2 = rl*x + Wo*att (+ xl*x0)   ane/train_full.go:414-426
       g.A = a.att; g.B = wop(s_wo_[l].off); g.C = a.x2;
       g.M = M; g.N = D_; g.K = QD_; g.lda = QD_; g.ldb = QD_; g.ldc = D_; g.out = GEMM_OUT_F32;
-      g.res1 = xs_[l]; g.s1 = rl; g.ldres = D_;
-      if (isN_) { g.res2 = x0_; g.s2 = xl; }
+      g.res1 = isN_ ? dxn_ : xs_[l]; g.s1 = isN_ ? d_one_ : rl; g.ldres = D_;
       count_launch();
       if ((rc = gemm(g)) != 0) return rc;
     }
     count_launch();
-    rmsnorm_forward<T>(a.x2, w_ffn, a.x2n, a.rstd2, M, D_, stream_);
+    rmsnorm_forward<T>(a.x2, w_ffn, a.x2n, a.rstd2, M, D_, stream_, blend);
     {
       GemmDesc g;
       g.A = a.x2n; g.B = wop(s_w13_[l].off); g.C = a.h13;
@@ -948,8 +950,7 @@ int EngineT<T>::forward(const uint16_t* d_tok, int B, int Tl, int pos0) {
       GemmDesc g;  // out = rl*x2 + W2*gate (+ xl*x0)   ane/train_full.go:434-445
       g.A = a.gate; g.B = wop(s_w2_[l].off); g.C = xs_[l + 1];
       g.M = M; g.N = D_; g.K = Hd_; g.lda = Hd_; g.ldb = Hd_; g.ldc = D_; g.out = GEMM_OUT_F32;
-      g.res1 = a.x2; g.s1 = rl; g.ldres = D_;
-      if (isN_) { g.res2 = x0_; g.s2 = xl; }
+      g.res1 = isN_ ? dxn_ : a.x2; g.s1 = isN_ ? d_one_ : rl; g.ldres = D_;
       count_launch();
       if ((rc = gemm(g)) != 0) return rc;
     }
@@ -1110,7 +1111,6 @@ int EngineT<T>::backward_layers(int B) {
     dot_accumulate(dcur_[cur], xs_[L_ / 2], MD, -1.f, G_ + s_backout_l_.off, stream_);
     count_launch();
     axpy_dev(gmid_, dcur_[cur], P_ + s_backout_l_.off, -1.f, MD, true, stream_);
-    cudaMemsetAsync(gx0_, 0, sizeof(float) * MD, stream_);
   }
   for (int l = L_ - 1; l >= 0; --l) {
     Act<T>& a = acts_[l];
@@ -1198,16 +1198,6 @@ int EngineT<T>::backward_layers(int B) {
         if ((rc = gemm(g, dws)) != 0) return rc;
         count_launch();
         if ((rc = gemm(g2, dws)) != 0) return rc;
-      }
-    }
-    if (isN_) {  // lambda gradients, FFN residual (ane/train_full.go:732-748)
-      count_launch(3);
-      if (MD % 4 == 0) {
-        lambda_grads(dcur, a.x2, x0_, gx0_, xl, MD, G_ + s_resid_.off + l, G_ + s_x0l_.off + l, stream_);
-      } else {
-        dot_accumulate(dcur, a.x2, MD, 1.f, G_ + s_resid_.off + l, stream_);
-        dot_accumulate(dcur, x0_, MD, 1.f, G_ + s_x0l_.off + l, stream_);
-        axpy_dev(gx0_, dcur, xl, 1.f, MD, false, stream_);
       }
     }
     // ---- attention backward
@@ -1320,15 +1310,9 @@ int EngineT<T>::backward_layers(int B) {
       }
       if (dws != stream_) cudaEventRecord(ev_dw_done_[l], dws);
     }
-    if (isN_) {  // lambda gradients, attention residual (ane/train_full.go:770-782)
-      count_launch(3);
-      if (MD % 4 == 0) {
-        lambda_grads(dx2, xs_[l], x0_, gx0_, xl, MD, G_ + s_resid_.off + l, G_ + s_x0l_.off + l, stream_);
-      } else {
-        dot_accumulate(dx2, xs_[l], MD, 1.f, G_ + s_resid_.off + l, stream_);
-        dot_accumulate(dx2, x0_, MD, 1.f, G_ + s_x0l_.off + l, stream_);
-        axpy_dev(gx0_, dx2, xl, 1.f, MD, false, stream_);
-      }
+    if (isN_) {  // lambda gradients of both residuals (ane/train_full.go:732-748, :770-782); MD % 4 == 0 (dim % 8 == 0)
+      count_launch();
+      lambda_grads(dcur, a.x2, dx2, xs_[l], x0_, gx0_, l == L_ - 1, xl, MD, G_ + s_resid_.off + l, G_ + s_x0l_.off + l, stream_);
       if (l == L_ / 2) {  // gradient of the backout term joins at the output of layer L/2-1
         count_launch();
         add_inplace(dprev, gmid_, MD, stream_);

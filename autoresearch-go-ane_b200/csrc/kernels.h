@@ -28,8 +28,13 @@ void embed_forward(const uint16_t* tok, const float* embed, float* x, float* x_r
 void embed_backward(const uint16_t* tok, const float* dx, float* g_embed, int M, int D, int vocab, cudaStream_t s);
 
 // y = x * rstd (* w); rstd = (mean(x^2)+1e-5)^-1/2.  ane/common.go:107-174, ane/stories/cpu.go:97-127.
+// With a blend: also blend.out = *s1 * x + *s2 * other ([M, D] fp32, device scalars).
+struct RmsBlend {
+  const float *other = nullptr, *s1 = nullptr, *s2 = nullptr;
+  float* out = nullptr;
+};
 template <typename T>
-void rmsnorm_forward(const float* x, const float* w, T* y, float* rstd, int M, int D, cudaStream_t s);
+void rmsnorm_forward(const float* x, const float* w, T* y, float* rstd, int M, int D, cudaStream_t s, RmsBlend blend = RmsBlend());
 // dx = rms_bwd(dy; x, w) + res_scale * res   (ane/common.go:176-197; ane/stories/cpu.go:129-150)
 //   dy: fp32 [M,D];  res/res_scale optional;  dx_f32 and dx_t outputs (dx_t optional copy in T);
 //   dw (optional, weighted norm): dw[i] += sum_m dy*x*rstd.
@@ -204,9 +209,10 @@ void smear_forward(const float* x_pre, const float* gate_pre, const float* lambd
 void smear_backward(const float* d_out, const float* x_pre, const float* gate_pre, const float* lambda,
                     float* d_gate_pre, float* dx, float* g_lambda, int M, int seq, int D, cudaStream_t s);
 // out[0] += alpha * sum(a*b)  (double accumulation; ane/train_full.go:733-782, ane/common.go:396-400)
-// out_a += sum(d*a), out_b += sum(d*b), y += *alpha * d in one pass (n % 4 == 0, 16-byte aligned buffers).
-void lambda_grads(const float* d, const float* a, const float* b, float* y, const float* alpha, uint64_t n, float* out_a,
-                  float* out_b, cudaStream_t s);
+// Both residuals of a layer in one pass (n % 4 == 0, 16-byte aligned buffers):
+// out_a += sum(d1*a1 + d2*a2), out_b += sum((d1+d2)*b), y (+)= *alpha * (d1+d2).
+void lambda_grads(const float* d1, const float* a1, const float* d2, const float* a2, const float* b, float* y, bool assign,
+                  const float* alpha, uint64_t n, float* out_a, float* out_b, cudaStream_t s);
 void dot_accumulate(const float* a, const float* b, uint64_t n, float alpha, float* out, cudaStream_t s);
 // y += (*alpha) * x  and  y = (*alpha) * x   (alpha is a device scalar; sign flips it)
 void axpy_dev(float* y, const float* x, const float* alpha, float sign, uint64_t n, bool assign, cudaStream_t s);
