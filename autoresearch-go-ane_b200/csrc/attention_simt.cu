@@ -160,6 +160,8 @@ __device__ __forceinline__ void zero(float (&a)[4][HDP / 16]) {
 template <int HDP, typename T, typename TO>
 __global__ void __launch_bounds__(kSimtThreads)
 attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, float* __restrict__ lse, int seq, int H, int KV, int hd, float scale) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) float simt_smem[];
   float* Qs = simt_smem;
   float* Ks = Qs + Simt<HDP>::kResFloats;
@@ -236,6 +238,8 @@ template <int HDP, typename T, typename TD>
 __global__ void __launch_bounds__(kSimtThreads)
 attention_dq_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_out, float* __restrict__ dqkv, float* __restrict__ stats, int rows, int seq,
                          int H, int KV, int hd, float scale) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) float simt_smem[];
   float* Qs = simt_smem;
   float* dOs = Qs + Simt<HDP>::kResFloats;
@@ -343,6 +347,8 @@ template <int HDP, typename T, typename TD>
 __global__ void __launch_bounds__(kSimtThreads)
 attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_out, float* __restrict__ dqkv, const float* __restrict__ stats, int rows,
                           int seq, int H, int KV, int hd, float scale) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) float simt_smem[];
   float* Ks = simt_smem;
   float* Vs = Ks + Simt<HDP>::kResFloats;
@@ -415,7 +421,7 @@ void forward_hdp(const T* qkv, TO* out, float* lse, int B, int seq, int H, int K
   auto kern = attention_forward_simt_kernel<HDP, T, TO>;
   static unsigned long long done = 0;
   smem_opt_in(kern, Simt<HDP>::kFwdSmem, done);
-  kern<<<dim3(B * H, (seq + kRes - 1) / kRes), kSimtThreads, Simt<HDP>::kFwdSmem, s>>>(qkv, out, lse, seq, H, KV, hd, scale);
+  launch_pdl(kern, dim3(B * H, (seq + kRes - 1) / kRes), dim3(kSimtThreads), Simt<HDP>::kFwdSmem, s, qkv, out, lse, seq, H, KV, hd, scale);
 }
 template <int HDP, typename T, typename TD>
 void backward_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
@@ -425,8 +431,8 @@ void backward_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int 
   smem_opt_in(dq, Simt<HDP>::kDqSmem, done_q);
   smem_opt_in(dkv, Simt<HDP>::kDkvSmem, done_k);
   const int tiles = (seq + kRes - 1) / kRes, rows = B * H * seq;
-  dq<<<dim3(B * H, tiles), kSimtThreads, Simt<HDP>::kDqSmem, s>>>(qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
-  dkv<<<dim3(B * KV, tiles), kSimtThreads, Simt<HDP>::kDkvSmem, s>>>(qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
+  launch_pdl(dq, dim3(B * H, tiles), dim3(kSimtThreads), Simt<HDP>::kDqSmem, s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
+  launch_pdl(dkv, dim3(B * KV, tiles), dim3(kSimtThreads), Simt<HDP>::kDkvSmem, s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
 }
 
 }  // namespace

@@ -168,6 +168,8 @@ template <class C>
 __global__ void __launch_bounds__(C::THREADS)
 attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf16* __restrict__ out_lo,
                         float* __restrict__ lse, int T, int H, int KV, float scale) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int HD = C::HD, BR = C::BR, LDS = C::LDS;
   extern __shared__ __align__(16) uint8_t att_smem[];
   bf16* Qs = reinterpret_cast<bf16*>(att_smem);   // [BR][LDS]
@@ -274,6 +276,8 @@ attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf
 // delta[b,h,t] = sum_d dO * O  (one warp per (token, head))
 __global__ void attention_delta_kernel(const bf16* __restrict__ d_out, const bf16* __restrict__ out,
                                        const bf16* __restrict__ out_lo, float* __restrict__ delta, int B, int T, int H, int HD) {
+  pdl_trigger();
+  pdl_wait();
   const long long wid = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (wid >= (long long)B * T * H) return;
@@ -303,6 +307,8 @@ __global__ void __launch_bounds__(C::THREADS)
 attention_bwd_dq_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ d_out, const float* __restrict__ lse,
                            const float* __restrict__ delta, bf16* __restrict__ dqkv, const float* __restrict__ cosb,
                            const float* __restrict__ sinb, int T, int H, int KV, float scale) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int HD = C::HD, BR = C::BR, LDS = C::LDS;
   extern __shared__ __align__(16) uint8_t att_smem[];
   bf16* Qs = reinterpret_cast<bf16*>(att_smem);   // [BR][LDS]
@@ -383,6 +389,8 @@ attention_bwd_dkv_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict
                             const float* __restrict__ lse, const float* __restrict__ delta, bf16* __restrict__ dqkv,
                             const float* __restrict__ cosb, const float* __restrict__ sinb, int T, int H, int KV,
                             float scale) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int HD = C::HD, BR = C::BR, LDS = C::LDS;
   extern __shared__ __align__(16) uint8_t att_smem[];
   bf16* Ks = reinterpret_cast<bf16*>(att_smem);   // [BR][LDS]
@@ -480,7 +488,7 @@ bool launch_forward(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B,
   static unsigned long long done = 0;
   if (!smem_opt_in(attention_fwd_tc_kernel<C>, C::kFwdSmem, done)) return false;
   dim3 grid((seq + C::BR - 1) / C::BR, B * H);
-  attention_fwd_tc_kernel<C><<<grid, C::THREADS, C::kFwdSmem, s>>>(qkv, out, out_lo, lse, seq, H, KV, scale);
+  launch_pdl(attention_fwd_tc_kernel<C>, grid, dim3(C::THREADS), C::kFwdSmem, s, qkv, out, out_lo, lse, seq, H, KV, scale);
   return true;
 }
 template <class CQ, class CK>
@@ -490,9 +498,9 @@ bool launch_backward(const bf16* qkv, const bf16* d_out, const float* lse, const
   if (!smem_opt_in(attention_bwd_dq_tc_kernel<CQ>, CQ::kDqSmem, done_q) || !smem_opt_in(attention_bwd_dkv_tc_kernel<CK>, CK::kDkvSmem, done_k))
     return false;
   dim3 gq((seq + CQ::BR - 1) / CQ::BR, B * H);
-  attention_bwd_dq_tc_kernel<CQ><<<gq, CQ::THREADS, CQ::kDqSmem, s>>>(qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV, scale);
+  launch_pdl(attention_bwd_dq_tc_kernel<CQ>, gq, dim3(CQ::THREADS), CQ::kDqSmem, s, qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV, scale);
   dim3 gk((seq + CK::BR - 1) / CK::BR, B * KV);
-  attention_bwd_dkv_tc_kernel<CK><<<gk, CK::THREADS, CK::kDkvSmem, s>>>(qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV, scale);
+  launch_pdl(attention_bwd_dkv_tc_kernel<CK>, gk, dim3(CK::THREADS), CK::kDkvSmem, s, qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV, scale);
   return true;
 }
 
@@ -540,7 +548,7 @@ int attention_backward_tc(const bf16* qkv, const bf16* out, const bf16* out_lo, 
     if (n > 0) return n;
   }
   const long long warps = (long long)B * seq * H;
-  attention_delta_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(d_out, out, out_lo, delta, B, seq, H, hd);
+  launch_pdl(attention_delta_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, s, d_out, out, out_lo, delta, B, seq, H, hd);
   if (hd == 64) backward_hd<64>(qkv, d_out, lse, delta, dqkv, cosb, sinb, B, seq, H, KV, scale, s);
   else if (hd == 48) backward_hd<48>(qkv, d_out, lse, delta, dqkv, cosb, sinb, B, seq, H, KV, scale, s);
   else backward_hd<32>(qkv, d_out, lse, delta, dqkv, cosb, sinb, B, seq, H, KV, scale, s);

@@ -33,6 +33,8 @@ static inline int grid_for(uint64_t n, int block) {
 // hi = bf16(x), lo = bf16(x - hi): two bf16 tensors that together carry ~16 mantissa bits of x.
 __global__ void split_f32_to_bf16x2_kernel(const float* __restrict__ src, bf16* __restrict__ hi, bf16* __restrict__ lo,
                                            uint64_t n4) {
+  pdl_trigger();
+  pdl_wait();
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (; i < n4; i += stride) {
@@ -50,7 +52,7 @@ __global__ void split_f32_to_bf16x2_kernel(const float* __restrict__ src, bf16* 
 }
 void split_f32_to_bf16x2(const float* src, bf16* hi, bf16* lo, uint64_t n, cudaStream_t s) {
   if (!n) return;  // n must be a multiple of 4
-  split_f32_to_bf16x2_kernel<<<grid_for(n / 4, 256), 256, 0, s>>>(src, hi, lo, n / 4);
+  launch_pdl(split_f32_to_bf16x2_kernel, dim3(grid_for(n / 4, 256)), dim3(256), 0, s, src, hi, lo, n / 4);
 }
 
 void cast_f32_to_bf16(const float* src, bf16* dst, uint64_t n, cudaStream_t s) {
@@ -88,6 +90,8 @@ template <typename T>
 __global__ void rope_qknorm_forward_kernel(T* __restrict__ qkv, T* __restrict__ qk_pre,
                                            const float* __restrict__ cosb, const float* __restrict__ sinb, int M,
                                            int seq, int H, int KV, int hd, int qk_norm, int pos0) {
+  pdl_trigger();
+  pdl_wait();
   const int heads = H + KV;
   const long long wid = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -177,7 +181,7 @@ void rope_qknorm_forward(T* qkv, T* qk_pre, const float* cosb, const float* sinb
   const long long warps = (long long)M * (H + KV);
   if (warps <= 0) return;
   const int wpb = 8;
-  rope_qknorm_forward_kernel<T><<<(unsigned)((warps + wpb - 1) / wpb), wpb * 32, 0, s>>>(
+  launch_pdl(rope_qknorm_forward_kernel<T>, dim3((unsigned)((warps + wpb - 1) / wpb)), dim3(wpb * 32), 0, s, 
       qkv, qk_pre, cosb, sinb, M, seq, H, KV, hd, qk_norm, pos0);
 }
 template void rope_qknorm_forward<float>(float*, float*, const float*, const float*, int, int, int, int, int, bool, int,
@@ -190,6 +194,8 @@ __global__ void rope_qknorm_backward_kernel(T* __restrict__ dqkv, const T* __res
                                             const float* __restrict__ cosb, const float* __restrict__ sinb, int M,
                                             int seq, int H, int KV, int hd, int qk_norm, int reference_coeff,
                                             int skip_rope, TO* __restrict__ out_t, int write_back) {
+  pdl_trigger();
+  pdl_wait();
   const int heads = H + KV;
   const int slots = out_t ? H + 2 * KV : heads;  // with a typed copy, the v heads are converted too
   const long long wid = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -262,7 +268,7 @@ void rope_qknorm_backward(T* dqkv, const T* qk_pre, const float* cosb, const flo
   const long long warps = (long long)M * (out_t ? H + 2 * KV : H + KV);
   if (warps <= 0) return;
   const int wpb = 8;
-  rope_qknorm_backward_kernel<T, TO><<<(unsigned)((warps + wpb - 1) / wpb), wpb * 32, 0, s>>>(
+  launch_pdl(rope_qknorm_backward_kernel<T, TO>, dim3((unsigned)((warps + wpb - 1) / wpb)), dim3(wpb * 32), 0, s, 
       dqkv, qk_pre, cosb, sinb, M, seq, H, KV, hd, qk_norm, reference_coeff, skip_rope, out_t, write_back ? 1 : 0);
 }
 template void rope_qknorm_backward<float, float>(float*, const float*, const float*, const float*, int, int, int, int,
@@ -299,6 +305,8 @@ __global__ void __launch_bounds__(256)
 rope_qknorm_forward_hd64_kernel(float* qkv, float* __restrict__ qk_pre, const float* __restrict__ cosb,
                                 const float* __restrict__ sinb, int M, int seq, int H, int KV, int qk_norm, int pos0,
                                 bf16* __restrict__ hi_out) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int HD = 64, G = 4;
   const int heads = H + KV, slots = H + 2 * KV;
   const int groups = (slots + G - 1) / G;
@@ -343,7 +351,7 @@ void rope_qknorm_forward_hd64(float* qkv, float* qk_pre, const float* cosb, cons
   const long long warps = (long long)M * ((H + 2 * KV + 3) / 4);
   if (warps <= 0) return;
   const int wpb = 8;
-  rope_qknorm_forward_hd64_kernel<<<(unsigned)((warps + wpb - 1) / wpb), wpb * 32, 0, s>>>(qkv, qk_pre, cosb, sinb, M, seq, H,
+  launch_pdl(rope_qknorm_forward_hd64_kernel, dim3((unsigned)((warps + wpb - 1) / wpb)), dim3(wpb * 32), 0, s, qkv, qk_pre, cosb, sinb, M, seq, H,
                                                                                          KV, qk_norm, pos0, hi_out);
 }
 
@@ -392,6 +400,8 @@ __global__ void __launch_bounds__(256)
 rope_qknorm_backward_hd64_kernel(const TI* din, float* out_f32, const float* __restrict__ qk_pre,
                                  const float* __restrict__ cosb, const float* __restrict__ sinb, int M, int seq, int H,
                                  int KV, int qk_norm, int reference_coeff, int skip_rope, TO* __restrict__ out_t) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int HD = 64, G = 4;
   const int heads = H + KV, slots = H + 2 * KV;
   const int groups = (slots + G - 1) / G;
@@ -454,7 +464,7 @@ void rope_qknorm_backward_hd64(const TI* din, float* out_f32, const float* qk_pr
   const long long warps = (long long)M * ((H + 2 * KV + 3) / 4);
   if (warps <= 0) return;
   const int wpb = 8;
-  rope_qknorm_backward_hd64_kernel<TI, TO><<<(unsigned)((warps + wpb - 1) / wpb), wpb * 32, 0, s>>>(
+  launch_pdl(rope_qknorm_backward_hd64_kernel<TI, TO>, dim3((unsigned)((warps + wpb - 1) / wpb)), dim3(wpb * 32), 0, s, 
       din, out_f32, qk_pre, cosb, sinb, M, seq, H, KV, qk_norm, reference_coeff, skip_rope, out_t);
 }
 template void rope_qknorm_backward_hd64<float, float>(const float*, float*, const float*, const float*, const float*, int,
@@ -470,6 +480,8 @@ template void rope_qknorm_backward_hd64<bf16, bf16>(const bf16*, float*, const f
 // 16 bytes per access (8 bf16 or 4 floats) over the aligned body, element-wise over the tail.
 template <typename T>
 __global__ void relu2_forward_kernel(const T* __restrict__ h1, T* __restrict__ gate, uint64_t n) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int VN = Vec16<T>::N;
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -495,6 +507,8 @@ __global__ void relu2_forward_kernel(const T* __restrict__ h1, T* __restrict__ g
 template <typename T>
 __global__ void relu2_backward_kernel(const T* __restrict__ dgate, const T* __restrict__ h1, T* __restrict__ dh1,
                                       uint64_t n) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int VN = Vec16<T>::N;
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -590,12 +604,12 @@ __global__ void swiglu_backward_kernel(const T* __restrict__ dgate, const T* __r
 template <typename T>
 void relu2_forward(const T* h1, T* gate, uint64_t n, cudaStream_t s) {
   if (!n) return;
-  relu2_forward_kernel<T><<<grid_for((n + Vec16<T>::N - 1) / Vec16<T>::N, 256), 256, 0, s>>>(h1, gate, n);
+  launch_pdl(relu2_forward_kernel<T>, dim3(grid_for((n + Vec16<T>::N - 1) / Vec16<T>::N, 256)), dim3(256), 0, s, h1, gate, n);
 }
 template <typename T>
 void relu2_backward(const T* dgate, const T* h1, T* dh1, uint64_t n, cudaStream_t s) {
   if (!n) return;
-  relu2_backward_kernel<T><<<grid_for((n + Vec16<T>::N - 1) / Vec16<T>::N, 256), 256, 0, s>>>(dgate, h1, dh1, n);
+  launch_pdl(relu2_backward_kernel<T>, dim3(grid_for((n + Vec16<T>::N - 1) / Vec16<T>::N, 256)), dim3(256), 0, s, dgate, h1, dh1, n);
 }
 template <typename T>
 void swiglu_forward(const T* h13, T* gate, int M, int Hd, cudaStream_t s) {
@@ -625,6 +639,8 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf
 
 __global__ void smear_forward_kernel(const float* __restrict__ x_pre, const float* __restrict__ gate_pre,
                                      const float* __restrict__ lambda, float* __restrict__ x, int M, int seq, int D) {
+  pdl_trigger();
+  pdl_wait();
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t n = (uint64_t)M * D, stride = (uint64_t)gridDim.x * blockDim.x;
   const float lam = *lambda;
@@ -639,13 +655,15 @@ void smear_forward(const float* x_pre, const float* gate_pre, const float* lambd
                    cudaStream_t s) {
   const uint64_t n = (uint64_t)M * D;
   if (!n) return;
-  smear_forward_kernel<<<grid_for(n, 256), 256, 0, s>>>(x_pre, gate_pre, lambda, x, M, seq, D);
+  launch_pdl(smear_forward_kernel, dim3(grid_for(n, 256)), dim3(256), 0, s, x_pre, gate_pre, lambda, x, M, seq, D);
 }
 
 __global__ void smear_backward_kernel(const float* __restrict__ d_out, const float* __restrict__ x_pre,
                                       const float* __restrict__ gate_pre, const float* __restrict__ lambda,
                                       float* __restrict__ d_gate_pre, float* __restrict__ dx,
                                       float* __restrict__ g_lambda, int M, int seq, int D) {
+  pdl_trigger();
+  pdl_wait();
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t n = (uint64_t)M * D, stride = (uint64_t)gridDim.x * blockDim.x;
   const float lam = *lambda;
@@ -677,7 +695,7 @@ void smear_backward(const float* d_out, const float* x_pre, const float* gate_pr
                     float* d_gate_pre, float* dx, float* g_lambda, int M, int seq, int D, cudaStream_t s) {
   const uint64_t n = (uint64_t)M * D;
   if (!n) return;
-  smear_backward_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_out, x_pre, gate_pre, lambda, d_gate_pre, dx, g_lambda, M,
+  launch_pdl(smear_backward_kernel, dim3(grid_for(n, 256)), dim3(256), 0, s, d_out, x_pre, gate_pre, lambda, d_gate_pre, dx, g_lambda, M,
                                                          seq, D);
 }
 
@@ -687,6 +705,8 @@ void smear_backward(const float* d_out, const float* x_pre, const float* gate_pr
 __global__ void __launch_bounds__(256)
 dot_accumulate_kernel(const float* __restrict__ a, const float* __restrict__ b, uint64_t n, float alpha,
                       float* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   double local = 0.0;
@@ -722,7 +742,7 @@ void dot_accumulate(const float* a, const float* b, uint64_t n, float alpha, flo
   if (!n) return;
   int grid = grid_for((n + 3) / 4, 256);
   if (grid > 148 * 8) grid = 148 * 8;
-  dot_accumulate_kernel<<<grid, 256, 0, s>>>(a, b, n, alpha, out);
+  launch_pdl(dot_accumulate_kernel, grid, dim3(256), 0, s, a, b, n, alpha, out);
 }
 
 // The three reductions / updates that both residuals of a layer contribute to the lambda gradients and the x0 gradient,
@@ -731,6 +751,8 @@ __global__ void __launch_bounds__(256)
 lambda_grads_kernel(const float4* __restrict__ d1, const float4* __restrict__ a1, const float4* __restrict__ d2,
                     const float4* __restrict__ a2, const float4* __restrict__ b, float4* __restrict__ y, int assign,
                     const float* __restrict__ alpha, uint64_t n4, float* __restrict__ out_a, float* __restrict__ out_b) {
+  pdl_trigger();
+  pdl_wait();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const float al = *alpha;
   double sa = 0.0, sb = 0.0;
@@ -771,12 +793,14 @@ void lambda_grads(const float* d1, const float* a1, const float* d2, const float
   int grid = grid_for(n / 4, 256);
   if (grid > 148 * 8) grid = 148 * 8;
   auto v = [](const float* p) { return reinterpret_cast<const float4*>(p); };
-  lambda_grads_kernel<<<grid, 256, 0, s>>>(v(d1), v(a1), v(d2), v(a2), v(b), reinterpret_cast<float4*>(y), assign ? 1 : 0, alpha, n / 4,
+  launch_pdl(lambda_grads_kernel, grid, dim3(256), 0, s, v(d1), v(a1), v(d2), v(a2), v(b), reinterpret_cast<float4*>(y), assign ? 1 : 0, alpha, n / 4,
                                            out_a, out_b);
 }
 
 __global__ void axpy_dev_kernel(float* __restrict__ y, const float* __restrict__ x, const float* __restrict__ alpha,
                                 float sign, uint64_t n, int assign) {
+  pdl_trigger();
+  pdl_wait();
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const float a = sign * (alpha ? *alpha : 1.f);
@@ -784,7 +808,7 @@ __global__ void axpy_dev_kernel(float* __restrict__ y, const float* __restrict__
 }
 void axpy_dev(float* y, const float* x, const float* alpha, float sign, uint64_t n, bool assign, cudaStream_t s) {
   if (!n) return;
-  axpy_dev_kernel<<<grid_for(n, 256), 256, 0, s>>>(y, x, alpha, sign, n, assign ? 1 : 0);
+  launch_pdl(axpy_dev_kernel, dim3(grid_for(n, 256)), dim3(256), 0, s, y, x, alpha, sign, n, assign ? 1 : 0);
 }
 void add_inplace(float* y, const float* x, uint64_t n, cudaStream_t s) { axpy_dev(y, x, nullptr, 1.f, n, false, s); }
 
@@ -797,6 +821,8 @@ template <typename T>
 __global__ void ve_forward_kernel(T* __restrict__ qkv, const float* __restrict__ x, const uint16_t* __restrict__ tok,
                                   const float* __restrict__ ve_embed, const float* __restrict__ ve_gate,
                                   float* __restrict__ gate_act, int M, int D, int H, int KV, int hd, int vocab) {
+  pdl_trigger();
+  pdl_wait();
   const long long wid = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (wid >= (long long)M * H) return;
@@ -818,7 +844,7 @@ void ve_forward(T* qkv, const float* x, const uint16_t* tok, const float* ve_emb
                 float* gate_act, int M, int D, int H, int KV, int hd, int vocab, cudaStream_t s) {
   const long long warps = (long long)M * H;
   if (warps <= 0) return;
-  ve_forward_kernel<T><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(qkv, x, tok, ve_embed, ve_gate, gate_act, M, D, H,
+  launch_pdl(ve_forward_kernel<T>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, s, qkv, x, tok, ve_embed, ve_gate, gate_act, M, D, H,
                                                                     KV, hd, vocab);
 }
 template void ve_forward<float>(float*, const float*, const uint16_t*, const float*, const float*, float*, int, int,
@@ -835,6 +861,8 @@ __global__ void ve_backward_kernel(const T* __restrict__ dqkv, const float* __re
                                    const float* __restrict__ ve_gate, const float* __restrict__ gate_act,
                                    float* __restrict__ g_ve_embed, float* __restrict__ g_ve_gate,
                                    float* __restrict__ d_prev, int M, int D, int H, int KV, int hd, int vocab) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ float s_gate[];  // [H][kVEGateChannels]
   for (int i = threadIdx.x; i < H * kVEGateChannels; i += blockDim.x) s_gate[i] = 0.f;
   __syncthreads();
@@ -876,7 +904,7 @@ void ve_backward(const T* dqkv, const float* x, const uint16_t* tok, const float
   if (warps <= 0) return;
   long long blocks = (warps + 7) / 8;
   if (blocks > 148 * 4) blocks = 148 * 4;
-  ve_backward_kernel<T><<<(unsigned)blocks, 256, sizeof(float) * H * kVEGateChannels, s>>>(
+  launch_pdl(ve_backward_kernel<T>, dim3((unsigned)blocks), dim3(256), sizeof(float) * H * kVEGateChannels, s, 
       dqkv, x, tok, ve_embed, ve_gate, gate_act, g_ve_embed, g_ve_gate, d_prev, M, D, H, KV, hd, vocab);
 }
 template void ve_backward<float>(const float*, const float*, const uint16_t*, const float*, const float*,

@@ -56,6 +56,93 @@ inline int64_t now_ns() {
 }
 
 
+// EvalLogits into ordinary memory: device -> page-locked staging (full PCIe rate) -> caller's array.  The download is
+// cut into pieces and the host copies what has landed while the rest is still crossing PCIe.  One core copies about
+// 10 GB/s, a fifth of the PCIe rate (32.8 MB cross in 0.6 ms), so all cores copy (ANE_B200_EVAL_COPY_THREADS; default: the
+// host's cores, at most 16), in blocks of 64 KB that they claim in order: when the last piece lands only its own blocks are
+// left, one per thread (whole pieces dealt to threads left a megabyte per thread: 0.1 - 0.2 ms).  The calling thread only
+// follows the download and says how far it is.  The threads live as long as the call.
+class LogitsCopy {
+ public:
+  LogitsCopy(float* out, uint64_t per_window, uint32_t windows, float* staging, cudaEvent_t* events)
+      : out_(out), n_(per_window), staging_(staging), events_(events), order_(windows) {
+    static const int want = [] {
+      const char* e = getenv("ANE_B200_EVAL_PIECES");
+      const int v = e ? atoi(e) : 16;
+      return v < 1 ? 1 : (v > 64 ? 64 : v);
+    }();
+    static const int cores = [] {
+      const char* e = getenv("ANE_B200_EVAL_COPY_THREADS");
+      const unsigned hw = std::thread::hardware_concurrency();
+      const int v = e ? atoi(e) : (hw == 0 ? 4 : (int)hw);
+      return v < 1 ? 1 : (v > 16 ? 16 : v);
+    }();
+    piece_ = ((n_ + want - 1) / want + kBlock - 1) / kBlock * kBlock;  // whole blocks
+    pieces_ = (int)((n_ + piece_ - 1) / piece_);
+    blocks_ = (int)((n_ + kBlock - 1) / kBlock);
+    helpers_wanted_ = n_ * sizeof(float) < (1u << 20) ? 0 : std::min(cores - 1, blocks_);  // under 1 MiB: not worth a thread start
+  }
+  ~LogitsCopy() {
+    stop_.store(true);
+    for (auto& h : helpers_) h.join();
+  }
+  // Window `w` of the output from `logits` on the device, once `stream` has reached this point; returns when it is there.
+  cudaError_t window(uint32_t w, const float* logits, cudaStream_t stream) {
+    const long long round = rounds_++;
+    order_[round] = w;  // read only after `landed_` has reached this round
+    while ((int)helpers_.size() < helpers_wanted_) helpers_.emplace_back([this] { helper(); });
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < pieces_ && e == cudaSuccess; ++i) {
+      const uint64_t off = (uint64_t)i * piece_, n = std::min(piece_, n_ - off);
+      e = cudaMemcpyAsync(staging_ + off, logits + off, sizeof(float) * n, cudaMemcpyDeviceToHost, stream);
+      if (e == cudaSuccess) e = cudaEventRecord(events_[i], stream);
+    }
+    for (int i = 0; i < pieces_ && e == cudaSuccess; ++i) {
+      e = cudaEventSynchronize(events_[i]);
+      if (e == cudaSuccess) landed_.store(round * pieces_ + i + 1, std::memory_order_release);
+    }
+    if (e != cudaSuccess) return e;
+    if (helpers_wanted_ == 0) {
+      for (int k = 0; k < blocks_; ++k) copy_block(w, k);
+      return cudaSuccess;
+    }
+    while (done_.load(std::memory_order_acquire) < (round + 1) * blocks_) std::this_thread::yield();
+    return cudaSuccess;
+  }
+
+ private:
+  static constexpr uint64_t kBlock = 16384;  // floats
+  void copy_block(uint32_t w, int k) {
+    const uint64_t off = (uint64_t)k * kBlock, n = std::min(kBlock, n_ - off);
+    memcpy(out_ + (size_t)w * n_ + off, staging_ + off, sizeof(float) * n);
+  }
+  void helper() {  // blocks are numbered through all windows of the call
+    const int per_piece = (int)(piece_ / kBlock);
+    for (;;) {
+      const long long id = next_.fetch_add(1), round = id / blocks_;
+      const int k = (int)(id - round * blocks_);
+      const long long need = round * pieces_ + k / per_piece;
+      for (int idle = 0; landed_.load(std::memory_order_acquire) <= need; ++idle) {
+        if (stop_.load()) return;
+        if (idle < 64) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds(5));
+      }
+      copy_block(order_[round], k);
+      done_.fetch_add(1, std::memory_order_release);
+    }
+  }
+  float* out_;
+  uint64_t n_, piece_ = 0;
+  float* staging_;
+  cudaEvent_t* events_;
+  int pieces_ = 0, blocks_ = 0, helpers_wanted_ = 0;
+  long long rounds_ = 0;
+  std::vector<uint32_t> order_;  // window of every round
+  std::vector<std::thread> helpers_;
+  std::atomic<long long> landed_{0}, next_{0}, done_{0};
+  std::atomic<bool> stop_{false};
+};
+
 template <typename T>
 struct Act {  // saved activations of one layer (ane/train_full.go:12-37)
   float* x2 = nullptr;
@@ -80,6 +167,8 @@ struct Act {  // saved activations of one layer (ane/train_full.go:12-37)
 
 __global__ void gather_windows_kernel(const uint16_t* __restrict__ tokens, const uint64_t* __restrict__ pos,
                                       uint16_t* __restrict__ in, uint16_t* __restrict__ tgt, int B, int seq) {
+  pdl_trigger();
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B * seq) return;
   const int b = i / seq, t = i - b * seq;
@@ -103,6 +192,8 @@ __global__ void export_tap_kernel(const TS* __restrict__ src, int ld, int col0, 
 
 // next-token targets inside each window for the evaluation loss: tgt[b,t] = tok[b,t+1], last = invalid.
 __global__ void shift_targets_kernel(const uint16_t* __restrict__ tok, uint16_t* __restrict__ tgt, int B, int seq) {
+  pdl_trigger();
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B * seq) return;
   const int t = i % seq;
@@ -117,6 +208,8 @@ __global__ void to_f32_kernel(const TS* __restrict__ src, float* __restrict__ ds
 }
 template <typename TD>
 __global__ void from_f32_kernel(const float* __restrict__ src, TD* __restrict__ dst, uint64_t n) {
+  pdl_trigger();
+  pdl_wait();
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (; i < n; i += stride) dst[i] = from_f<TD>(src[i]);
@@ -240,7 +333,7 @@ class EngineT final : public EngineBase {
   void cast_to_t(const float* src, T* dst, uint64_t n) {
     if constexpr (!kIsF32) {
       count_launch();
-      from_f32_kernel<T><<<ew_grid(n), 256, 0, stream_>>>(src, dst, n);
+      launch_pdl(from_f32_kernel<T>, dim3(ew_grid(n)), dim3(256), 0, stream_, src, dst, n);
     }
   }
   int layout_params();
@@ -248,7 +341,8 @@ class EngineT final : public EngineBase {
   int refresh_shadow();
   int forward(const uint16_t* d_tok, int B, int Tl, int pos0);
   int head_and_backward(int B);
-  int head_eval_loss(int B, double* loss_sum, uint64_t* n_pos);
+  int loss_pass(int nb);
+  int enqueue_loss(int nb);
   int backward_layers(int B);
   int do_flush();
   int check_device_status(int* out_status);
@@ -349,6 +443,12 @@ class EngineT final : public EngineBase {
   uint16_t *h_in_ = nullptr, *h_tgt_ = nullptr;  // pinned
   uint64_t *d_pos_ = nullptr, *h_pos_ = nullptr;
   float* h_loss_ = nullptr;  // pinned
+  float* h_rows_ = nullptr;  // pinned: per-position losses of an evaluation pass
+  struct LossGraph {
+    cudaGraphExec_t exec = nullptr;
+    int passes = 0, launches = 0;
+  };
+  std::vector<LossGraph> loss_graphs_;  // by number of windows
   uint64_t n_tokens_ = 0, rng_ = 0;
   // ---- state
   ane_state st_{};
@@ -402,6 +502,11 @@ void EngineT<T>::destroy() {
   if (h_tgt_) cudaFreeHost(h_tgt_);
   if (h_pos_) cudaFreeHost(h_pos_);
   if (h_loss_) cudaFreeHost(h_loss_);
+  if (h_rows_) cudaFreeHost(h_rows_);
+  h_rows_ = nullptr;
+  for (auto& g : loss_graphs_)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+  loss_graphs_.clear();
   if (h_logits_) cudaFreeHost(h_logits_);
   h_logits_ = nullptr;
   h_in_ = h_tgt_ = nullptr;
@@ -720,6 +825,7 @@ int EngineT<T>::open(const ane_options& opts, const uint16_t* tokens, uint64_t n
   if ((rc = cuda_check(cudaMallocHost(&h_tgt_, sizeof(uint16_t) * M_), "cudaMallocHost")) != 0) return rc;
   if ((rc = cuda_check(cudaMallocHost(&h_pos_, sizeof(uint64_t) * B_), "cudaMallocHost")) != 0) return rc;
   if ((rc = cuda_check(cudaMallocHost(&h_loss_, sizeof(float) * 4), "cudaMallocHost")) != 0) return rc;
+  if ((rc = cuda_check(cudaMallocHost(&h_rows_, sizeof(float) * M_), "cudaMallocHost")) != 0) return rc;
   if ((rc = cuda_check(cudaMallocHost(&h_logits_, sizeof(float) * (size_t)V_ * S_), "cudaMallocHost")) != 0) return rc;
   for (float* p : {P_, G_, Mo_, Vo_})
     if ((rc = cuda_check(cudaMemsetAsync(p, 0, sizeof(float) * n_params_, stream_), "memset")) != 0) return rc;
@@ -1565,7 +1671,7 @@ int EngineT<T>::step(const uint16_t* input, const uint16_t* target, uint32_t n_s
     st_.token_pos = h_pos_[B_ - 1] + (uint64_t)S_;
     cudaMemcpyAsync(d_pos_, h_pos_, sizeof(uint64_t) * B_, cudaMemcpyHostToDevice, stream_);
     count_launch();
-    gather_windows_kernel<<<(M_ + 255) / 256, 256, 0, stream_>>>(d_tokens_, d_pos_, d_in_, d_tgt_, B_, S_);
+    launch_pdl(gather_windows_kernel, dim3((M_ + 255) / 256), dim3(256), 0, stream_, d_tokens_, d_pos_, d_in_, d_tgt_, B_, S_);
   }
   overlap_reduce_ = dp_.active() && (int)micro_steps_ + 1 >= o_.accum_steps;
   reduced_lo_ = r_mat1_;
@@ -1620,6 +1726,7 @@ int EngineT<T>::eval_logits(const uint16_t* tokens, uint32_t n_seq, float* out, 
   if ((rc = cuda_check(cudaSetDevice(o_.device), "cudaSetDevice")) != 0) return rc;
   const uint64_t per_seq = (uint64_t)V_ * S_;
   if (cap < per_seq * n_seq) return fail(ANE_ERR_ARG, "storiesane eval logits: output buffer too small");
+  LogitsCopy copy(out, per_seq, n_seq, h_logits_, ev_logits_);
   for (uint32_t s0 = 0; s0 < n_seq; s0 += (uint32_t)B_) {
     const int nb = (int)std::min<uint32_t>((uint32_t)B_, n_seq - s0);
     const int M = nb * S_;
@@ -1642,70 +1749,19 @@ int EngineT<T>::eval_logits(const uint16_t* tokens, uint32_t n_seq, float* out, 
         count_launch();
         softcap_inplace(logits_, per_seq, stream_);
       }
-      // device -> pinned staging (full PCIe rate) -> caller's buffer, in pieces: the host copies piece i
-      // out of the staging buffer while pieces i+1.. are still crossing PCIe.  One core copies ~10 GB/s, a
-      // fifth of the PCIe rate (32.8 MB cross in 0.6-0.7 ms), so the pieces are dealt to several threads
-      // (ANE_B200_EVAL_COPY_THREADS; default: the host's cores, at most 16) - measured per call with 2 / 4 / 8 /
-      // 12 / 16 threads: 2.54 / 2.10 / 1.99 / 1.91 / 1.75 ms, of which 0.83 ms is the forward pass.
       float* dst = out + (size_t)(s0 + b) * per_seq;
-      {
-        // A page-locked destination (ane_host_malloc, or memory the caller registered) takes the copy directly.
-        cudaPointerAttributes pa;
-        if (cudaPointerGetAttributes(&pa, dst) == cudaSuccess && pa.type == cudaMemoryTypeHost) {
-          if ((rc = cuda_check(cudaMemcpyAsync(dst, logits_, sizeof(float) * per_seq, cudaMemcpyDeviceToHost, stream_),
-                               "logits download")) != 0)
-            return rc;
-          if ((rc = cuda_check(cudaStreamSynchronize(stream_), "logits sync")) != 0) return rc;
-          continue;
-        }
-        cudaGetLastError();  // an ordinary pointer may leave an error code behind on older drivers
-      }
-      static const int kPieces = [] {
-        const char* e = getenv("ANE_B200_EVAL_PIECES");
-        const int v = e ? atoi(e) : 32;
-        return v < 1 ? 1 : (v > 64 ? 64 : v);
-      }();
-      const uint64_t piece = (per_seq + kPieces - 1) / kPieces;
-      int n_pieces = 0;
-      for (int pi = 0; pi < kPieces; ++pi) {
-        const uint64_t off = (uint64_t)pi * piece;
-        if (off >= per_seq) break;
-        const uint64_t n = std::min(piece, per_seq - off);
-        if ((rc = cuda_check(cudaMemcpyAsync(h_logits_ + off, logits_ + off, sizeof(float) * n, cudaMemcpyDeviceToHost,
-                                             stream_), "logits download")) != 0)
+      // A page-locked destination (ane_host_malloc, or memory the caller registered) takes the copy directly.
+      cudaPointerAttributes pa;
+      if (cudaPointerGetAttributes(&pa, dst) == cudaSuccess && pa.type == cudaMemoryTypeHost) {
+        if ((rc = cuda_check(cudaMemcpyAsync(dst, logits_, sizeof(float) * per_seq, cudaMemcpyDeviceToHost, stream_),
+                             "logits download")) != 0)
           return rc;
-        cudaEventRecord(ev_logits_[pi], stream_);
-        ++n_pieces;
+        if ((rc = cuda_check(cudaStreamSynchronize(stream_), "logits sync")) != 0) return rc;
+        continue;
       }
-      static const int copy_threads = [] {
-        const char* e = getenv("ANE_B200_EVAL_COPY_THREADS");
-        const unsigned hw = std::thread::hardware_concurrency();
-        const int v = e ? atoi(e) : (hw == 0 ? 4 : (int)hw);
-        return v < 1 ? 1 : (v > 16 ? 16 : v);
-      }();
-      // small outputs (under 1 MiB) are not worth a thread start
-      const int use_threads = per_seq * sizeof(float) < (1u << 20) ? 1 : copy_threads;
-      std::atomic<int> copy_err{0};
-      auto copy_share = [&](int t) {  // pieces t, t + threads, ...: every thread's last piece is a late one
-        if (t > 0 && cudaSetDevice(o_.device) != cudaSuccess) {
-          copy_err.store(1);
-          return;
-        }
-        for (int pi = t; pi < n_pieces; pi += use_threads) {
-          const uint64_t off = (uint64_t)pi * piece;
-          const uint64_t n = std::min(piece, per_seq - off);
-          if (cudaEventSynchronize(ev_logits_[pi]) != cudaSuccess) {
-            copy_err.store(1);
-            return;
-          }
-          memcpy(dst + off, h_logits_ + off, sizeof(float) * n);
-        }
-      };
-      std::vector<std::thread> helpers;
-      for (int t = 1; t < use_threads && t < n_pieces; ++t) helpers.emplace_back(copy_share, t);
-      copy_share(0);
-      for (auto& h : helpers) h.join();
-      if (copy_err.load() != 0) return cuda_check(cudaErrorUnknown, "logits sync");
+      cudaGetLastError();  // an ordinary pointer may leave an error code behind on older drivers
+      const cudaError_t e = copy.window(s0 + (uint32_t)b, logits_, stream_);
+      if (e != cudaSuccess) return cuda_check(e, "logits download");
     }
   }
   return check_device_status(nullptr);
@@ -1722,9 +1778,62 @@ int EngineT<T>::eval_loss(const uint16_t* tokens, uint32_t n_seq, double* loss_s
     const int nb = (int)std::min<uint32_t>((uint32_t)B_, n_seq - s0);
     const int M = nb * S_;
     memcpy(h_in_, tokens + (size_t)s0 * S_, sizeof(uint16_t) * M);
+    if ((rc = loss_pass(nb)) != 0) return rc;
+    if ((rc = cuda_check(cudaStreamSynchronize(stream_), "eval loss sync")) != 0) return rc;
+    for (int i = 0; i < M; ++i) {
+      const int t = i % S_;
+      if (t + 1 >= S_) continue;
+      if (h_in_[i + 1] >= V_) continue;
+      total += (double)h_rows_[i];
+      count++;
+    }
+  }
+  if (loss_sum) *loss_sum = total;
+  if (n_pos) *n_pos = count;
+  return check_device_status(nullptr);
+}
+
+// Enqueues the loss of nb windows in h_in_ -> h_rows_.  The pass is 45 to 110 short kernels at fixed addresses; issuing them
+// costs 4 us each, more than a small model's kernels take (217 of 280 us for one window of 100 tokens at dim 288), so from
+// the second pass over the same number of windows on it is replayed from a CUDA graph.
+template <typename T>
+int EngineT<T>::loss_pass(int nb) {
+  int rc;
+  const bool graphs = !profiling_ && !dp_.active();
+  if (graphs && (int)loss_graphs_.size() <= nb) loss_graphs_.resize((size_t)nb + 1);
+  if (graphs && loss_graphs_[nb].exec) {
+    count_launch(loss_graphs_[nb].launches);
+    last_B_ = nb;
+    return cuda_check(cudaGraphLaunch(loss_graphs_[nb].exec, stream_), "eval loss graph");
+  }
+  if (!graphs || loss_graphs_[nb].passes++ != 1) return enqueue_loss(nb);
+  const uint64_t before = launches();
+  if (cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+    cudaGetLastError();
+    return enqueue_loss(nb);
+  }
+  rc = enqueue_loss(nb);
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  const bool ok = cudaStreamEndCapture(stream_, &graph) == cudaSuccess && rc == 0 && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+  if (graph) cudaGraphDestroy(graph);
+  if (!ok) {  // eager from now on
+    cudaGetLastError();
+    return enqueue_loss(nb);
+  }
+  loss_graphs_[nb].exec = exec;
+  loss_graphs_[nb].launches = (int)(launches() - before);
+  return cuda_check(cudaGraphLaunch(exec, stream_), "eval loss graph");
+}
+
+template <typename T>
+int EngineT<T>::enqueue_loss(int nb) {
+  int rc;
+  const int M = nb * S_;
+  {
     cudaMemcpyAsync(d_in_, h_in_, sizeof(uint16_t) * M, cudaMemcpyHostToDevice, stream_);
     count_launch();
-    shift_targets_kernel<<<(M + 255) / 256, 256, 0, stream_>>>(d_in_, d_tgt_, nb, S_);
+    launch_pdl(shift_targets_kernel, dim3((M + 255) / 256), dim3(256), 0, stream_, d_in_, d_tgt_, nb, S_);
     if ((rc = forward(d_in_, nb, S_, 0)) != 0) return rc;
     cudaMemsetAsync(loss_rows_, 0, sizeof(float) * M, stream_);
     bool fused_done = false;
@@ -1754,22 +1863,10 @@ int EngineT<T>::eval_loss(const uint16_t* tokens, uint32_t n_seq, double* loss_s
       count_launch();
       cross_entropy_rows<T>(logits_, d_tgt_, d_one_ - 0, (T*)nullptr, loss_rows_, rows, r0, M + 1, V_, isN_, 0.f, stream_);
     }
-    std::vector<float> rows_host(M);
-    if ((rc = cuda_check(cudaMemcpyAsync(rows_host.data(), loss_rows_, sizeof(float) * M, cudaMemcpyDeviceToHost, stream_),
-                         "loss rows")) != 0)
+    if ((rc = cuda_check(cudaMemcpyAsync(h_rows_, loss_rows_, sizeof(float) * M, cudaMemcpyDeviceToHost, stream_), "loss rows")) != 0)
       return rc;
-    if ((rc = cuda_check(cudaStreamSynchronize(stream_), "eval loss sync")) != 0) return rc;
-    for (int i = 0; i < M; ++i) {
-      const int t = i % S_;
-      if (t + 1 >= S_) continue;
-      if (h_in_[i + 1] >= V_) continue;
-      total += (double)rows_host[i];
-      count++;
-    }
   }
-  if (loss_sum) *loss_sum = total;
-  if (n_pos) *n_pos = count;
-  return check_device_status(nullptr);
+  return 0;
 }
 
 // ------------------------------------------------------------------------------------------------

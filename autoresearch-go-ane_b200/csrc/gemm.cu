@@ -7,10 +7,9 @@
 #include <string.h>
 
 #include <algorithm>
-#include <map>
 #include <mutex>
 #include <string>
-#include <tuple>
+#include <vector>
 
 #include "gemm_tc.cuh"
 
@@ -67,17 +66,35 @@ static EncodeTiledFn get_encode_fn() {
 // 2-D tensor [outer, inner] with row pitch ld (elements); box = [box_outer, box_inner]; 128B swizzle.
 static bool make_tmap(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld,
                       uint32_t box_inner, uint32_t box_outer, bool is_f32 = false) {
-  typedef std::tuple<int, const void*, uint64_t, uint64_t, uint64_t, uint32_t, uint32_t, bool> Key;
-  static std::map<Key, CUtensorMap> cache;
-  static std::mutex mu;
+  // Encoding takes about a microsecond and a step asks for some 700 maps of buffers that never move: a small direct-mapped
+  // cache per thread (no lock; a shared std::map behind a mutex cost several tenths of a microsecond per map).
+  struct Key {
+    const void* ptr;
+    uint64_t inner, outer, ld;
+    uint32_t box_inner, box_outer;
+    int dev, f32;
+    bool operator==(const Key& o) const {
+      return ptr == o.ptr && inner == o.inner && outer == o.outer && ld == o.ld && box_inner == o.box_inner && box_outer == o.box_outer &&
+             dev == o.dev && f32 == o.f32;
+    }
+  };
+  struct Entry {
+    CUtensorMap tm;
+    Key key;
+  };
+  constexpr size_t kEntries = 2048;
+  static thread_local std::vector<Entry> cache;
+  if (cache.empty()) cache.resize(kEntries);  // zero keys match no call: a null pointer is refused below
   int dev = 0;
   cudaGetDevice(&dev);
-  Key key(dev, ptr, inner, outer, ld, box_inner, box_outer, is_f32);
+  const Key key{ptr, inner, outer, ld, box_inner, box_outer, dev, is_f32 ? 1 : 0};
+  uint64_t h = reinterpret_cast<uintptr_t>(ptr) >> 4;
+  for (uint64_t v : {inner, outer, ld, (uint64_t)box_inner << 32 | box_outer, (uint64_t)dev << 1 | (uint64_t)key.f32})
+    h = (h ^ v) * 0x9E3779B97F4A7C15ull;
+  Entry& entry = cache[(h >> 40) % kEntries];
   const uint64_t esz = is_f32 ? 4 : 2;
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find(key);
-  if (it != cache.end()) {
-    *out = it->second;
+  if (ptr != nullptr && entry.key == key) {
+    *out = entry.tm;
     return true;
   }
   EncodeTiledFn fn = get_encode_fn();
@@ -85,7 +102,7 @@ static bool make_tmap(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_
     g_gemm_err = "cuTensorMapEncodeTiled entry point not available";
     return false;
   }
-  if ((reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || (ld * esz) % 16 != 0) {
+  if (ptr == nullptr || (reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || (ld * esz) % 16 != 0) {
     g_gemm_err = "TMA operand must be 16-byte aligned with a 16-byte multiple row pitch";
     return false;
   }
@@ -104,7 +121,8 @@ static bool make_tmap(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_
     g_gemm_err = buf;
     return false;
   }
-  cache[key] = tm;
+  entry.tm = tm;
+  entry.key = key;
   *out = tm;
   return true;
 }
@@ -685,6 +703,8 @@ struct SplitOperand {
   int rows, cols, kp, pitch, k_major, vec;  // vec: float4 reads are aligned
 };
 __global__ void split_operands_kernel(const SplitOperand a, const SplitOperand b) {
+  pdl_trigger();
+  pdl_wait();
   const SplitOperand& o = blockIdx.y == 0 ? a : b;
   const int out_rows = o.k_major ? o.rows : o.kp, out_cols = o.k_major ? o.kp : o.pitch, per = out_cols / 4;
   const size_t lo = o.k_major ? (size_t)o.kp : (size_t)o.kp * o.pitch;
@@ -727,8 +747,8 @@ void SplitScratch::release() {
   }
 }
 
-// The three products run as one: its contraction is three passes of kp over (hi, hi), (hi, lo) and (lo, hi), so the
-// accumulators stay in tensor memory between them.  (Three launches, the second and third adding to C in memory, and
+// The three products run as one: its contraction is three passes of kp over (hi, lo), (lo, hi) and (hi, hi), so the
+// accumulators stay in tensor memory between them; the small cross terms come first, while the accumulators are small too.  (Three launches, the second and third adding to C in memory, and
 // two scalar conversion launches before them took 9.8 us each for 512 token rows.)
 int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t stream) {
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return 0;
@@ -770,7 +790,7 @@ int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t
   const long long most = std::max((long long)(o[0].k_major ? o[0].rows : kp) * (o[0].k_major ? kp : o[0].pitch),
                                   (long long)(o[1].k_major ? o[1].rows : kp) * (o[1].k_major ? kp : o[1].pitch));
   const unsigned blocks = (unsigned)std::min<long long>(148 * 8, (most / 4 + 255) / 256);
-  split_operands_kernel<<<dim3(blocks, 2), 256, 0, stream>>>(o[0], o[1]);
+  launch_pdl(split_operands_kernel, dim3(blocks, 2), dim3(256), 0, stream, o[0], o[1]);
   if (cudaGetLastError() != cudaSuccess) {
     g_gemm_err = "split-precision GEMM: operand split launch failed";
     return -4;

@@ -195,7 +195,7 @@ struct EpiParams {
   int ce_rows;           // row count of the statistics buffer
   int ce_col0;           // vocabulary column of this product's column 0
   int ce_softcap;        // z = 15 tanh(logit / 15) (ane/common.go:272-287)
-  int seg_kb;            // > 0: operands are (hi | lo) halves of seg_kb k-blocks each, three passes hi*hi, hi*lo, lo*hi
+  int seg_kb;            // > 0: operands are (hi | lo) halves of seg_kb k-blocks each, three passes hi*lo, lo*hi, hi*hi
 };
 
 // Several accumulating products with one contraction length, run by one launch (the four weight gradients of a
@@ -401,8 +401,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           int ka = kb * BK, kb_ = ka;  // first k of this block in A and B
           if (epi.seg_kb > 0) {
             const int pass = kb / epi.seg_kb, in_pass = kb - pass * epi.seg_kb;
-            ka = (in_pass + (pass == 2 ? epi.seg_kb : 0)) * BK;
-            kb_ = (in_pass + (pass == 1 ? epi.seg_kb : 0)) * BK;
+            ka = (in_pass + (pass == 1 ? epi.seg_kb : 0)) * BK;
+            kb_ = (in_pass + (pass == 0 ? epi.seg_kb : 0)) * BK;
           }
           if constexpr (PAIR) {
             // both CTAs' bytes complete on the leader's barrier, which expects the sum

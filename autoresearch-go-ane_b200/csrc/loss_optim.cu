@@ -433,22 +433,34 @@ template void cross_entropy_rows<bf16>(const float*, const uint16_t*, const floa
 // (log2 domain) combine to the row's log2-sum-exp; the loss of the row follows from its target logit
 // (ane/stories/cpu.go:212-292: -log(max(p[target], 1e-10)); rows whose target lies outside the vocabulary
 // count nothing and get a zero gradient row), and coef = grad_scale * inv_valid[sequence] is what pass 2
-// multiplies (softmax - onehot) by.  One thread per row; stats is [n_tiles][rows].
-__global__ void ce_merge_stats_kernel(const float2* __restrict__ stats, int n_tiles, int rows, const float* __restrict__ tgt_logit,
-                                      const uint16_t* __restrict__ targets, const float* __restrict__ inv_valid, int seq, int V,
-                                      int softcap, float grad_scale, float* __restrict__ lse2, float* __restrict__ coef,
-                                      float* __restrict__ loss_rows) {
+// multiplies (softmax - onehot) by.  stats is [n_tiles][rows]; 32 rows per block, eight warps share the tiles of a row (one
+// thread per row is a chain of n_tiles exponentials: 21 us for 125 tiles whatever the rows).
+__global__ void __launch_bounds__(256)
+ce_merge_stats_kernel(const float2* __restrict__ stats, int n_tiles, int rows, const float* __restrict__ tgt_logit,
+                      const uint16_t* __restrict__ targets, const float* __restrict__ inv_valid, int seq, int V,
+                      int softcap, float grad_scale, float* __restrict__ lse2, float* __restrict__ coef,
+                      float* __restrict__ loss_rows) {
   pdl_trigger();
   pdl_wait();
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
+  __shared__ float2 s_part[8][32];
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+  const int r = blockIdx.x * 32 + lane;
   float m = -INFINITY, s = 0.f;
-  for (int t = 0; t < n_tiles; ++t) {
-    const float2 v = stats[(size_t)t * rows + r];
+  auto merge = [&](float2 v) {
     const float mn = fmaxf(m, v.x);
+    if (mn == -INFINITY) return;
     s = s * exp2f(m - mn) + v.y * exp2f(v.x - mn);
     m = mn;
+  };
+  if (r < rows) {
+#pragma unroll 4
+    for (int t = part; t < n_tiles; t += 8) merge(stats[(size_t)t * rows + r]);
   }
+  s_part[part][lane] = make_float2(m, s);
+  __syncthreads();
+  if (part != 0 || r >= rows) return;
+#pragma unroll
+  for (int p = 1; p < 8; ++p) merge(s_part[p][lane]);
   const float l2 = m + log2f(s);
   lse2[r] = l2;
   const int tgt = targets[r];
@@ -468,7 +480,7 @@ void ce_merge_stats(const float* stats, int n_tiles, int rows, const float* tgt_
                     const float* inv_valid, int seq, int V, bool softcap, float grad_scale, float* lse2, float* coef,
                     float* loss_rows, cudaStream_t s) {
   if (rows <= 0) return;
-  launch_pdl(ce_merge_stats_kernel, dim3((rows + 127) / 128), dim3(128), 0, s, reinterpret_cast<const float2*>(stats), n_tiles,
+  launch_pdl(ce_merge_stats_kernel, dim3((rows + 31) / 32), dim3(256), 0, s, reinterpret_cast<const float2*>(stats), n_tiles,
              rows, tgt_logit, targets, inv_valid, seq, V, softcap ? 1 : 0, grad_scale, lse2, coef, loss_rows);
 }
 

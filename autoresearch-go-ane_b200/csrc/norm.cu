@@ -219,6 +219,8 @@ __global__ void rmsnorm_backward_kernel(const float* __restrict__ dy, const floa
                                         const float* __restrict__ res, const float* __restrict__ res_scale,
                                         float* __restrict__ dx_f32, T* __restrict__ dx_t, float* __restrict__ dw,
                                         int M, int D) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ float s_dw[];  // [D] when dw != nullptr
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -405,7 +407,7 @@ void rmsnorm_backward(const float* dy, const float* x, const float* w, const flo
   if (dw && blocks > 148 * 2) blocks = 148 * 2;  // bound the number of global atomic passes
   const size_t smem = dw ? sizeof(float) * (size_t)D : 0;
   // dx_t may alias dx_f32 only when T == float; callers pass nullptr instead.
-  rmsnorm_backward_kernel<T><<<blocks, kWarpsPerBlock * 32, smem, s>>>(dy, x, w, rstd, res, res_scale, dx_f32, dx_t,
+  launch_pdl(rmsnorm_backward_kernel<T>, dim3(blocks), dim3(kWarpsPerBlock * 32), smem, s, dy, x, w, rstd, res, res_scale, dx_f32, dx_t,
                                                                          dw, M, D);
 }
 template void rmsnorm_backward<float>(const float*, const float*, const float*, const float*, const float*,
