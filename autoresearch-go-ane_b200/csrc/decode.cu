@@ -449,6 +449,26 @@ __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16*
     const bf16* kb = kc + (size_t)b * a.S * kvd + (size_t)kvh * a.hd;
     const bf16* vb = vc + (size_t)b * a.S * kvd + (size_t)kvh * a.hd;
     const uint2* wk = nullptr;  // words of the new key
+    // 16 bytes of a key's or value's dims d..d+7 from the cache (R8 = 1: all but the newest, which put_new() adds).  The
+    // registers of a tile are requested again as soon as its MMAs have read them: keys load under the softmax and P * V,
+    // values under the next scores; the first tiles (the cache does not depend on q) before q is there.
+    const int cached = R8 == 1 ? pos : pos + 1;
+    uint4 kr[2][2 * PANELS], vr[4][PANELS];
+    auto fetch = [&](const bf16* base, int j, int d) { return ld_l2_if(base + (size_t)j * kvd + d, d < a.hd && j < cached); };
+    auto load_k = [&](int j0) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int i = 0; i < 2 * PANELS; ++i) kr[t][i] = fetch(kb, j0 + t * 8 + g, i * 32 + c * 8);
+    };
+    auto load_v = [&](int j0) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int p = 0; p < PANELS; ++p) vr[t][p] = fetch(vb, j0 + 2 * c + (t & 1) + (t >> 1) * 8, p * 64 + g * 8);
+    };
+    load_k(warp * 16);
+    load_v(warp * 16);
     uint4 q[PANELS][2];
     if constexpr (R8 == 1) {
       const uint2* row = a.w_qkv + (size_t)b * ((qd + 2 * kvd) / 2);
@@ -482,9 +502,6 @@ __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16*
         q[i >> 1][i & 1] = ld_l2_if(a.q + (size_t)b * qd + (size_t)(h0 + g) * a.hd + d, g < G && d < a.hd);
       }
     }
-    // 16 bytes of a key's or value's dims d..d+7 from the cache (R8 = 1: all but the newest, which put_new() adds)
-    const int cached = R8 == 1 ? pos : pos + 1;
-    auto fetch = [&](const bf16* base, int j, int d) { return ld_l2_if(base + (size_t)j * kvd + d, d < a.hd && j < cached); };
     auto put_new = [&](uint4& v, int off, int j, int d) {
       if (R8 == 1 && j == pos && d < a.hd) {
         const uint4 x = get_words(wk + (off + d) / 2), y = get_words(wk + (off + d) / 2 + 2);
@@ -494,15 +511,6 @@ __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16*
     float m = -INFINITY, l = 0.f, acc[PANELS][8][2] = {};
 #pragma unroll 1
     for (int j0 = warp * 16; j0 <= pos; j0 += kWarps * 16) {
-      uint4 kr[2][2 * PANELS], vr[4][PANELS];
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int i = 0; i < 2 * PANELS; ++i) kr[t][i] = fetch(kb, j0 + t * 8 + g, i * 32 + c * 8);
-#pragma unroll
-      for (int t = 0; t < 4; ++t)
-#pragma unroll
-        for (int p = 0; p < PANELS; ++p) vr[t][p] = fetch(vb, j0 + 2 * c + (t & 1) + (t >> 1) * 8, p * 64 + g * 8);
       if (R8 == 1 && j0 + 16 > pos) {  // this warp holds the newest key
 #pragma unroll
         for (int t = 0; t < 2; ++t)
@@ -522,6 +530,10 @@ __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16*
           mma16816_top(s[t][0], s[t][1], x.x, x.y, k.x, k.y);
           mma16816_top(s[t][0], s[t][1], x.z, x.w, k.z, k.w);
         }
+      }
+      load_k(j0 + kWarps * 16);
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           s[t][e] = j0 + t * 8 + 2 * c + e <= pos ? s[t][e] * sc : -INFINITY;
@@ -561,6 +573,7 @@ __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16*
           mma16816_top(acc[p][j][0], acc[p][j][1], lo[0], lo[1], b0, b1);
         }
       }
+      load_v(j0 + kWarps * 16);
     }
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
@@ -700,6 +713,20 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
       const Prod& p = s_prod[kind];
       const uint32_t epoch = (uint32_t)(step * a.L + l + 1);
       const bool direct = kind == kWo || kind == kW2;
+      if (R8 > 1 && kind == kQkv) {
+        // The cached keys and values that this CTA will attend to, from DRAM into L2 while q|k|v are computed: 164 KB per
+        // item at 640 positions, more than all of it fits at once, and the attention's own loads are a chain of a few.
+        const int group_heads = a.group, hgroups = a.H / group_heads, row_bytes = a.hd * 2, lines = (row_bytes + 127) / 128;
+        for (int item = blockIdx.x; item < a.B * hgroups; item += gridDim.x) {
+          const int b = item / hgroups, kvh = (item - b * hgroups) * group_heads / (a.H / a.KV);
+          const size_t base = (size_t)l * a.kv_layer + (size_t)b * a.S * KVD + (size_t)kvh * a.hd;
+          for (int i = threadIdx.x; i < 2 * pos * lines; i += kThreads) {
+            const int j = i / (2 * lines), part = i - j * 2 * lines;
+            const bf16* from = (part < lines ? a.kcache : a.vcache) + base + (size_t)j * KVD + (part % lines) * 64;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(from));
+          }
+        }
+      }
       Source src{nullptr, nullptr, nullptr, a.B, epoch};
       float2 old = make_float2(0.f, 0.f);  // residual of this thread's first pair
       const float* xrow = kind == kWo && l == 0 ? a.p + a.off_embed_f32 + (size_t)s_tok[live ? row : 0] * D : a.x + (size_t)row * D;
