@@ -362,8 +362,6 @@ class EngineT final : public EngineBase {
   bool decoding_ = false;  // forward() runs one KV-cached decode step
   std::vector<T*> kcache_, vcache_;  // [B, S_, KV*hd] per layer (one block each for all layers), allocated by the first decode
   // scratch of the persistent decode kernel (bf16 engines)
-  float* dec_x_ = nullptr;
-  bf16 *dec_q_ = nullptr, *dec_att_ = nullptr, *dec_gate_ = nullptr;
   unsigned long long* dec_best_ = nullptr;
   double* dec_psum_ = nullptr;
   unsigned* dec_bar_ = nullptr;
@@ -1912,10 +1910,9 @@ int EngineT<T>::decode(const uint16_t* prompts, uint32_t n_seq, uint32_t prompt_
     }
     if constexpr (!kIsF32) {
       const size_t rows = std::min(B_, 32);  // the persistent kernel takes up to 32 sequences at a time
-      if ((rc = dalloc(&dec_x_, rows * D_)) != 0 || (rc = dalloc(&dec_q_, rows * QD_)) != 0 || (rc = dalloc(&dec_att_, rows * QD_)) != 0 ||
-          (rc = dalloc(&dec_gate_, rows * Hd_)) != 0 || (rc = dalloc(&dec_best_, 3 * rows)) != 0 ||
+      if ((rc = dalloc(&dec_best_, 3 * rows)) != 0 ||
           (rc = dalloc(&dec_psum_, rows * gemm_num_sms())) != 0 || (rc = dalloc(&dec_bar_, 1)) != 0 ||
-          (rc = dalloc(&dec_words_, decode_words_bytes(D_, Hd_, H_, KV_, hd_))) != 0)
+          (rc = dalloc(&dec_words_, decode_words_bytes(D_, Hd_, H_, KV_, hd_, (int)rows, gemm_num_sms()))) != 0)
         return rc;
     }
     if ((rc = dalloc(&d_argmax_, B_)) != 0) return rc;
@@ -1963,7 +1960,6 @@ int EngineT<T>::decode(const uint16_t* prompts, uint32_t n_seq, uint32_t prompt_
         a.cosb = rope_cos_; a.sinb = rope_sin_;
         a.kcache = kcache_[0] + (size_t)b0 * S_ * KVD_; a.vcache = vcache_[0] + (size_t)b0 * S_ * KVD_;
         a.kv_layer = (size_t)B_ * S_ * KVD_;
-        a.x = dec_x_; a.q = dec_q_; a.att = dec_att_; a.gate = dec_gate_;
         a.logits = logits_; a.best = dec_best_; a.psum = dec_psum_;
         a.u = d_dec_u_ + b0; a.u_stride = B;
         a.tok = d_dec_tok_ + b0; a.out = d_dec_out_ + (size_t)b0 * n_new;

@@ -132,6 +132,23 @@ bool make_tmap_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t ou
   return make_tmap(out, ptr, inner, outer, ld, box_inner, box_outer, is_f32);
 }
 
+// [layer][row][column] bf16 matrices, dense rows, `layer_stride` elements apart; boxes of box_rows x box_inner, not swizzled.
+bool make_tmap_weights(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t rows, uint64_t layers, uint64_t layer_stride,
+                       uint32_t box_inner, uint32_t box_rows) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) {
+    g_gemm_err = "cuTensorMapEncodeTiled entry point not available";
+    return false;
+  }
+  cuuint64_t gdim[3] = {inner, rows, layers}, gstride[2] = {inner * 2, (layers > 1 ? layer_stride : rows * inner) * 2};
+  cuuint32_t box[3] = {box_inner, box_rows, 1}, estr[3] = {1, 1, 1};
+  if (fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
+    return true;
+  g_gemm_err = "cuTensorMapEncodeTiled failed for a weight matrix";
+  return false;
+}
+
 template <int BN, int MT, bool A_MN, bool B_MN, int EPI>
 static int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& td,
                      const EpiParams& epi,

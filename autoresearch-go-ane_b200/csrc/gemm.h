@@ -109,6 +109,8 @@ size_t gemm_group_slot_bytes();
 int gemm_num_sms();
 // 2-D tensor map over a row-major [outer, inner] buffer (row pitch ld elements) of bf16 (or fp32) with a
 // 128B-swizzled [box_outer, box_inner] box; cached per (device, arguments).  False + gemm_last_error() on failure.
+bool make_tmap_weights(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t rows, uint64_t layers, uint64_t layer_stride,
+                       uint32_t box_inner, uint32_t box_rows);
 bool make_tmap_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner,
                   uint32_t box_outer, bool is_f32);
 const char* gemm_last_error();

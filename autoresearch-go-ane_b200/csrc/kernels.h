@@ -114,8 +114,6 @@ struct DecodeArgs {
   const float *cosb, *sinb;      // rotation tables [positions, hd / 2]
   bf16 *kcache, *vcache;         // [L][B, S, KV * hd] with kv_layer elements per layer
   size_t kv_layer;
-  float* x;                      // scratch: residual stream [B, D]
-  bf16 *q, *att, *gate;          // scratch: [B, H * hd], [B, H * hd], [B, Hd]
   float* logits;                 // scratch [B, V], written when sampling
   unsigned long long* best;      // scratch [3][B]
   double* psum;                  // scratch [CTAs][B]
@@ -125,13 +123,16 @@ struct DecodeArgs {
   int* status;
   float temperature;             // <= 1e-6: argmax
   int B, D, Hd, L, H, KV, hd, V, S, prompt, n_new, u_stride;
-  int group, stage_bytes, slot_bytes;  // set by decode_steps
+  int group, stage_bytes, slot_bytes, slots, units, units_w2;  // set by decode_steps
   unsigned hd_magic;
   uint2 *w_x0, *w_x1, *w_qkv, *w_att, *w_gate;
 };
 bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int batch, int sms);
-size_t decode_words_bytes(int D, int Hd, int H, int KV, int hd);  // size of `words`, scratch for exchanges between SMs
+size_t decode_words_bytes(int D, int Hd, int H, int KV, int hd, int batch, int sms);  // size of `words`, scratch for exchanges between SMs
 int decode_steps(DecodeArgs a, void* words, int sms, cudaStream_t s);
+// with clusters (called by the two above)
+bool decode_batch_supported(int D, int Hd, int hd, int batch, int sms);
+int decode_batch_steps(DecodeArgs a, int sms, cudaStream_t s);
 
 // Tensor-core causal attention (bf16 operands; head_dim 32, 48 or 64; see attention_tc.cu).
 bool attention_tc_supported(int hd);

@@ -157,3 +157,43 @@ def test_decode_sample_fp32_matches_oracle_full_recompute():
     with pytest.raises(ane.EngineError):
         e.decode_sample(prompts, n_new, temp, u[:, :2])
     e.close()
+
+
+@pytest.mark.parametrize("batch,dim,heads,kv,hidden,vocab,prompt,temp", [
+    (1, 128, 2, 1, 256, 512, 5, 0.0),       # one sequence; and the largest of its kernel
+    (8, 192, 4, 2, 256, 504, 40, 0.9),      # head size 48
+    (9, 128, 2, 1, 256, 512, 33, 0.0),      # smallest batch of the kernel for more, sixteen-row tile half empty
+    (16, 64, 1, 1, 64, 96, 130, 0.9),       # fewer units of work than clusters; more keys than one round of the warps
+    (17, 288, 6, 6, 768, 1000, 17, 0.0),    # contraction of 9 chunks: the last CTA of a cluster has none
+    (32, 200, 5, 5, 544, 512, 12, 0.9),     # head size 40, contraction not a multiple of 32
+    (32, 256, 2, 1, 2304, 512, 70, 0.0),    # head size 128; W2 in two boxes a row
+    (33, 1280, 20, 4, 1024, 512, 20, 0.0),  # a second pass with one sequence; a norm read in two pieces
+])
+def test_decode_bf16_kernels_match_own_full_forward(batch, dim, heads, kv, hidden, vocab, prompt, temp):
+    """Tokens of the persistent kernels against the engine's full forward over prompt + generated tokens.
+
+    Two chains of bf16 roundings of the same values differ in a logit by about 2^-8 sqrt(dim) std (an element of the
+    normalised row is 1, of the classifier std) times the root of some 8 roundings per layer that feed it; `tol` is six of
+    that.  Greedy: the token's logit is within tol of the best (a wrong value somewhere costs units).  Sampled: the draw
+    lies in the token's interval of the distribution, whose edges move by at most a factor e^(2 tol / T)."""
+    layers, new, std = 3, 12, 0.08
+    seq = (prompt + new + 63) // 64 * 64
+    cfg = dict(dim=dim, hidden=hidden, heads=heads, kv_heads=kv, layers=layers, vocab=vocab, seq=seq)
+    _, e = make_pair(ane, cfg, arch=O.ARCH_L, quirks=0, dtype=ane.DTYPE_BF16, batch=batch, std=std, debug_taps=False)
+    prompts = O.zipf_tokens(batch * prompt, vocab, 3).reshape(batch, prompt)
+    u = np.random.default_rng(5).random((new, batch))
+    got = e.decode_sample(prompts, new, temp, u) if temp > 0 else e.decode_greedy(prompts, new)
+    full = np.zeros((batch, seq), np.uint16)
+    full[:, :prompt], full[:, prompt:prompt + new] = prompts, got
+    tol = 6 * 2.0 ** -8 * np.sqrt(dim) * std * np.sqrt(8 * layers)
+    for b in range(batch):
+        logits = e.eval_logits(full[b])[0][:, prompt - 1:prompt + new - 1].astype(np.float64)
+        for step in range(new):
+            col, tok = logits[:, step], int(got[b, step])
+            if temp == 0:
+                assert col.max() - col[tok] <= tol, (b, step)
+            else:
+                p = np.exp((col - col.max()) / temp)
+                at, total = np.cumsum(p), p.sum()
+                slack = np.expm1(2 * tol / temp)
+                assert (at[tok] - p[tok]) / total - slack <= u[step, b] <= at[tok] / total + slack, (b, step)
