@@ -367,8 +367,8 @@ __global__ void __launch_bounds__(kLaunch, 1) decode_batch_kernel(const __grid_c
               if (live && (int)threadIdx.x < min(p.group, p.nu) * EL) old = residual(p.row0(threadIdx.x / EL) + 2 * (threadIdx.x & 3));  // of this thread's first pair
             } else {
               // Normalised rows, bf16(x * rms^-1 * gain), rounded like the training forward's.  A thread's part of a row stays
-              // in registers between the sum of squares and the conversion for dim <= 1024; wider rows are read twice.
-              constexpr int V = 8, Per = kThreads / BP, Seg = Per * 4 * V;
+              // in registers between the sum of squares and the conversion for dim <= 768; wider rows are read twice.
+              constexpr int V = 6, Per = kThreads / BP, Seg = Per * 4 * V;
               const int r = threadIdx.x / Per, sub = threadIdx.x % Per, nseg = max(1, (p.kn + Seg - 1) / Seg);
               const bool has = r < a.B;
               const bool embed = kind == kQkv && l == 0;

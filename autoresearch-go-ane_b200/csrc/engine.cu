@@ -66,20 +66,27 @@ class LogitsCopy {
  public:
   LogitsCopy(float* out, uint64_t per_window, uint32_t windows, float* staging, cudaEvent_t* events)
       : out_(out), n_(per_window), staging_(staging), events_(events), order_(windows) {
-    static const int want = [] {
+    // An output above 32 MiB (malloc's largest threshold) is memory fresh from the kernel, in huge pages where its owner asks
+    // for them: helpers that copy neighbouring 64 KiB wait for the first touch of the same page, so they take 2 MiB each
+    // (65 MB: 4.5 -> 3.1-3.6 ms; three windows of 33 MB: 7.9 -> 6.4).  Smaller outputs are mostly warm, and the last
+    // piece is over sooner in small blocks (1.53 ms against 1.67 at 32.8 MB).
+    const bool fresh = per_window * windows * sizeof(float) > (32u << 20);
+    block_ = fresh ? 524288 : 16384;
+    static const int pieces = [] {
       const char* e = getenv("ANE_B200_EVAL_PIECES");
-      const int v = e ? atoi(e) : 16;
-      return v < 1 ? 1 : (v > 64 ? 64 : v);
+      const int v = e ? atoi(e) : 0;
+      return v > 64 ? 64 : v;
     }();
+    const int want = pieces > 0 ? pieces : fresh ? 32 : 16;
     static const int cores = [] {
       const char* e = getenv("ANE_B200_EVAL_COPY_THREADS");
       const unsigned hw = std::thread::hardware_concurrency();
       const int v = e ? atoi(e) : (hw == 0 ? 4 : (int)hw);
       return v < 1 ? 1 : (v > 16 ? 16 : v);
     }();
-    piece_ = ((n_ + want - 1) / want + kBlock - 1) / kBlock * kBlock;  // whole blocks
+    piece_ = ((n_ + want - 1) / want + block_ - 1) / block_ * block_;  // whole blocks
     pieces_ = (int)((n_ + piece_ - 1) / piece_);
-    blocks_ = (int)((n_ + kBlock - 1) / kBlock);
+    blocks_ = (int)((n_ + block_ - 1) / block_);
     helpers_wanted_ = n_ * sizeof(float) < (1u << 20) ? 0 : std::min(cores - 1, blocks_);  // under 1 MiB: not worth a thread start
   }
   ~LogitsCopy() {
@@ -111,13 +118,12 @@ class LogitsCopy {
   }
 
  private:
-  static constexpr uint64_t kBlock = 16384;  // floats
   void copy_block(uint32_t w, int k) {
-    const uint64_t off = (uint64_t)k * kBlock, n = std::min(kBlock, n_ - off);
+    const uint64_t off = (uint64_t)k * block_, n = std::min(block_, n_ - off);
     memcpy(out_ + (size_t)w * n_ + off, staging_ + off, sizeof(float) * n);
   }
   void helper() {  // blocks are numbered through all windows of the call
-    const int per_piece = (int)(piece_ / kBlock);
+    const int per_piece = (int)(piece_ / block_);
     for (;;) {
       const long long id = next_.fetch_add(1), round = id / blocks_;
       const int k = (int)(id - round * blocks_);
@@ -132,7 +138,7 @@ class LogitsCopy {
     }
   }
   float* out_;
-  uint64_t n_, piece_ = 0;
+  uint64_t n_, block_ = 16384, piece_ = 0;  // floats
   float* staging_;
   cudaEvent_t* events_;
   int pieces_ = 0, blocks_ = 0, helpers_wanted_ = 0;
