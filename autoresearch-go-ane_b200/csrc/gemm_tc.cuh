@@ -400,7 +400,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const uint32_t sb = smem_b0 + stage * Cfg::B_BYTES;
           int ka = kb * BK, kb_ = ka;  // first k of this block in A and B
           if (epi.seg_kb > 0) {
-            const int pass = kb / epi.seg_kb, in_pass = kb - pass * epi.seg_kb;
+            // (two compares; the other products only test seg_kb)
+            const int pass = (kb >= epi.seg_kb) + (kb >= 2 * epi.seg_kb), in_pass = kb - pass * epi.seg_kb;
             ka = (in_pass + (pass == 1 ? epi.seg_kb : 0)) * BK;
             kb_ = (in_pass + (pass == 0 ? epi.seg_kb : 0)) * BK;
           }
