@@ -746,7 +746,8 @@ void dot_accumulate(const float* a, const float* b, uint64_t n, float alpha, flo
 }
 
 // The three reductions / updates that both residuals of a layer contribute to the lambda gradients and the x0 gradient,
-// (ane/train_full.go:733-782; products rounded to fp32, summed in double) in one pass over seven tensors (one pass per residual read ten: 21 us each at 8192 x 768, at the memory's rate).
+// (ane/train_full.go:733-782; products rounded to fp32, summed in double) in one pass over seven tensors (one pass per
+// residual read ten: 21 us each at 8192 x 768, at the memory's rate).
 __global__ void __launch_bounds__(256)
 lambda_grads_kernel(const float4* __restrict__ d1, const float4* __restrict__ a1, const float4* __restrict__ d2,
                     const float4* __restrict__ a2, const float4* __restrict__ b, float4* __restrict__ y, int assign,
