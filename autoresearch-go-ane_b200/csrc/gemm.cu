@@ -514,9 +514,13 @@ static int resident_clusters(int size) {
 // exchange costs about as much as four).  The bf16 epilogues without input pieces are short and have only two 64-column
 // pieces to share (SwiGLU forward: one pair), so there the exchange costs more than it saves for short K: excluded; measured
 // on the one-window step with the bf16 store / SwiGLU left out, 2552 -> 2535 / 2522 us.
+// Split-precision products keep one accumulator for the whole contraction.  Parts have less of the tensor core's truncation, so
+// a product would depend on the tiles there are beside it, and the unscaled scores of the reference's backward carry that
+// far: after two updates of the reference network at 2 x 256 gradients were up to 2.2e-3 from those of whole tiles, where
+// the mode is to hold 1e-3 (6.5 ms a step with clusters, 7.8 without).
 static int cluster_split(const GemmDesc& d) {
   static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_CLUSTER_SPLIT"); return e && e[0] == '0'; }();  // A/B measurements
-  if (off || d.a_mn) return 0;
+  if (off || d.a_mn || d.seg_kb > 0) return 0;
   if (d.out != GEMM_OUT_F32 && d.out != GEMM_OUT_BF16_ROPE && d.out != GEMM_OUT_DSWIGLU && d.out != GEMM_OUT_DRELU2) return 0;
   const long tiles = (long)((d.M + 127) / 128) * ((d.N + 127) / 128);
   const int kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;

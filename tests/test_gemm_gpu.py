@@ -150,6 +150,20 @@ def test_split_precision_gemm_carries_fp32_operands_through_the_tensor_cores():
     assert rel_l2(got, C0 + At.astype(np.float64).T @ B.astype(np.float64)) < 2e-5
 
 
+@pytest.mark.parametrize("b_mn", [0, 1])
+@pytest.mark.parametrize("n,k", [(768, 768), (2304, 768), (768, 2048), (768, 2304)])
+def test_split_precision_rows_do_not_depend_on_the_number_of_rows(b_mn, n, k):
+    """A split-precision product has one accumulator for the whole contraction, whatever tiles there are beside it: the rows of
+    a small product are those of a large one, bit for bit."""
+    rng = np.random.default_rng(n + k)
+    A = rng.standard_normal((4096, k)).astype(np.float32)
+    B = rng.standard_normal((k, n) if b_mn else (n, k)).astype(np.float32)
+    large = _gemm(ane.DTYPE_BF16X3, A, B, np.zeros((4096, n), np.float32), 4096, n, k, 0, b_mn, 1)
+    for m in (100, 256, 512):
+        small = _gemm(ane.DTYPE_BF16X3, A[:m], B, np.zeros((m, n), np.float32), m, n, k, 0, b_mn, 1)
+        np.testing.assert_array_equal(small, large[:m])
+
+
 @pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 1), (1, 0)])
 @pytest.mark.parametrize("m,n,k", [(128, 96, 16), (4, 4, 4), (100, 92, 60), (288, 96, 2048), (97 * 4, 132, 1000), (2048, 288, 288), (20000, 128, 36)])
 def test_fp32_tiles_and_cluster_splits(a_mn, b_mn, m, n, k):
