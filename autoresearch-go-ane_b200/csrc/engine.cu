@@ -451,6 +451,7 @@ class EngineT final : public EngineBase {
   struct LossGraph {
     cudaGraphExec_t exec = nullptr;
     int passes = 0, launches = 0;
+    uint64_t scratch = 0;  // split_.generation at its capture: the pass reads and writes that scratch
   };
   std::vector<LossGraph> loss_graphs_;  // by number of windows
   uint64_t n_tokens_ = 0, rng_ = 0;
@@ -1797,14 +1798,21 @@ int EngineT<T>::eval_loss(const uint16_t* tokens, uint32_t n_seq, double* loss_s
   return check_device_status(nullptr);
 }
 
-// Enqueues the loss of nb windows in h_in_ -> h_rows_.  The pass is 45 to 110 short kernels at fixed addresses; issuing them
-// costs 4 us each, more than a small model's kernels take (217 of 280 us for one window of 100 tokens at dim 288), so from
-// the second pass over the same number of windows on it is replayed from a CUDA graph.
+// Enqueues the loss of nb windows in h_in_ -> h_rows_.  The pass is 45 to 110 short kernels; issuing them costs 4 us each, more
+// than a small model's kernels take (217 of 280 us for one window of 100 tokens at dim 288), so from the second pass over the
+// same number of windows on it is replayed from a CUDA graph.  Its buffers are those of the engine, which never move, and in
+// the split-precision mode the operand halves, which do: a graph is good for the scratch that it was captured with.
 template <typename T>
 int EngineT<T>::loss_pass(int nb) {
   int rc;
   const bool graphs = !profiling_ && !dp_.active();
   if (graphs && (int)loss_graphs_.size() <= nb) loss_graphs_.resize((size_t)nb + 1);
+  if (graphs && loss_graphs_[nb].exec && loss_graphs_[nb].scratch != split_.generation) {
+    // a larger product (a step's, EvalLogits', more windows') has moved the operand halves since: capture again
+    cudaGraphExecDestroy(loss_graphs_[nb].exec);
+    loss_graphs_[nb].exec = nullptr;
+    loss_graphs_[nb].passes = 1;
+  }
   if (graphs && loss_graphs_[nb].exec) {
     count_launch(loss_graphs_[nb].launches);
     last_B_ = nb;
@@ -1827,6 +1835,7 @@ int EngineT<T>::loss_pass(int nb) {
   }
   loss_graphs_[nb].exec = exec;
   loss_graphs_[nb].launches = (int)(launches() - before);
+  loss_graphs_[nb].scratch = split_.generation;
   return cuda_check(cudaGraphLaunch(exec, stream_), "eval loss graph");
 }
 

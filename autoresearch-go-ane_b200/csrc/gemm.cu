@@ -792,6 +792,7 @@ int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t
     o[i].vec = o[i].ld % 4 == 0 && (reinterpret_cast<uintptr_t>(o[i].src) & 15) == 0;
     const size_t need = sizeof(bf16) * (size_t)(mn ? 2 * kp : outer) * o[i].pitch;
     if (sc->cap[i] < need) {
+      ++sc->generation;
       // the previous, smaller buffer may still be read by GEMMs in flight on this stream
       if (sc->buf[i]) {
         cudaStreamSynchronize(stream);

@@ -96,6 +96,7 @@ int gemm_f32(const GemmDesc& d, cudaStream_t stream);
 struct SplitScratch {
   void* buf[2] = {nullptr, nullptr};  // A, B
   size_t cap[2] = {0, 0};             // bytes
+  uint64_t generation = 0;            // counts the times that a buffer moved: what was captured before holds old addresses
   void release();
 };
 int gemm_bf16x3(const GemmDesc& d, SplitScratch* scratch, int* d_status, cudaStream_t stream);

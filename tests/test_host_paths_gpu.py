@@ -163,3 +163,32 @@ def test_open_with_a_model_path_reads_a_model_file_or_a_checkpoint(tmp_path):
     junk.write_bytes(b"\x01" * 64)
     with pytest.raises(ane.EngineError, match="load model"):
         ane.open(_options(cfg, arch=ane.ARCH_LLAMA, compute_dtype=ane.DTYPE_F32, batch=1, model_path=str(junk)))
+
+
+@pytest.mark.parametrize("dtype", [ane.DTYPE_BF16, ane.DTYPE_F32, ane.DTYPE_BF16X3])
+def test_eval_loss_between_calls_that_need_more_scratch(dtype):
+    """The evaluation loss is replayed from a graph from the second pass of a window count on; a step, EvalLogits and another
+    window count in between (in split precision each has larger operands, whose scratch moves) must not change what it
+    reads.  The same kernels on the same weights in the same order: equal to a fresh engine's first, eager pass."""
+    toks = O.zipf_tokens(4096, CFG["vocab"], 29)
+    seq = CFG["seq"]
+    two, one = np.ascontiguousarray(toks[:2 * seq]), np.ascontiguousarray(toks[7 * seq:8 * seq])
+
+    def fresh_loss(e, windows):
+        _, f = make_pair(ane, CFG, arch=O.ARCH_N, quirks=0, dtype=dtype, batch=2, debug_taps=False)
+        for tid, layer, a in m.tensors(O.W):
+            f.import_tensor(tid, layer, e.export_tensor(tid, layer))
+        loss = f.eval_loss(windows)
+        f.close()
+        return loss
+
+    m, e = make_pair(ane, CFG, arch=O.ARCH_N, quirks=0, dtype=dtype, batch=2, hyper=dict(lr=1e-2, accum_steps=1), std=0.1,
+                     tokens=toks, debug_taps=False)
+    for _ in range(3):
+        assert e.eval_loss(one) == fresh_loss(e, one)
+    for between in (lambda: e.eval_loss(two), lambda: e.eval_logits(one, layout=1), lambda: e.eval_logits(one), e.step):
+        between()
+        for windows in (one, two):
+            for _ in range(3):
+                assert e.eval_loss(windows) == fresh_loss(e, windows)
+    e.close()
