@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
         __syncthreads();  // the partial sums of the phase before have been read
         src.words = kind == kWo ? a.w_att : a.w_gate;
         if (live && j0 < p.nu * 4) old = residual(p.row0(j0 >> 2) + 2 * (j0 & 3));
-      } else {
+      } else if (p.nu > 0) {  // (a CTA beyond the units of a small vocabulary has no group to wait for)
         // x before this layer (after W2 of the one below; the embedding row for layer 0), or after Wo for W1|W3
         const bool embed = kind == kQkv && l == 0;
         const uint2* words = embed ? nullptr : kind == kW13 ? a.w_x1 : a.w_x0;

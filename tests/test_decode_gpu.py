@@ -168,6 +168,8 @@ def test_decode_sample_fp32_matches_oracle_full_recompute():
     (32, 200, 5, 5, 544, 512, 12, 0.9),     # head size 40, contraction not a multiple of 32
     (32, 256, 2, 1, 2304, 512, 70, 0.0),    # head size 128; W2 in two boxes a row
     (33, 1280, 20, 4, 1024, 512, 20, 0.0),  # a second pass with one sequence; a norm read in two pieces
+    (2, 512, 8, 8, 1376, 256, 5, 0.0),      # fewer units of the vocabulary than CTAs: some own none
+    (12, 512, 8, 8, 1376, 96, 5, 0.0),      # and fewer than clusters
 ])
 def test_decode_bf16_kernels_match_own_full_forward(batch, dim, heads, kv, hidden, vocab, prompt, temp):
     """Tokens of the persistent kernels against the engine's full forward over prompt + generated tokens.
