@@ -199,3 +199,49 @@ def test_decode_bf16_kernels_match_own_full_forward(batch, dim, heads, kv, hidde
                 at, total = np.cumsum(p), p.sum()
                 slack = np.expm1(2 * tol / temp)
                 assert (at[tok] - p[tok]) / total - slack <= u[step, b] <= at[tok] / total + slack, (b, step)
+
+
+@pytest.mark.parametrize("batch,dim,heads,kv,hidden,vocab,new,temp", [
+    (1, 288, 6, 2, 768, 32000, 24, 1.0),     # kernel for up to eight sequences, fewer CTAs than SMs
+    (8, 288, 6, 3, 768, 4096, 24, 0.7),
+    (4, 768, 12, 4, 2048, 32000, 24, 1.0),   # on all SMs
+    (9, 288, 6, 6, 768, 32000, 24, 1.0),     # cluster kernel
+    (20, 288, 6, 2, 768, 4096, 24, 0.7),
+    (32, 768, 12, 4, 2048, 32000, 24, 1.0),
+    (2, 512, 8, 8, 1376, 256, 24, 1.0),      # fewer units of the vocabulary than CTAs: some own none
+    (2, 512, 8, 8, 1376, 256, 2, 0.7),
+    (12, 512, 8, 8, 1376, 96, 24, 0.7),
+])
+def test_sampled_tokens_are_the_serial_walks(batch, dim, heads, kv, hidden, vocab, new, temp):
+    """The sampler of the persistent kernels, index by index.  All weights but the embedding are zero, so the stream stays the
+    token's embedding; its elements are +-1/64, normalised they are +-c for one bf16 number c, and a logit is c / 64 times a whole
+    number: exact in fp32 in any order of addition.  The token must be the one of the serial walk in double over those logits
+    (ane/train_full.go:318-342).  Draws: 0, the largest below 1, 1e-9 to either side of the edges of CTA ranges (sums in another
+    order move an edge by 1e-13), and random ones."""
+    a, prompt = 1.0 / 64, 3
+    rng = np.random.default_rng(vocab + batch)
+    signs = rng.integers(0, 2, (vocab, dim)).astype(np.float32) * 2 - 1
+    x = np.float32(a) * (np.float32(1) / np.sqrt(np.float32(a * a) + np.float32(1e-5)))
+    c = float(np.float32(np.round(float(x) * 256) / 256))  # 8 bits in [1/2, 1)
+    assert abs(abs(float(x) - c) - 1 / 512) > 1e-4         # clear of a rounding edge
+    e = ane.open(ane.Options(dim=dim, hidden=hidden, n_layers=2, n_heads=heads, n_kv_heads=kv, vocab=vocab, seq=64, batch=batch,
+                             arch=ane.ARCH_LLAMA, quirks=0, compute_dtype=ane.DTYPE_BF16))
+    e.import_tensor(ane.T_EMBED, 0, signs * np.float32(a))
+    prompts = rng.integers(0, vocab, (batch, prompt)).astype(np.uint16)
+    units = vocab // 8
+    edges = sorted({8 * (units * i // n) for n in (60, 132, 136, 140, 144, 148) for i in range(1, n)} - {0})
+    u, want = np.zeros((new, batch)), np.zeros((batch, new), np.uint16)
+    last = prompts[:, -1].astype(int)
+    inv_temp = float(np.float32(1) / np.float32(temp))
+    for step in range(new):
+        logits = (signs @ signs[last].T).astype(np.float64) * (c * a)  # whole numbers up to dim: exact
+        cdf = np.cumsum(np.exp((logits - logits.max(0)) * inv_temp), 0)
+        for b in range(batch):
+            kind = (step + b) % 6
+            at = cdf[edges[rng.integers(len(edges))] - 1, b] / cdf[-1, b]
+            u[step, b] = (0.0, 1 - 2.0 ** -53, at - 1e-9, at + 1e-9, rng.random(), rng.random())[kind]
+            want[b, step] = min(int(np.searchsorted(cdf[:, b], u[step, b] * cdf[-1, b])), vocab - 1)
+        last = want[:, step].astype(int)
+    got = e.decode_sample(prompts, new, temp, u)
+    e.close()
+    np.testing.assert_array_equal(got, want)
