@@ -344,6 +344,7 @@ class EngineT final : public EngineBase {
   }
   int layout_params();
   int alloc_buffers();
+  int alloc_decode();
   int refresh_shadow();
   int forward(const uint16_t* d_tok, int B, int Tl, int pos0);
   int head_and_backward(int B);
@@ -1898,6 +1899,37 @@ __global__ void store_tokens_kernel(const int32_t* __restrict__ arg, uint16_t* _
   out[(size_t)b * n_new + step] = t;
 }
 
+// Caches and scratch of decode(): all of them or, when memory runs out, none, so that a later call starts afresh.
+template <typename T>
+int EngineT<T>::alloc_decode() {
+  const size_t held = allocs_.size(), per_layer = (size_t)B_ * S_ * KVD_;
+  T *kc = nullptr, *vc = nullptr;
+  const int rc = [&]() -> int {
+    int r;
+    if ((r = dalloc(&kc, per_layer * L_)) != 0 || (r = dalloc(&vc, per_layer * L_)) != 0) return r;
+    if constexpr (!kIsF32) {
+      const size_t rows = std::min(B_, 32);  // the persistent kernel takes up to 32 sequences at a time
+      if ((r = dalloc(&dec_best_, 3 * rows)) != 0 || (r = dalloc(&dec_psum_, rows * gemm_num_sms())) != 0 || (r = dalloc(&dec_bar_, 1)) != 0 ||
+          (r = dalloc(&dec_words_, decode_words_bytes(D_, Hd_, H_, KV_, hd_, (int)rows, gemm_num_sms()))) != 0)
+        return r;
+    }
+    if ((r = dalloc(&d_argmax_, B_)) != 0 || (r = dalloc(&d_dec_tok_, B_)) != 0 || (r = dalloc(&d_dec_out_, (size_t)B_ * S_)) != 0 ||
+        (r = dalloc(&d_dec_u_, (size_t)B_ * S_)) != 0)
+      return r;
+    return 0;
+  }();
+  if (rc != 0) {
+    for (; allocs_.size() > held; allocs_.pop_back()) cudaFree(allocs_.back());
+    cudaGetLastError();
+    return rc;
+  }
+  for (int l = 0; l < L_; ++l) {
+    kcache_.push_back(kc + per_layer * l);
+    vcache_.push_back(vc + per_layer * l);
+  }
+  return 0;
+}
+
 template <typename T>
 int EngineT<T>::decode(const uint16_t* prompts, uint32_t n_seq, uint32_t prompt_len, uint32_t n_new,
                        float temperature, const double* uniforms, uint16_t* out) {
@@ -1910,31 +1942,7 @@ int EngineT<T>::decode(const uint16_t* prompts, uint32_t n_seq, uint32_t prompt_
     return fail(ANE_ERR_ARG, "storiesane decode: prompt_len + n_new must fit the engine's seq");
   if ((rc = cuda_check(cudaSetDevice(o_.device), "cudaSetDevice")) != 0) return rc;
   const int B = (int)n_seq, P = (int)prompt_len;
-  if (kcache_.empty()) {
-    kcache_.assign(L_, nullptr);
-    vcache_.assign(L_, nullptr);
-    T *kc = nullptr, *vc = nullptr;
-    const size_t per_layer = (size_t)B_ * S_ * KVD_;
-    if ((rc = dalloc(&kc, per_layer * L_)) != 0 || (rc = dalloc(&vc, per_layer * L_)) != 0) {
-      kcache_.clear();
-      return rc;
-    }
-    for (int l = 0; l < L_; ++l) {
-      kcache_[l] = kc + per_layer * l;
-      vcache_[l] = vc + per_layer * l;
-    }
-    if constexpr (!kIsF32) {
-      const size_t rows = std::min(B_, 32);  // the persistent kernel takes up to 32 sequences at a time
-      if ((rc = dalloc(&dec_best_, 3 * rows)) != 0 ||
-          (rc = dalloc(&dec_psum_, rows * gemm_num_sms())) != 0 || (rc = dalloc(&dec_bar_, 1)) != 0 ||
-          (rc = dalloc(&dec_words_, decode_words_bytes(D_, Hd_, H_, KV_, hd_, (int)rows, gemm_num_sms()))) != 0)
-        return rc;
-    }
-    if ((rc = dalloc(&d_argmax_, B_)) != 0) return rc;
-    if ((rc = dalloc(&d_dec_tok_, B_)) != 0) return rc;
-    if ((rc = dalloc(&d_dec_out_, (size_t)B_ * S_)) != 0) return rc;
-    if ((rc = dalloc(&d_dec_u_, (size_t)B_ * S_)) != 0) return rc;
-  }
+  if (kcache_.empty() && (rc = alloc_decode()) != 0) return rc;
   if (sampling)  // [n_new][n_seq]: the draws of one step are contiguous
     cudaMemcpyAsync(d_dec_u_, uniforms, sizeof(double) * (size_t)n_seq * n_new, cudaMemcpyHostToDevice, stream_);
   // The prompt does not fit the pinned window buffer in general (B*P <= B_*S_ does hold).

@@ -245,3 +245,39 @@ def test_sampled_tokens_are_the_serial_walks(batch, dim, heads, kv, hidden, voca
     got = e.decode_sample(prompts, new, temp, u)
     e.close()
     np.testing.assert_array_equal(got, want)
+
+
+def test_decode_after_its_buffers_could_not_be_allocated():
+    """The first decode allocates the caches and its scratch.  With memory left for the two caches (128 MiB each) but not for
+    all of the rest (8 MiB of draws) it reports an error and keeps nothing; when there is memory again it decodes."""
+    from ane import _ffi
+    lib = _ffi.lib
+    opts = ane.Options(dim=64, hidden=64, n_layers=1, n_heads=1, n_kv_heads=1, vocab=96, seq=512, batch=2048, arch=ane.ARCH_LLAMA,
+                       quirks=0, compute_dtype=ane.DTYPE_BF16)
+    weights = np.random.default_rng(3).standard_normal((96, 64)).astype(np.float32)
+    prompts = O.zipf_tokens(2 * 8, 96, 3).reshape(2, 8)
+    e = ane.open(opts)
+    e.import_tensor(ane.T_EMBED, 0, weights)
+    room = lib.ane_dev_malloc(260 << 20)
+    held, size = [], 1 << 34
+    while size >= 1 << 20:
+        p = lib.ane_dev_malloc(size)
+        if p:
+            held.append(p)
+        else:
+            size >>= 1
+    lib.ane_dev_free(room)
+    try:
+        with pytest.raises(ane.EngineError, match="cudaMalloc"):
+            e.decode_greedy(prompts, 4)
+        with pytest.raises(ane.EngineError, match="cudaMalloc"):
+            e.decode_greedy(prompts, 4)
+    finally:
+        for p in held:
+            lib.ane_dev_free(p)
+    got = e.decode_greedy(prompts, 4)
+    e.close()
+    e = ane.open(opts)
+    e.import_tensor(ane.T_EMBED, 0, weights)
+    np.testing.assert_array_equal(got, e.decode_greedy(prompts, 4))
+    e.close()
