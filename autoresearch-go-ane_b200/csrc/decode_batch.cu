@@ -630,6 +630,7 @@ int decode_batch_steps(DecodeArgs a, int sms, cudaStream_t s) {
   attr[1].id = cudaLaunchAttributeCooperative;  // all CTAs are resident together, so the waits on one another complete
   attr[1].val.cooperative = 1;
   cudaLaunchConfig_t cfg = {};
+  if (sms < kCluster) return -4;
   cfg.gridDim = dim3((unsigned)(sms / kCluster * kCluster));
   cfg.blockDim = dim3(kLaunch);
   cfg.dynamicSmemBytes = p.smem;

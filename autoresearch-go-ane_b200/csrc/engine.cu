@@ -1991,10 +1991,16 @@ int EngineT<T>::decode(const uint16_t* prompts, uint32_t n_seq, uint32_t prompt_
         a.B = std::min(32, B - b0); a.D = D_; a.Hd = Hd_; a.L = L_; a.H = H_; a.KV = KV_; a.hd = hd_; a.V = V_; a.S = S_;
         a.prompt = P; a.n_new = (int)n_new;
         count_launch();
-        if (decode_steps(a, dec_words_, gemm_num_sms(), stream_) != 0)
-          return fail(ANE_ERR_KERNEL, "storiesane decode: persistent kernel launch failed");
+        done = decode_steps(a, dec_words_, gemm_num_sms(), stream_) == 0;
+        if (!done) break;
       }
-      done = true;
+      if (!done) {  // not all of its CTAs fit this GPU (a share of one, a cap on the SMs): one step after the other
+        cudaGetLastError();
+        // first tokens again: a sampling kernel has moved those of the sequences before on
+        if ((rc = cuda_check(cudaMemcpy2DAsync(d_dec_tok_, sizeof(uint16_t), d_dec_out_, sizeof(uint16_t) * n_new, sizeof(uint16_t), B,
+                                               cudaMemcpyDeviceToDevice, stream_), "decode first tokens")) != 0)
+          return rc;
+      }
     }
   }
   decoding_ = true;

@@ -281,3 +281,42 @@ def test_decode_after_its_buffers_could_not_be_allocated():
     e.import_tensor(ane.T_EMBED, 0, weights)
     np.testing.assert_array_equal(got, e.decode_greedy(prompts, 4))
     e.close()
+
+
+def _decode_in_a_child(env):
+    """Tokens of 2 greedy and 36 sampled sequences, from a process with `env`."""
+    import json
+    import os
+    import subprocess
+    import sys
+    code = """
+import json, sys
+import numpy as np
+import ane
+rng = np.random.default_rng(4)
+out = []
+for batch, temp in ((2, 0.0), (36, 0.9)):
+    e = ane.open(ane.Options(dim=128, hidden=256, n_layers=2, n_heads=2, n_kv_heads=1, vocab=512, seq=64, batch=batch, arch=ane.ARCH_LLAMA,
+                             quirks=0, compute_dtype=ane.DTYPE_BF16))
+    e.import_tensor(ane.T_EMBED, 0, (rng.integers(0, 2, (512, 128)) * 2 - 1).astype(np.float32) / 64)
+    prompts = rng.integers(0, 512, (batch, 5)).astype(np.uint16)
+    before = e.launch_count()
+    tokens = e.decode_sample(prompts, 9, temp, rng.random((9, batch)))
+    out.append([tokens.tolist(), e.launch_count() - before])
+    e.close()
+print(json.dumps(out))
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.path.join(root, "autoresearch-go-ane_b200"), **env)
+    done = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
+    return json.loads(done.stdout.strip().splitlines()[-1])
+
+
+def test_decode_where_the_persistent_kernel_does_not_fit():
+    """On two SMs (ANE_B200_GEMM_SMS) there is no cluster of four CTAs to launch, a launch that the host refuses; decoding goes
+    one step after the other then.  Zero weights but the embedding: logits are exact, so the tokens are the same."""
+    whole, two = _decode_in_a_child({}), _decode_in_a_child({"ANE_B200_GEMM_SMS": "2"})
+    for (tokens, launches), (same, more) in zip(whole, two):
+        assert same == tokens
+        assert more > 2 * launches
