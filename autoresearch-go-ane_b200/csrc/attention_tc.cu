@@ -98,23 +98,37 @@ __device__ __forceinline__ void gemm_a_smem_b_nk(float (&acc)[8][4], const bf16*
   }
 }
 
-// acc (16 x HD) += P (16 x 64 in registers, accumulator layout, rounded to bf16) * B, with B stored [k][n] (64 rows).
+// acc (16 x HD) += P (16 x 64 in registers, accumulator layout) * B, with B stored [k][n] (64 rows).  For head sizes 32 and 48,
+// which fp32 kernels served before these, P (in the backward also dS) enters as bf16 hi and lo parts, two MMAs: against
+// attention in double on the same operands the results are off by their own rounding to bf16 alone (1.0000 to 1.0001 of it over
+// head sizes 32 and 48, 63 to 1024 tokens, uniform to peaked rows), with one part by 1.01 to 1.16 of it (out), 1.10 to 1.63
+// (dq, dk) and 1.00 to 1.34 (dv).  It costs 5 % of a small model's update (5 x 200 tokens, three micro-steps: 3158 -> 3315 us).
+// Head size 64 keeps one part, as the tcgen05 kernels do.
 template <class C>
 __device__ __forceinline__ void gemm_a_regs_b_kn(float (&acc)[C::NT][4], const float (&p)[8][4], const bf16* b_tile,
                                                  int lane) {
 #pragma unroll
   for (int kk = 0; kk < KT / 16; ++kk) {
-    uint32_t a[4];
-    a[0] = pack_bf16(p[2 * kk][0], p[2 * kk][1]);
-    a[1] = pack_bf16(p[2 * kk][2], p[2 * kk][3]);
-    a[2] = pack_bf16(p[2 * kk + 1][0], p[2 * kk + 1][1]);
-    a[3] = pack_bf16(p[2 * kk + 1][2], p[2 * kk + 1][3]);
+    uint32_t a[4], lo[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float x = p[2 * kk + (e >> 1)][2 * (e & 1)], y = p[2 * kk + (e >> 1)][2 * (e & 1) + 1];
+      a[e] = pack_bf16(x, y);
+      if constexpr (C::HD != 64) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[e]));
+        lo[e] = pack_bf16(x - f.x, y - f.y);
+      }
+    }
 #pragma unroll
     for (int np = 0; np < C::HD / 16; ++np) {
       uint32_t b[4];
       ldsm_x4_t(b, b_tile + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * C::LDS + np * 16 + (lane >> 4) * 8);
       mma_bf16(acc[2 * np], a, b[0], b[1]);
       mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
+      if constexpr (C::HD != 64) {
+        mma_bf16(acc[2 * np], lo, b[0], b[1]);
+        mma_bf16(acc[2 * np + 1], lo, b[2], b[3]);
+      }
     }
   }
 }

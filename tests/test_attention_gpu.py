@@ -48,3 +48,48 @@ def test_bf16_tiles(hd, heads, kv, seq, batch):
             err = np.linalg.norm(got - want) / np.linalg.norm(want)
             assert err < tol, (layer, tap, err)
     e.close()
+
+
+def _bf16(x):
+    """float64 -> nearest bf16, as float64."""
+    u = np.asarray(x, np.float32).view(np.uint32).astype(np.uint64)
+    return (((u + 0x7FFF + ((u >> 16) & 1)) >> 16) << 16).astype(np.uint32).view(np.float32).astype(np.float64)
+
+
+def attention_error_over_rounding(hd, heads, kv, seq, batch, std):
+    """{tensor: error of the engine's attention / the error that rounding the exact result to bf16 makes}, where exact is
+    attention in float64 on the engine's own bf16 operands (Wo = 1, so that d att is bf16(d x2))."""
+    cfg, m, e, inp, tgt = _step(ane.DTYPE_BF16, O.ARCH_L, 0, hd, heads, kv, seq, batch, std)
+    e.import_tensor(ane.T_WO, 0, np.eye(hd * heads, dtype=np.float32))
+    e.import_tensor(ane.T_WO, 1, np.eye(hd * heads, dtype=np.float32))
+    e.step_tokens(inp, tgt)
+    tap = lambda t, h: e.tap(t, 0).reshape(batch, h, hd, seq).astype(np.float64).transpose(0, 1, 3, 2)  # noqa: E731
+    q, k, v, do = tap(O.TAP_Q, heads), tap(O.TAP_K, kv), tap(O.TAP_V, kv), _bf16(tap(O.TAP_DX2, heads))
+    got = {"att": tap(O.TAP_ATT, heads), "dq": tap(O.TAP_DQ, heads), "dk": tap(O.TAP_DK, kv), "dv": tap(O.TAP_DV, kv)}
+    e.close()
+    rep = heads // kv
+    kr, vr = k.repeat(rep, 1), v.repeat(rep, 1)
+    s = q @ kr.transpose(0, 1, 3, 2) / np.sqrt(hd)
+    s[..., np.triu(np.ones((seq, seq), bool), 1)] = -np.inf
+    p = np.exp(s - s.max(-1, keepdims=True))
+    p /= p.sum(-1, keepdims=True)
+    dp = do @ vr.transpose(0, 1, 3, 2)
+    ds = p * (dp - (p * dp).sum(-1, keepdims=True)) / np.sqrt(hd)
+    shared = lambda x: x.reshape(batch, kv, rep, seq, hd).sum(2)  # noqa: E731
+    want = {"att": p @ vr, "dq": ds @ kr, "dk": shared(ds.transpose(0, 1, 3, 2) @ q), "dv": shared(p.transpose(0, 1, 3, 2) @ do)}
+    angle = np.arange(seq)[:, None] * 10000.0 ** (-np.arange(0, hd, 2) / hd)
+    c, sn = np.cos(angle), np.sin(angle)
+    for name in ("dq", "dk"):  # the rotation undone
+        x, y = want[name][..., ::2].copy(), want[name][..., 1::2].copy()
+        want[name][..., ::2], want[name][..., 1::2] = x * c + y * sn, y * c - x * sn
+    return {n: np.linalg.norm(got[n] - want[n]) / np.linalg.norm(_bf16(want[n]) - want[n]) for n in got}
+
+
+@pytest.mark.parametrize("hd,heads,kv,seq,batch", [(32, 2, 1, 63, 2), (48, 2, 2, 65, 2), (48, 4, 2, 200, 2), (48, 2, 2, 257, 50)])
+@pytest.mark.parametrize("std", [0.02, 0.15])
+def test_probabilities_keep_sixteen_bits(hd, heads, kv, seq, batch, std):
+    """Probabilities and score gradients enter their products as bf16 hi + lo (2^-17 each), so that the result is off by its
+    own rounding (2^-9) and little else: 2 % more is 2^-9 sqrt(1.02^2 - 1) = 2^-11.3 of the result, ten times what their
+    2^-17 and the 2^-17 of delta's O leave after the differences they enter.  Rounded to bf16 alone they exceed it."""
+    off = attention_error_over_rounding(hd, heads, kv, seq, batch, std)
+    assert max(off.values()) < 1.02, off
