@@ -102,7 +102,7 @@ __device__ __forceinline__ void gemm_a_smem_b_nk(float (&acc)[8][4], const bf16*
 // which fp32 kernels served before these, P (in the backward also dS) enters as bf16 hi and lo parts, two MMAs: against
 // attention in double on the same operands the results are off by their own rounding to bf16 alone (1.0000 to 1.0001 of it over
 // head sizes 32 and 48, 63 to 1024 tokens, uniform to peaked rows), with one part by 1.01 to 1.16 of it (out), 1.10 to 1.63
-// (dq, dk) and 1.00 to 1.34 (dv).  It costs 5 % of a small model's update (5 x 200 tokens, three micro-steps: 3158 -> 3315 us).
+// (dq, dk) and 1.00 to 1.34 (dv).  It costs 5 % of a small model's update (5 x 200 tokens, three micro-steps: 3160 -> 3270 us).
 // Head size 64 keeps one part, as the tcgen05 kernels do.
 template <class C>
 __device__ __forceinline__ void gemm_a_regs_b_kn(float (&acc)[C::NT][4], const float (&p)[8][4], const bf16* b_tile,
@@ -176,7 +176,8 @@ __device__ __forceinline__ void store_grad_bf16(bf16* base, int ld, int row_lo, 
 }
 
 // ------------------------------------------------------------------------------------------------
-// Forward: grid (query tiles of BR, B*H); 16 query rows per warp; key/value tiles of 64 streamed.
+// Forward: grid (B*H, query tiles of BR, the longest first); 16 query rows per warp; key/value tiles of 64 streamed.
+// (Heads along x, as everywhere here: many short windows have more than the 65535 that y takes.)
 // ------------------------------------------------------------------------------------------------
 template <class C>
 __global__ void __launch_bounds__(C::THREADS)
@@ -189,7 +190,7 @@ attention_fwd_tc_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ out, bf
   bf16* Qs = reinterpret_cast<bf16*>(att_smem);   // [BR][LDS]
   bf16* Ks = Qs + BR * LDS;                       // [2][KT][LDS]
   bf16* Vs = Ks + 2 * KT * LDS;                   // [2][KT][LDS]
-  const int qt = blockIdx.x, bh = blockIdx.y;
+  const int qt = (int)(gridDim.y - 1 - blockIdx.y), bh = blockIdx.x;
   const int b = bh / H, h = bh - b * H, kvh = h / (H / KV);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int ld = (H + 2 * KV) * HD;
@@ -314,7 +315,7 @@ __global__ void attention_delta_kernel(const bf16* __restrict__ d_out, const bf1
 }
 
 // ------------------------------------------------------------------------------------------------
-// Backward, dQ: grid (query tiles of BR, B*H); key/value tiles streamed.
+// Backward, dQ: grid (B*H, query tiles of BR, the longest first); key/value tiles streamed.
 // ------------------------------------------------------------------------------------------------
 template <class C>
 __global__ void __launch_bounds__(C::THREADS)
@@ -329,7 +330,7 @@ attention_bwd_dq_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
   bf16* dOs = Qs + BR * LDS;                      // [BR][LDS]
   bf16* Ks = dOs + BR * LDS;                      // [2][KT][LDS]
   bf16* Vs = Ks + 2 * KT * LDS;                   // [2][KT][LDS]
-  const int qt = blockIdx.x, bh = blockIdx.y;
+  const int qt = (int)(gridDim.y - 1 - blockIdx.y), bh = blockIdx.x;
   const int b = bh / H, h = bh - b * H, kvh = h / (H / KV);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int ld = (H + 2 * KV) * HD;
@@ -394,7 +395,7 @@ attention_bwd_dq_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
 }
 
 // ------------------------------------------------------------------------------------------------
-// Backward, dK/dV: grid (key tiles of BR, B*KV); 16 key rows per warp; streams the query/dO tiles
+// Backward, dK/dV: grid (B*KV, key tiles of BR); 16 key rows per warp; streams the query/dO tiles
 // of every query head that shares this KV head, so no atomics are needed.
 // ------------------------------------------------------------------------------------------------
 template <class C>
@@ -413,7 +414,7 @@ attention_bwd_dkv_tc_kernel(const bf16* __restrict__ qkv, const bf16* __restrict
   bf16* dOs = Qs + 2 * KT * LDS;                  // [2][KT][LDS]
   float* lse_s = reinterpret_cast<float*>(dOs + 2 * KT * LDS);  // [2][KT]
   float* del_s = lse_s + 2 * KT;                                // [2][KT]
-  const int kt = blockIdx.x, bk = blockIdx.y;
+  const int kt = blockIdx.y, bk = blockIdx.x;
   const int b = bk / KV, kvh = bk - b * KV;
   const int group = H / KV;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
@@ -501,7 +502,7 @@ template <class C>
 bool launch_forward(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B, int seq, int H, int KV, float scale, cudaStream_t s) {
   static unsigned long long done = 0;
   if (!smem_opt_in(attention_fwd_tc_kernel<C>, C::kFwdSmem, done)) return false;
-  dim3 grid((seq + C::BR - 1) / C::BR, B * H);
+  dim3 grid(B * H, (seq + C::BR - 1) / C::BR);
   launch_pdl(attention_fwd_tc_kernel<C>, grid, dim3(C::THREADS), C::kFwdSmem, s, qkv, out, out_lo, lse, seq, H, KV, scale);
   return true;
 }
@@ -511,9 +512,9 @@ bool launch_backward(const bf16* qkv, const bf16* d_out, const float* lse, const
   static unsigned long long done_q = 0, done_k = 0;
   if (!smem_opt_in(attention_bwd_dq_tc_kernel<CQ>, CQ::kDqSmem, done_q) || !smem_opt_in(attention_bwd_dkv_tc_kernel<CK>, CK::kDkvSmem, done_k))
     return false;
-  dim3 gq((seq + CQ::BR - 1) / CQ::BR, B * H);
+  dim3 gq(B * H, (seq + CQ::BR - 1) / CQ::BR);
   launch_pdl(attention_bwd_dq_tc_kernel<CQ>, gq, dim3(CQ::THREADS), CQ::kDqSmem, s, qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV, scale);
-  dim3 gk((seq + CK::BR - 1) / CK::BR, B * KV);
+  dim3 gk(B * KV, (seq + CK::BR - 1) / CK::BR);
   launch_pdl(attention_bwd_dkv_tc_kernel<CK>, gk, dim3(CK::THREADS), CK::kDkvSmem, s, qkv, d_out, lse, delta, dqkv, cosb, sinb, seq, H, KV, scale);
   return true;
 }

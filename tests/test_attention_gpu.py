@@ -50,6 +50,26 @@ def test_bf16_tiles(hd, heads, kv, seq, batch):
     e.close()
 
 
+@pytest.mark.parametrize("hd", [48, 64])
+def test_more_heads_than_a_grid_dimension_takes(hd):
+    """33000 windows of two tokens with two heads: 66000 heads in one launch.  Every window is the same, and so must be its
+    attention output and gradients."""
+    batch, seq, heads = 33000, 2, 2
+    e = ane.open(ane.Options(dim=hd * heads, hidden=32, n_layers=1, n_heads=heads, n_kv_heads=heads, vocab=96, seq=seq, batch=batch,
+                             arch=ane.ARCH_LLAMA, quirks=0, compute_dtype=ane.DTYPE_BF16, accum_steps=1000, debug_taps=True))
+    rng = np.random.default_rng(2)
+    for tid, layer in ((ane.T_EMBED, 0), (ane.T_WQ, 0), (ane.T_WK, 0), (ane.T_WV, 0), (ane.T_WO, 0)):
+        e.import_tensor(tid, layer, (0.2 * rng.standard_normal(e.tensor_size(tid, layer))).astype(np.float32))
+    toks = np.tile(np.array([3, 7], np.uint16), (batch, 1))
+    r = e.step_tokens(toks, toks[:, ::-1].copy())
+    assert r.device_status == 0 and np.isfinite(r.loss)
+    for tap in (O.TAP_ATT, O.TAP_DQ, O.TAP_DK, O.TAP_DV):
+        out = e.tap(tap, 0).reshape(batch, -1)
+        assert np.abs(out[0]).max() > 0
+        np.testing.assert_array_equal(out, np.broadcast_to(out[0], out.shape))
+    e.close()
+
+
 def _bf16(x):
     """float64 -> nearest bf16, as float64."""
     u = np.asarray(x, np.float32).view(np.uint32).astype(np.uint64)
