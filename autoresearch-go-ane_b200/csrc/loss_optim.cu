@@ -447,8 +447,8 @@ ce_merge_stats_kernel(const float2* __restrict__ stats, int n_tiles, int rows, c
   const int r = blockIdx.x * 32 + lane;
   float m = -INFINITY, s = 0.f;
   auto merge = [&](float2 v) {
+    if (v.x == -INFINITY && v.y == 0.f) return;  // a warp without tiles (a tile of nothing but NaN has a sum of NaN, which counts)
     const float mn = fmaxf(m, v.x);
-    if (mn == -INFINITY) return;
     s = s * exp2f(m - mn) + v.y * exp2f(v.x - mn);
     m = mn;
   };

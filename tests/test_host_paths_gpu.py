@@ -192,3 +192,22 @@ def test_eval_loss_between_calls_that_need_more_scratch(dtype):
             for _ in range(3):
                 assert e.eval_loss(windows) == fresh_loss(e, windows)
     e.close()
+
+
+def test_evaluation_loss_counts_a_tile_of_nan_logits():
+    """256 embedding rows of NaN make a whole tile of the classifier's statistics NaN, without a maximum.  The softmax over the
+    vocabulary is NaN then, and the loss of every position -log of the probability's floor of 1e-10 (ane/stories/cpu.go:212-292)."""
+    e = ane.open(ane.Options(dim=64, hidden=64, n_layers=1, n_heads=1, n_kv_heads=1, vocab=1024, seq=32, batch=1, arch=ane.ARCH_LLAMA,
+                             quirks=0, compute_dtype=ane.DTYPE_BF16))
+    embed = (0.02 * np.random.default_rng(1).standard_normal((1024, 64))).astype(np.float32)
+    window = np.arange(32, dtype=np.uint16)
+    e.import_tensor(ane.T_EMBED, 0, embed)
+    loss, n = e.eval_loss(window)
+    assert n == 31 and loss / n == pytest.approx(np.log(1024), abs=0.1)
+    for tile in range(1, 4):
+        bad = embed.copy()
+        bad[256 * tile:256 * (tile + 1)] = np.nan
+        e.import_tensor(ane.T_EMBED, 0, bad)
+        loss, n = e.eval_loss(window)
+        assert n == 31 and loss / n == pytest.approx(-np.log(1e-10), abs=1e-3)
+    e.close()
