@@ -59,32 +59,34 @@ inline int64_t now_ns() {
 // EvalLogits into ordinary memory: device -> page-locked staging (full PCIe rate) -> caller's array.  The download is
 // cut into pieces and the host copies what has landed while the rest is still crossing PCIe.  One core copies about
 // 10 GB/s, a fifth of the PCIe rate (32.8 MB cross in 0.6 ms), so all cores copy (ANE_B200_EVAL_COPY_THREADS; default: the
-// host's cores, at most 16), in blocks of 64 KB that they claim in order: when the last piece lands only its own blocks are
-// left, one per thread (whole pieces dealt to threads left a megabyte per thread: 0.1 - 0.2 ms).  The calling thread only
-// follows the download and says how far it is.  The threads live as long as the call.
+// host's cores, at most 16), in blocks that they claim in order: when the last piece lands only its own blocks are left, one
+// per thread (whole pieces dealt to threads left a megabyte per thread: 0.1 - 0.2 ms).  The calling thread only follows the
+// download and says how far it is.  The threads live as long as the call.
+// Memory that nobody has touched yet (what an allocator has just got from the kernel; most arrays above 32 MiB) is mapped at the
+// first write, which takes longer than the copy, and threads that copy neighbouring blocks wait for one another's page.  The
+// helpers therefore touch the output first, a huge page at a time, while the GPU is still at the first window's logits (values
+// stay as they are); what has been touched before costs them next to nothing.  Fresh / touched arrays, against pieces dealt
+// to 16 threads: one window of 65 MB 3.2 -> 2.5 / 2.5 -> 2.3 ms, three of 33 MB 6.9 -> 5.6 / 5.0 -> 4.3, one of 33 MB 1.65 ->
+// 1.56 (both).  Blocks of 256 KB lose 0.08 of 2.9 ms against 64 KB in three windows of 4 MB, blocks of 64 KB lose 2 of 16 ms
+// against 256 KB in 262 MB of fresh memory.
 class LogitsCopy {
  public:
   LogitsCopy(float* out, uint64_t per_window, uint32_t windows, float* staging, cudaEvent_t* events)
       : out_(out), n_(per_window), staging_(staging), events_(events), order_(windows) {
-    // An output above 32 MiB (malloc's largest threshold) is memory fresh from the kernel, in huge pages where its owner asks
-    // for them: helpers that copy neighbouring 64 KiB wait for the first touch of the same page, so they take 2 MiB each
-    // (65 MB: 4.5 -> 3.1-3.6 ms; three windows of 33 MB: 7.9 -> 6.4).  Smaller outputs are mostly warm, and the last
-    // piece is over sooner in small blocks (1.53 ms against 1.67 at 32.8 MB).
-    const bool fresh = per_window * windows * sizeof(float) > (32u << 20);
-    block_ = fresh ? 524288 : 16384;
     static const int pieces = [] {
       const char* e = getenv("ANE_B200_EVAL_PIECES");
-      const int v = e ? atoi(e) : 0;
-      return v > 64 ? 64 : v;
+      const int v = e ? atoi(e) : 16;
+      return v < 1 ? 1 : (v > 64 ? 64 : v);
     }();
-    const int want = pieces > 0 ? pieces : fresh ? 32 : 16;
     static const int cores = [] {
       const char* e = getenv("ANE_B200_EVAL_COPY_THREADS");
       const unsigned hw = std::thread::hardware_concurrency();
       const int v = e ? atoi(e) : (hw == 0 ? 4 : (int)hw);
       return v < 1 ? 1 : (v > 16 ? 16 : v);
     }();
-    piece_ = ((n_ + want - 1) / want + block_ - 1) / block_ * block_;  // whole blocks
+    // a quarter of a piece, so that several threads share the last one, in bounds that the comment above gives
+    block_ = std::min<uint64_t>(65536, std::max<uint64_t>(16384, n_ / (4 * pieces)));
+    piece_ = ((n_ + pieces - 1) / pieces + block_ - 1) / block_ * block_;  // whole blocks
     pieces_ = (int)((n_ + piece_ - 1) / piece_);
     blocks_ = (int)((n_ + block_ - 1) / block_);
     helpers_wanted_ = n_ * sizeof(float) < (1u << 20) ? 0 : std::min(cores - 1, blocks_);  // under 1 MiB: not worth a thread start
@@ -95,40 +97,63 @@ class LogitsCopy {
   }
   // Window `w` of the output from `logits` on the device, once `stream` has reached this point; returns when it is there.
   cudaError_t window(uint32_t w, const float* logits, cudaStream_t stream) {
+    if (rounds_ == 0) start();
     const long long round = rounds_++;
     order_[round] = w;  // read only after `landed_` has reached this round
-    while ((int)helpers_.size() < helpers_wanted_) helpers_.emplace_back([this] { helper(); });
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < pieces_ && e == cudaSuccess; ++i) {
       const uint64_t off = (uint64_t)i * piece_, n = std::min(piece_, n_ - off);
       e = cudaMemcpyAsync(staging_ + off, logits + off, sizeof(float) * n, cudaMemcpyDeviceToHost, stream);
       if (e == cudaSuccess) e = cudaEventRecord(events_[i], stream);
     }
+    const int per_piece = (int)(piece_ / block_);
     for (int i = 0; i < pieces_ && e == cudaSuccess; ++i) {
       e = cudaEventSynchronize(events_[i]);
-      if (e == cudaSuccess) landed_.store(round * pieces_ + i + 1, std::memory_order_release);
+      if (e != cudaSuccess) break;
+      landed_.store(round * pieces_ + i + 1, std::memory_order_release);
+      if (helpers_wanted_ == 0)
+        for (int k = i * per_piece; k < std::min((i + 1) * per_piece, blocks_); ++k) copy_block(w, k);
     }
-    if (e != cudaSuccess) return e;
-    if (helpers_wanted_ == 0) {
-      for (int k = 0; k < blocks_; ++k) copy_block(w, k);
-      return cudaSuccess;
-    }
+    if (e != cudaSuccess || helpers_wanted_ == 0) return e;
     while (done_.load(std::memory_order_acquire) < (round + 1) * blocks_) std::this_thread::yield();
     return cudaSuccess;
   }
 
  private:
+  void start() {
+    touching_.store(helpers_wanted_);
+    try {
+      while ((int)helpers_.size() < helpers_wanted_) helpers_.emplace_back([this] { helper(); });
+    } catch (...) {  // no more threads to be had: those that there are, or the calling one
+      touching_.fetch_sub(helpers_wanted_ - (int)helpers_.size());
+      helpers_wanted_ = (int)helpers_.size();
+    }
+  }
   void copy_block(uint32_t w, int k) {
     const uint64_t off = (uint64_t)k * block_, n = std::min(block_, n_ - off);
     memcpy(out_ + (size_t)w * n_ + off, staging_ + off, sizeof(float) * n);
   }
+  // The output's pages, 2 MiB (a huge page) at a time, until the first piece has landed.
+  void touch() {
+    constexpr uint64_t kSpan = 2u << 20, kPage = 4096;
+    const uint64_t first = reinterpret_cast<uintptr_t>(out_), last = first + n_ * order_.size() * sizeof(float);
+    while (landed_.load(std::memory_order_relaxed) == 0 && !stop_.load()) {
+      const uint64_t from = (first / kSpan + spans_.fetch_add(1)) * kSpan;
+      if (from >= last) return;
+      for (uint64_t p = std::max(from, first); p < std::min(from + kSpan, last); p = (p / kPage + 1) * kPage)
+        __atomic_fetch_or(reinterpret_cast<unsigned char*>(p), 0, __ATOMIC_RELAXED);
+    }
+  }
   void helper() {  // blocks are numbered through all windows of the call
+    touch();
+    touching_.fetch_sub(1);
     const int per_piece = (int)(piece_ / block_);
     for (;;) {
       const long long id = next_.fetch_add(1), round = id / blocks_;
       const int k = (int)(id - round * blocks_);
       const long long need = round * pieces_ + k / per_piece;
-      for (int idle = 0; landed_.load(std::memory_order_acquire) <= need; ++idle) {
+      // (nobody copies while another may still touch)
+      for (int idle = 0; landed_.load(std::memory_order_acquire) <= need || touching_.load(std::memory_order_acquire) > 0; ++idle) {
         if (stop_.load()) return;
         if (idle < 64) std::this_thread::yield();
         else std::this_thread::sleep_for(std::chrono::microseconds(5));
@@ -138,7 +163,7 @@ class LogitsCopy {
     }
   }
   float* out_;
-  uint64_t n_, block_ = 16384, piece_ = 0;  // floats
+  uint64_t n_, block_ = 0, piece_ = 0;  // floats
   float* staging_;
   cudaEvent_t* events_;
   int pieces_ = 0, blocks_ = 0, helpers_wanted_ = 0;
@@ -146,6 +171,8 @@ class LogitsCopy {
   std::vector<uint32_t> order_;  // window of every round
   std::vector<std::thread> helpers_;
   std::atomic<long long> landed_{0}, next_{0}, done_{0};
+  std::atomic<uint64_t> spans_{0};
+  std::atomic<int> touching_{0};
   std::atomic<bool> stop_{false};
 };
 

@@ -211,3 +211,22 @@ def test_evaluation_loss_counts_a_tile_of_nan_logits():
         loss, n = e.eval_loss(window)
         assert n == 31 and loss / n == pytest.approx(-np.log(1e-10), abs=1e-3)
     e.close()
+
+
+@pytest.mark.parametrize("vocab,seq", [(2048, 132), (4096, 96), (20008, 128)])
+def test_eval_logits_by_several_threads(vocab, seq):
+    """Windows of 1 to 10 MiB, copied by several threads in pieces and blocks that the size is no multiple of, into fresh memory and
+    into the middle of an array whose other values must stay; against page-locked memory, which takes the download directly."""
+    e = ane.open(ane.Options(dim=64, hidden=64, n_layers=1, n_heads=1, n_kv_heads=1, vocab=vocab, seq=seq, batch=2, arch=ane.ARCH_LLAMA,
+                             quirks=0, compute_dtype=ane.DTYPE_BF16))
+    e.import_tensor(ane.T_EMBED, 0, np.random.default_rng(7).standard_normal((vocab, 64)).astype(np.float32))
+    for count in (1, 3):
+        windows = O.zipf_tokens(count * seq, vocab, 11)
+        want = e.eval_logits(windows, out=ane.pinned_empty((count, vocab, seq)))
+        for _ in range(3):
+            np.testing.assert_array_equal(e.eval_logits(windows), want)
+            held = np.full(want.size + 12, -7.0, np.float32)
+            e.eval_logits(windows, out=held[5:5 + want.size].reshape(want.shape))
+            np.testing.assert_array_equal(held[5:-7], want.ravel())
+            assert (held[:5] == -7).all() and (held[-7:] == -7).all()
+    e.close()
