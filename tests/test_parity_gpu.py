@@ -206,8 +206,8 @@ def test_split_precision_step_meets_the_stated_tolerance(arch, quirks, extra):
 def test_split_precision_reference_network_full_size_two_steps():
     """The reference's own network at its own size and hyperparameters (see
     test_bf16_reference_network_full_size_two_steps), backward quirks on, in the split-precision mode: every
-    parameter gradient within 1e-2 and the loss within 1e-3 nats before and after an optimizer step -- the
-    stated tolerance on the tensor-core path, where plain bf16 operands give up to 5e-2."""
+    parameter gradient within 5e-4 (1.25e-4 measured: two operands of 2^-17 each and what the unscaled scores make of
+    them) and the loss within 1e-3 nats before and after an optimizer step, where plain bf16 operands give up to 5e-2."""
     cfg = dict(dim=768, hidden=2048, heads=12, layers=12, vocab=32000, seq=256)
     hyper = dict(lr=3e-4, adam_beta1=0.8, adam_beta2=0.95, adam_eps=1e-10, weight_decay=0.0, grad_clip=1.0,
                  loss_scale=256.0, accum_steps=1000)
@@ -225,7 +225,7 @@ def test_split_precision_reference_network_full_size_two_steps():
             rep = []
             worst = compare_grads(m, e, rep)
             print("worst gradients", sorted(rep, key=lambda x: -x[2])[:6])
-            assert worst < BF16_TOL, sorted(rep, key=lambda x: -x[2])[:5]
+            assert worst < 5e-4, sorted(rep, key=lambda x: -x[2])[:5]
         m.flush()
         e.flush()
     e.close()
