@@ -10,7 +10,7 @@
 // ANE graphs materialise [heads, seq, seq] probabilities (ane/mil_stories.go:383-432); these
 // kernels replace them.
 //
-// Layout: q|k|v packed token-major [M, (H+2KV)*64]; out [M, H*64]; lse, delta [B, H, seq].
+// Layout: q|k|v packed token-major [M, (H+2KV)*hd]; out [M, H*hd]; lse, delta [B, H, seq].
 #include <stdlib.h>
 
 #include "common.cuh"

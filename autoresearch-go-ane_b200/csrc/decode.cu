@@ -502,8 +502,10 @@ constexpr size_t kSmemLimit = 224 * 1024;  // beside the static arrays
 int decode_ctas(int sms, int Hd, int H, int KV, int hd) { return std::min(std::min(sms, 148), std::min((H + 2 * KV) * hd / 8, Hd / 8)) & ~3; }
 
 // Up to 8 sequences go to the kernel above where its whole rows fit (dim <= 1100 or so): one SM's part of a contraction costs
-// it little then, and nothing has to be exchanged in a cluster (16.4 ms against 19.9 for one sequence of the 110M model,
-// 19.9 against 21.0 for eight).  The others take the clusters.
+// it little then, and nothing has to be exchanged in a cluster.  Prompts of 37 tokens and 64 new ones, this kernel against
+// clusters, for 1 / 4 / 8 sequences: 13.2 / 13.6 / 14.6 against 18.6 / 18.8 / 19.2 ms (110M model), 8.5 / 8.6 / 8.9 against
+// 11.9 / 12.0 / 12.1 (dim 512), 6.7 / 6.5 / 6.6 against 8.2 / 8.4 / 8.5 (dim 288); with prompts of 512 and with grouped heads
+// alike.  The others take the clusters.
 bool in_clusters(int D, int Hd, int H, int KV, int hd, int batch, int sms) {
   const int ctas = decode_ctas(sms, Hd, H, KV, hd);
   return batch > kRows || ctas <= 0 || smem_bytes(D, Hd, hd, ctas, batch) > kSmemLimit;

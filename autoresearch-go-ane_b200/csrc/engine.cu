@@ -390,7 +390,7 @@ class EngineT final : public EngineBase {
   // The reference architecture's backward recomputes attention with unscaled scores
   // (ane/train_full.go:268-269), which amplifies operand rounding; its q/k/v stay in fp32.
   bool qkv_f32_ = false;
-  bool att_tc_ = false;  // tensor-core attention kernels (bf16 operands, head_dim 64)
+  bool att_tc_ = false;  // tensor-core attention kernels (bf16 operands, head_dim 32, 48 or 64)
   bool x3_ = false;      // fp32 engine whose GEMMs run as three bf16 tensor-core products (ANE_DTYPE_BF16X3)
   SplitScratch split_;   // its operand halves (one stream at a time: no side stream in this mode)
   bool decoding_ = false;  // forward() runs one KV-cached decode step

@@ -108,12 +108,15 @@ int gemm_bf16_grouped(const GemmDesc* ds, int n, void* slot, bool* built, int* d
 size_t gemm_group_slot_bytes();
 
 int gemm_num_sms();
+// Both: false + gemm_last_error() on failure.
 // 2-D tensor map over a row-major [outer, inner] buffer (row pitch ld elements) of bf16 (or fp32) with a
-// 128B-swizzled [box_outer, box_inner] box; cached per (device, arguments).  False + gemm_last_error() on failure.
-bool make_tmap_weights(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t rows, uint64_t layers, uint64_t layer_stride,
-                       uint32_t box_inner, uint32_t box_rows);
+// 128B-swizzled [box_outer, box_inner] box; cached per thread and (device, arguments).
 bool make_tmap_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner,
                   uint32_t box_outer, bool is_f32);
+// 3-D tensor map over bf16 matrices [layers][rows][inner] with dense rows, layer_stride elements from one to the next; boxes of
+// [1][box_rows][box_inner], not swizzled, not cached.
+bool make_tmap_weights(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t rows, uint64_t layers, uint64_t layer_stride,
+                       uint32_t box_inner, uint32_t box_rows);
 const char* gemm_last_error();
 
 }  // namespace ane

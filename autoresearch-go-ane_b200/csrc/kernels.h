@@ -136,7 +136,7 @@ int decode_batch_steps(DecodeArgs a, int sms, cudaStream_t s);
 
 // Tensor-core causal attention (bf16 operands; head_dim 32, 48 or 64; see attention_tc.cu).
 bool attention_tc_supported(int hd);
-// `out_lo` (optional, [M, H*64] like `out`) receives bf16(O - bf16(O)): given to the backward as well, it makes
+// `out_lo` (optional, [M, H*hd] like `out`) receives bf16(O - bf16(O)): given to the backward as well, it makes
 // delta = rowsum(dO * O) as accurate as an fp32 O would (with bf16 O alone that rounding is the largest
 // error of dQ).
 void attention_forward_tc(const bf16* qkv, bf16* out, bf16* out_lo, float* lse, int B, int seq, int H, int KV, int hd, float scale,
