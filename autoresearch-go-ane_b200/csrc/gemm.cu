@@ -240,8 +240,13 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   const int whole = GemmCfg<BN, MT>::SPLIT ? split_k : 1;  // schedule of the epilogues that need whole tiles
   CUtensorMap tc;
   if (d.out == GEMM_OUT_BF16) {
-    if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false)) return -2;
-    return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
+    if constexpr (!GemmCfg<BN, MT>::SPLIT) {
+      if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false)) return -2;
+      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
+    } else {
+      g_gemm_err = "tiles shared by a cluster are built for the fp32 store and the activations' backward";
+      return -2;
+    }
   }
   if (d.out == GEMM_OUT_BF16_TGT) {
     if constexpr (!A_MN && !B_MN) {
@@ -355,7 +360,11 @@ static int dispatch_layout(const GemmDesc& d, int split_k, int* d_status, cudaSt
   if (!d.b_mn) ok = make_tmap(&tb, d.B, k_extent, d.N, d.ldb, GEMM_BK, GemmCfg<BN, MT>::PAIR ? BN / 2 : BN);
   else         ok = make_tmap(&tb, d.B, d.N, k_extent, d.ldb, 64, GEMM_BK);
   if (!ok) return -2;
-  if constexpr (GemmCfg<BN, MT>::PAIR || GemmCfg<BN, MT>::SPLIT) {  // forward and dX forms only (A K-major)
+  if constexpr (GemmCfg<BN, MT>::SPLIT) {  // dX form only: see cluster_split()
+    if (!d.a_mn && d.b_mn) return dispatch_epi<BN, MT, false, true>(ta, tb, d, split_k, d_status, stream);
+    g_gemm_err = "tiles shared by a cluster: unsupported operand layout";
+    return -2;
+  } else if constexpr (GemmCfg<BN, MT>::PAIR) {  // forward and dX forms only (A K-major)
     if (!d.a_mn && !d.b_mn) return dispatch_epi<BN, MT, false, false>(ta, tb, d, split_k, d_status, stream);
     if (!d.a_mn && d.b_mn) return dispatch_epi<BN, MT, false, true>(ta, tb, d, split_k, d_status, stream);
     g_gemm_err = "cluster tiles: unsupported operand layout";
@@ -488,7 +497,7 @@ static int resident_clusters(int size) {
   const int at = size == 8 ? 3 : size == 4 ? 2 : 1;
   if (known[at] == 0) {
     using Cfg = GemmCfg<128, GEMM_MT_SPLIT>;
-    auto kern = gemm_tc_kernel<128, GEMM_MT_SPLIT, false, false, EPI_STORE_F32>;
+    auto kern = gemm_tc_kernel<128, GEMM_MT_SPLIT, false, true, EPI_STORE_F32>;
     const int bytes = (int)Cfg::smem_bytes(false);
     int n = 0;
     cudaLaunchConfig_t q = {};
@@ -511,17 +520,19 @@ static int resident_clusters(int size) {
   return known[at];
 }
 // How many CTAs share a 128 x 128 tile (0: none): as many as stay resident together with at least four k-blocks each (the
-// exchange costs about as much as four).  The bf16 epilogues without input pieces are short and have only two 64-column
-// pieces to share (SwiGLU forward: one pair), so there the exchange costs more than it saves for short K: excluded; measured
-// on the one-window step with the bf16 store / SwiGLU left out, 2552 -> 2535 / 2522 us.
-// Split-precision products keep one accumulator for the whole contraction.  Parts have less of the tensor core's truncation, so
-// a product would depend on the tiles there are beside it, and the unscaled scores of the reference's backward carry that
-// far: after two updates of the reference network at 2 x 256 gradients were up to 2.2e-3 from those of whole tiles, where
-// the mode is to hold 1e-3 (6.5 ms a step with clusters, 7.8 without).
+// exchange costs about as much as four).  Parts of a contraction have less of the tensor core's truncation than the whole, so
+// a product then depends, by its rounding, on how many tiles there are beside it.  Where that may be:
+//   * Backward products towards the inputs (B MN-major, with or without an activation's backward in the epilogue): one window of
+//     the 110M model 3.05 -> 2.62 ms a step, two 3.15 -> 2.75, four 3.30 -> 3.19.
+//   * Not the forward ones.  A window's activations are the same whatever batch it comes in; shared tiles for q|k|v and the
+//     fp32 stores would give 2.47, 2.61 and 3.08 ms, but moved the logits of one window by 4e-3 from those of a large batch.
+//   * Not split precision, whose backward carries a difference far through unscaled scores: after two updates of the reference
+//     network at 2 x 256 gradients were up to 2.2e-3 from those of whole tiles, where the mode is to hold 1e-3 (6.5 ms a step
+//     with clusters, 7.8 without).
 static int cluster_split(const GemmDesc& d) {
   static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_CLUSTER_SPLIT"); return e && e[0] == '0'; }();  // A/B measurements
-  if (off || d.a_mn || d.seg_kb > 0) return 0;
-  if (d.out != GEMM_OUT_F32 && d.out != GEMM_OUT_BF16_ROPE && d.out != GEMM_OUT_DSWIGLU && d.out != GEMM_OUT_DRELU2) return 0;
+  if (off || d.a_mn || !d.b_mn || d.seg_kb > 0) return 0;
+  if (d.out != GEMM_OUT_F32 && d.out != GEMM_OUT_DSWIGLU && d.out != GEMM_OUT_DRELU2) return 0;
   const long tiles = (long)((d.M + 127) / 128) * ((d.N + 127) / 128);
   const int kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;
   for (int s : {8, 4, 2})

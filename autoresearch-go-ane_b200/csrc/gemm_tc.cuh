@@ -47,7 +47,7 @@ static constexpr int GEMM_MT_PAIR2 = 5;
 // token rows: 12 tiles of 128 x 128 for N = 768) the k-blocks of a tile are a serial chain on one SM, 64 of them for
 // K = 4096; split, each CTA runs its share, parks its fp32 accumulators in its own shared memory (the pipeline stages
 // are free by then), and after one cluster barrier every CTA finishes its share of the tile's pieces, summing the
-// partial sums over distributed shared memory in rank order.  No workspace, no atomics; every epilogue kind works.
+// partial sums over distributed shared memory in rank order.  No workspace, no atomics.  Built for the dX form: see cluster_split().
 static constexpr int GEMM_MT_SPLIT = 6;
 static constexpr uint32_t GEMM_TMARES_BYTES = 4 * 2 * 4096;
 static constexpr uint32_t GEMM_SMEM_LIMIT = 232448u;
@@ -539,11 +539,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t res_base = smem_stage0 + Cfg::staging_bytes(EW) + (uint32_t)(warp - 2) * (uint32_t)(RD * 4096);
     // with eight warps, warps 2-5 take the first half of the tile's columns and warps 6-9 the second
     constexpr int CSPAN = BN / (EW / 4);
-    // CTAs that share a tile take its pieces in turns (SwiGLU forward: pairs of pieces, which make one gate piece)
-    constexpr int CGRP = EPI == EPI_STORE_BF16_SWIGLU ? 2 * CW : CW;
+    // CTAs that share a tile take its pieces in turns
     const int part = SPLIT ? (int)blockIdx.x % parts : 0;
-    const int c_begin = ((warp - 2) >> 2) * CSPAN + part * CGRP, c_end = ((warp - 2) >> 2) * CSPAN + CSPAN;
-    auto c_next = [&](int c) { return (!SPLIT || (CGRP > CW && ((c / CW) & 1) == 0)) ? c + CW : c + CW + (parts - 1) * CGRP; };
+    const int c_begin = ((warp - 2) >> 2) * CSPAN + part * CW, c_end = ((warp - 2) >> 2) * CSPAN + CSPAN;
+    auto c_next = [&](int c) { return c + CW * parts; };
     const uint8_t* res_ptr = smem_raw + (res_base - smem_u32(smem_raw));
     uint32_t res_uses = 0;  // pieces consumed so far (buffer = uses % RD, phase = (uses / RD) & 1)
     GemmSched sched;

@@ -230,3 +230,23 @@ def test_eval_logits_by_several_threads(vocab, seq):
             np.testing.assert_array_equal(held[5:-7], want.ravel())
             assert (held[:5] == -7).all() and (held[-7:] == -7).all()
     e.close()
+
+
+@pytest.mark.parametrize("arch,dtype", [(ane.ARCH_LLAMA, ane.DTYPE_BF16), (ane.ARCH_REFERENCE, ane.DTYPE_BF16), (ane.ARCH_LLAMA, ane.DTYPE_BF16X3)])
+def test_logits_of_a_window_do_not_depend_on_its_batch(arch, dtype):
+    """Forward products on the tensor cores have one accumulator for the whole contraction, and the other kernels go row by row or
+    head by head: the logits of a window are the same, bit for bit, alone and among others."""
+    cfg = dict(dim=768, hidden=2048, heads=12, layers=2, vocab=512, seq=256)
+    rng = np.random.default_rng(9)
+    windows = O.zipf_tokens(24 * cfg["seq"], cfg["vocab"], 13)
+    logits = []
+    for batch in (1, 2, 24):
+        e = ane.open(_options(cfg, batch=batch, arch=arch, quirks=0, compute_dtype=dtype))
+        rng = np.random.default_rng(9)
+        for tid in (ane.T_EMBED, ane.T_WQ, ane.T_WK, ane.T_WV, ane.T_WO, ane.T_W1, ane.T_W2) + ((ane.T_W3,) if arch == ane.ARCH_LLAMA else ()):
+            for layer in range(1 if tid == ane.T_EMBED else cfg["layers"]):
+                e.import_tensor(tid, layer, (0.05 * rng.standard_normal(e.tensor_size(tid, layer))).astype(np.float32))
+        logits.append(e.eval_logits(windows)[:2])
+        e.close()
+    np.testing.assert_array_equal(logits[0], logits[1])
+    np.testing.assert_array_equal(logits[0], logits[2])
