@@ -493,9 +493,9 @@ static GemmPlan plan_gemm(const GemmDesc& d, int sms) {
 
 // Clusters of `size` CTAs of the split kernels that the device holds at once (one CTA per SM).
 static int resident_clusters(int size) {
-  static int known[4] = {0, 0, 0, 0};
+  static int known[4] = {-1, -1, -1, -1};
   const int at = size == 8 ? 3 : size == 4 ? 2 : 1;
-  if (known[at] == 0) {
+  if (known[at] < 0) {
     using Cfg = GemmCfg<128, GEMM_MT_SPLIT>;
     auto kern = gemm_tc_kernel<128, GEMM_MT_SPLIT, false, true, EPI_STORE_F32>;
     const int bytes = (int)Cfg::smem_bytes(false);
@@ -512,8 +512,8 @@ static int resident_clusters(int size) {
     q.attrs = a;
     q.numAttrs = 1;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, kern, &q) != cudaSuccess || n <= 0)
-      n = gemm_num_sms() / size;
+        cudaOccupancyMaxActiveClusters(&n, kern, &q) != cudaSuccess)
+      n = 0;  // a part of a GPU may hold no cluster of this size: products take whole tiles there
     cudaGetLastError();
     known[at] = std::min(n, gemm_num_sms() / size);
   }
