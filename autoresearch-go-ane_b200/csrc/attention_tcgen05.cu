@@ -191,7 +191,7 @@ attn5_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv_r, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       for (int it = 2; it < n_it; ++it) {
         const int s = it & 1;
         const uint32_t ph = (uint32_t)(it >> 1) & 1u;
@@ -201,7 +201,7 @@ attn5_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv_r, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_kk = a5_idesc(false, false);  // both operands K-major
       constexpr uint32_t idesc_kn = a5_idesc(false, true);   // B stored [k][n]
       bool ok = mbar_wait(smem_u32(&bar_r), 0, status, DEV_MBAR_TIMEOUT_MMA);
@@ -531,7 +531,7 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv_r, const __grid_cons
   const uint32_t tmem_base = tmem_slot;  // S[0] S[1] O[0] O[1], 64 columns each
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int it = 2; it < n_it; ++it) {
         const int s = it & 1;
         const uint32_t ph = (uint32_t)(it >> 1) & 1u;
@@ -540,7 +540,7 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv_r, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_kk = a5_idesc(false, false);
       constexpr uint32_t idesc_kn = a5_idesc(false, true);
       auto issue_scores = [&](int it) -> bool {
@@ -781,7 +781,7 @@ attn5_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_qkv_r, const __g
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int g = 0;  // blocks issued so far, over all units
       bool ok = true;
       for (int k = 0; ok; ++k) {
@@ -814,7 +814,7 @@ attn5_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_qkv_r, const __g
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_kk = a5_idesc(false, false);
       constexpr uint32_t idesc_kn = a5_idesc(false, true);
       auto issue_scores = [&](int gg) -> bool {
@@ -1101,7 +1101,7 @@ attn5_bwd_head_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       auto load = [&](uint32_t dst, const CUtensorMap* tm, uint32_t bar, int col, int row) {
         tma_load_2d(dst, tm, bar, col, row);
@@ -1189,7 +1189,7 @@ attn5_bwd_head_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t id_s = a5_idesc_n(false, false, 128);  // S, dP: both operands K-major, N = 128 keys
       constexpr uint32_t id_t = a5_idesc_n(true, true, 64);     // dV, dK: A = P^T / dS^T read M-major, B stored [k][n]
       constexpr uint32_t id_q = a5_idesc_n(false, true, 64);    // dQ: A = dS K-major, B = K stored [k][n]
@@ -1643,7 +1643,7 @@ attn5_bwd_split_kernel(const __grid_constant__ CUtensorMap tm_hi_r, const __grid
   const uint32_t tS = tmem_base, tDP = tmem_base + 64, tA1 = tmem_base + 128, tA2 = tmem_base + 192;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int it = 2; it < n_it; ++it) {
         const int s = it & 1;
         const uint32_t ph = (uint32_t)(it >> 1) & 1u;
@@ -1652,7 +1652,7 @@ attn5_bwd_split_kernel(const __grid_constant__ CUtensorMap tm_hi_r, const __grid
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_kk = a5_idesc(false, false);
       constexpr uint32_t idesc_kn = a5_idesc(false, true);
       bool ok = mbar_wait(smem_u32(&bar_r), 0, status, DEV_MBAR_TIMEOUT_MMA);

@@ -381,7 +381,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -459,7 +459,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((A_MN ? 1u : 0u) << 15) |
                                  ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(BN >> 3) << 17) |
                                  ((uint32_t)((PAIR ? 2 * GEMM_BM : GEMM_BM) >> 4) << 24);
@@ -579,7 +579,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       auto issue_res = [&](int m_w, int n0r) {
         if constexpr (kTmaRes) {
           if (n0r < N && n0r < tn * BN + c_end && m_w < M) {
-            if (lane == 0) {
+            if (elect_one()) {
               const uint32_t b = res_issued % (uint32_t)RD;
               const uint32_t bar = smem_u32(&bar_res[warp - 2][b]);
               mbar_expect_tx(bar, 4096);
@@ -754,7 +754,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         // The piece staged SBUF iterations ago must have been read by its TMA store before its
         // buffer is rewritten.
-        if (lane == 0) tma_store_wait_read<SBUF - 1>();
+        if (elect_one()) tma_store_wait_read<SBUF - 1>();
         __syncwarp();
         uint8_t* row_ptr = stage_ptr + sbuf * 4096 + lane * 128;
         if constexpr (EPI == EPI_CE_GRAD) {
@@ -892,7 +892,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               }
               fence_proxy_async_smem();
               __syncwarp();
-              if (lane == 0) {
+              if (elect_one()) {
                 tma_store_2d(&tmD, stage_base + (uint32_t)sbuf * 4096u, (n0 - CW) >> 1, m_warp);
                 tma_store_commit();
                 tma_store_wait_read<SBUF - 1>();  // the next buffer in the rotation is free again
@@ -917,7 +917,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) {
+            if (elect_one()) {
               tma_store_2d(&tmD, stage_base + (uint32_t)sbuf * 4096u, n0, m_warp);
               tma_store_commit();
               tma_store_wait_read<SBUF - 1>();  // the next buffer in the rotation is free again
@@ -996,7 +996,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           ++res_uses;
           issue_res(m_warp, n0 + RD * CW * parts);
         }
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t src = stage_base + (uint32_t)sbuf * 4096u;
           if constexpr (EPI == EPI_REDUCE_F32) tma_reduce_add_2d(pC, src, n0, m_warp);
           else if constexpr (EPI == EPI_DSWIGLU) tma_store_2d(&tmC, src, 2 * n0, m_warp);
@@ -1018,7 +1018,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
       ++local;
     }
-    if (lane == 0) tma_store_wait<0>();
+    if (elect_one()) tma_store_wait<0>();
   }
 
   tc_fence_before();
