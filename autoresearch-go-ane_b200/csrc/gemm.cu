@@ -154,12 +154,9 @@ static int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
                      const EpiParams& epi,
                      const GemmDesc& d, int split_k, int* d_status, cudaStream_t stream) {
   auto kern = gemm_tc_kernel<BN, MT, A_MN, B_MN, EPI>;
-  constexpr bool tma_res = (EPI == EPI_STORE_F32_TMARES || EPI == EPI_DSWIGLU || EPI == EPI_DRELU2);
-  constexpr int depth = GemmCfg<BN, MT>::res_depth(EPI);
-  constexpr int ew = GemmCfg<BN, MT>::epi_warps(EPI);
-  constexpr int threads = 64 + 32 * ew;
-  constexpr uint32_t smem_bytes = GemmCfg<BN, MT>::smem_bytes(tma_res, EPI == EPI_DSWIGLU || EPI == EPI_DRELU2, depth, ew);
-  static_assert(smem_bytes <= GEMM_SMEM_LIMIT && GemmCfg<BN, MT>::stages(tma_res, EPI == EPI_DSWIGLU || EPI == EPI_DRELU2, depth, ew) >= 3, "pipeline does not fit");
+  constexpr int threads = 64 + 32 * GemmCfg<BN, MT>::epi_warps(EPI);
+  constexpr uint32_t smem_bytes = GemmCfg<BN, MT>::smem_bytes(EPI);
+  static_assert(GemmCfg<BN, MT>::fits(EPI), "pipeline does not fit");
   static bool attr_set = false;  // per template instantiation
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
@@ -236,20 +233,22 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
                         int* d_status, cudaStream_t stream) {
   EpiParams epi{d.alpha, d.res1, d.s1, d.res2, d.s2, d.ldres, reinterpret_cast<bf16*>(d.aux), d.ldaux,
                 d.rope_cos, d.rope_sin, d.rope_seq, d.rope_pos0, d.rope_cols, d.tgt, d.tgt_out, d.tgt_row0,
-                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, d.seg_kb};
+                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, reinterpret_cast<float*>(d.C), d.ldc, d.seg_kb};
   const int whole = GemmCfg<BN, MT>::SPLIT ? split_k : 1;  // schedule of the epilogues that need whole tiles
+  constexpr bool NARROW = GemmCfg<BN, MT>::NARROW;
   CUtensorMap tc;
-  if (d.out == GEMM_OUT_BF16) {
-    if constexpr (!GemmCfg<BN, MT>::SPLIT) {
-      if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false)) return -2;
-      return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
-    } else {
-      g_gemm_err = "tiles shared by a cluster are built for the fp32 store and the activations' backward";
+  if constexpr (BN == 32 || GemmCfg<BN, MT>::SPLIT) {
+    if (d.out != GEMM_OUT_F32) {
+      g_gemm_err = "32-column tiles and tiles shared by a cluster are built for the fp32 store";
       return -2;
     }
+  } else {
+  if (d.out == GEMM_OUT_BF16) {
+    if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false)) return -2;
+    return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
   }
   if (d.out == GEMM_OUT_BF16_TGT) {
-    if constexpr (!A_MN && !B_MN) {
+    if constexpr (!A_MN && !B_MN && !NARROW) {
       if (d.tgt == nullptr || d.tgt_out == nullptr) {
         g_gemm_err = "target-logit epilogue: missing target pointers";
         return -2;
@@ -257,7 +256,7 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
       if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false)) return -2;
       return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_BF16_TGT>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
     } else {
-      g_gemm_err = "the target-logit epilogue takes K-major operands only";
+      g_gemm_err = "the target-logit epilogue takes K-major operands and tiles of at least 128 columns";
       return -2;
     }
   }
@@ -305,32 +304,33 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
     }
   }
   if (d.out == GEMM_OUT_DSWIGLU) {
-    if constexpr (!A_MN && B_MN && ((BN == 256 && (MT == 1 || MT == GEMM_MT_PAIR)) || MT == GEMM_MT_SPLIT)) {
+    if constexpr (!A_MN && B_MN && ((BN == 256 && (MT == 1 || MT == GEMM_MT_PAIR)) || NARROW)) {
       CUtensorMap td;  // h13 in, d h13 out: [M, 2N] bf16, pieces of 32 rows x 64 columns
       if (!make_tmap(&tc, d.C, 2 * (uint64_t)d.N, d.M, d.ldc, 64, 32, false) ||
           !make_tmap(&td, d.aux, 2 * (uint64_t)d.N, d.M, d.ldaux, 64, 32, false))
         return -2;
       return launch_tc<BN, MT, A_MN, B_MN, EPI_DSWIGLU>(ta, tb, tc, td, epi, d, whole, d_status, stream);
     } else {
-      g_gemm_err = "the SwiGLU-backward epilogue takes the dX form (A K-major, B MN-major) on 256-column tiles";
+      g_gemm_err = "the SwiGLU-backward epilogue takes the dX form (A K-major, B MN-major) on 64- and 256-column tiles";
       return -2;
     }
   }
   if (d.out == GEMM_OUT_DRELU2) {
-    if constexpr (!A_MN && B_MN && ((BN == 256 && (MT == 1 || MT == GEMM_MT_PAIR)) || MT == GEMM_MT_SPLIT)) {
+    if constexpr (!A_MN && B_MN && ((BN == 256 && (MT == 1 || MT == GEMM_MT_PAIR)) || NARROW)) {
       CUtensorMap td;  // h in, d h out: [M, N] bf16, pieces of 32 rows x 64 columns
       if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 64, 32, false) || !make_tmap(&td, d.aux, d.N, d.M, d.ldaux, 64, 32, false))
         return -2;
       return launch_tc<BN, MT, A_MN, B_MN, EPI_DRELU2>(ta, tb, tc, td, epi, d, whole, d_status, stream);
     } else {
-      g_gemm_err = "the ReLU^2-backward epilogue takes the dX form (A K-major, B MN-major) on 256-column tiles";
+      g_gemm_err = "the ReLU^2-backward epilogue takes the dX form (A K-major, B MN-major) on 64- and 256-column tiles";
       return -2;
     }
+  }
   }
   if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 32, 32, true)) return -2;
   if (d.out == GEMM_OUT_F32) {
     // One residual, K-major operands and room for the residual buffers: let TMA fetch the residual pieces.
-    if constexpr (!A_MN && !B_MN && GemmCfg<BN, MT>::smem_bytes(true) <= GEMM_SMEM_LIMIT && GemmCfg<BN, MT>::stages(true) >= 3) {
+    if constexpr (!A_MN && !B_MN && GemmCfg<BN, MT>::fits(EPI_STORE_F32_TMARES)) {
       static const bool no_tma_res = getenv("ANE_B200_NO_TMA_RES") != nullptr;  // A/B measurements
       if (d.res1 != nullptr && d.res2 == nullptr && !no_tma_res) {
         CUtensorMap td;
@@ -340,8 +340,8 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
     }
     return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_F32>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
   }
-  if constexpr (GemmCfg<BN, MT>::PAIR || GemmCfg<BN, MT>::SPLIT) {
-    g_gemm_err = "cluster tiles are built for the non-accumulating epilogues";
+  if constexpr (GemmCfg<BN, MT>::PAIR || GemmCfg<BN, MT>::SPLIT || BN == 32) {
+    g_gemm_err = "cluster tiles and 32-column tiles are built for the non-accumulating epilogues";
     return -2;
   } else {
     return launch_tc<BN, MT, A_MN, B_MN, EPI_REDUCE_F32>(ta, tb, tc, tc, epi, d, split_k, d_status, stream);
@@ -363,6 +363,10 @@ static int dispatch_layout(const GemmDesc& d, int split_k, int* d_status, cudaSt
   if constexpr (GemmCfg<BN, MT>::SPLIT) {  // dX form only: see cluster_split()
     if (!d.a_mn && d.b_mn) return dispatch_epi<BN, MT, false, true>(ta, tb, d, split_k, d_status, stream);
     g_gemm_err = "tiles shared by a cluster: unsupported operand layout";
+    return -2;
+  } else if constexpr (BN == 32) {
+    if (!d.a_mn && !d.b_mn) return dispatch_epi<BN, MT, false, false>(ta, tb, d, split_k, d_status, stream);
+    g_gemm_err = "32-column tiles: unsupported operand layout";
     return -2;
   } else if constexpr (GemmCfg<BN, MT>::PAIR) {  // forward and dX forms only (A K-major)
     if (!d.a_mn && !d.b_mn) return dispatch_epi<BN, MT, false, false>(ta, tb, d, split_k, d_status, stream);
@@ -498,7 +502,7 @@ static int resident_clusters(int size) {
   if (known[at] < 0) {
     using Cfg = GemmCfg<128, GEMM_MT_SPLIT>;
     auto kern = gemm_tc_kernel<128, GEMM_MT_SPLIT, false, true, EPI_STORE_F32>;
-    const int bytes = (int)Cfg::smem_bytes(false);
+    const int bytes = (int)Cfg::smem_bytes(EPI_STORE_F32);
     int n = 0;
     cudaLaunchConfig_t q = {};
     q.gridDim = dim3((unsigned)(size * 148));
@@ -519,24 +523,58 @@ static int resident_clusters(int size) {
   }
   return known[at];
 }
-// How many CTAs share a 128 x 128 tile (0: none): as many as stay resident together with at least four k-blocks each (the
-// exchange costs about as much as four).  Parts of a contraction have less of the tensor core's truncation than the whole, so
-// a product then depends, by its rounding, on how many tiles there are beside it.  Where that may be:
-//   * Backward products towards the inputs (B MN-major, with or without an activation's backward in the epilogue): one window of
-//     the 110M model 3.05 -> 2.62 ms a step, two 3.15 -> 2.75, four 3.30 -> 3.19.
-//   * Not the forward ones.  A window's activations are the same whatever batch it comes in; shared tiles for q|k|v and the
-//     fp32 stores would give 2.47, 2.61 and 3.08 ms, but moved the logits of one window by 4e-3 from those of a large batch.
+// Width of a narrow tile (64 or 32 columns; 0: none) for a product with less than a wave of 128 x 128 tiles.  One CTA per SM
+// then, and its time is that of its own chain: k-blocks of about 310 cycles at 32 columns, 340 at 64 and 370 at 128 (more SMs pull
+// operands, each of them less), and an epilogue of about 700 cycles per staged piece, four of them for 128 fp32 columns.  Every
+// element is the same sum in the same order whatever the width.  us, 128 columns -> narrow: 256 x 2304 x 768 (bf16) 6.7 -> 6.1,
+// 256 x 768 x 768 (fp32 + residual) 9.9 -> 5.5, 256 x 768 x 2048 13.7 -> 9.3, 512 x 768 x 6144 26.0 -> 20.9, 1000 x 288 x 288 8.7 -> 4.4,
+// SwiGLU backward of 256 x 2048 x 768 9.2 -> 7.5.
+static int narrow_width(const GemmDesc& d) {
+  static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_NARROW"); return e && e[0] == '0'; }();  // A/B measurements
+  if (off || d.split_k > 1) return 0;
+  const bool f32 = d.out == GEMM_OUT_F32 || d.out == GEMM_OUT_ACCUM;
+  if (!f32 && d.out != GEMM_OUT_DSWIGLU && d.out != GEMM_OUT_DRELU2 && d.out != GEMM_OUT_BF16 && d.out != GEMM_OUT_BF16_ROPE &&
+      d.out != GEMM_OUT_BF16_SWIGLU && d.out != GEMM_OUT_BF16_RELU2)
+    return 0;
+  const int sms = gemm_num_sms();
+  const long tiles_m = (d.M + GEMM_BM - 1) / GEMM_BM, kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;
+  if (tiles_m * ((d.N + 127) / 128) > sms) return 0;
+  // weight gradients over eight k-blocks or more share out the contraction instead (plan_gemm)
+  if (d.out == GEMM_OUT_ACCUM && kblocks >= 8) return 0;
+  int best_bn = 0;
+  long best = 0;
+  for (int bn : {128, 64, 32}) {
+    if (bn == 32 && (d.out != GEMM_OUT_F32 || d.a_mn || d.b_mn)) continue;
+    const long waves = (tiles_m * ((d.N + bn - 1) / bn) + sms - 1) / sms;
+    const long cost = waves * kblocks * (290 + 5 * bn / 8) + bn / (f32 || d.out == GEMM_OUT_DSWIGLU ? 32 : 64) * 700;
+    if (best == 0 || cost < best) {
+      best = cost;
+      best_bn = bn;
+    }
+  }
+  return best_bn < 128 ? best_bn : 0;
+}
+// How many CTAs share a 128 x 128 tile (0: none): as many as stay resident together with at least four k-blocks each, where that
+// beats one CTA per tile.  ns, fitted to the dX forms of 256, 512 and 1024 rows with 12 to 64 k-blocks: a split tile takes
+// 7000 + 256 per own k-block (the exchange takes about 2000 of them) and 700 more in halves (64 columns of direct stores per
+// thread), a narrow one 5000 + 180 per k-block.  us, whole -> split: 256 x 768 x 4096 16.4 -> 9.0 in eighths, 512 x 768 x 2304 11.5 ->
+// 9.5 in quarters, 1024 x 768 x 4096 17.3 -> 16.0 in halves.  (12.4, 11.3 and 18.0 while every CTA fetched the parts of its columns
+// from the others' shared memory, one after the other, and an eighth was 32 columns for four of them and none for the rest.)
+// Parts of a contraction have less of the tensor core's truncation than the whole, so a product then depends, by its rounding, on how
+// many tiles there are beside it.  Where that may be:
+//   * Backward products towards the inputs (B MN-major).
+//   * Not the forward ones.  A window's activations are the same whatever batch it comes in; shared tiles moved the logits of
+//     one window by 4e-3 from those of a large batch.
 //   * Not split precision, whose backward carries a difference far through unscaled scores: after two updates of the reference
-//     network at 2 x 256 gradients were up to 2.2e-3 from those of whole tiles, where the mode is to hold 1e-3 (6.5 ms a step
-//     with clusters, 7.8 without).
+//     network at 2 x 256 gradients were up to 2.2e-3 from those of whole tiles, where the mode is to hold 1e-3.
 static int cluster_split(const GemmDesc& d) {
   static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_CLUSTER_SPLIT"); return e && e[0] == '0'; }();  // A/B measurements
-  if (off || d.a_mn || !d.b_mn || d.seg_kb > 0) return 0;
-  if (d.out != GEMM_OUT_F32 && d.out != GEMM_OUT_DSWIGLU && d.out != GEMM_OUT_DRELU2) return 0;
+  if (off || d.a_mn || !d.b_mn || d.seg_kb > 0 || d.out != GEMM_OUT_F32) return 0;
   const long tiles = (long)((d.M + 127) / 128) * ((d.N + 127) / 128);
   const int kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;
+  const int whole = narrow_width(d) ? 5000 + 180 * kblocks : 6500 + 210 * kblocks;
   for (int s : {8, 4, 2})
-    if (kblocks >= 4 * s && tiles <= resident_clusters(s)) return s;
+    if (kblocks >= 4 * s && tiles <= resident_clusters(s) && 7000 + 256 * kblocks / s + (s == 2 ? 700 : 0) < whole) return s;
   return 0;
 }
 
@@ -569,7 +607,7 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
                    "output 16-byte aligned with pitches % 8 == 0";
       return -2;
     }
-    if (const int s = cluster_split(d)) return dispatch_layout<128, GEMM_MT_SPLIT>(d, -s, d_status, stream);
+    if (narrow_width(d) == 64) return dispatch_layout<64, 1>(d, 1, d_status, stream);
     // 256-column tiles: CTA pairs when they fill their waves (the step's shape), else one CTA per tile
     const int pairs = gemm_num_sms() / 2;
     const long tiles = (long)((d.M + 255) / 256) * ((d.N + 255) / 256);
@@ -595,6 +633,8 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
     return dispatch_layout<256, 1>(d, 1, d_status, stream);
   }
   if (const int s = cluster_split(d)) return dispatch_layout<128, GEMM_MT_SPLIT>(d, -s, d_status, stream);
+  if (const int bn = narrow_width(d))
+    return bn == 64 ? dispatch_layout<64, 1>(d, 1, d_status, stream) : dispatch_layout<32, 1>(d, 1, d_status, stream);
   GemmPlan p = plan_gemm(d, gemm_num_sms());
   if (d.out == GEMM_OUT_BF16_SWIGLU && p.bn == 192) p.bn = 256;  // gate rows pair up two 64-column pieces
   // CTA-pair tiles (256 x 256 per two SMs, half of the B tile per CTA): measured faster than both single-CTA
@@ -691,7 +731,7 @@ int gemm_bf16_grouped(const GemmDesc* ds, int n, void* slot, bool* built, int* d
     *built = true;
   }
   auto kern = gemm_tc_kernel<BN, MT, true, true, EPI_REDUCE_F32>;
-  constexpr uint32_t smem_bytes = GemmCfg<BN, MT>::smem_bytes(false);
+  constexpr uint32_t smem_bytes = GemmCfg<BN, MT>::smem_bytes(EPI_REDUCE_F32);
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess) {

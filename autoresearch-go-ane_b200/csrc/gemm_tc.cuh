@@ -46,73 +46,11 @@ static constexpr int GEMM_MT_PAIR2 = 5;
 // MT = GEMM_MT_SPLIT: a cluster of 2, 4 or 8 CTAs shares one 128 x BN tile along the contraction.  With few tiles (256
 // token rows: 12 tiles of 128 x 128 for N = 768) the k-blocks of a tile are a serial chain on one SM, 64 of them for
 // K = 4096; split, each CTA runs its share, parks its fp32 accumulators in its own shared memory (the pipeline stages
-// are free by then), and after one cluster barrier every CTA finishes its share of the tile's pieces, summing the
-// partial sums over distributed shared memory in rank order.  No workspace, no atomics.  Built for the dX form: see cluster_split().
+// are free by then) and copies to every CTA of the cluster the columns which that one finishes (bulk copies, each warp its own
+// rows, counted by the receiver's mbarrier); a CTA sums what it receives in rank order and stores its columns.  No
+// workspace, no atomics.  Built for the dX form: see cluster_split().
 static constexpr int GEMM_MT_SPLIT = 6;
-static constexpr uint32_t GEMM_TMARES_BYTES = 4 * 2 * 4096;
 static constexpr uint32_t GEMM_SMEM_LIMIT = 232448u;
-template <int BN, int MT>
-struct GemmCfg {
-  static constexpr bool PAIR = MT == GEMM_MT_PAIR || MT == GEMM_MT_PAIR2;
-  static constexpr bool SPLIT = MT == GEMM_MT_SPLIT;
-  static constexpr int SUBS = (MT == GEMM_MT_PAIR || SPLIT) ? 1 : (MT == GEMM_MT_PAIR2 ? 2 : MT);  // 128-row sub-tiles per CTA
-  static constexpr int BM_TILE = (PAIR ? 2 : 1) * SUBS * GEMM_BM;       // rows of a scheduled tile
-  static constexpr uint32_t A_BYTES = SUBS * GEMM_BM * GEMM_BK * 2;     // per CTA and stage
-  // a CTA of a pair holds half of the tile's B rows, rounded up to whole 64-column chunks (an MN-major half of
-  // 96 columns is loaded as two chunks, the second half used)
-  static constexpr int B_ROWS = PAIR ? ((BN / 2 + 63) / 64) * 64 : BN;
-  static constexpr uint32_t B_BYTES = B_ROWS * GEMM_BK * 2;
-  // Staged output pieces per epilogue warp (a buffer is reused once its TMA store has read it; four buffers
-  // measured no faster than two and cost a pipeline stage).
-  static constexpr int SBUF = 2;
-  static constexpr uint32_t STAGING_BYTES = 4 * SBUF * 4096;  // 4 epilogue warps x SBUF buffers x (32 rows x 128 B)
-  // Epilogue warps.  The epilogues that do arithmetic per element and move more than one piece per 64 accumulator
-  // columns (SwiGLU forward: h13 + gate; SwiGLU backward: h13 in, d h13 out) take longer than the 12-k-block main
-  // loop of their products with four warps (one per scheduler, ~750 cycles of fixed cost per piece).  With eight,
-  // two warps share each TMEM lane group and split the tile's columns (256-column CTA-pair tiles only).  Measured
-  // with ANE_B200_GEMM_EW8=1: the two warps of a scheduler then share its exponential unit and the pipeline drops
-  // to three stages, W2-dX 51 -> 46 us, W1|W3 forward 51 -> 56 us, the step unchanged; hence off by default.
-  __host__ __device__ static constexpr int epi_warps(int epi_kind) {
-    return (ANE_B200_GEMM_EW8 && PAIR && SUBS == 1 && BN == 256 && (epi_kind == 3 || epi_kind == 8)) ? 8 : 4;
-  }
-  __host__ __device__ static constexpr uint32_t staging_bytes(int ew) { return (uint32_t)ew * SBUF * 4096; }
-  // Pipeline depth.  Single-CTA kernels take what fits beside the staging buffers and use the TMA-fed residual
-  // epilogue only if its buffers still fit; pair kernels give up stages for them instead.
-  // `room`: also a single-CTA kernel gives up stages for the TMA-fed input pieces (an epilogue that cannot do without them)
-  // `depth`: input pieces each epilogue warp keeps in flight; `ew`: epilogue warps
-  __host__ __device__ static constexpr int stages(bool tma_res, bool room = false, int depth = 2, int ew = 4) {
-    const uint32_t res = (uint32_t)(ew * depth) * 4096u;
-    const uint32_t avail = GEMM_SMEM_LIMIT - 1024u - staging_bytes(ew) - (((PAIR || SPLIT || room) && tma_res) ? res : 0u);
-    const int n = (int)(avail / (A_BYTES + B_BYTES));
-    return n > 6 ? 6 : n;
-  }
-  __host__ __device__ static constexpr uint32_t smem_bytes(bool tma_res, bool room = false, int depth = 2, int ew = 4) {  // +1024: alignment
-    return stages(tma_res, room, depth, ew) * (A_BYTES + B_BYTES) + staging_bytes(ew) + 1024 +
-           (tma_res ? (uint32_t)(ew * depth) * 4096u : 0u);
-  }
-  // Input pieces (residual, h13) each epilogue warp keeps in flight.  Four instead of two measured no faster for the
-  // SwiGLU backward (its pieces arrive in time; the epilogue is bound by its arithmetic), so two everywhere.
-  __host__ __device__ static constexpr int res_depth(int) { return 2; }
-  static constexpr int ACC_COLS = SUBS * BN;                     // one accumulator set
-  static constexpr int NBUF = (2 * ACC_COLS <= 512) ? 2 : 1;     // TMEM accumulator sets
-  static constexpr uint32_t TMEM_COLS = (NBUF * ACC_COLS <= 256) ? 256 : 512;
-};
-
-// 64-bit shared-memory matrix descriptor (sm_100 format, version field = 1).
-__device__ __forceinline__ uint32_t pack2_bf16(float lo, float hi) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);            // start address, bits [0,14)
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;   // leading byte offset, bits [16,30)
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;   // stride byte offset, bits [32,46)
-  d |= (uint64_t)1 << 46;                              // descriptor version (Blackwell)
-  d |= (uint64_t)2 << 61;                              // layout type: 128-byte swizzle
-  return d;
-}
 
 // Epilogue kinds.  Every kind stages 32-row x 128-byte pieces of the accumulator in 128B-swizzled
 // shared memory and hands them to TMA, so global writes are full lines and edge tiles are clipped by
@@ -129,7 +67,7 @@ enum EpiKind : int {
   EPI_STORE_BF16_ROPE = 4,
   // C(fp32) = alpha*acc + s1*res1 with the residual pieces fetched by TMA (two 32-row x 128-byte buffers
   // per epilogue warp, two pieces ahead) instead of by per-thread row loads: the residual read then costs
-  // one bulk copy per piece.  Needs GEMM_TMARES_BYTES of shared memory beside the pipeline stages.
+  // one bulk copy per piece.  Needs shared memory for the pieces beside the pipeline stages.
   EPI_STORE_F32_TMARES = 5,
   // EPI_STORE_BF16 that also writes the accumulator of each row's target column in fp32.
   EPI_STORE_BF16_TGT = 6,
@@ -152,6 +90,75 @@ enum EpiKind : int {
   // map, one 32-row x 64-column piece per output piece: the ReLU^2 backward (ane/common.go:146) in the W2-dX epilogue.
   EPI_DRELU2 = 11,
 };
+template <int BN, int MT>
+struct GemmCfg {
+  static constexpr bool PAIR = MT == GEMM_MT_PAIR || MT == GEMM_MT_PAIR2;
+  static constexpr bool SPLIT = MT == GEMM_MT_SPLIT;
+  static constexpr int SUBS = (MT == GEMM_MT_PAIR || SPLIT) ? 1 : (MT == GEMM_MT_PAIR2 ? 2 : MT);  // 128-row sub-tiles per CTA
+  static constexpr int BM_TILE = (PAIR ? 2 : 1) * SUBS * GEMM_BM;       // rows of a scheduled tile
+  static constexpr uint32_t A_BYTES = SUBS * GEMM_BM * GEMM_BK * 2;     // per CTA and stage
+  // a CTA of a pair holds half of the tile's B rows, rounded up to whole 64-column chunks (an MN-major half of
+  // 96 columns is loaded as two chunks, the second half used)
+  static constexpr int B_ROWS = PAIR ? ((BN / 2 + 63) / 64) * 64 : BN;
+  static constexpr uint32_t B_BYTES = B_ROWS * GEMM_BK * 2;
+  // Narrow tiles (32 or 64 columns, one CTA): the forms for products with few tiles, see narrow_width().  They stage no more
+  // pieces than a tile has and spend the room on stages: a stage holds 20 or 24 KB, and what hides the latency of operands from
+  // DRAM is the bytes in flight (K = 6144 on 32 columns: 28.9 us with four stages, 20.8 with eight).
+  static constexpr bool NARROW = BN < 128;
+  // Staged output pieces per epilogue warp (a buffer is reused once its TMA store has read it; four buffers
+  // measured no faster than two and cost a pipeline stage).
+  __host__ __device__ static constexpr int sbuf(int epi) { return NARROW && epi != EPI_STORE_BF16_RELU2 ? 1 : 2; }
+  // Epilogue warps.  The epilogues that do arithmetic per element and move more than one piece per 64 accumulator
+  // columns (SwiGLU forward: h13 + gate; SwiGLU backward: h13 in, d h13 out) take longer than the 12-k-block main
+  // loop of their products with four warps (one per scheduler, ~750 cycles of fixed cost per piece).  With eight,
+  // two warps share each TMEM lane group and split the tile's columns (256-column CTA-pair tiles only).  Measured
+  // with ANE_B200_GEMM_EW8=1: the two warps of a scheduler then share its exponential unit and the pipeline drops
+  // to three stages, W2-dX 51 -> 46 us, W1|W3 forward 51 -> 56 us, the step unchanged; hence off by default.
+  __host__ __device__ static constexpr int epi_warps(int epi) {
+    return (ANE_B200_GEMM_EW8 && PAIR && SUBS == 1 && BN == 256 && (epi == EPI_STORE_BF16_SWIGLU || epi == EPI_DSWIGLU)) ? 8 : 4;
+  }
+  // Epilogues that read an input piece per output piece by TMA (residual, h13, h), and those of them that cannot do without.
+  __host__ __device__ static constexpr bool tma_in(int epi) { return epi == EPI_STORE_F32_TMARES || epi == EPI_DSWIGLU || epi == EPI_DRELU2; }
+  __host__ __device__ static constexpr bool needs_in(int epi) { return epi == EPI_DSWIGLU || epi == EPI_DRELU2; }
+  // Input pieces each epilogue warp keeps in flight.  Four instead of two measured no faster for the SwiGLU backward (its
+  // pieces arrive in time; the epilogue is bound by its arithmetic), so two, or all that a narrow tile has.
+  __host__ __device__ static constexpr int res_depth(int epi) { return BN <= (epi == EPI_DRELU2 ? 64 : 32) ? 1 : 2; }
+  __host__ __device__ static constexpr uint32_t staging_bytes(int epi) { return (uint32_t)(epi_warps(epi) * sbuf(epi)) * 4096u; }
+  __host__ __device__ static constexpr uint32_t in_bytes(int epi) { return tma_in(epi) ? (uint32_t)(epi_warps(epi) * res_depth(epi)) * 4096u : 0u; }
+  static constexpr uint32_t EXCHANGE_BYTES = SPLIT ? GEMM_BM * BN * 4u : 0u;  // partial sums that a CTA of a split tile receives
+  // Pipeline depth.  Single-CTA kernels take what fits beside the staging buffers and use the TMA-fed residual epilogue only if
+  // its buffers still fit; pair kernels and narrow tiles give up stages for them instead.  Split tiles keep the exchange beside
+  // the stages and stage no output.
+  __host__ __device__ static constexpr int stages(int epi) {
+    const uint32_t own = SPLIT ? 1024u + EXCHANGE_BYTES : 1024u + staging_bytes(epi) + (PAIR || NARROW || needs_in(epi) ? in_bytes(epi) : 0u);
+    const int n = (int)((GEMM_SMEM_LIMIT - own) / (A_BYTES + B_BYTES)), most = NARROW ? 8 : 6;
+    return n > most ? most : n;
+  }
+  __host__ __device__ static constexpr uint32_t smem_bytes(int epi) {  // +1024: alignment
+    return stages(epi) * (A_BYTES + B_BYTES) + 1024 + (SPLIT ? EXCHANGE_BYTES : staging_bytes(epi) + in_bytes(epi));
+  }
+  __host__ __device__ static constexpr bool fits(int epi) { return smem_bytes(epi) <= GEMM_SMEM_LIMIT && stages(epi) >= 3; }
+  static constexpr int ACC_COLS = SUBS * BN;                     // one accumulator set
+  static constexpr int NBUF = (2 * ACC_COLS <= 512) ? 2 : 1;     // TMEM accumulator sets
+  static constexpr uint32_t TMEM_COLS = NARROW ? 2 * BN : (NBUF * ACC_COLS <= 256) ? 256 : 512;
+};
+
+// 64-bit shared-memory matrix descriptor (sm_100 format, version field = 1).
+__device__ __forceinline__ uint32_t pack2_bf16(float lo, float hi) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+
+__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);            // start address, bits [0,14)
+  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;   // leading byte offset, bits [16,30)
+  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;   // stride byte offset, bits [32,46)
+  d |= (uint64_t)1 << 46;                              // descriptor version (Blackwell)
+  d |= (uint64_t)2 << 61;                              // layout type: 128-byte swizzle
+  return d;
+}
+
 __device__ __forceinline__ float epi_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -174,6 +181,19 @@ __device__ __forceinline__ float epi_sigmoid(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * x));
   return fmaf(0.5f, t, 0.5f);
 }
+__device__ __forceinline__ float2 unpack2_bf16(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); }
+// Two elements of the activations' backward: d gate (fp32) and the saved h1 | h3 (h) to d h1 | d h3 (d h), packed bf16.
+__device__ __forceinline__ void dswiglu_pair(float dg0, float dg1, uint32_t h1, uint32_t h3, uint32_t& o1, uint32_t& o3) {
+  const float2 x = unpack2_bf16(h1), h = unpack2_bf16(h3);
+  // d silu = s (1 + x (1 - s)) with s = sigmoid(x)
+  const float s0 = epi_sigmoid(x.x), s1 = epi_sigmoid(x.y);
+  o1 = pack2_bf16(dg0 * h.x * s0 * (1.f + x.x * (1.f - s0)), dg1 * h.y * s1 * (1.f + x.y * (1.f - s1)));
+  o3 = pack2_bf16(dg0 * x.x * s0, dg1 * x.y * s1);
+}
+__device__ __forceinline__ uint32_t drelu2_pair(float two_alpha, float dg0, float dg1, uint32_t hv) {
+  const float2 h = unpack2_bf16(hv);
+  return pack2_bf16(two_alpha * dg0 * fmaxf(h.x, 0.f), two_alpha * dg1 * fmaxf(h.y, 0.f));
+}
 struct EpiParams {
   float alpha;
   const float* res1;  // optional fp32 [M, ldres]
@@ -195,6 +215,8 @@ struct EpiParams {
   int ce_rows;           // row count of the statistics buffer
   int ce_col0;           // vocabulary column of this product's column 0
   int ce_softcap;        // z = 15 tanh(logit / 15) (ane/common.go:272-287)
+  float* out;            // C and its pitch: split tiles store without a tensor map
+  int ldout;
   int seg_kb;            // > 0: operands are (hi | lo) halves of seg_kb k-blocks each, three passes hi*lo, lo*hi, hi*hi
 };
 
@@ -305,10 +327,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const int parts = SPLIT ? -split_k : 1;  // CTAs that share a tile
   const GemmGroup* grp = kGroup ? group : nullptr;
   int M = M0, N = N0;  // the epilogue of a grouped launch sets them per tile
-  constexpr bool kTmaRes = (EPI == EPI_STORE_F32_TMARES || EPI == EPI_DSWIGLU || EPI == EPI_DRELU2);  // an input piece per output piece, by TMA
+  constexpr bool kTmaRes = Cfg::tma_in(EPI);  // an input piece per output piece, by TMA
   constexpr int RD = Cfg::res_depth(EPI);  // input pieces in flight per epilogue warp
   constexpr int EW = Cfg::epi_warps(EPI);  // epilogue warps: 4, or 8 (two per TMEM lane group, half of the columns each)
-  constexpr int STAGES = Cfg::stages(kTmaRes, EPI == EPI_DSWIGLU || EPI == EPI_DRELU2, RD, EW);
+  constexpr int STAGES = Cfg::stages(EPI);
   constexpr int BM = Cfg::BM_TILE, BK = GEMM_BK;
   constexpr int NBUF = Cfg::NBUF;
   constexpr bool PAIR = Cfg::PAIR;
@@ -323,7 +345,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __shared__ __align__(8) uint64_t bar_tfull[NBUF];
   __shared__ __align__(8) uint64_t bar_tempty[NBUF];
   __shared__ uint32_t tmem_slot;
-  __shared__ __align__(8) uint64_t bar_res[8][4];  // TMA-fed input pieces (residual, h13): piece landed
+  __shared__ __align__(8) uint64_t bar_res[8][4];  // TMA-fed input pieces (residual, h13): piece landed; [0]: split tiles, sums landed
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_a0 = smem_base;
@@ -353,6 +375,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int b = 0; b < RD; ++b) mbar_init(smem_u32(&bar_res[w][b]), 1);
       tma_prefetch_desc(&tmD);
     }
+    if constexpr (SPLIT)
+      for (int w = 0; w < 4; ++w) {
+        mbar_init(smem_u32(&bar_res[0][w]), 1);
+        mbar_expect_tx(smem_u32(&bar_res[0][w]), Cfg::EXCHANGE_BYTES / 4);
+      }
     for (int b = 0; b < NBUF; ++b) {
       mbar_init(smem_u32(&bar_tfull[b]), 1);
       mbar_init(smem_u32(&bar_tempty[b]), (PAIR ? 2 : 1) * EW);  // the epilogue warps of both CTAs
@@ -374,7 +401,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   pdl_trigger();
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();  // the peer's barriers exist before anything signals them
+  if constexpr (PAIR || SPLIT) cluster_sync_all();  // the peers' barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
   pdl_wait();  // operands, residuals and C belong to earlier kernels: nothing above touched them
@@ -453,10 +480,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
       }
     }
-    if constexpr (SPLIT) {
-      __syncwarp();
-      cluster_sync_all();  // the epilogue warps' exchange
-    }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
     if (rank == 0 && elect_one()) {
@@ -512,10 +535,107 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         ++local;
       }
     }
-    if constexpr (SPLIT) {
+  } else if constexpr (SPLIT) {
+    // ------------------------------ epilogue warps of a split tile ------------------------------
+    const int g = warp & 3;  // TMEM lanes, and rows of the tile, [32 g, 32 g + 32)
+    const int part = (int)blockIdx.x % parts, cols = BN / parts;
+    GemmSched sched;
+    sched.init(M, N, K, BM, BN, split_k, sched_id, sched_n, grp);
+    int tm, tn, kb0, kb1;
+    sched.next(tm, tn, kb0, kb1);
+    const int m = tm * BM + g * 32 + lane, n_begin = tn * BN + part * cols;  // this thread's row and first column to finish
+    const float a1 = epi.res1 && epi.s1 ? *epi.s1 : 1.f, a2 = epi.res2 && epi.s2 ? *epi.s2 : 1.f;
+    bool ok = mbar_wait(smem_u32(&bar_tfull[0]), 0u, status, DEV_MBAR_TIMEOUT_EPILOGUE);
+    tc_fence_after();
+    // Partial sums as [row group][column / 4][row in the group] float4 over the pipeline stages, which the MMAs no longer need:
+    // the columns of one receiver are one piece of 512 * cols / 4 bytes per group.
+    const uint32_t parked = smem_base + (uint32_t)g * (BN / 4 * 512u), landed = smem_stage0 + (uint32_t)g * (BN / 4 * 512u);
+    const uint32_t piece = (uint32_t)cols / 4 * 512u;
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 32) {
+      float v[32];
       __syncwarp();
-      cluster_sync_all();
+      tmem_ld_32x32(tmem_base + ((uint32_t)(g * 32) << 16) + (uint32_t)c, v);
+      tmem_ld_wait();
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(parked + (uint32_t)(c / 4 + q) * 512u + (uint32_t)lane * 16u), "f"(v[4 * q]),
+                     "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
+                     : "memory");
     }
+    tc_fence_before();
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane < parts) {  // one copy per lane; every CTA receives the parts in rank order
+      const uint32_t to = (uint32_t)((lane + part) % parts);
+      bulk_copy_to_cta(map_to_cta(landed + (uint32_t)part * piece, to), parked + to * piece, piece, map_to_cta(smem_u32(&bar_res[0][g]), to));
+    }
+    __syncwarp();
+    // 16 columns at a time; what they are combined with is requested before the wait for the sums
+    static_assert(!SPLIT || EPI == EPI_STORE_F32, "split tiles are built for the fp32 store");
+    bool waited = false;
+#pragma unroll 1
+    for (int c = 0; c < cols; c += 16) {
+      const int n0 = n_begin + c;
+      const bool in = m < M && n0 < N;
+      float4 r1[4], r2[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        r1[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        r2[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      auto request = [&](float4 (&r)[4], const float* res) {
+        if (res == nullptr || !in) return;
+        const float* rp = res + (size_t)m * epi.ldres + n0;
+        if (n0 + 16 <= N) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) r[q] = *reinterpret_cast<const float4*>(rp + 4 * q);
+        } else {
+          float* f = reinterpret_cast<float*>(r);
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            if (n0 + e < N) f[e] = rp[e];
+        }
+      };
+      request(r1, epi.res1);
+      request(r2, epi.res2);
+      if (!waited) {
+        ok = mbar_wait(smem_u32(&bar_res[0][g]), 0u, status, DEV_MBAR_TIMEOUT_EPILOGUE) && ok;
+        waited = true;
+      }
+      float acc[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) acc[e] = 0.f;
+#pragma unroll 2
+      for (int p = 0; p < parts; ++p) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float4 t;
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
+                       : "r"(landed + (uint32_t)p * piece + (uint32_t)(c / 4 + q) * 512u + (uint32_t)lane * 16u) : "memory");
+          acc[4 * q] += t.x; acc[4 * q + 1] += t.y; acc[4 * q + 2] += t.z; acc[4 * q + 3] += t.w;
+        }
+      }
+      if (!in || !ok) continue;
+      float* out = epi.out + (size_t)m * epi.ldout + n0;
+      const float *f1 = reinterpret_cast<const float*>(r1), *f2 = reinterpret_cast<const float*>(r2);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        acc[e] *= epi.alpha;
+        if (epi.res1) acc[e] += a1 * f1[e];
+        if (epi.res2) acc[e] += a2 * f2[e];
+      }
+      if (n0 + 16 <= N) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          *reinterpret_cast<float4*>(out + 4 * q) = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+          if (n0 + e < N) out[e] = acc[e];
+      }
+    }
+    if (!waited) mbar_wait(smem_u32(&bar_res[0][g]), 0u, status, DEV_MBAR_TIMEOUT_EPILOGUE);
   } else {
     // ------------------------------ epilogue warps ------------------------------
     const int lane_group = warp & 3;  // TMEM lanes [32*lane_group, 32*lane_group+32)
@@ -524,7 +644,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                EPI == EPI_STORE_BF16_TGT || EPI == EPI_STORE_BF16_RELU2 || EPI == EPI_CE_STATS ||
                                EPI == EPI_CE_GRAD || EPI == EPI_DRELU2);
     constexpr int CW = kBf16Out ? 64 : 32;
-    constexpr int SBUF = Cfg::SBUF;
+    constexpr int SBUF = Cfg::sbuf(EPI);
     const uint32_t stage_base = smem_stage0 + (uint32_t)(warp - 2) * (uint32_t)(SBUF * 4096);
     uint8_t* stage_ptr = smem_raw + (stage_base - smem_u32(smem_raw));
     int local = 0;
@@ -536,13 +656,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (epi.res2) a2 = epi.s2 ? *epi.s2 : 1.f;
     }
     // EPI_STORE_F32_TMARES: this warp's two residual buffers, behind the store staging of all four warps
-    const uint32_t res_base = smem_stage0 + Cfg::staging_bytes(EW) + (uint32_t)(warp - 2) * (uint32_t)(RD * 4096);
+    const uint32_t res_base = smem_stage0 + Cfg::staging_bytes(EPI) + (uint32_t)(warp - 2) * (uint32_t)(RD * 4096);
     // with eight warps, warps 2-5 take the first half of the tile's columns and warps 6-9 the second
     constexpr int CSPAN = BN / (EW / 4);
-    // CTAs that share a tile take its pieces in turns
-    const int part = SPLIT ? (int)blockIdx.x % parts : 0;
-    const int c_begin = ((warp - 2) >> 2) * CSPAN + part * CW, c_end = ((warp - 2) >> 2) * CSPAN + CSPAN;
-    auto c_next = [&](int c) { return c + CW * parts; };
+    const int c_begin = ((warp - 2) >> 2) * CSPAN, c_end = c_begin + CSPAN;
     const uint8_t* res_ptr = smem_raw + (res_base - smem_u32(smem_raw));
     uint32_t res_uses = 0;  // pieces consumed so far (buffer = uses % RD, phase = (uses / RD) & 1)
     GemmSched sched;
@@ -591,32 +708,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       };
       if constexpr (kTmaRes) {  // first two pieces of sub-tile 0, while the MMAs still run
 #pragma unroll
-        for (int k = 0; k < RD; ++k) issue_res(tm * BM + sub_row(0) + lane_group * 32, tn * BN + c_begin + k * CW * parts);
+        for (int k = 0; k < RD; ++k) issue_res(tm * BM + sub_row(0) + lane_group * 32, tn * BN + c_begin + k * CW);
       }
-      const bool landed = mbar_wait(smem_u32(&bar_tfull[buf]), tphase, status, DEV_MBAR_TIMEOUT_EPILOGUE);
-      if (!SPLIT && !landed) {
+      if (!mbar_wait(smem_u32(&bar_tfull[buf]), tphase, status, DEV_MBAR_TIMEOUT_EPILOGUE)) {
         ok = false;
         break;
       }
       tc_fence_after();
-      if constexpr (SPLIT) {
-        // this CTA's partial sums as [column / 4][row] float4 over the pipeline stages, which the MMAs no longer need
-        const uint32_t mine = smem_base + (uint32_t)((lane_group * 32 + lane) * 16);
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          float v[32];
-          __syncwarp();
-          tmem_ld_32x32(tmem_base + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)c, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(mine + (uint32_t)((c / 4 + q) * GEMM_BM * 16)), "f"(v[4 * q]),
-                         "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
-                         : "memory");
-        }
-        __syncwarp();
-        cluster_sync_all();
-      }
 #pragma unroll 1
       for (int sub = 0; sub < SUBS; ++sub) {
       const int m_warp = tm * BM + sub_row(sub) + lane_group * 32;
@@ -625,7 +723,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         prefetch_first(m);
         if constexpr (kTmaRes) {
 #pragma unroll
-          for (int k = 0; k < RD; ++k) issue_res(m_warp, tn * BN + c_begin + k * CW * parts);
+          for (int k = 0; k < RD; ++k) issue_res(m_warp, tn * BN + c_begin + k * CW);
         }
       }
       int tgt_col = -1;        // EPI_STORE_BF16_TGT: this row's target column
@@ -657,30 +755,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const uint32_t taddr = tmem_base + ((uint32_t)(lane_group * 32) << 16) +
                              (uint32_t)(buf * Cfg::ACC_COLS + sub * BN);
 #pragma unroll 1
-      for (int c = c_begin; c < c_end; c = c_next(c)) {
+      for (int c = c_begin; c < c_end; c += CW) {
         const int n0 = tn * BN + c;
         if (n0 >= N || m_warp >= M) break;  // warp-uniform
         float acc[CW];
         __syncwarp();
-        if constexpr (SPLIT) {  // all CTAs' partial sums, in rank order
-          const uint32_t at = smem_base + (uint32_t)((c / 4 * GEMM_BM + lane_group * 32 + lane) * 16);
-#pragma unroll
-          for (int e = 0; e < CW; ++e) acc[e] = 0.f;
-#pragma unroll 1
-          for (int p = 0; p < parts; ++p) {
-            const uint32_t from = map_to_cta(at, (uint32_t)p);
-#pragma unroll
-            for (int q = 0; q < CW / 4; ++q) {
-              float4 t;
-              asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
-                           : "r"(from + (uint32_t)(q * GEMM_BM * 16)) : "memory");
-              acc[4 * q] += t.x; acc[4 * q + 1] += t.y; acc[4 * q + 2] += t.z; acc[4 * q + 3] += t.w;
-            }
-          }
-        } else {
-          tmem_ld_32x32(taddr + (uint32_t)c, acc);
-          if constexpr (CW == 64) tmem_ld_32x32(taddr + (uint32_t)c + 32u, acc + 32);
-        }
+        tmem_ld_32x32(taddr + (uint32_t)c, acc);
+        if constexpr (CW == 64) tmem_ld_32x32(taddr + (uint32_t)c + 32u, acc + 32);
         float4 cur[8];
         bool cur_ok = false;
         if constexpr (EPI == EPI_STORE_F32) {
@@ -688,15 +769,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
           for (int q = 0; q < 8; ++q) cur[q] = pre[q];
           pre_ok = false;
-          const int nn = tn * BN + c_next(c);
-          if (epi.res1 && m < M && c_next(c) < c_end && nn + 32 <= N) {
+          const int nn = n0 + CW;
+          if (epi.res1 && m < M && c + CW < c_end && nn + 32 <= N) {
             const float4* rp = reinterpret_cast<const float4*>(epi.res1 + (size_t)m * epi.ldres + nn);
 #pragma unroll
             for (int q = 0; q < 8; ++q) pre[q] = rp[q];
             pre_ok = true;
           }
         }
-        if constexpr (!SPLIT) tmem_ld_wait();
+        tmem_ld_wait();
         if constexpr (EPI == EPI_CE_STATS) {
           constexpr float kL2e = 1.4426950408889634f;
           const int t = tgt_col - epi.ce_col0 - n0;
@@ -809,18 +890,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           for (int q = 0; q < 8; ++q) hraw[q] = *reinterpret_cast<const uint4*>(hrow + ((q ^ (lane & 7)) << 4));
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const __nv_bfloat162* h1p = reinterpret_cast<const __nv_bfloat162*>(&hraw[q]);
-            const __nv_bfloat162* h3p = reinterpret_cast<const __nv_bfloat162*>(&hraw[q + 4]);
+            const uint32_t* h1p = reinterpret_cast<const uint32_t*>(&hraw[q]);
+            const uint32_t* h3p = reinterpret_cast<const uint32_t*>(&hraw[q + 4]);
             uint32_t o1[4], o3[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 x = __bfloat1622float2(h1p[e]), h = __bfloat1622float2(h3p[e]);
-              const float dg0 = epi.alpha * acc[8 * q + 2 * e], dg1 = epi.alpha * acc[8 * q + 2 * e + 1];
-              // d silu = s (1 + x (1 - s)) with s = sigmoid(x)
-              const float s0 = epi_sigmoid(x.x), s1 = epi_sigmoid(x.y);
-              o1[e] = pack2_bf16(dg0 * h.x * s0 * (1.f + x.x * (1.f - s0)), dg1 * h.y * s1 * (1.f + x.y * (1.f - s1)));
-              o3[e] = pack2_bf16(dg0 * x.x * s0, dg1 * x.y * s1);
-            }
+            for (int e = 0; e < 4; ++e)
+              dswiglu_pair(epi.alpha * acc[8 * q + 2 * e], epi.alpha * acc[8 * q + 2 * e + 1], h1p[e], h3p[e], o1[e], o3[e]);
             *reinterpret_cast<uint4*>(row_ptr + ((q ^ (lane & 7)) << 4)) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
             *reinterpret_cast<uint4*>(row_ptr + (((q + 4) ^ (lane & 7)) << 4)) = make_uint4(o3[0], o3[1], o3[2], o3[3]);
           }
@@ -834,14 +909,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const uint4 hraw = *reinterpret_cast<const uint4*>(hrow + ((q ^ (lane & 7)) << 4));
-            const __nv_bfloat162* hp = reinterpret_cast<const __nv_bfloat162*>(&hraw);
+            const uint32_t* hp = reinterpret_cast<const uint32_t*>(&hraw);
             uint32_t o[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 h = __bfloat1622float2(hp[e]);
-              const float two_a = 2.f * epi.alpha;
-              o[e] = pack2_bf16(two_a * acc[8 * q + 2 * e] * fmaxf(h.x, 0.f), two_a * acc[8 * q + 2 * e + 1] * fmaxf(h.y, 0.f));
-            }
+            for (int e = 0; e < 4; ++e) o[e] = drelu2_pair(2.f * epi.alpha, acc[8 * q + 2 * e], acc[8 * q + 2 * e + 1], hp[e]);
             *reinterpret_cast<uint4*>(row_ptr + ((q ^ (lane & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
           }
         } else if constexpr (kBf16Out) {
@@ -879,7 +950,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               const float h0 = epi.alpha * acc[32 + 2 * e], h1 = epi.alpha * acc[32 + 2 * e + 1];
               gcur[e] = pack2_bf16(x0 * h0 * epi_sigmoid(x0), x1 * h1 * epi_sigmoid(x1));
             }
-            if (((c / CW) & 1) == 0) {
+            if constexpr (Cfg::NARROW) {  // one piece per tile, half of a gate row: 64 bytes straight to memory
+              static_assert(BN == CW || !Cfg::NARROW, "narrow SwiGLU tiles hold one piece");
+              if (m < M) {
+                uint4* gp = reinterpret_cast<uint4*>(epi.aux + (size_t)m * epi.ldaux + (n0 >> 1));
+#pragma unroll
+                for (int q = 0; q < 4; ++q) gp[q] = make_uint4(gcur[4 * q], gcur[4 * q + 1], gcur[4 * q + 2], gcur[4 * q + 3]);
+              }
+            } else if (((c / CW) & 1) == 0) {
 #pragma unroll
               for (int e = 0; e < 16; ++e) gate_even[e] = gcur[e];
             } else {
@@ -994,7 +1072,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         __syncwarp();
         if constexpr (kTmaRes) {  // this residual buffer is free: fetch the piece after next
           ++res_uses;
-          issue_res(m_warp, n0 + RD * CW * parts);
+          issue_res(m_warp, n0 + RD * CW);
         }
         if (elect_one()) {
           const uint32_t src = stage_base + (uint32_t)sbuf * 4096u;

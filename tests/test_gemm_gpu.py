@@ -313,6 +313,40 @@ def test_activation_backward_on_tiles_shared_by_a_cluster(M, Hd, K):
     test_relu2_backward_fused_into_the_dx_product(M, Hd, K)
 
 
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn,out", [(1, 8, 72, 0, 0, 1), (129, 72, 520, 0, 0, 1), (256, 768, 2048, 0, 0, 1), (300, 40, 64, 0, 0, 0),
+                                                 (256, 2304, 768, 0, 0, 0), (200, 136, 520, 0, 1, 1), (256, 768, 768, 0, 1, 0),
+                                                 (136, 72, 200, 1, 1, 2), (768, 768, 256, 1, 1, 2)])
+def test_narrow_tiles_give_the_sums_of_wide_ones(M, N, K, a_mn, b_mn, out):
+    """Products with few tiles run on 64- or 32-column tiles (fp32 store, bf16 store, accumulation): against float64, and bit for bit
+    the same as those rows of a product large enough for wide tiles."""
+    rng = np.random.default_rng(M + N + K + out)
+    big = 32768 if a_mn else 8192
+    A = _bf16_round(rng.standard_normal((K, big) if a_mn else (big, K)).astype(np.float32) * 0.1)
+    B = _bf16_round(rng.standard_normal((K, N) if b_mn else (N, K)).astype(np.float32) * 0.1)
+    few = np.ascontiguousarray(A[:, :M] if a_mn else A[:M])
+    C = np.ones((big, N), np.float32)
+    run = lambda a, m: _bf16_result(a, B, m, N, K, b_mn) if out == 0 else _gemm(ane.DTYPE_BF16, a, B, C[:m], m, N, K, a_mn, b_mn, out)  # noqa: E731
+    got = run(few, M)
+    want = (few.T if a_mn else few).astype(np.float64) @ (B if b_mn else B.T).astype(np.float64) + (1.0 if out == 2 else 0.0)
+    assert rel_l2(got, want) < (4e-3 if out == 0 else 1e-5)
+    np.testing.assert_array_equal(got, run(A, big)[:M])
+
+
+def _bf16_result(A, B, M, N, K, b_mn):
+    dA, dB, dC = _up_bf16(A), _up_bf16(B), lib.ane_dev_malloc(M * N * 2)
+    g = _ffi.GemmArgs()
+    g.struct_size = ctypes.sizeof(_ffi.GemmArgs)
+    g.dtype = ane.DTYPE_BF16
+    g.d_a, g.d_b, g.d_c = dA, dB, dC
+    g.m, g.n, g.k, g.lda, g.ldb, g.ldc = M, N, K, K, N if b_mn else K, N
+    g.b_mn, g.out_mode, g.alpha = b_mn, 0, 1.0
+    _ck(lib.ane_op_gemm(ctypes.byref(g)))
+    got = _down_bf16(dC, (M, N))
+    for p in (dA, dB, dC):
+        lib.ane_dev_free(p)
+    return got
+
+
 def test_gemm_rejects_misaligned_pitch():
     A = np.zeros((16, 20), np.float32)  # 20 bf16 = 40 bytes per row: not a 16-byte multiple
     dA, dB, dC = _up_bf16(A), _up_bf16(A), _up(np.zeros((16, 16), np.float32))
