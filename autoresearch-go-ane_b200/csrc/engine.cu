@@ -319,7 +319,7 @@ class EngineT final : public EngineBase {
       cudaEventCreate(&e1);
       cudaEventRecord(e0, st);
     }
-    if constexpr (kIsF32) rc = x3_ ? gemm_bf16x3(d, &split_, d_status_, st) : gemm_f32(d, st);
+    if constexpr (kIsF32) rc = x3_ ? gemm_bf16x3(d, &split_, d_status_, st) : gemm_f32(d, st == stream_ ? &split_ : &dw_split_, d_status_, st);
     else rc = gemm_bf16(d, d_status_, st);
     if (profiling_) {
       cudaEventRecord(e1, st);
@@ -393,7 +393,9 @@ class EngineT final : public EngineBase {
   bool qkv_f32_ = false;
   bool att_tc_ = false;  // tensor-core attention kernels (bf16 operands, head_dim 32, 48 or 64)
   bool x3_ = false;      // fp32 engine whose GEMMs run as three bf16 tensor-core products (ANE_DTYPE_BF16X3)
-  SplitScratch split_;   // its operand halves (one stream at a time: no side stream in this mode)
+  SplitScratch split_;   // its operand halves, or the fp32 mode's operands in three parts (one stream at a time: no side stream in
+                         // the first of the two modes)
+  SplitScratch dw_split_;  // the same for the weight-gradient stream
   bool decoding_ = false;  // forward() runs one KV-cached decode step
   std::vector<T*> kcache_, vcache_;  // [B, S_, KV*hd] per layer (one block each for all layers), allocated by the first decode
   // scratch of the persistent decode kernel (bf16 engines)
@@ -529,7 +531,9 @@ void EngineT<T>::destroy() {
   if (stream_) cudaStreamSynchronize(stream_);
   if (comm_stream_) cudaStreamSynchronize(comm_stream_);  // weight gathers of the last update may still run
   dp_.shutdown();
+  if (dw_stream_) cudaStreamSynchronize(dw_stream_);
   split_.release();
+  dw_split_.release();
   for (void* p : allocs_) cudaFree(p);
   allocs_.clear();
   if (h_in_) cudaFreeHost(h_in_);

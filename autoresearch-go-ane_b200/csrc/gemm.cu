@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "gemm_f32_tc.cuh"
 #include "gemm_tc.cuh"
 
 namespace ane {
@@ -495,18 +496,15 @@ static GemmPlan plan_gemm(const GemmDesc& d, int sms) {
   return p;
 }
 
-// Clusters of `size` CTAs of the split kernels that the device holds at once (one CTA per SM).
-static int resident_clusters(int size) {
-  static int known[4] = {-1, -1, -1, -1};
+// Clusters of `size` (2, 4 or 8) CTAs of a kernel that takes an SM's shared memory that the device holds at once.
+template <class K>
+static int resident_clusters(K kern, int threads, uint32_t bytes, int size, int (&known)[4]) {
   const int at = size == 8 ? 3 : size == 4 ? 2 : 1;
   if (known[at] < 0) {
-    using Cfg = GemmCfg<128, GEMM_MT_SPLIT>;
-    auto kern = gemm_tc_kernel<128, GEMM_MT_SPLIT, false, true, EPI_STORE_F32>;
-    const int bytes = (int)Cfg::smem_bytes(EPI_STORE_F32);
     int n = 0;
     cudaLaunchConfig_t q = {};
     q.gridDim = dim3((unsigned)(size * 148));
-    q.blockDim = dim3(GEMM_THREADS);
+    q.blockDim = dim3((unsigned)threads);
     q.dynamicSmemBytes = bytes;
     cudaLaunchAttribute a[1];
     a[0].id = cudaLaunchAttributeClusterDimension;
@@ -515,13 +513,22 @@ static int resident_clusters(int size) {
     a[0].val.clusterDim.z = 1;
     q.attrs = a;
     q.numAttrs = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kern, &q) != cudaSuccess)
       n = 0;  // a part of a GPU may hold no cluster of this size: products take whole tiles there
     cudaGetLastError();
     known[at] = std::min(n, gemm_num_sms() / size);
   }
   return known[at];
+}
+static int resident_clusters(int size) {
+  static int known[4] = {-1, -1, -1, -1};
+  return resident_clusters(gemm_tc_kernel<128, GEMM_MT_SPLIT, false, true, EPI_STORE_F32>, GEMM_THREADS,
+                           GemmCfg<128, GEMM_MT_SPLIT>::smem_bytes(EPI_STORE_F32), size, known);
+}
+static int resident_clusters_f32(int size) {
+  static int known[4] = {-1, -1, -1, -1};
+  return resident_clusters(gemm_f32_tc_kernel<true, true, true>, F32TC_THREADS, F32TC_SMEM, size, known);
 }
 // Width of a narrow tile (64 or 32 columns; 0: none) for a product with less than a wave of 128 x 128 tiles.  One CTA per SM
 // then, and its time is that of its own chain: k-blocks of about 310 cycles at 32 columns, 340 at 64 and 370 at 128 (more SMs pull
@@ -765,24 +772,26 @@ size_t gemm_group_slot_bytes() { return sizeof(GemmGroup); }
 // Split-precision GEMM: fp32 operands as bf16 (hi, lo) pairs, three tensor-core products.
 // ------------------------------------------------------------------------------------------
 // Both operands of a product in one launch (blockIdx.y), four values per thread and step.  Operand [rows, cols] fp32
-// with row pitch ld; its halves lie behind one another along the contraction: for a K-major operand (k = cols)
+// with row pitch ld; its parts (hi, lo or hi, mid, lo) lie behind one another along the contraction: for a K-major operand (k = cols)
 // [rows][hi (kp) | lo (kp)], for an MN-major one (k = rows) [hi (kp rows) | lo (kp rows)][cols rounded up to 8].  kp =
-// k rounded up to a whole k-block; what lies past k is zero.
+// k rounded up to a whole k-block; what lies past k is zero.  Three parts are exactly the fp32 value (down to 2^-133, the last bit
+// of a bf16): what rounds to infinity is cut off instead, what is not finite has no further parts.
 struct SplitOperand {
   const float* src;
   bf16* dst;
   long long ld;
   int rows, cols, kp, pitch, k_major, vec;  // vec: float4 reads are aligned
 };
+template <int PARTS>
 __global__ void split_operands_kernel(const SplitOperand a, const SplitOperand b) {
   pdl_trigger();
   pdl_wait();
   const SplitOperand& o = blockIdx.y == 0 ? a : b;
   const int out_rows = o.k_major ? o.rows : o.kp, out_cols = o.k_major ? o.kp : o.pitch, per = out_cols / 4;
-  const size_t lo = o.k_major ? (size_t)o.kp : (size_t)o.kp * o.pitch;
+  const size_t next = o.k_major ? (size_t)o.kp : (size_t)o.kp * o.pitch;
   const long long total = (long long)out_rows * per;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(i / per), c = (int)(i - (long long)r * per) * 4;
+    const int r = total <= 0xFFFFFFFFll ? (int)((unsigned)i / (unsigned)per) : (int)(i / per), c = (int)(i - (long long)r * per) * 4;
     float x[4] = {0.f, 0.f, 0.f, 0.f};
     if (r < o.rows) {
       const float* p = o.src + (size_t)r * o.ld + c;
@@ -795,19 +804,29 @@ __global__ void split_operands_kernel(const SplitOperand a, const SplitOperand b
           if (c + e < o.cols) x[e] = p[e];
       }
     }
-    uint2 h, l;
-    uint32_t* hp = &h.x;
-    uint32_t* lp = &l.x;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const __nv_bfloat162 v = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
-      const __nv_bfloat162 w = __floats2bfloat162_rn(x[2 * e] - __bfloat162float(v.x), x[2 * e + 1] - __bfloat162float(v.y));
-      hp[e] = *reinterpret_cast<const uint32_t*>(&v);
-      lp[e] = *reinterpret_cast<const uint32_t*>(&w);
-    }
     bf16* q = o.dst + (size_t)r * o.pitch + c;
-    *reinterpret_cast<uint2*>(q) = h;
-    *reinterpret_cast<uint2*>(q + lo) = l;
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p, q += next) {
+      __nv_bfloat162 v[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        v[e] = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
+        if constexpr (PARTS == 3) {
+          bf16* part[2] = {&v[e].x, &v[e].y};
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            float& f = x[2 * e + t];
+            const bool finite = fabsf(f) <= 3.402823466e38f;
+            if (p == 0 && finite && fabsf(f) >= 3.3895e38f) *part[t] = __float2bfloat16_rz(f);
+            f = finite ? f - __bfloat162float(*part[t]) : 0.f;
+          }
+        } else {
+          x[2 * e] -= __bfloat162float(v[e].x);
+          x[2 * e + 1] -= __bfloat162float(v[e].y);
+        }
+      }
+      *reinterpret_cast<uint2*>(q) = make_uint2(*reinterpret_cast<const uint32_t*>(&v[0]), *reinterpret_cast<const uint32_t*>(&v[1]));
+    }
   }
 }
 
@@ -819,17 +838,10 @@ void SplitScratch::release() {
   }
 }
 
-// The three products run as one: its contraction is three passes of kp over (hi, lo), (lo, hi) and (hi, hi), so the
-// accumulators stay in tensor memory between them; the small cross terms come first, while the accumulators are small too.  (Three launches, the second and third adding to C in memory, and
-// two scalar conversion launches before them took 9.8 us each for 512 token rows.)
-int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t stream) {
-  if (d.M <= 0 || d.N <= 0 || d.K <= 0) return 0;
-  if (d.out != GEMM_OUT_F32 && d.out != GEMM_OUT_ACCUM) {
-    g_gemm_err = "split-precision GEMM writes fp32 (store or accumulate) only";
-    return -2;
-  }
+static constexpr int kNoScratch = -3;
+// The operands of `d` in `parts` bf16 parts each, in the scratch (which grows on demand).
+static int split_operands(const GemmDesc& d, int parts, SplitScratch* sc, SplitOperand (&o)[2], cudaStream_t stream) {
   const int kp = (d.K + GEMM_BK - 1) / GEMM_BK * GEMM_BK;
-  SplitOperand o[2];
   for (int i = 0; i < 2; ++i) {
     const bool mn = i == 0 ? d.a_mn : d.b_mn;
     const int outer = i == 0 ? d.M : d.N;
@@ -839,9 +851,9 @@ int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t
     o[i].cols = mn ? outer : d.K;
     o[i].kp = kp;
     o[i].k_major = mn ? 0 : 1;
-    o[i].pitch = mn ? (outer + 7) / 8 * 8 : 2 * kp;
+    o[i].pitch = mn ? (outer + 7) / 8 * 8 : parts * kp;
     o[i].vec = o[i].ld % 4 == 0 && (reinterpret_cast<uintptr_t>(o[i].src) & 15) == 0;
-    const size_t need = sizeof(bf16) * (size_t)(mn ? 2 * kp : outer) * o[i].pitch;
+    const size_t need = sizeof(bf16) * (size_t)(mn ? parts * kp : outer) * o[i].pitch;
     if (sc->cap[i] < need) {
       ++sc->generation;
       // the previous, smaller buffer may still be read by GEMMs in flight on this stream
@@ -853,8 +865,9 @@ int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t
       }
       const size_t bytes = need + need / 4 + 256;
       if (cudaMalloc(&sc->buf[i], bytes) != cudaSuccess) {
-        g_gemm_err = "split-precision GEMM: out of memory for the operand halves";
-        return -3;
+        cudaGetLastError();
+        g_gemm_err = "split-precision GEMM: out of memory for the operands' parts";
+        return kNoScratch;
       }
       sc->cap[i] = bytes;
     }
@@ -863,11 +876,28 @@ int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t
   const long long most = std::max((long long)(o[0].k_major ? o[0].rows : kp) * (o[0].k_major ? kp : o[0].pitch),
                                   (long long)(o[1].k_major ? o[1].rows : kp) * (o[1].k_major ? kp : o[1].pitch));
   const unsigned blocks = (unsigned)std::min<long long>(148 * 8, (most / 4 + 255) / 256);
-  launch_pdl(split_operands_kernel, dim3(blocks, 2), dim3(256), 0, stream, o[0], o[1]);
-  if (cudaGetLastError() != cudaSuccess) {
+  const cudaError_t e = parts == 2 ? launch_pdl(split_operands_kernel<2>, dim3(blocks, 2), dim3(256), 0, stream, o[0], o[1])
+                                   : launch_pdl(split_operands_kernel<3>, dim3(blocks, 2), dim3(256), 0, stream, o[0], o[1]);
+  if (e != cudaSuccess) {
     g_gemm_err = "split-precision GEMM: operand split launch failed";
     return -4;
   }
+  return 0;
+}
+
+// The three products run as one: its contraction is three passes of kp over (hi, lo), (lo, hi) and (hi, hi), so the
+// accumulators stay in tensor memory between them; the small cross terms come first, while the accumulators are small too.  (Three launches, the second and third adding to C in memory, and
+// two scalar conversion launches before them took 9.8 us each for 512 token rows.)
+int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t stream) {
+  if (d.M <= 0 || d.N <= 0 || d.K <= 0) return 0;
+  if (d.out != GEMM_OUT_F32 && d.out != GEMM_OUT_ACCUM) {
+    g_gemm_err = "split-precision GEMM writes fp32 (store or accumulate) only";
+    return -2;
+  }
+  SplitOperand o[2];
+  const int rc = split_operands(d, 2, sc, o, stream);
+  if (rc != 0) return rc;
+  const int kp = o[0].kp;
   GemmDesc g = d;
   g.A = o[0].dst; g.B = o[1].dst; g.lda = o[0].pitch; g.ldb = o[1].pitch;
   g.K = 3 * kp;
@@ -1182,11 +1212,76 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
   }
 }
 
-int gemm_f32(const GemmDesc& d, cudaStream_t stream) {
+// CTAs per tile of the tensor-core form: what gives the shortest chain, counting a start and end of about two k-blocks and two
+// more for the exchange; 0: the FMA kernels are faster (or have to take it).
+static int f32_on_tensor_cores(const GemmDesc& d) {
+  static const bool off = [] { const char* e = getenv("ANE_B200_F32_TC"); return e && e[0] == '0'; }();  // A/B measurements
+  if (off || !f32_aligned(d) || d.K < 128 || (d.out != GEMM_OUT_F32 && d.out != GEMM_OUT_ACCUM)) return 0;
+  const int sms = gemm_num_sms();
+  const long tiles = (long)((d.M + 127) / 128) * ((d.N + 127) / 128), kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;
+  long best = 0;
+  int parts = 1;
+  for (int p : {1, 2, 4, 8}) {
+    if (p > 1 && (kblocks < 2 * p || tiles > resident_clusters_f32(p))) continue;
+    const long cost = (tiles * p + sms - 1) / sms * ((kblocks + p - 1) / p) + 2 + (p > 1 ? 2 : 0);
+    if (best == 0 || cost < best) {
+      best = cost;
+      parts = p;
+    }
+  }
+  // us: k-blocks at 1.25, the cut (4 bytes read, 6 written per element) and its launch; the FMA kernels at about 40 TFLOP/s
+  const double tc = 1.25 * best + ((double)d.M + d.N) * d.K * 10.0 / 5e6 + 4.0, fma = 2.0 * d.M * d.N * d.K / 40e6 + 5.0;
+  return tc < fma ? parts : 0;
+}
+
+template <bool A_MN, bool B_MN, bool SPLIT>
+static cudaError_t launch_f32_tc(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const F32TcArgs& a, int* d_status, cudaStream_t stream) {
+  auto kern = gemm_f32_tc_kernel<A_MN, B_MN, SPLIT>;
+  static unsigned long long done = 0;
+  if (!smem_opt_in(kern, F32TC_SMEM, done)) return cudaErrorInvalidValue;
+  const int tiles = ((a.M + 127) / 128) * ((a.N + 127) / 128);
+  if constexpr (SPLIT)
+    return launch_pdl_cluster(kern, dim3((unsigned)(tiles * a.parts)), dim3(F32TC_THREADS), F32TC_SMEM, stream, (unsigned)a.parts, ta, tb, tc, a, d_status);
+  else
+    return launch_pdl(kern, dim3((unsigned)std::min(tiles, gemm_num_sms())), dim3(F32TC_THREADS), F32TC_SMEM, stream, ta, tb, tc, a, d_status);
+}
+template <bool SPLIT>
+static cudaError_t launch_f32_tc_layout(const GemmDesc& d, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const F32TcArgs& a, int* d_status, cudaStream_t stream) {
+  if (!d.a_mn && !d.b_mn) return launch_f32_tc<false, false, SPLIT>(ta, tb, tc, a, d_status, stream);
+  if (!d.a_mn) return launch_f32_tc<false, true, SPLIT>(ta, tb, tc, a, d_status, stream);
+  if (d.b_mn) return launch_f32_tc<true, true, SPLIT>(ta, tb, tc, a, d_status, stream);
+  return launch_f32_tc<true, false, SPLIT>(ta, tb, tc, a, d_status, stream);
+}
+static int gemm_f32_tc(const GemmDesc& d, int parts, SplitScratch* sc, int* d_status, cudaStream_t stream) {
+  SplitOperand o[2];
+  const int rc = split_operands(d, 3, sc, o, stream);
+  if (rc != 0) return rc;
+  const int kp = o[0].kp;
+  CUtensorMap ta, tb, tc;
+  bool ok = d.a_mn ? make_tmap(&ta, o[0].dst, d.M, 3 * kp, o[0].pitch, 64, GEMM_BK) : make_tmap(&ta, o[0].dst, 3 * kp, d.M, o[0].pitch, GEMM_BK, 128);
+  ok = ok && (d.b_mn ? make_tmap(&tb, o[1].dst, d.N, 3 * kp, o[1].pitch, 64, GEMM_BK) : make_tmap(&tb, o[1].dst, 3 * kp, d.N, o[1].pitch, GEMM_BK, 128));
+  ok = ok && make_tmap(&tc, d.C, d.N, d.M, d.ldc, 32, 32, true);
+  if (!ok) return -2;
+  const bool accum = d.out == GEMM_OUT_ACCUM;
+  const F32TcArgs a{d.M, d.N, d.K, kp, accum ? 1 : 0, parts, d.alpha, accum ? nullptr : d.res1, d.s1, accum ? nullptr : d.res2, d.s2, d.ldres,
+                    reinterpret_cast<float*>(d.C), d.ldc, reinterpret_cast<const float*>(d.A), reinterpret_cast<const float*>(d.B), d.lda, d.ldb};
+  const cudaError_t e = parts > 1 ? launch_f32_tc_layout<true>(d, ta, tb, tc, a, d_status, stream) : launch_f32_tc_layout<false>(d, ta, tb, tc, a, d_status, stream);
+  if (e != cudaSuccess) {
+    g_gemm_err = std::string("gemm_f32 tensor-core launch: ") + cudaGetErrorString(e);
+    return -4;
+  }
+  return 0;
+}
+
+int gemm_f32(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t stream) {
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return 0;
   if (d.out == GEMM_OUT_BF16) {
     g_gemm_err = "fp32 GEMM cannot write bf16";
     return -2;
+  }
+  if (const int parts = f32_on_tensor_cores(d)) {
+    const int rc = gemm_f32_tc(d, parts, sc, d_status, stream);
+    if (rc != kNoScratch) return rc;  // no memory for the parts: the FMA kernels need none
   }
   if (f32_aligned(d)) {
     const cudaError_t e = launch_f32(d, stream);

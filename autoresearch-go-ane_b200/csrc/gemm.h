@@ -85,21 +85,21 @@ struct GemmDesc {
 
 // bf16 operands, tcgen05 tensor cores.  Returns 0 or a negative error code.
 int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream);
-// fp32 operands, SIMT FMA (the fp32 parity mode).
-int gemm_f32(const GemmDesc& d, cudaStream_t stream);
-
 // fp32 operands at split precision on the tensor cores: A and B are each cut into a bf16 (hi, lo) pair
 // (hi = bf16(x), lo = bf16(x - hi): together ~16 significand bits) and the product is formed as Ah*Bh + Ah*Bl + Al*Bh
 // with fp32 accumulation, one GEMM over a contraction of three passes (the dropped Al*Bl term is ~2^-18 relative).
 // Output kinds GEMM_OUT_F32 (with residuals) and GEMM_OUT_ACCUM.  The scratch holds both operands' halves and grows on
 // demand; one scratch serves one stream at a time.
 struct SplitScratch {
-  void* buf[2] = {nullptr, nullptr};  // A, B
+  void* buf[2] = {nullptr, nullptr};  // A, B, in two or three parts
   size_t cap[2] = {0, 0};             // bytes
   uint64_t generation = 0;            // counts the times that a buffer moved: what was captured before holds old addresses
   void release();
 };
 int gemm_bf16x3(const GemmDesc& d, SplitScratch* scratch, int* d_status, cudaStream_t stream);
+// fp32 operands with the error of fp32 sums (the fp32 parity mode): on the FMA units or, for products that are large enough, as six
+// products of bf16 parts (hi, mid, lo) on the tensor cores.
+int gemm_f32(const GemmDesc& d, SplitScratch* scratch, int* d_status, cudaStream_t stream);
 
 // Up to four accumulating products C_p += A_p^T B_p (both operands stored [K, .], the same K: the weight gradients of
 // one layer) in one stream-K launch.  `slot` = gemm_group_slot_bytes() of device memory (64-byte aligned) that keeps

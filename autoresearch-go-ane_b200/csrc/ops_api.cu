@@ -214,13 +214,13 @@ int32_t ane_op_gemm(const ane_gemm_args* a) {
   d.aux = const_cast<void*>(a->d_aux);
   d.ldaux = a->ldaux;
   int rc;
-  if (a->dtype == ANE_DTYPE_BF16X3) {
-    SplitScratch sc;  // operand halves for this call only
-    rc = gemm_bf16x3(d, &sc, status, 0);
-    cudaStreamSynchronize(0);
+  if (a->dtype == ANE_DTYPE_BF16X3 || a->dtype == ANE_DTYPE_F32) {
+    SplitScratch sc;  // operand parts for this call only (fp32: none for products that the FMA units take)
+    rc = a->dtype == ANE_DTYPE_F32 ? gemm_f32(d, &sc, status, 0) : gemm_bf16x3(d, &sc, status, 0);
+    if (sc.buf[0]) cudaStreamSynchronize(0);
     sc.release();
   } else {
-    rc = (a->dtype == ANE_DTYPE_F32) ? gemm_f32(d, 0) : gemm_bf16(d, status, 0);
+    rc = gemm_bf16(d, status, 0);
   }
   if (rc != 0) return set_err(ANE_ERR_KERNEL, gemm_last_error());
   return 0;

@@ -347,6 +347,30 @@ def _bf16_result(A, B, M, N, K, b_mn):
     return got
 
 
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn,out", [(513, 4096, 136, 0, 0, 1), (1025, 1000, 288, 0, 1, 1), (2048, 288, 768, 0, 0, 1), (1000, 2304, 264, 1, 0, 1),
+                                                 (864, 288, 2048, 1, 1, 2), (520, 264, 8200, 1, 1, 2), (2048, 288, 4096, 0, 1, 1)])
+def test_fp32_products_on_the_tensor_cores(M, N, K, a_mn, b_mn, out):
+    """Large fp32 products (all of these sizes) run as six products of bf16 parts, whole tiles and tiles shared by a cluster, with residuals and as
+    accumulation.  The error of a sum of K fp32 products in any order is about sqrt(K) / 2 roundings of 2^-24 in the 2-norm;
+    held to a quarter of that, and for terms of one sign to 2^-23.  Elements that an infinite or NaN operand touches are what fp32 FMAs give."""
+    rng = np.random.default_rng(M + N + K)
+    for positive in (False, True):
+        draw = (lambda *s: rng.random(s, dtype=np.float32)) if positive else (lambda *s: rng.standard_normal(s, dtype=np.float32))  # noqa: E731
+        A, B, R = draw(*((K, M) if a_mn else (M, K))), draw(*((K, N) if b_mn else (N, K))), draw(M, N)
+        want = (A.T if a_mn else A).astype(np.float64) @ (B if b_mn else B.T).astype(np.float64)
+        got = _gemm(ane.DTYPE_F32, A, B, R, M, N, K, a_mn, b_mn, 2) if out == 2 else _gemm(ane.DTYPE_F32, A, B, np.zeros_like(R), M, N, K, a_mn, b_mn, 1, res=R)
+        assert rel_l2(got, want + R) < (2.0**-23 if positive else max(np.sqrt(K) / 8, 2.0) * 2.0**-24)
+    at = (A.T if a_mn else A), (B if b_mn else B.T)  # views: [M, K] and [K, N]
+    at[0][3, 5], at[0][7, 1], at[1][4, 2], at[0][9, 0] = np.inf, np.nan, -np.inf, 3.4e38
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = np.vstack([at[0][r].astype(np.float64) @ at[1].astype(np.float64) for r in (3, 7, 9, 11)]).astype(np.float32)
+    got = _gemm(ane.DTYPE_F32, A, B, np.zeros_like(R), M, N, K, a_mn, b_mn, out)[[3, 7, 9, 11]]
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+    far = ~np.isfinite(want)
+    np.testing.assert_array_equal(got[far], want[far])
+    np.testing.assert_allclose(got[~far], want[~far], rtol=1e-4)
+
+
 def test_gemm_rejects_misaligned_pitch():
     A = np.zeros((16, 20), np.float32)  # 20 bf16 = 40 bytes per row: not a 16-byte multiple
     dA, dB, dC = _up_bf16(A), _up_bf16(A), _up(np.zeros((16, 16), np.float32))
