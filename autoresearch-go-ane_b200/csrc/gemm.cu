@@ -331,7 +331,7 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 32, 32, true)) return -2;
   if (d.out == GEMM_OUT_F32) {
     // One residual, K-major operands and room for the residual buffers: let TMA fetch the residual pieces.
-    if constexpr (!A_MN && !B_MN && GemmCfg<BN, MT>::fits(EPI_STORE_F32_TMARES)) {
+    if constexpr (!A_MN && !B_MN && MT != GEMM_MT_PAIR2 && GemmCfg<BN, MT>::fits(EPI_STORE_F32_TMARES)) {
       static const bool no_tma_res = getenv("ANE_B200_NO_TMA_RES") != nullptr;  // A/B measurements
       if (d.res1 != nullptr && d.res2 == nullptr && !no_tma_res) {
         CUtensorMap td;
@@ -673,8 +673,13 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
         const long waves2 = (tiles2 + pairs - 1) / pairs;
         const double eff2 =
             (double)tiles2 / (double)(waves2 * pairs) * ((double)d.N / (double)(((d.N + 191) / 192) * 192));
-        const bool exposed_residual = kblocks < 32 && (d.res1 != nullptr || d.res2 != nullptr);
-        if (eff2 >= 0.85 && !exposed_residual) bn = 512;
+        const bool residual = d.res1 != nullptr || d.res2 != nullptr;
+        if (eff2 >= 0.85 && !(kblocks < 32 && residual)) bn = 512;
+        // A long K with a residual that TMA can fetch: 256 x 192 tiles, two waves of them, whose first epilogue hides behind the
+        // second tile (W2 forward, 8192 x 768 x 2048: 32 -> 28.7 us; of 16384 rows 86 -> 71).
+        const long tiles3 = (long)((d.M + 255) / 256) * ((d.N + 191) / 192);
+        const double eff3 = (double)tiles3 / (double)((tiles3 + pairs - 1) / pairs * pairs) * ((double)d.N / (double)(((d.N + 191) / 192) * 192));
+        if (kblocks >= 32 && d.res1 != nullptr && d.res2 == nullptr && !d.b_mn && eff3 >= 0.8) bn = 192;
       }
     }
     if (bn == 512 && d.out != GEMM_OUT_BF16_SWIGLU) return dispatch_layout<192, GEMM_MT_PAIR2>(d, 1, d_status, stream);

@@ -105,9 +105,13 @@ struct GemmCfg {
   // pieces than a tile has and spend the room on stages: a stage holds 20 or 24 KB, and what hides the latency of operands from
   // DRAM is the bytes in flight (K = 6144 on 32 columns: 28.9 us with four stages, 20.8 with eight).
   static constexpr bool NARROW = BN < 128;
+  // Epilogues with nothing to hide behind, as there is one accumulator set: fp32 stores of the 512-row pair tiles, twelve pieces of
+  // 1200 cycles for each of four warps.  Eight warps, with one staging buffer each, take half of the columns: W1|W3 dX of 8192
+  // rows 46.1 -> 44.4 us, q|k|v dX 31.6 -> 28.8.
+  __host__ __device__ static constexpr bool exposed(int epi) { return MT == GEMM_MT_PAIR2 && epi == EPI_STORE_F32; }
   // Staged output pieces per epilogue warp (a buffer is reused once its TMA store has read it; four buffers
   // measured no faster than two and cost a pipeline stage).
-  __host__ __device__ static constexpr int sbuf(int epi) { return NARROW && epi != EPI_STORE_BF16_RELU2 ? 1 : 2; }
+  __host__ __device__ static constexpr int sbuf(int epi) { return (NARROW && epi != EPI_STORE_BF16_RELU2) || exposed(epi) ? 1 : 2; }
   // Epilogue warps.  The epilogues that do arithmetic per element and move more than one piece per 64 accumulator
   // columns (SwiGLU forward: h13 + gate; SwiGLU backward: h13 in, d h13 out) take longer than the 12-k-block main
   // loop of their products with four warps (one per scheduler, ~750 cycles of fixed cost per piece).  With eight,
@@ -115,7 +119,7 @@ struct GemmCfg {
   // with ANE_B200_GEMM_EW8=1: the two warps of a scheduler then share its exponential unit and the pipeline drops
   // to three stages, W2-dX 51 -> 46 us, W1|W3 forward 51 -> 56 us, the step unchanged; hence off by default.
   __host__ __device__ static constexpr int epi_warps(int epi) {
-    return (ANE_B200_GEMM_EW8 && PAIR && SUBS == 1 && BN == 256 && (epi == EPI_STORE_BF16_SWIGLU || epi == EPI_DSWIGLU)) ? 8 : 4;
+    return exposed(epi) || (ANE_B200_GEMM_EW8 && PAIR && SUBS == 1 && BN == 256 && (epi == EPI_STORE_BF16_SWIGLU || epi == EPI_DSWIGLU)) ? 8 : 4;
   }
   // Epilogues that read an input piece per output piece by TMA (residual, h13, h), and those of them that cannot do without.
   __host__ __device__ static constexpr bool tma_in(int epi) { return epi == EPI_STORE_F32_TMARES || epi == EPI_DSWIGLU || epi == EPI_DRELU2; }
