@@ -575,8 +575,10 @@ static int narrow_width(const GemmDesc& d) {
 //   * Not split precision, whose backward carries a difference far through unscaled scores: after two updates of the reference
 //     network at 2 x 256 gradients were up to 2.2e-3 from those of whole tiles, where the mode is to hold 1e-3.
 static int cluster_split(const GemmDesc& d) {
-  static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_CLUSTER_SPLIT"); return e && e[0] == '0'; }();  // A/B measurements
-  if (off || d.a_mn || !d.b_mn || d.seg_kb > 0 || d.out != GEMM_OUT_F32) return 0;
+  // Off unless ANE_B200_GEMM_CLUSTER_SPLIT=1: over 20 updates of the 110M model at 2 x 256 the loss was up to 5.1e-3 from the
+  // fp32 oracle's with shared tiles and 1.8e-3 with whole ones.
+  static const bool on = [] { const char* e = getenv("ANE_B200_GEMM_CLUSTER_SPLIT"); return e && e[0] == '1'; }();
+  if (!on || d.a_mn || !d.b_mn || d.seg_kb > 0 || d.out != GEMM_OUT_F32) return 0;
   const long tiles = (long)((d.M + 127) / 128) * ((d.N + 127) / 128);
   const int kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;
   const int whole = narrow_width(d) ? 5000 + 180 * kblocks : 6500 + 210 * kblocks;
