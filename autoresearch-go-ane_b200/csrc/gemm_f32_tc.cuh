@@ -16,7 +16,7 @@
 // operands), warp 1 the MMAs (1536 cycles a k-block; the latency and fill of 96 KB behind two stages bound it, about 2250 cycles),
 // warps 2 - 9 hold the sums, 64 columns of a row per thread.  SPLIT: a cluster shares a tile along the contraction (products with
 // few tiles and a long one, dW and the head's dX) and exchanges its sums as the split tiles of gemm_tc.cuh do, in rank order.
-// An operand that is infinite or NaN makes the sums NaN (inf * 0 in the other parts); such elements are computed again as a chain of
+// An operand that is infinite or NaN makes the sums NaN (inf * 0 in the other parts); such elements are computed again with
 // fp32 FMAs, so that what is infinite stays infinite.
 #pragma once
 
@@ -41,12 +41,69 @@ static constexpr uint32_t F32TC_PART = GEMM_BM * GEMM_BK * 2, F32TC_STAGE = 6 * 
 static constexpr uint32_t F32TC_SMEM = 2 * F32TC_STAGE + 8 * 4096 + 1024;
 static_assert(F32TC_SMEM <= GEMM_SMEM_LIMIT, "pipeline does not fit");
 
+// Sums of 32 rows (from m0, a row per lane) and `cols` columns (from n0, up to 32, a multiple of 4), column e of lane r in dword
+// 32 e + r of the warp's 4 KB of shared memory at `at`: those whose bit e is set in `wanted` are formed again as fp32 FMAs.  The lanes share
+// the contraction of a row and eight columns and stop where all that is wanted of them is NaN, as a sum is from its first NaN term on.
+// (One thread per sum, to the end of the contraction, took 37 ms for 2048 x 1536 x 2048 of NaN, 0.1 ms of finite numbers; for
+// K = 32000 it is longer than the MMA warp's bounded wait.)
+__device__ __forceinline__ void f32tc_park(uint32_t at, int lane, int e, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)(e * 128 + lane * 4)), "f"(v) : "memory");
+}
+__device__ __forceinline__ float f32tc_parked(uint32_t at, int lane, int e) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at + (uint32_t)(e * 128 + lane * 4)) : "memory");
+  return v;
+}
 template <bool A_MN, bool B_MN>
-__device__ __noinline__ float f32tc_dot(const F32TcArgs& a, int m, int n) {
-  float s = 0.f;
-  for (int k = 0; k < a.K; ++k)
-    s = fmaf(A_MN ? a.A[(size_t)k * a.lda + m] : a.A[(size_t)m * a.lda + k], B_MN ? a.B[(size_t)k * a.ldb + n] : a.B[(size_t)n * a.ldb + k], s);
-  return s;
+__device__ __forceinline__ void f32tc_again(const F32TcArgs& a, int m0, int n0, int cols, uint32_t wanted, uint32_t at) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  for (uint32_t rows = __ballot_sync(0xffffffffu, wanted != 0); rows != 0; rows &= rows - 1) {
+    const int r = __ffs((int)rows) - 1, m = m0 + r;
+    const uint32_t of_row = __shfl_sync(0xffffffffu, wanted, r);
+#pragma unroll 1
+    for (int c = 0; c < cols; c += 8) {
+      const uint32_t want = of_row >> c & 0xffu;
+      if (want == 0) continue;
+      const bool both = c + 4 < cols;  // the second four columns exist
+      float s[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s[e] = 0.f;
+#pragma unroll 1
+      for (int k0 = 0, k1 = 128;; k0 = k1, k1 += 1024) {
+        const int end = min(k1, a.K);
+#pragma unroll 4
+        for (int k = k0 + lane; k < end; k += 32) {
+          const float x = A_MN ? a.A[(size_t)k * a.lda + m] : a.A[(size_t)m * a.lda + k];
+          float y[8];
+          if constexpr (B_MN) {
+            const float4* b = reinterpret_cast<const float4*>(a.B + (size_t)k * a.ldb + n0 + c);
+            *reinterpret_cast<float4*>(y) = b[0];
+            *reinterpret_cast<float4*>(y + 4) = b[both ? 1 : 0];
+          } else {
+            const float* b = a.B + (size_t)(n0 + c) * a.ldb + k;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] = b[(size_t)(e < 4 || both ? e : 0) * a.ldb];
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) s[e] = fmaf(x, y[e], s[e]);
+        }
+        __syncwarp();
+        uint32_t nan = 0;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) nan |= __any_sync(0xffffffffu, s[e] != s[e]) ? 1u << e : 0u;
+        if (end == a.K || (want & ~nan) == 0) break;
+      }
+      float mine = 0.f;  // lane e's column is c + e
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float t = warp_sum(s[e]);
+        if (lane == e) mine = t;
+      }
+      if (lane < 8 && (want >> lane & 1u) != 0) f32tc_park(at, r, c + lane, mine);
+    }
+  }
+  __syncwarp();
 }
 
 template <bool A_MN, bool B_MN, bool SPLIT>
@@ -205,10 +262,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           bool nan = false;
 #pragma unroll
           for (int e = 0; e < 32; ++e) nan = nan || acc[32 * p + e] != acc[32 * p + e];
-          if (nan && m < a.M) {
+          if (__any_sync(0xffffffffu, nan)) {
+            uint32_t wanted = 0;
 #pragma unroll
             for (int e = 0; e < 32; ++e)
-              if (n0 + e < a.N && acc[32 * p + e] != acc[32 * p + e]) acc[32 * p + e] = f32tc_dot<A_MN, B_MN>(a, m, n0 + e);
+              if (m < a.M && n0 + e < a.N && acc[32 * p + e] != acc[32 * p + e]) wanted |= 1u << e;
+            if (elect_one()) tma_store_wait_read<0>();
+            __syncwarp();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) f32tc_park(stage, lane, e, acc[32 * p + e]);
+            f32tc_again<A_MN, B_MN>(a, m - lane, n0, min(32, a.N - n0), wanted, stage);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) acc[32 * p + e] = f32tc_parked(stage, lane, e);
+            __syncwarp();
           }
           float4 r1[8], r2[8];
 #pragma unroll
@@ -269,24 +335,55 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           in2[q] = in && a.res2 ? *reinterpret_cast<const float4*>(a.res2 + (size_t)m * a.ldres + n) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         ok = mbar_wait(smem_u32(&bar_sums[warp - 2]), 0u, status, DEV_MBAR_TIMEOUT_EPILOGUE) && ok;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int n = n_begin + 4 * q;
-          if (4 * q >= cols || !ok || m >= a.M || n >= a.N) continue;
-          float s[4] = {0.f, 0.f, 0.f, 0.f};
+        auto received = [&](int q, float (&s)[4]) {  // in rank order
+          s[0] = s[1] = s[2] = s[3] = 0.f;
           for (int p = 0; p < parts; ++p) {
             float4 t;
             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
                          : "r"(landed + (uint32_t)p * piece + (uint32_t)q * 512u + (uint32_t)lane * 16u) : "memory");
             s[0] += t.x; s[1] += t.y; s[2] += t.z; s[3] += t.w;
           }
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (s[e] != s[e]) s[e] = f32tc_dot<A_MN, B_MN>(a, m, n + e);
+        };
+        auto finish = [&](int n, const float (&s)[4], const float4& i1, const float4& i2) {
           float4 v = make_float4(a.alpha * s[0], a.alpha * s[1], a.alpha * s[2], a.alpha * s[3]);
-          if (base1) { v.x += a1 * in1[q].x; v.y += a1 * in1[q].y; v.z += a1 * in1[q].z; v.w += a1 * in1[q].w; }
-          if (a.res2) { v.x += a2 * in2[q].x; v.y += a2 * in2[q].y; v.z += a2 * in2[q].z; v.w += a2 * in2[q].w; }
+          if (base1) { v.x += a1 * i1.x; v.y += a1 * i1.y; v.z += a1 * i1.z; v.w += a1 * i1.w; }
+          if (a.res2) { v.x += a2 * i2.x; v.y += a2 * i2.y; v.z += a2 * i2.z; v.w += a2 * i2.w; }
           *reinterpret_cast<float4*>(a.C + (size_t)m * a.ldc + n) = v;
+        };
+        uint32_t left = 0;  // columns with a NaN among their four: after the others
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int n = n_begin + 4 * q;
+          if (4 * q >= cols || !ok || m >= a.M || n >= a.N) continue;
+          float s[4];
+          received(q, s);
+          if (s[0] != s[0] || s[1] != s[1] || s[2] != s[2] || s[3] != s[3]) left |= 1u << q;
+          else finish(n, s, in1[q], in2[q]);
+        }
+        if (__any_sync(0xffffffffu, left != 0)) {
+          uint32_t wanted = 0;
+#pragma unroll 1
+          for (int q = 0; q < 8; ++q) {
+            float s[4];
+            if ((left >> q & 1u) == 0) continue;
+            received(q, s);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              f32tc_park(stage, lane, 4 * q + e, s[e]);
+              if (s[e] != s[e]) wanted |= 1u << (4 * q + e);
+            }
+          }
+          f32tc_again<A_MN, B_MN>(a, m - lane, n_begin, min(cols, a.N - n_begin), wanted, stage);
+#pragma unroll 1
+          for (int q = 0; q < 8; ++q) {
+            const int n = n_begin + 4 * q;
+            if ((left >> q & 1u) == 0) continue;
+            const float s[4] = {f32tc_parked(stage, lane, 4 * q), f32tc_parked(stage, lane, 4 * q + 1), f32tc_parked(stage, lane, 4 * q + 2),
+                                f32tc_parked(stage, lane, 4 * q + 3)};
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            finish(n, s, base1 ? *reinterpret_cast<const float4*>(base1 + (size_t)m * ld1 + n) : zero,
+                   a.res2 ? *reinterpret_cast<const float4*>(a.res2 + (size_t)m * a.ldres + n) : zero);
+          }
         }
       }
     }

@@ -371,6 +371,44 @@ def test_fp32_products_on_the_tensor_cores(M, N, K, a_mn, b_mn, out):
     np.testing.assert_allclose(got[~far], want[~far], rtol=1e-4)
 
 
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(2048, 1544, 4096, 0, 0), (2048, 1544, 4096, 0, 1), (520, 264, 8200, 1, 1), (520, 264, 8200, 1, 0)])
+def test_fp32_products_of_nan_and_infinities_cost_about_what_finite_ones_do(M, N, K, a_mn, b_mn):
+    """Sums that the tensor cores leave NaN are formed again; a whole operand of NaN and a row of infinities, on more tiles than SMs and on
+    tiles shared by a cluster.  One thread per sum to the end of the contraction took 50 times as long as finite numbers, and ever longer with K."""
+    rng = np.random.default_rng(M + K)
+    A, B = rng.random((K, M) if a_mn else (M, K), dtype=np.float32), rng.random((K, N) if b_mn else (N, K), dtype=np.float32)
+    row = A.copy()
+    (row.T if a_mn else row)[77] = np.inf
+    dB, dC = _up(B), _up(np.zeros((M, N), np.float32))
+    g = _ffi.GemmArgs()
+    g.struct_size = ctypes.sizeof(_ffi.GemmArgs)
+    g.dtype, g.d_b, g.d_c = ane.DTYPE_F32, dB, dC
+    g.m, g.n, g.k, g.lda, g.ldb, g.ldc = M, N, K, A.shape[1], B.shape[1], N
+    g.a_mn, g.b_mn, g.out_mode, g.alpha = a_mn, b_mn, 1, 1.0
+    times, results = [], []
+    for a in (A, np.full_like(A, np.nan), row):
+        g.d_a = _up(a)
+        took = []
+        for _ in range(4):
+            ms = ctypes.c_float(0)
+            _ck(lib.ane_timer_begin())
+            _ck(lib.ane_op_gemm(ctypes.byref(g)))
+            _ck(lib.ane_timer_end(ctypes.byref(ms)))
+            took.append(ms.value)
+        st = ctypes.c_int32(0)
+        _ck(lib.ane_ops_device_status(ctypes.byref(st)))
+        assert st.value == 0
+        times.append(min(took))
+        results.append(_down(dC, (M, N)))
+        lib.ane_dev_free(g.d_a)
+    lib.ane_dev_free(dB)
+    lib.ane_dev_free(dC)
+    assert np.isnan(results[1]).all()
+    assert (results[2][77] == np.inf).all()
+    np.testing.assert_array_equal(np.delete(results[2], 77, 0), np.delete(results[0], 77, 0))
+    assert times[1] < 8 * times[0] and times[2] < 8 * times[0], times
+
+
 def test_gemm_rejects_misaligned_pitch():
     A = np.zeros((16, 20), np.float32)  # 20 bf16 = 40 bytes per row: not a 16-byte multiple
     dA, dB, dC = _up_bf16(A), _up_bf16(A), _up(np.zeros((16, 16), np.float32))
