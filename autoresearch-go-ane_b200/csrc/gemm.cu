@@ -781,8 +781,8 @@ size_t gemm_group_slot_bytes() { return sizeof(GemmGroup); }
 // Both operands of a product in one launch (blockIdx.y), four values per thread and step.  Operand [rows, cols] fp32
 // with row pitch ld; its parts (hi, lo or hi, mid, lo) lie behind one another along the contraction: for a K-major operand (k = cols)
 // [rows][hi (kp) | lo (kp)], for an MN-major one (k = rows) [hi (kp rows) | lo (kp rows)][cols rounded up to 8].  kp =
-// k rounded up to a whole k-block; what lies past k is zero.  Three parts are exactly the fp32 value (down to 2^-133, the last bit
-// of a bf16): what rounds to infinity is cut off instead, what is not finite has no further parts.
+// k rounded up to a whole k-block; what lies past k is zero.  Three parts are exactly F32TC_SCALE times the fp32 value; where that is not
+// finite, or its first part is not, the others are not either.
 struct SplitOperand {
   const float* src;
   bf16* dst;
@@ -811,6 +811,10 @@ __global__ void split_operands_kernel(const SplitOperand a, const SplitOperand b
           if (c + e < o.cols) x[e] = p[e];
       }
     }
+    if constexpr (PARTS == 3) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] *= F32TC_SCALE;
+    }
     bf16* q = o.dst + (size_t)r * o.pitch + c;
 #pragma unroll
     for (int p = 0; p < PARTS; ++p, q += next) {
@@ -818,19 +822,8 @@ __global__ void split_operands_kernel(const SplitOperand a, const SplitOperand b
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         v[e] = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
-        if constexpr (PARTS == 3) {
-          bf16* part[2] = {&v[e].x, &v[e].y};
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            float& f = x[2 * e + t];
-            const bool finite = fabsf(f) <= 3.402823466e38f;
-            if (p == 0 && finite && fabsf(f) >= 3.3895e38f) *part[t] = __float2bfloat16_rz(f);
-            f = finite ? f - __bfloat162float(*part[t]) : 0.f;
-          }
-        } else {
-          x[2 * e] -= __bfloat162float(v[e].x);
-          x[2 * e + 1] -= __bfloat162float(v[e].y);
-        }
+        x[2 * e] -= __bfloat162float(v[e].x);
+        x[2 * e + 1] -= __bfloat162float(v[e].y);
       }
       *reinterpret_cast<uint2*>(q) = make_uint2(*reinterpret_cast<const uint32_t*>(&v[0]), *reinterpret_cast<const uint32_t*>(&v[1]));
     }

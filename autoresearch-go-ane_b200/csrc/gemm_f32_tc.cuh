@@ -1,8 +1,9 @@
 // fp32 products on the tensor cores, with the error of fp32 sums.
 //
-//   * Operands are cut into three bf16 parts, hi + mid + lo, which together are the fp32 value (3 x 8 significand bits, rounded to
-//     nearest at each cut).  Six of the nine products of parts are formed; the three that are left out (mid lo, lo mid, lo lo) are
-//     below 2^-25 of the product.
+//   * Operands are cut into three bf16 parts, hi + mid + lo, which together are 2^16 times the fp32 value (3 x 8 significand bits,
+//     rounded to nearest at each cut).  The factor is for the low bits of small values, which would fall below the last bit of a bf16,
+//     2^-133; 2^-149, the last one of an fp32, comes to lie there.  (Without it operands of 2^-115 had errors of 1.1e-6, of 2^-130 3.6e-2.)
+//     Six of the nine products of parts are formed; the three that are left out (mid lo, lo mid, lo lo) are below 2^-25 of the product.
 //   * The tensor core truncates what it adds to its accumulator, which over a whole contraction would be a bias of several
 //     units in the last place.  An accumulator therefore lives for half a k-block, 32 terms: six passes, the small products first,
 //     12 MMAs, and only the last two of them at the size of the sum.  Eight warps then add it to the running sums in registers
@@ -16,8 +17,8 @@
 // operands), warp 1 the MMAs (1536 cycles a k-block; the latency and fill of 96 KB behind two stages bound it, about 2250 cycles),
 // warps 2 - 9 hold the sums, 64 columns of a row per thread.  SPLIT: a cluster shares a tile along the contraction (products with
 // few tiles and a long one, dW and the head's dX) and exchanges its sums as the split tiles of gemm_tc.cuh do, in rank order.
-// An operand that is infinite or NaN makes the sums NaN (inf * 0 in the other parts); such elements are computed again with
-// fp32 FMAs, so that what is infinite stays infinite.
+// An operand that is not finite, or not after the factor, makes the sums infinite or NaN (its other parts are NaN), and so does a sum
+// above 2^96; such elements are computed again with fp32 FMAs.
 #pragma once
 
 #include "gemm_tc.cuh"
@@ -40,6 +41,9 @@ static constexpr int F32TC_THREADS = 64 + 8 * 32;
 static constexpr uint32_t F32TC_PART = GEMM_BM * GEMM_BK * 2, F32TC_STAGE = 6 * F32TC_PART;
 static constexpr uint32_t F32TC_SMEM = 2 * F32TC_STAGE + 8 * 4096 + 1024;
 static_assert(F32TC_SMEM <= GEMM_SMEM_LIMIT, "pipeline does not fit");
+static constexpr float F32TC_SCALE = 65536.f, F32TC_UNSCALE = 1.f / (65536.f * 65536.f);  // of an operand, of a product
+
+__device__ __forceinline__ bool f32tc_bad(float v) { return !(fabsf(v) <= 3.402823466e38f); }
 
 // Sums of 32 rows (from m0, a row per lane) and `cols` columns (from n0, up to 32, a multiple of 4), column e of lane r in dword
 // 32 e + r of the warp's 4 KB of shared memory at `at`: those whose bit e is set in `wanted` are formed again as fp32 FMAs.  The lanes share
@@ -259,14 +263,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         for (int p = 0; p < 2; ++p) {
           const int n0 = n_tile + half * 64 + p * 32;
           if (n0 >= a.N || m - lane >= a.M) break;  // warp-uniform
-          bool nan = false;
+          bool bad = false;
 #pragma unroll
-          for (int e = 0; e < 32; ++e) nan = nan || acc[32 * p + e] != acc[32 * p + e];
-          if (__any_sync(0xffffffffu, nan)) {
+          for (int e = 0; e < 32; ++e) {
+            acc[32 * p + e] *= F32TC_UNSCALE;
+            bad = bad || f32tc_bad(acc[32 * p + e]);
+          }
+          if (__any_sync(0xffffffffu, bad)) {
             uint32_t wanted = 0;
 #pragma unroll
             for (int e = 0; e < 32; ++e)
-              if (m < a.M && n0 + e < a.N && acc[32 * p + e] != acc[32 * p + e]) wanted |= 1u << e;
+              if (m < a.M && n0 + e < a.N && f32tc_bad(acc[32 * p + e])) wanted |= 1u << e;
             if (elect_one()) tma_store_wait_read<0>();
             __syncwarp();
 #pragma unroll
@@ -343,6 +350,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                          : "r"(landed + (uint32_t)p * piece + (uint32_t)q * 512u + (uint32_t)lane * 16u) : "memory");
             s[0] += t.x; s[1] += t.y; s[2] += t.z; s[3] += t.w;
           }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[e] *= F32TC_UNSCALE;
         };
         auto finish = [&](int n, const float (&s)[4], const float4& i1, const float4& i2) {
           float4 v = make_float4(a.alpha * s[0], a.alpha * s[1], a.alpha * s[2], a.alpha * s[3]);
@@ -350,14 +359,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           if (a.res2) { v.x += a2 * i2.x; v.y += a2 * i2.y; v.z += a2 * i2.z; v.w += a2 * i2.w; }
           *reinterpret_cast<float4*>(a.C + (size_t)m * a.ldc + n) = v;
         };
-        uint32_t left = 0;  // columns with a NaN among their four: after the others
+        uint32_t left = 0;  // columns with a sum among their four that is not finite: after the others
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int n = n_begin + 4 * q;
           if (4 * q >= cols || !ok || m >= a.M || n >= a.N) continue;
           float s[4];
           received(q, s);
-          if (s[0] != s[0] || s[1] != s[1] || s[2] != s[2] || s[3] != s[3]) left |= 1u << q;
+          if (f32tc_bad(s[0]) || f32tc_bad(s[1]) || f32tc_bad(s[2]) || f32tc_bad(s[3])) left |= 1u << q;
           else finish(n, s, in1[q], in2[q]);
         }
         if (__any_sync(0xffffffffu, left != 0)) {
@@ -370,7 +379,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               f32tc_park(stage, lane, 4 * q + e, s[e]);
-              if (s[e] != s[e]) wanted |= 1u << (4 * q + e);
+              if (f32tc_bad(s[e])) wanted |= 1u << (4 * q + e);
             }
           }
           f32tc_again<A_MN, B_MN>(a, m - lane, n_begin, min(cols, a.N - n_begin), wanted, stage);

@@ -371,6 +371,19 @@ def test_fp32_products_on_the_tensor_cores(M, N, K, a_mn, b_mn, out):
     np.testing.assert_allclose(got[~far], want[~far], rtol=1e-4)
 
 
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn,out", [(1025, 1000, 288, 0, 1, 1), (864, 288, 2048, 1, 1, 2), (520, 264, 8200, 0, 0, 1)])
+def test_fp32_products_keep_their_precision_over_the_range_of_fp32(M, N, K, a_mn, b_mn, out):
+    """Operands far from one, down to subnormal ones and up to where products overflow, have the error bound of those around one (see above); sums
+    that are formed again, K / 32 terms a lane, stay below it.  Products of powers of two scale exactly, so the reference does too."""
+    rng = np.random.default_rng(M + K)
+    A, B = rng.standard_normal((K, M) if a_mn else (M, K)), rng.standard_normal((K, N) if b_mn else (N, K))
+    for ea, eb in ((-115, 40), (40, -122), (-130, 60), (-146, 90), (-60, -60), (60, 50), (118, -100), (-20, 123)):
+        a, b = (A * 2.0**ea).astype(np.float32), (B * 2.0**eb).astype(np.float32)
+        want = (np.ldexp(a.astype(np.float64), -ea).T if a_mn else np.ldexp(a.astype(np.float64), -ea)) @ (np.ldexp(b.astype(np.float64), -eb) if b_mn else np.ldexp(b.astype(np.float64), -eb).T)
+        got = np.ldexp(_gemm(ane.DTYPE_F32, a, b, np.zeros((M, N), np.float32), M, N, K, a_mn, b_mn, out).astype(np.float64), -ea - eb)
+        assert rel_l2(got, want) < max(np.sqrt(K) / 8, 2.0) * 2.0**-24, (ea, eb)
+
+
 @pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(2048, 1544, 4096, 0, 0), (2048, 1544, 4096, 0, 1), (520, 264, 8200, 1, 1), (520, 264, 8200, 1, 0)])
 def test_fp32_products_of_nan_and_infinities_cost_about_what_finite_ones_do(M, N, K, a_mn, b_mn):
     """Sums that the tensor cores leave NaN are formed again; a whole operand of NaN and a row of infinities, on more tiles than SMs and on
