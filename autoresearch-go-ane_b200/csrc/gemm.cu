@@ -839,9 +839,10 @@ void SplitScratch::release() {
 }
 
 static constexpr int kNoScratch = -3;
-// The operands of `d` in `parts` bf16 parts each, in the scratch (which grows on demand).
+// The operands of `d` in `parts` bf16 parts each, in the scratch.
 static int split_operands(const GemmDesc& d, int parts, SplitScratch* sc, SplitOperand (&o)[2], cudaStream_t stream) {
   const int kp = (d.K + GEMM_BK - 1) / GEMM_BK * GEMM_BK;
+  size_t used = 0;  // of an arena
   for (int i = 0; i < 2; ++i) {
     const bool mn = i == 0 ? d.a_mn : d.b_mn;
     const int outer = i == 0 ? d.M : d.N;
@@ -854,6 +855,15 @@ static int split_operands(const GemmDesc& d, int parts, SplitScratch* sc, SplitO
     o[i].pitch = mn ? (outer + 7) / 8 * 8 : parts * kp;
     o[i].vec = o[i].ld % 4 == 0 && (reinterpret_cast<uintptr_t>(o[i].src) & 15) == 0;
     const size_t need = sizeof(bf16) * (size_t)(mn ? parts * kp : outer) * o[i].pitch;
+    if (sc->arena != nullptr) {
+      o[i].dst = reinterpret_cast<bf16*>(static_cast<char*>(sc->arena) + used);
+      used += (need + 255) / 256 * 256;
+      if (used > sc->arena_bytes) {
+        g_gemm_err = "split-precision GEMM: the operands' parts do not fit the arena";
+        return kNoScratch;
+      }
+      continue;
+    }
     if (sc->cap[i] < need) {
       ++sc->generation;
       // the previous, smaller buffer may still be read by GEMMs in flight on this stream
@@ -1234,6 +1244,8 @@ static int f32_on_tensor_cores(const GemmDesc& d) {
   return tc < fma ? parts : 0;
 }
 
+bool gemm_f32_needs_parts(const GemmDesc& d) { return d.M > 0 && d.N > 0 && d.K > 0 && f32_on_tensor_cores(d) != 0; }
+
 template <bool A_MN, bool B_MN, bool SPLIT>
 static cudaError_t launch_f32_tc(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const F32TcArgs& a, int* d_status, cudaStream_t stream) {
   auto kern = gemm_f32_tc_kernel<A_MN, B_MN, SPLIT>;
@@ -1279,7 +1291,7 @@ int gemm_f32(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t st
     g_gemm_err = "fp32 GEMM cannot write bf16";
     return -2;
   }
-  if (const int parts = f32_on_tensor_cores(d)) {
+  if (const int parts = sc != nullptr ? f32_on_tensor_cores(d) : 0) {
     const int rc = gemm_f32_tc(d, parts, sc, d_status, stream);
     if (rc != kNoScratch) return rc;  // no memory for the parts: the FMA kernels need none
   }

@@ -95,7 +95,12 @@ const char* ane_op_sumsq_noalloc_last_error(void);
  */
 typedef struct ane_gemm_args {
   uint32_t struct_size;
-  int32_t dtype; /* operands: ANE_DTYPE_BF16 (tcgen05), ANE_DTYPE_F32 (SIMT), ANE_DTYPE_BF16X3 (fp32 in, split tcgen05) */
+  /* operands: ANE_DTYPE_BF16 (tcgen05), ANE_DTYPE_F32 (FMA units; large products as six tcgen05 products of three bf16 parts, with no
+   * larger error), ANE_DTYPE_BF16X3 (fp32 in, split tcgen05).  Calls only queue work on the default stream, except that
+   * ANE_DTYPE_BF16X3 allocates for the call and waits.  The first large ANE_DTYPE_F32 product on a device takes 64 MiB there, for
+   * the parts of this and later ones, which is given back when ane_dev_malloc finds no memory otherwise; products whose parts need
+   * more stay on the FMA units. */
+  int32_t dtype;
   const void* d_a;
   const void* d_b;
   void* d_c;

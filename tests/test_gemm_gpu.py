@@ -422,6 +422,55 @@ def test_fp32_products_of_nan_and_infinities_cost_about_what_finite_ones_do(M, N
     assert times[1] < 8 * times[0] and times[2] < 8 * times[0], times
 
 
+def test_fp32_products_are_queued_without_waiting_or_allocating():
+    """A large fp32 product beside a sleeping stream returns at once, as the other products do, also by two threads with operands of their own, and
+    does not disturb what another stream of the thread captures."""
+    import threading
+
+    import torch
+    M, N, K = 1024, 768, 768
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    jobs = []
+    for _ in range(2):
+        a, b = torch.randn(M, K, device="cuda", generator=gen), torch.randn(N, K, device="cuda", generator=gen)
+        c = torch.zeros(M, N, device="cuda")
+        g = _ffi.GemmArgs()
+        g.struct_size = ctypes.sizeof(_ffi.GemmArgs)
+        g.dtype, g.d_a, g.d_b, g.d_c = ane.DTYPE_F32, a.data_ptr(), b.data_ptr(), c.data_ptr()
+        g.m, g.n, g.k, g.lda, g.ldb, g.ldc, g.out_mode, g.alpha = M, N, K, K, K, N, 1, 1.0
+        _ck(lib.ane_op_gemm(ctypes.byref(g)))
+        jobs.append((g, a, b, c, c.clone()))
+    torch.cuda.synchronize()
+    for _, a, b, _, first in jobs:
+        assert rel_l2(first.cpu().numpy(), (a.double() @ b.double().T).cpu().numpy()) < 4e-7
+    torch.cuda._sleep(200_000_000)  # about 0.1 s on the default stream
+    for g, *_ in jobs:
+        _ck(lib.ane_op_gemm(ctypes.byref(g)))
+    assert not torch.cuda.current_stream().query()
+    torch.cuda.synchronize()
+
+    def many(g, a, b, c, first):
+        for _ in range(50):
+            lib.ane_op_gemm(ctypes.byref(g))
+
+    threads = [threading.Thread(target=many, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for _, _, _, c, first in jobs:
+        assert torch.equal(c, first)
+    x, graph = torch.zeros(4, device="cuda"), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x += 1
+        _ck(lib.ane_op_gemm(ctypes.byref(jobs[0][0])))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [1.0] * 4 and torch.equal(jobs[0][3], jobs[0][4])
+
+
 def test_gemm_rejects_misaligned_pitch():
     A = np.zeros((16, 20), np.float32)  # 20 bf16 = 40 bytes per row: not a 16-byte multiple
     dA, dB, dC = _up_bf16(A), _up_bf16(A), _up(np.zeros((16, 16), np.float32))
