@@ -373,6 +373,7 @@ class EngineT final : public EngineBase {
   int layout_params();
   int alloc_buffers();
   int alloc_decode();
+  void reserve_parts();
   int refresh_shadow();
   int forward(const uint16_t* d_tok, int B, int Tl, int pos0);
   int head_and_backward(int B);
@@ -393,8 +394,8 @@ class EngineT final : public EngineBase {
   bool qkv_f32_ = false;
   bool att_tc_ = false;  // tensor-core attention kernels (bf16 operands, head_dim 32, 48 or 64)
   bool x3_ = false;      // fp32 engine whose GEMMs run as three bf16 tensor-core products (ANE_DTYPE_BF16X3)
-  SplitScratch split_;   // its operand halves, or the fp32 mode's operands in three parts (one stream at a time: no side stream in
-                         // the first of the two modes)
+  SplitScratch split_;   // its operand halves, which grow on demand (no side stream in this mode), or the fp32 mode's operands in three
+                         // parts: reserve_parts()
   SplitScratch dw_split_;  // the same for the weight-gradient stream
   bool decoding_ = false;  // forward() runs one KV-cached decode step
   std::vector<T*> kcache_, vcache_;  // [B, S_, KV*hd] per layer (one block each for all layers), allocated by the first decode
@@ -917,10 +918,44 @@ int EngineT<T>::open(const ane_options& opts, const uint16_t* tokens, uint64_t n
     for (auto& ev : ev_gather_)
       if ((rc = cuda_check(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event")) != 0) return rc;
   }
+  reserve_parts();
   if ((rc = cuda_check(cudaStreamSynchronize(stream_), "open sync")) != 0) return rc;
   t_open_ns_ = now_ns();
   st_.struct_size = sizeof(ane_state);
   return 0;
+}
+
+// fp32 mode: room for the operands' parts of every product that the tensor cores take, in full batches: smaller ones need less.
+// Taken here and not by the first update, which waited, freed and allocated for each product larger than those before (first update
+// of 8 x 256 tokens 8.5 ms, later ones 3.6).  The largest operand is the chunk of d logits, three parts of [ce_rows, V] for
+// each stream: 2 x 393 MB at 2048 x 32000.  Where there is no memory for it all products stay on the FMA units.
+template <typename T>
+void EngineT<T>::reserve_parts() {
+  if (!kIsF32 || x3_) return;
+  size_t all[2] = {0, 0}, dw[2] = {0, 0};
+  auto product = [&](int M, int N, int K, bool a_mn, bool b_mn) {
+    GemmDesc g;
+    g.M = M; g.N = N; g.K = K; g.lda = a_mn ? M : K; g.ldb = b_mn ? N : K; g.ldc = N; g.a_mn = a_mn; g.b_mn = b_mn;
+    g.out = a_mn ? GEMM_OUT_ACCUM : GEMM_OUT_F32;
+    size_t bytes[2];
+    if (!gemm_f32_parts(g, bytes)) return;
+    for (int i = 0; i < 2; ++i) {
+      all[i] = std::max(all[i], bytes[i]);  // a profiled step has its weight gradients on the main stream
+      if (a_mn) dw[i] = std::max(dw[i], bytes[i]);
+    }
+  };
+  const int layer[5][2] = {{QKVD_, D_}, {D_, QD_}, {N13_, D_}, {D_, Hd_}, {isN_ ? D_ : 0, D_}};  // q|k|v, Wo, W1|W3, W2, smear gate
+  for (const auto& w : layer) {
+    product(M_, w[0], w[1], false, false);
+    product(M_, w[1], w[0], false, true);
+    product(w[0], w[1], M_, true, true);
+  }
+  product(ce_rows_, V_, D_, false, false);
+  product(ce_rows_, D_, V_, false, true);
+  product(V_, D_, ce_rows_, true, true);
+  product(V_, S_, D_, false, false);  // EvalLogits, both layouts
+  product(S_, V_, D_, false, false);
+  if (split_.reserve(all) && dw_overlap_) dw_split_.reserve(dw);
 }
 
 template <typename T>

@@ -830,7 +830,25 @@ __global__ void split_operands_kernel(const SplitOperand a, const SplitOperand b
   }
 }
 
+bool SplitScratch::reserve(const size_t (&bytes)[2]) {
+  for (int i = 0; i < 2; ++i) {
+    if (cap[i] >= bytes[i]) continue;
+    ++generation;
+    if (buf[i]) cudaFree(buf[i]);
+    buf[i] = nullptr;
+    cap[i] = 0;
+    if (cudaMalloc(&buf[i], bytes[i]) != cudaSuccess) {
+      cudaGetLastError();
+      buf[i] = nullptr;
+      release();
+      return false;
+    }
+    cap[i] = bytes[i];
+  }
+  return true;
+}
 void SplitScratch::release() {
+  if (buf[0] || buf[1]) ++generation;
   for (int i = 0; i < 2; ++i) {
     if (buf[i]) cudaFree(buf[i]);
     buf[i] = nullptr;
@@ -839,6 +857,13 @@ void SplitScratch::release() {
 }
 
 static constexpr int kNoScratch = -3;
+// Bytes of operand `i` of `d` in `parts` bf16 parts, and their pitch.
+static size_t parts_bytes(const GemmDesc& d, int parts, int i, int* pitch) {
+  const bool mn = i == 0 ? d.a_mn : d.b_mn;
+  const int outer = i == 0 ? d.M : d.N, kp = (d.K + GEMM_BK - 1) / GEMM_BK * GEMM_BK;
+  *pitch = mn ? (outer + 7) / 8 * 8 : parts * kp;
+  return sizeof(bf16) * (size_t)(mn ? parts * kp : outer) * *pitch;
+}
 // The operands of `d` in `parts` bf16 parts each, in the scratch.
 static int split_operands(const GemmDesc& d, int parts, SplitScratch* sc, SplitOperand (&o)[2], cudaStream_t stream) {
   const int kp = (d.K + GEMM_BK - 1) / GEMM_BK * GEMM_BK;
@@ -852,9 +877,8 @@ static int split_operands(const GemmDesc& d, int parts, SplitScratch* sc, SplitO
     o[i].cols = mn ? outer : d.K;
     o[i].kp = kp;
     o[i].k_major = mn ? 0 : 1;
-    o[i].pitch = mn ? (outer + 7) / 8 * 8 : parts * kp;
+    const size_t need = parts_bytes(d, parts, i, &o[i].pitch);
     o[i].vec = o[i].ld % 4 == 0 && (reinterpret_cast<uintptr_t>(o[i].src) & 15) == 0;
-    const size_t need = sizeof(bf16) * (size_t)(mn ? parts * kp : outer) * o[i].pitch;
     if (sc->arena != nullptr) {
       o[i].dst = reinterpret_cast<bf16*>(static_cast<char*>(sc->arena) + used);
       used += (need + 255) / 256 * 256;
@@ -864,6 +888,7 @@ static int split_operands(const GemmDesc& d, int parts, SplitScratch* sc, SplitO
       }
       continue;
     }
+    if (sc->cap[i] < need && parts == 3) return kNoScratch;
     if (sc->cap[i] < need) {
       ++sc->generation;
       // the previous, smaller buffer may still be read by GEMMs in flight on this stream
@@ -1244,13 +1269,15 @@ static int f32_on_tensor_cores(const GemmDesc& d) {
   return tc < fma ? parts : 0;
 }
 
-bool gemm_f32_needs_parts(const GemmDesc& d) { return d.M > 0 && d.N > 0 && d.K > 0 && f32_on_tensor_cores(d) != 0; }
-
+template <bool A_MN, bool B_MN, bool SPLIT>
+static bool load_f32_tc() {
+  static unsigned long long done = 0;
+  return smem_opt_in(gemm_f32_tc_kernel<A_MN, B_MN, SPLIT>, F32TC_SMEM, done);
+}
 template <bool A_MN, bool B_MN, bool SPLIT>
 static cudaError_t launch_f32_tc(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const F32TcArgs& a, int* d_status, cudaStream_t stream) {
   auto kern = gemm_f32_tc_kernel<A_MN, B_MN, SPLIT>;
-  static unsigned long long done = 0;
-  if (!smem_opt_in(kern, F32TC_SMEM, done)) return cudaErrorInvalidValue;
+  if (!load_f32_tc<A_MN, B_MN, SPLIT>()) return cudaErrorInvalidValue;
   const int tiles = ((a.M + 127) / 128) * ((a.N + 127) / 128);
   if constexpr (SPLIT)
     return launch_pdl_cluster(kern, dim3((unsigned)(tiles * a.parts)), dim3(F32TC_THREADS), F32TC_SMEM, stream, (unsigned)a.parts, ta, tb, tc, a, d_status);
@@ -1283,6 +1310,20 @@ static int gemm_f32_tc(const GemmDesc& d, int parts, SplitScratch* sc, int* d_st
     return -4;
   }
   return 0;
+}
+
+bool gemm_f32_parts(const GemmDesc& d, size_t (&bytes)[2]) {
+  const int parts = d.M > 0 && d.N > 0 && d.K > 0 ? f32_on_tensor_cores(d) : 0;
+  if (parts == 0) return false;
+  int pitch;
+  for (int i = 0; i < 2; ++i) bytes[i] = parts_bytes(d, 3, i, &pitch);
+  cudaFuncAttributes attr;
+  cudaFuncGetAttributes(&attr, split_operands_kernel<3>);
+  if (parts > 1) d.a_mn ? (d.b_mn ? load_f32_tc<true, true, true>() : load_f32_tc<true, false, true>())
+                        : (d.b_mn ? load_f32_tc<false, true, true>() : load_f32_tc<false, false, true>());
+  else d.a_mn ? (d.b_mn ? load_f32_tc<true, true, false>() : load_f32_tc<true, false, false>())
+              : (d.b_mn ? load_f32_tc<false, true, false>() : load_f32_tc<false, false, false>());
+  return true;
 }
 
 int gemm_f32(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t stream) {

@@ -88,20 +88,23 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream);
 // fp32 operands at split precision on the tensor cores: A and B are each cut into a bf16 (hi, lo) pair
 // (hi = bf16(x), lo = bf16(x - hi): together ~16 significand bits) and the product is formed as Ah*Bh + Ah*Bl + Al*Bh
 // with fp32 accumulation, one GEMM over a contraction of three passes (the dropped Al*Bl term is ~2^-18 relative).
-// Output kinds GEMM_OUT_F32 (with residuals) and GEMM_OUT_ACCUM.  The scratch holds both operands' halves and grows on
-// demand, or lays them out in an arena that somebody else owns and that does not grow; one scratch serves one stream at a time.
+// Output kinds GEMM_OUT_F32 (with residuals) and GEMM_OUT_ACCUM.  The scratch holds both operands' halves and grows on demand.
+// (gemm_f32 takes what has been reserved, or lays the parts out in an arena that somebody else owns, and does not grow either.)
+// One scratch serves one stream at a time.
 struct SplitScratch {
   void* arena = nullptr;
   size_t arena_bytes = 0;
   void* buf[2] = {nullptr, nullptr};  // A, B, in two or three parts
   size_t cap[2] = {0, 0};             // bytes
   uint64_t generation = 0;            // counts the times that a buffer moved: what was captured before holds old addresses
+  bool reserve(const size_t (&bytes)[2]);  // both buffers or none
   void release();
 };
 int gemm_bf16x3(const GemmDesc& d, SplitScratch* scratch, int* d_status, cudaStream_t stream);
 // fp32 operands with the error of fp32 sums (the fp32 parity mode): on the FMA units or, for products that are large enough, as six
 // products of bf16 parts (hi, mid, lo) on the tensor cores: none without a scratch for the parts (nullptr, or no memory for it).
-bool gemm_f32_needs_parts(const GemmDesc& d);
+// gemm_f32_parts: the bytes of both operands' parts, false for a product that the FMA units take; it also loads the kernels.
+bool gemm_f32_parts(const GemmDesc& d, size_t (&bytes)[2]);
 int gemm_f32(const GemmDesc& d, SplitScratch* scratch, int* d_status, cudaStream_t stream);
 
 // Up to four accumulating products C_p += A_p^T B_p (both operands stored [K, .], the same K: the weight gradients of

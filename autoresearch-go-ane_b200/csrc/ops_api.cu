@@ -240,7 +240,8 @@ int32_t ane_op_gemm(const ane_gemm_args* a) {
     if (int r = current_device(&dev)) return r;
     std::lock_guard<std::mutex> lock(g_parts_mutex);
     auto& parts = g_parts_dev[dev];
-    if (!parts.block && !parts.refused && gemm_f32_needs_parts(d)) {
+    size_t bytes[2];
+    if (!parts.block && !parts.refused && gemm_f32_parts(d, bytes) && bytes[0] + bytes[1] <= kPartsBytes) {
       cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // another stream of this thread may be capturing
       cudaThreadExchangeStreamCaptureMode(&mode);
       parts.refused = cudaMalloc(&parts.block, kPartsBytes) != cudaSuccess;

@@ -250,3 +250,55 @@ def test_logits_of_a_window_do_not_depend_on_its_batch(arch, dtype):
         e.close()
     np.testing.assert_array_equal(logits[0], logits[1])
     np.testing.assert_array_equal(logits[0], logits[2])
+
+
+F32_CFG = dict(dim=288, hidden=768, heads=6, layers=2, vocab=32000, seq=256)  # products that the tensor cores take in three parts
+
+
+def _free_mib():
+    import torch
+    return torch.cuda.mem_get_info()[0] / 2**20
+
+
+def _f32_engine(toks):
+    e = ane.open(_options(F32_CFG, tokens=toks, batch=4, arch=ane.ARCH_LLAMA, quirks=0, compute_dtype=ane.DTYPE_F32, accum_steps=1))
+    C.random_init(e, 6)
+    return e
+
+
+def test_fp32_engines_take_their_memory_when_they_are_opened():
+    """Updates, evaluation losses and logits of an fp32 engine allocate nothing (16 MiB for kernels that are loaded on their first
+    launch), and it leaves nothing behind."""
+    toks = O.zipf_tokens(1 << 14, F32_CFG["vocab"], 31)
+    _f32_engine(toks).close()
+    before = _free_mib()
+    e = _f32_engine(toks)
+    opened = _free_mib()
+    for use in (e.step, lambda: e.eval_loss(toks[:1024]), lambda: e.eval_logits(toks[:256]), lambda: e.eval_logits(toks[:256], layout=1), e.step):
+        use()
+        assert abs(_free_mib() - opened) < 16
+    e.close()
+    assert abs(_free_mib() - before) < 16
+
+
+def test_fp32_engine_without_memory_for_the_parts_of_its_operands():
+    """An engine that fits without the parts opens where they do not fit, and stays on the FMA units without asking for memory again."""
+    toks = O.zipf_tokens(1 << 14, F32_CFG["vocab"], 31)
+    e = _f32_engine(toks)
+    losses = [e.step().loss for _ in range(3)]
+    held = _free_mib()
+    e.close()
+    free = _free_mib()
+    parts = 2 * 6 * 1024 * 32000 / 2**20  # of d logits alone, on both streams
+    filler = ane._ffi.lib.ane_dev_malloc(int((held + parts - 100) * 2**20))  # leaves the engine, and 100 MiB of these 375
+    assert filler
+    try:
+        e = _f32_engine(toks)
+        opened = _free_mib()
+        assert opened > 40 and free - held > parts
+        for want in losses:
+            assert e.step().loss == pytest.approx(want, abs=1e-4)
+            assert abs(_free_mib() - opened) < 16
+        e.close()
+    finally:
+        ane._ffi.lib.ane_dev_free(filler)
