@@ -299,6 +299,15 @@ class EngineT final : public EngineBase {
   int dalloc(U** p, size_t count) {
     void* q = nullptr;
     cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(U));
+    if (e == cudaErrorMemoryAllocation && kIsF32 && !x3_ && (split_.buf[0] || split_.buf[1])) {
+      // The fp32 mode can do without the room for its operands' parts, what is asked for here it cannot.
+      cudaGetLastError();
+      cudaStreamSynchronize(stream_);
+      cudaStreamSynchronize(dw_stream_);
+      split_.release();
+      dw_split_.release();
+      e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(U));
+    }
     if (e != cudaSuccess) return cuda_check(e, "cudaMalloc");
     allocs_.push_back(q);
     *p = reinterpret_cast<U*>(q);

@@ -302,3 +302,29 @@ def test_fp32_engine_without_memory_for_the_parts_of_its_operands():
         e.close()
     finally:
         ane._ffi.lib.ane_dev_free(filler)
+
+
+def test_fp32_engine_gives_the_parts_of_its_operands_back_for_a_decode():
+    """The caches of the first decode come after the parts: where only one of them fits, it is the caches.  Same tokens as with both, and
+    the evaluation loss, a graph of the former scratch by then, within the rounding of the FMA units."""
+    toks = O.zipf_tokens(1 << 14, F32_CFG["vocab"], 31)
+    prompts = np.ascontiguousarray(toks[:64]).reshape(4, 16)
+    cfg = dict(F32_CFG, seq=12288, vocab=512)  # caches of 216 MiB, logits of 24
+    e = ane.open(_options(cfg, batch=4, arch=ane.ARCH_LLAMA, quirks=0, compute_dtype=ane.DTYPE_F32))
+    C.random_init(e, 6)
+    tokens = e.decode_greedy(prompts % 512, 6)
+    e.close()
+    e = ane.open(_options(cfg, batch=4, arch=ane.ARCH_LLAMA, quirks=0, compute_dtype=ane.DTYPE_F32))
+    C.random_init(e, 6)
+    window = np.ascontiguousarray(toks[:cfg["seq"]] % 512)
+    losses = [e.eval_loss(window)[0] for _ in range(3)]
+    caches = 2 * 4 * 4 * 2 * cfg["seq"] * cfg["dim"] / 2**20
+    filler = ane._ffi.lib.ane_dev_malloc(int((_free_mib() - caches / 2) * 2**20))
+    assert filler
+    try:
+        np.testing.assert_array_equal(e.decode_greedy(prompts % 512, 6), tokens)
+        for _ in range(3):
+            assert e.eval_loss(window)[0] == pytest.approx(losses[0], rel=1e-5)
+        e.close()
+    finally:
+        ane._ffi.lib.ane_dev_free(filler)
