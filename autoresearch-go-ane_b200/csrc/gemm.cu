@@ -200,15 +200,6 @@ static int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
     }
     return 0;
   }
-  if constexpr (GemmCfg<BN, MT>::SPLIT) {  // split_k = -(CTAs per tile)
-    cudaError_t e = launch_pdl_cluster(kern, dim3((unsigned)(base_tiles * -split_k)), dim3(threads), smem_bytes, stream, (unsigned)-split_k, ta, tb,
-                                       tc, td, epi, d.M, d.N, d.K, split_k, d_status, (const GemmGroup*)nullptr);
-    if (e != cudaSuccess) {
-      g_gemm_err = std::string("gemm_tc split launch: ") + cudaGetErrorString(e);
-      return -4;
-    }
-    return 0;
-  }
   int grid;
   if (split_k > 0) {
     const int tiles = base_tiles * split_k;
@@ -234,13 +225,13 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
                         int* d_status, cudaStream_t stream) {
   EpiParams epi{d.alpha, d.res1, d.s1, d.res2, d.s2, d.ldres, reinterpret_cast<bf16*>(d.aux), d.ldaux,
                 d.rope_cos, d.rope_sin, d.rope_seq, d.rope_pos0, d.rope_cols, d.tgt, d.tgt_out, d.tgt_row0,
-                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, reinterpret_cast<float*>(d.C), d.ldc, d.seg_kb};
-  const int whole = GemmCfg<BN, MT>::SPLIT ? split_k : 1;  // schedule of the epilogues that need whole tiles
+                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, d.seg_kb};
+  constexpr int whole = 1;  // schedule of the epilogues that need whole tiles
   constexpr bool NARROW = GemmCfg<BN, MT>::NARROW;
   CUtensorMap tc;
-  if constexpr (BN == 32 || GemmCfg<BN, MT>::SPLIT) {
+  if constexpr (BN == 32) {
     if (d.out != GEMM_OUT_F32) {
-      g_gemm_err = "32-column tiles and tiles shared by a cluster are built for the fp32 store";
+      g_gemm_err = "32-column tiles are built for the fp32 store";
       return -2;
     }
   } else {
@@ -341,8 +332,8 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
     }
     return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_F32>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
   }
-  if constexpr (GemmCfg<BN, MT>::PAIR || GemmCfg<BN, MT>::SPLIT || BN == 32) {
-    g_gemm_err = "cluster tiles and 32-column tiles are built for the non-accumulating epilogues";
+  if constexpr (GemmCfg<BN, MT>::PAIR || BN == 32) {
+    g_gemm_err = "pair tiles and 32-column tiles are built for the non-accumulating epilogues";
     return -2;
   } else {
     return launch_tc<BN, MT, A_MN, B_MN, EPI_REDUCE_F32>(ta, tb, tc, tc, epi, d, split_k, d_status, stream);
@@ -361,11 +352,7 @@ static int dispatch_layout(const GemmDesc& d, int split_k, int* d_status, cudaSt
   if (!d.b_mn) ok = make_tmap(&tb, d.B, k_extent, d.N, d.ldb, GEMM_BK, GemmCfg<BN, MT>::PAIR ? BN / 2 : BN);
   else         ok = make_tmap(&tb, d.B, d.N, k_extent, d.ldb, 64, GEMM_BK);
   if (!ok) return -2;
-  if constexpr (GemmCfg<BN, MT>::SPLIT) {  // dX form only: see cluster_split()
-    if (!d.a_mn && d.b_mn) return dispatch_epi<BN, MT, false, true>(ta, tb, d, split_k, d_status, stream);
-    g_gemm_err = "tiles shared by a cluster: unsupported operand layout";
-    return -2;
-  } else if constexpr (BN == 32) {
+  if constexpr (BN == 32) {
     if (!d.a_mn && !d.b_mn) return dispatch_epi<BN, MT, false, false>(ta, tb, d, split_k, d_status, stream);
     g_gemm_err = "32-column tiles: unsupported operand layout";
     return -2;
@@ -496,16 +483,17 @@ static GemmPlan plan_gemm(const GemmDesc& d, int sms) {
   return p;
 }
 
-// Clusters of `size` (2, 4 or 8) CTAs of a kernel that takes an SM's shared memory that the device holds at once.
-template <class K>
-static int resident_clusters(K kern, int threads, uint32_t bytes, int size, int (&known)[4]) {
+// Clusters of `size` (2, 4 or 8) CTAs of the fp32 kernel, each with an SM's shared memory, that the device holds at once.
+static int resident_clusters_f32(int size) {
+  static int known[4] = {-1, -1, -1, -1};
+  auto kern = gemm_f32_tc_kernel<true, true, true>;
   const int at = size == 8 ? 3 : size == 4 ? 2 : 1;
   if (known[at] < 0) {
     int n = 0;
     cudaLaunchConfig_t q = {};
     q.gridDim = dim3((unsigned)(size * 148));
-    q.blockDim = dim3((unsigned)threads);
-    q.dynamicSmemBytes = bytes;
+    q.blockDim = dim3(F32TC_THREADS);
+    q.dynamicSmemBytes = F32TC_SMEM;
     cudaLaunchAttribute a[1];
     a[0].id = cudaLaunchAttributeClusterDimension;
     a[0].val.clusterDim.x = (unsigned)size;
@@ -513,7 +501,7 @@ static int resident_clusters(K kern, int threads, uint32_t bytes, int size, int 
     a[0].val.clusterDim.z = 1;
     q.attrs = a;
     q.numAttrs = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F32TC_SMEM) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kern, &q) != cudaSuccess)
       n = 0;  // a part of a GPU may hold no cluster of this size: products take whole tiles there
     cudaGetLastError();
@@ -521,17 +509,9 @@ static int resident_clusters(K kern, int threads, uint32_t bytes, int size, int 
   }
   return known[at];
 }
-static int resident_clusters(int size) {
-  static int known[4] = {-1, -1, -1, -1};
-  return resident_clusters(gemm_tc_kernel<128, GEMM_MT_SPLIT, false, true, EPI_STORE_F32>, GEMM_THREADS,
-                           GemmCfg<128, GEMM_MT_SPLIT>::smem_bytes(EPI_STORE_F32), size, known);
-}
-static int resident_clusters_f32(int size) {
-  static int known[4] = {-1, -1, -1, -1};
-  return resident_clusters(gemm_f32_tc_kernel<true, true, true>, F32TC_THREADS, F32TC_SMEM, size, known);
-}
+
 // Width of a narrow tile (64 or 32 columns; 0: none) for a product with less than a wave of 128 x 128 tiles.  One CTA per SM
-// then, and its time is that of its own chain: k-blocks of about 310 cycles at 32 columns, 340 at 64 and 370 at 128 (more SMs pull
+// then, and its time is that of its own chain: k-blocks of about 310 cycles at 32 columns, 330 at 64 and 370 at 128 (more SMs pull
 // operands, each of them less), and an epilogue of about 700 cycles per staged piece, four of them for 128 fp32 columns.  Every
 // element is the same sum in the same order whatever the width.  us, 128 columns -> narrow: 256 x 2304 x 768 (bf16) 6.7 -> 6.1,
 // 256 x 768 x 768 (fp32 + residual) 9.9 -> 5.5, 256 x 768 x 2048 13.7 -> 9.3, 512 x 768 x 6144 26.0 -> 20.9, 1000 x 288 x 288 8.7 -> 4.4,
@@ -561,32 +541,6 @@ static int narrow_width(const GemmDesc& d) {
   }
   return best_bn < 128 ? best_bn : 0;
 }
-// How many CTAs share a 128 x 128 tile (0: none): as many as stay resident together with at least four k-blocks each, where that
-// beats one CTA per tile.  ns, fitted to the dX forms of 256, 512 and 1024 rows with 12 to 64 k-blocks: a split tile takes
-// 7000 + 256 per own k-block (the exchange takes about 2000 of them) and 700 more in halves (64 columns of direct stores per
-// thread), a narrow one 5000 + 180 per k-block.  us, whole -> split: 256 x 768 x 4096 16.4 -> 9.0 in eighths, 512 x 768 x 2304 11.5 ->
-// 9.5 in quarters, 1024 x 768 x 4096 17.3 -> 16.0 in halves.  (12.4, 11.3 and 18.0 while every CTA fetched the parts of its columns
-// from the others' shared memory, one after the other, and an eighth was 32 columns for four of them and none for the rest.)
-// Parts of a contraction have less of the tensor core's truncation than the whole, so a product then depends, by its rounding, on how
-// many tiles there are beside it.  Where that may be:
-//   * Backward products towards the inputs (B MN-major).
-//   * Not the forward ones.  A window's activations are the same whatever batch it comes in; shared tiles moved the logits of
-//     one window by 4e-3 from those of a large batch.
-//   * Not split precision, whose backward carries a difference far through unscaled scores: after two updates of the reference
-//     network at 2 x 256 gradients were up to 2.2e-3 from those of whole tiles, where the mode is to hold 1e-3.
-static int cluster_split(const GemmDesc& d) {
-  // Off unless ANE_B200_GEMM_CLUSTER_SPLIT=1: over 20 updates of the 110M model at 2 x 256 the loss was up to 5.1e-3 from the
-  // fp32 oracle's with shared tiles and 1.8e-3 with whole ones.
-  static const bool on = [] { const char* e = getenv("ANE_B200_GEMM_CLUSTER_SPLIT"); return e && e[0] == '1'; }();
-  if (!on || d.a_mn || !d.b_mn || d.seg_kb > 0 || d.out != GEMM_OUT_F32) return 0;
-  const long tiles = (long)((d.M + 127) / 128) * ((d.N + 127) / 128);
-  const int kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;
-  const int whole = narrow_width(d) ? 5000 + 180 * kblocks : 6500 + 210 * kblocks;
-  for (int s : {8, 4, 2})
-    if (kblocks >= 4 * s && tiles <= resident_clusters(s) && 7000 + 256 * kblocks / s + (s == 2 ? 700 : 0) < whole) return s;
-  return 0;
-}
-
 int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return 0;
   if (d.out == GEMM_OUT_F32 && (d.res1 || d.res2) && (d.ldres % 4 != 0 ||
@@ -641,7 +595,6 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
     if (!no_pair && d.M >= 256 && eff >= 0.8) return dispatch_layout<256, GEMM_MT_PAIR>(d, 1, d_status, stream);
     return dispatch_layout<256, 1>(d, 1, d_status, stream);
   }
-  if (const int s = cluster_split(d)) return dispatch_layout<128, GEMM_MT_SPLIT>(d, -s, d_status, stream);
   if (const int bn = narrow_width(d))
     return bn == 64 ? dispatch_layout<64, 1>(d, 1, d_status, stream) : dispatch_layout<32, 1>(d, 1, d_status, stream);
   GemmPlan p = plan_gemm(d, gemm_num_sms());

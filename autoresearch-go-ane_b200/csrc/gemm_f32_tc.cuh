@@ -16,7 +16,8 @@
 // A CTA works on 128 x 128 tiles, persistent: warp 0 issues the copies (two stages of 96 KB, the three parts of both
 // operands), warp 1 the MMAs (1536 cycles a k-block; the latency and fill of 96 KB behind two stages bound it, about 2250 cycles),
 // warps 2 - 9 hold the sums, 64 columns of a row per thread.  SPLIT: a cluster shares a tile along the contraction (products with
-// few tiles and a long one, dW and the head's dX) and exchanges its sums as the split tiles of gemm_tc.cuh do, in rank order.
+// few tiles and a long one, dW and the head's dX): a CTA parks its sums in shared memory, each warp copies every CTA of the cluster the
+// columns which that one finishes (bulk copies, counted by the receiver's mbarrier), and what arrives is summed in rank order.
 // An operand that is not finite, or not after the factor, makes the sums infinite or NaN (its other parts are NaN), and so does a sum
 // above 2^96; such elements are computed again with fp32 FMAs.
 #pragma once

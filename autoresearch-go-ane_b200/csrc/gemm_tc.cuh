@@ -43,13 +43,6 @@ static constexpr int GEMM_THREADS = 192;  // TMA warp, MMA warp, four epilogue w
 // accumulator set): the least fill per FLOP, for long K with few columns.
 static constexpr int GEMM_MT_PAIR = 4;
 static constexpr int GEMM_MT_PAIR2 = 5;
-// MT = GEMM_MT_SPLIT: a cluster of 2, 4 or 8 CTAs shares one 128 x BN tile along the contraction.  With few tiles (256
-// token rows: 12 tiles of 128 x 128 for N = 768) the k-blocks of a tile are a serial chain on one SM, 64 of them for
-// K = 4096; split, each CTA runs its share, parks its fp32 accumulators in its own shared memory (the pipeline stages
-// are free by then) and copies to every CTA of the cluster the columns which that one finishes (bulk copies, each warp its own
-// rows, counted by the receiver's mbarrier); a CTA sums what it receives in rank order and stores its columns.  No
-// workspace, no atomics.  Built for the dX form: see cluster_split().
-static constexpr int GEMM_MT_SPLIT = 6;
 static constexpr uint32_t GEMM_SMEM_LIMIT = 232448u;
 
 // Epilogue kinds.  Every kind stages 32-row x 128-byte pieces of the accumulator in 128B-swizzled
@@ -93,8 +86,7 @@ enum EpiKind : int {
 template <int BN, int MT>
 struct GemmCfg {
   static constexpr bool PAIR = MT == GEMM_MT_PAIR || MT == GEMM_MT_PAIR2;
-  static constexpr bool SPLIT = MT == GEMM_MT_SPLIT;
-  static constexpr int SUBS = (MT == GEMM_MT_PAIR || SPLIT) ? 1 : (MT == GEMM_MT_PAIR2 ? 2 : MT);  // 128-row sub-tiles per CTA
+  static constexpr int SUBS = MT == GEMM_MT_PAIR ? 1 : (MT == GEMM_MT_PAIR2 ? 2 : MT);  // 128-row sub-tiles per CTA
   static constexpr int BM_TILE = (PAIR ? 2 : 1) * SUBS * GEMM_BM;       // rows of a scheduled tile
   static constexpr uint32_t A_BYTES = SUBS * GEMM_BM * GEMM_BK * 2;     // per CTA and stage
   // a CTA of a pair holds half of the tile's B rows, rounded up to whole 64-column chunks (an MN-major half of
@@ -129,17 +121,15 @@ struct GemmCfg {
   __host__ __device__ static constexpr int res_depth(int epi) { return BN <= (epi == EPI_DRELU2 ? 64 : 32) ? 1 : 2; }
   __host__ __device__ static constexpr uint32_t staging_bytes(int epi) { return (uint32_t)(epi_warps(epi) * sbuf(epi)) * 4096u; }
   __host__ __device__ static constexpr uint32_t in_bytes(int epi) { return tma_in(epi) ? (uint32_t)(epi_warps(epi) * res_depth(epi)) * 4096u : 0u; }
-  static constexpr uint32_t EXCHANGE_BYTES = SPLIT ? GEMM_BM * BN * 4u : 0u;  // partial sums that a CTA of a split tile receives
   // Pipeline depth.  Single-CTA kernels take what fits beside the staging buffers and use the TMA-fed residual epilogue only if
-  // its buffers still fit; pair kernels and narrow tiles give up stages for them instead.  Split tiles keep the exchange beside
-  // the stages and stage no output.
+  // its buffers still fit; pair kernels and narrow tiles give up stages for them instead.
   __host__ __device__ static constexpr int stages(int epi) {
-    const uint32_t own = SPLIT ? 1024u + EXCHANGE_BYTES : 1024u + staging_bytes(epi) + (PAIR || NARROW || needs_in(epi) ? in_bytes(epi) : 0u);
+    const uint32_t own = 1024u + staging_bytes(epi) + (PAIR || NARROW || needs_in(epi) ? in_bytes(epi) : 0u);
     const int n = (int)((GEMM_SMEM_LIMIT - own) / (A_BYTES + B_BYTES)), most = NARROW ? 8 : 6;
     return n > most ? most : n;
   }
   __host__ __device__ static constexpr uint32_t smem_bytes(int epi) {  // +1024: alignment
-    return stages(epi) * (A_BYTES + B_BYTES) + 1024 + (SPLIT ? EXCHANGE_BYTES : staging_bytes(epi) + in_bytes(epi));
+    return stages(epi) * (A_BYTES + B_BYTES) + 1024 + staging_bytes(epi) + in_bytes(epi);
   }
   __host__ __device__ static constexpr bool fits(int epi) { return smem_bytes(epi) <= GEMM_SMEM_LIMIT && stages(epi) >= 3; }
   static constexpr int ACC_COLS = SUBS * BN;                     // one accumulator set
@@ -219,8 +209,6 @@ struct EpiParams {
   int ce_rows;           // row count of the statistics buffer
   int ce_col0;           // vocabulary column of this product's column 0
   int ce_softcap;        // z = 15 tanh(logit / 15) (ane/common.go:272-287)
-  float* out;            // C and its pitch: split tiles store without a tensor map
-  int ldout;
   int seg_kb;            // > 0: operands are (hi | lo) halves of seg_kb k-blocks each, three passes hi*lo, lo*hi, hi*hi
 };
 
@@ -237,7 +225,6 @@ struct alignas(64) GemmGroup {
 
 // Work scheduler shared by the three warp roles (each role walks the same sequence).
 //   split_k > 0 : classic persistent schedule, work item = (k split, tile), stride gridDim.x.
-//   split_k < 0 : one tile per cluster of -split_k CTAs, each with an equal share of the k-blocks.
 //   split_k == 0: stream-K.  The tiles x k-blocks units are dealt out in equal contiguous ranges, one per
 //                 CTA; a range is cut into segments at tile boundaries and every segment ends in a
 //                 reduce-add, so it needs an accumulating epilogue.  Removes the partial last wave.
@@ -259,9 +246,7 @@ struct GemmSched {
     tiles = g ? g->tile0[g->n] : tiles_m * tiles_n;
     kblocks = (K + GEMM_BK - 1) / GEMM_BK;
     split_k = split;
-    if (split_k < 0) {
-      w = 0;
-    } else if (split_k > 0) {
+    if (split_k > 0) {
       kb_per_split = (kblocks + split_k - 1) / split_k;
       total_work = tiles * split_k;
       w = bid;
@@ -273,15 +258,6 @@ struct GemmSched {
   }
   // Next non-empty segment: tile (tm, tn) and k-block range [kb0, kb1).
   __device__ __forceinline__ bool next(int& tm, int& tn, int& kb0, int& kb1) {
-    if (split_k < 0) {
-      if (w != 0) return false;
-      w = 1;
-      const int part = bid % -split_k;
-      kb0 = kblocks * part / -split_k;
-      kb1 = kblocks * (part + 1) / -split_k;
-      place(bid / -split_k, tm, tn);
-      return true;
-    }
     if (split_k > 0) {
       while (w < total_work) {
         const int split = w / tiles;
@@ -327,8 +303,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   using Cfg = GemmCfg<BN, MT>;
   // grouped launches exist for the accumulating weight-gradient form on single-CTA tiles only
   constexpr bool kGroup = A_MN && B_MN && EPI == EPI_REDUCE_F32 && MT < GEMM_MT_PAIR;
-  constexpr bool SPLIT = Cfg::SPLIT;
-  const int parts = SPLIT ? -split_k : 1;  // CTAs that share a tile
   const GemmGroup* grp = kGroup ? group : nullptr;
   int M = M0, N = N0;  // the epilogue of a grouped launch sets them per tile
   constexpr bool kTmaRes = Cfg::tma_in(EPI);  // an input piece per output piece, by TMA
@@ -349,7 +323,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __shared__ __align__(8) uint64_t bar_tfull[NBUF];
   __shared__ __align__(8) uint64_t bar_tempty[NBUF];
   __shared__ uint32_t tmem_slot;
-  __shared__ __align__(8) uint64_t bar_res[8][4];  // TMA-fed input pieces (residual, h13): piece landed; [0]: split tiles, sums landed
+  __shared__ __align__(8) uint64_t bar_res[8][4];  // TMA-fed input pieces (residual, h13): piece landed
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_a0 = smem_base;
@@ -362,7 +336,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // A pipeline wait that gave up earlier in this stream poisons the status word: later launches
   // return at once instead of each running into its own time-out.
   // (a cluster always runs through: its CTAs must take the same path, and every wait below is bounded)
-  if (!PAIR && !SPLIT && status != nullptr && *reinterpret_cast<volatile int*>(status) != DEV_OK) return;
+  if (!PAIR && status != nullptr && *reinterpret_cast<volatile int*>(status) != DEV_OK) return;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;  // 0 = the CTA that issues the MMAs
   const int sched_id = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int sched_n = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -379,11 +353,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int b = 0; b < RD; ++b) mbar_init(smem_u32(&bar_res[w][b]), 1);
       tma_prefetch_desc(&tmD);
     }
-    if constexpr (SPLIT)
-      for (int w = 0; w < 4; ++w) {
-        mbar_init(smem_u32(&bar_res[0][w]), 1);
-        mbar_expect_tx(smem_u32(&bar_res[0][w]), Cfg::EXCHANGE_BYTES / 4);
-      }
     for (int b = 0; b < NBUF; ++b) {
       mbar_init(smem_u32(&bar_tfull[b]), 1);
       mbar_init(smem_u32(&bar_tempty[b]), (PAIR ? 2 : 1) * EW);  // the epilogue warps of both CTAs
@@ -405,7 +374,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   pdl_trigger();
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR || SPLIT) cluster_sync_all();  // the peers' barriers exist before anything signals them
+  if constexpr (PAIR) cluster_sync_all();  // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
   pdl_wait();  // operands, residuals and C belong to earlier kernels: nothing above touched them
@@ -539,107 +508,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         ++local;
       }
     }
-  } else if constexpr (SPLIT) {
-    // ------------------------------ epilogue warps of a split tile ------------------------------
-    const int g = warp & 3;  // TMEM lanes, and rows of the tile, [32 g, 32 g + 32)
-    const int part = (int)blockIdx.x % parts, cols = BN / parts;
-    GemmSched sched;
-    sched.init(M, N, K, BM, BN, split_k, sched_id, sched_n, grp);
-    int tm, tn, kb0, kb1;
-    sched.next(tm, tn, kb0, kb1);
-    const int m = tm * BM + g * 32 + lane, n_begin = tn * BN + part * cols;  // this thread's row and first column to finish
-    const float a1 = epi.res1 && epi.s1 ? *epi.s1 : 1.f, a2 = epi.res2 && epi.s2 ? *epi.s2 : 1.f;
-    bool ok = mbar_wait(smem_u32(&bar_tfull[0]), 0u, status, DEV_MBAR_TIMEOUT_EPILOGUE);
-    tc_fence_after();
-    // Partial sums as [row group][column / 4][row in the group] float4 over the pipeline stages, which the MMAs no longer need:
-    // the columns of one receiver are one piece of 512 * cols / 4 bytes per group.
-    const uint32_t parked = smem_base + (uint32_t)g * (BN / 4 * 512u), landed = smem_stage0 + (uint32_t)g * (BN / 4 * 512u);
-    const uint32_t piece = (uint32_t)cols / 4 * 512u;
-#pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
-      float v[32];
-      __syncwarp();
-      tmem_ld_32x32(tmem_base + ((uint32_t)(g * 32) << 16) + (uint32_t)c, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(parked + (uint32_t)(c / 4 + q) * 512u + (uint32_t)lane * 16u), "f"(v[4 * q]),
-                     "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
-                     : "memory");
-    }
-    tc_fence_before();
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane < parts) {  // one copy per lane; every CTA receives the parts in rank order
-      const uint32_t to = (uint32_t)((lane + part) % parts);
-      bulk_copy_to_cta(map_to_cta(landed + (uint32_t)part * piece, to), parked + to * piece, piece, map_to_cta(smem_u32(&bar_res[0][g]), to));
-    }
-    __syncwarp();
-    // 16 columns at a time; what they are combined with is requested before the wait for the sums
-    static_assert(!SPLIT || EPI == EPI_STORE_F32, "split tiles are built for the fp32 store");
-    bool waited = false;
-#pragma unroll 1
-    for (int c = 0; c < cols; c += 16) {
-      const int n0 = n_begin + c;
-      const bool in = m < M && n0 < N;
-      float4 r1[4], r2[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        r1[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        r2[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      auto request = [&](float4 (&r)[4], const float* res) {
-        if (res == nullptr || !in) return;
-        const float* rp = res + (size_t)m * epi.ldres + n0;
-        if (n0 + 16 <= N) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) r[q] = *reinterpret_cast<const float4*>(rp + 4 * q);
-        } else {
-          float* f = reinterpret_cast<float*>(r);
-#pragma unroll
-          for (int e = 0; e < 16; ++e)
-            if (n0 + e < N) f[e] = rp[e];
-        }
-      };
-      request(r1, epi.res1);
-      request(r2, epi.res2);
-      if (!waited) {
-        ok = mbar_wait(smem_u32(&bar_res[0][g]), 0u, status, DEV_MBAR_TIMEOUT_EPILOGUE) && ok;
-        waited = true;
-      }
-      float acc[16];
-#pragma unroll
-      for (int e = 0; e < 16; ++e) acc[e] = 0.f;
-#pragma unroll 2
-      for (int p = 0; p < parts; ++p) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float4 t;
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
-                       : "r"(landed + (uint32_t)p * piece + (uint32_t)(c / 4 + q) * 512u + (uint32_t)lane * 16u) : "memory");
-          acc[4 * q] += t.x; acc[4 * q + 1] += t.y; acc[4 * q + 2] += t.z; acc[4 * q + 3] += t.w;
-        }
-      }
-      if (!in || !ok) continue;
-      float* out = epi.out + (size_t)m * epi.ldout + n0;
-      const float *f1 = reinterpret_cast<const float*>(r1), *f2 = reinterpret_cast<const float*>(r2);
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        acc[e] *= epi.alpha;
-        if (epi.res1) acc[e] += a1 * f1[e];
-        if (epi.res2) acc[e] += a2 * f2[e];
-      }
-      if (n0 + 16 <= N) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<float4*>(out + 4 * q) = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 16; ++e)
-          if (n0 + e < N) out[e] = acc[e];
-      }
-    }
-    if (!waited) mbar_wait(smem_u32(&bar_res[0][g]), 0u, status, DEV_MBAR_TIMEOUT_EPILOGUE);
   } else {
     // ------------------------------ epilogue warps ------------------------------
     const int lane_group = warp & 3;  // TMEM lanes [32*lane_group, 32*lane_group+32)
@@ -1105,8 +973,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   tc_fence_before();
   __syncthreads();
-  // the peer has drained its accumulators and its last loads have landed; all partial sums have been read
-  if constexpr (PAIR || SPLIT) cluster_sync_all();
+  // the peer has drained its accumulators and its last loads have landed
+  if constexpr (PAIR) cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
     if constexpr (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);

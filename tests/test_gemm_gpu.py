@@ -295,9 +295,9 @@ def test_relu2_backward_fused_into_the_dx_product(M, Hd, K):
 
 @pytest.mark.parametrize("M,N,K,b_mn", [(1, 8, 256, 0), (37, 768, 768, 0), (128, 128, 1024, 1), (256, 768, 4096, 1), (129, 136, 520, 0),
                                         (300, 2304, 768, 0), (512, 1000, 264, 1)])
-def test_tiles_shared_by_a_cluster(M, N, K, b_mn):
-    """Few 128 x 128 tiles: two, four or eight CTAs share one along the contraction and meet in distributed shared memory
-    (uneven shares of the k-blocks, ragged rows and columns, more CTAs than pieces), plain and with a TMA-fed residual."""
+def test_products_of_few_tiles(M, N, K, b_mn):
+    """Less than a wave of 128 x 128 tiles: 32- and 64-column ones, ragged rows and columns, plain and with a residual that TMA feeds or the
+    threads read."""
     rng = np.random.default_rng(M + N + K)
     A = _bf16_round(rng.standard_normal((M, K)).astype(np.float32) * 0.1)
     B = _bf16_round(rng.standard_normal((K, N) if b_mn else (N, K)).astype(np.float32) * 0.1)
@@ -308,7 +308,8 @@ def test_tiles_shared_by_a_cluster(M, N, K, b_mn):
 
 
 @pytest.mark.parametrize("M,Hd,K", [(256, 2048, 768), (200, 320, 264), (100, 64, 512)])
-def test_activation_backward_on_tiles_shared_by_a_cluster(M, Hd, K):
+def test_activation_backward_on_narrow_tiles(M, Hd, K):
+    """Few enough tiles for 64-column ones, whose epilogues keep one input piece in flight, or two (SwiGLU)."""
     test_swiglu_backward_fused_into_the_dx_product(M, Hd, K)
     test_relu2_backward_fused_into_the_dx_product(M, Hd, K)
 
