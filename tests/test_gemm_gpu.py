@@ -361,6 +361,14 @@ def test_fp32_products_on_the_tensor_cores(M, N, K, a_mn, b_mn, out):
         want = (A.T if a_mn else A).astype(np.float64) @ (B if b_mn else B.T).astype(np.float64)
         got = _gemm(ane.DTYPE_F32, A, B, R, M, N, K, a_mn, b_mn, 2) if out == 2 else _gemm(ane.DTYPE_F32, A, B, np.zeros_like(R), M, N, K, a_mn, b_mn, 1, res=R)
         assert rel_l2(got, want + R) < (2.0**-23 if positive else max(np.sqrt(K) / 8, 2.0) * 2.0**-24)
+    # One term per sum: the FMA units would round the product of the two operands once, parts that are added and cut off are a bit off here and there.
+    one = np.zeros_like(A)
+    term = np.arange(M) % K
+    (one.T if a_mn else one)[np.arange(M), term] = draw(M)
+    exact = (one.T if a_mn else one)[np.arange(M), term][:, None] * (B if b_mn else B.T)[term]
+    got = _gemm(ane.DTYPE_F32, one, B, np.zeros_like(R), M, N, K, a_mn, b_mn, out)
+    assert (got != exact).any()
+    np.testing.assert_allclose(got, exact, rtol=2.0**-22)
     at = (A.T if a_mn else A), (B if b_mn else B.T)  # views: [M, K] and [K, N]
     at[0][3, 5], at[0][7, 1], at[1][4, 2], at[0][9, 0] = np.inf, np.nan, -np.inf, 3.4e38
     with np.errstate(invalid="ignore", over="ignore"):
