@@ -513,9 +513,10 @@ static int resident_clusters_f32(int size) {
 // Width of a narrow tile (64 or 32 columns; 0: none) for a product with less than a wave of 128 x 128 tiles.  One CTA per SM
 // then, and its time is that of its own chain: k-blocks of about 310 cycles at 32 columns, 330 at 64 and 370 at 128 (more SMs pull
 // operands, each of them less), and an epilogue of about 700 cycles per staged piece, four of them for 128 fp32 columns.  Every
-// element is the same sum in the same order whatever the width.  us, 128 columns -> narrow: 256 x 2304 x 768 (bf16) 6.7 -> 6.1,
-// 256 x 768 x 768 (fp32 + residual) 9.9 -> 5.5, 256 x 768 x 2048 13.7 -> 9.3, 512 x 768 x 6144 26.0 -> 20.9, 1000 x 288 x 288 8.7 -> 4.4,
-// SwiGLU backward of 256 x 2048 x 768 9.2 -> 7.5.
+// element is the same sum in the same order whatever the width.  us, 128 columns -> narrow: 256 x 2304 x 768 (bf16) 6.2 -> 5.8,
+// 256 x 768 x 768 (fp32 + residual) 8.8 -> 5.6, 256 x 768 x 2048 12.4 -> 9.0, 512 x 768 x 6144 26.0 -> 20.9, 1000 x 288 x 288 8.2 -> 4.4,
+// accumulated 768 x 768 x 256 7.3 -> 5.0, 2304 x 768 x 440 (the line: eight k-blocks) 8.7 both, SwiGLU backward of 256 x 2048 x 768
+// 9.2 -> 7.5; of 440 products of 48 to 2048 rows none was slower.
 static int narrow_width(const GemmDesc& d) {
   static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_NARROW"); return e && e[0] == '0'; }();  // A/B measurements
   if (off || d.split_k > 1) return 0;
@@ -630,11 +631,14 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
             (double)tiles2 / (double)(waves2 * pairs) * ((double)d.N / (double)(((d.N + 191) / 192) * 192));
         const bool residual = d.res1 != nullptr || d.res2 != nullptr;
         if (eff2 >= 0.85 && !(kblocks < 32 && residual)) bn = 512;
-        // A long K with a residual that TMA can fetch: 256 x 192 tiles, two waves of them, whose first epilogue hides behind the
-        // second tile (W2 forward, 8192 x 768 x 2048: 32 -> 28.7 us; of 16384 rows 86 -> 71).
+        // A long K with a residual that TMA can fetch: 256 x 192 tiles, whose first epilogues hide behind the tiles after them.  us, this
+        // against what is chosen otherwise: 8192 x 768 x 2048 32.1 / 40.3, 8192 x 2304 x 2048 80 / 114, 16384 x 768 x 2048 64 / 82,
+        // 12288 x 768 x 3072 62.7 / 62.3, 6144 x 512 x 2048 20.3 / 21.3 (34 products of 3000 to 16384 rows and K up to 3072: 0.99 to
+        // 1.48 times as fast).  From K = 4096 on, in several waves, an epilogue is a small part and the wider tiles' fill counts: 12288 x 768 x
+        // 4096 83 / 78, 8192 x 768 x 8192 96 / 86, 16384 x 768 x 8192 209 / 193.  In one wave these stay ahead: 4096 x 768 x 8192 45.6 / 52.1.
         const long tiles3 = (long)((d.M + 255) / 256) * ((d.N + 191) / 192);
         const double eff3 = (double)tiles3 / (double)((tiles3 + pairs - 1) / pairs * pairs) * ((double)d.N / (double)(((d.N + 191) / 192) * 192));
-        if (kblocks >= 32 && d.res1 != nullptr && d.res2 == nullptr && !d.b_mn && eff3 >= 0.8) bn = 192;
+        if (kblocks >= 32 && (kblocks < 64 || tiles3 <= pairs) && d.res1 != nullptr && d.res2 == nullptr && !d.b_mn && eff3 >= 0.8) bn = 192;
       }
     }
     if (bn == 512 && d.out != GEMM_OUT_BF16_SWIGLU) return dispatch_layout<192, GEMM_MT_PAIR2>(d, 1, d_status, stream);
@@ -1217,7 +1221,10 @@ static int f32_on_tensor_cores(const GemmDesc& d) {
       parts = p;
     }
   }
-  // us: k-blocks at 1.25, the cut (4 bytes read, 6 written per element) and its launch; the FMA kernels at about 40 TFLOP/s
+  // us: k-blocks at 1.25, the cut (4 bytes read, 6 written per element) and its launch; the FMA kernels at about 40 TFLOP/s.  Of 176
+  // products of 64 to 4096 rows, all layouts, those that this sends to the tensor cores are 1.28 to 5.1 times as fast there: next to
+  // the line 768 x 768 x 256 12.9 us (16.5 on the FMA units), 768 x 768 x 512 17.3 (22.7), 512 x 1536 x 288 14.5 (22.7), 1024 x 288 x
+  // 768 14.2 (20.6).  The other side may be up to 1.4 times too slow: 256 x 768 x 768 takes 20.6 where 400 x 768 x 768 takes 14.3.
   const double tc = 1.25 * best + ((double)d.M + d.N) * d.K * 10.0 / 5e6 + 4.0, fma = 2.0 * d.M * d.N * d.K / 40e6 + 5.0;
   return tc < fma ? parts : 0;
 }
