@@ -1,4 +1,4 @@
-"""tcgen05 GEMM (and the fp32 SIMT GEMM) against the oracle's naive loops, through the C ABI.
+"""tcgen05 GEMM (and fp32 products on the FMA units and the tensor cores) against the oracle's naive loops, through the C ABI.
 Shapes cover the step's three operand layouts, ragged edges and split-K accumulation."""
 import ctypes
 
@@ -478,6 +478,35 @@ def test_fp32_products_are_queued_without_waiting_or_allocating():
     graph.replay()
     torch.cuda.synchronize()
     assert x.tolist() == [1.0] * 4 and torch.equal(jobs[0][3], jobs[0][4])
+
+
+def test_fp32_products_give_their_memory_back_to_allocations():
+    """An allocation that only fits with the block for the parts succeeds, and products go on without one (in a process of its own: for good)."""
+    import os
+    import subprocess
+    import sys
+
+    body = """
+import numpy as np, torch
+import test_gemm_gpu as t
+rng = np.random.default_rng(5)
+A, B = rng.standard_normal((1024, 768)).astype(np.float32), rng.standard_normal((768, 768)).astype(np.float32)
+want = A.astype(np.float64) @ B.astype(np.float64).T
+run = lambda: t._gemm(t.ane.DTYPE_F32, A, B, np.zeros((1024, 768), np.float32), 1024, 768, 768, 0, 0, 1)
+first = run()
+room = [t.lib.ane_dev_malloc(32 << 20) for _ in range(2)]
+filler = t.lib.ane_dev_malloc(torch.cuda.mem_get_info()[0] + (32 << 20))
+assert filler
+for p in room:
+    t.lib.ane_dev_free(p)
+second = run()
+assert t.rel_l2(first, want) < 2e-7 and t.rel_l2(second, want) < 1e-6 and (first != second).any()
+t.lib.ane_dev_free(filler)
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    path = os.pathsep.join([here, os.path.dirname(here), os.path.dirname(os.path.dirname(os.path.abspath(ane.__file__)))])
+    r = subprocess.run([sys.executable, "-c", body], env=dict(os.environ, PYTHONPATH=path), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 def test_gemm_rejects_misaligned_pitch():
