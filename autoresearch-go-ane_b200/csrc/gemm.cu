@@ -1,4 +1,4 @@
-// GEMM launchers: tcgen05 bf16 path (gemm_tc.cuh) and the fp32 SIMT path.
+// GEMM launchers: tcgen05 bf16 path (gemm_tc.cuh), fp32 products on the tensor cores (gemm_f32_tc.cuh) and on the FMA units.
 #include "gemm.h"
 
 #include <cuda.h>

@@ -139,7 +139,7 @@ typedef struct ane_options {
   int32_t batch;          /* sequences per ane_step call (reference: 1) */
   int32_t arch;           /* ANE_ARCH_*                                  */
   int32_t quirks;         /* 1: reproduce the reference's backward exactly (ANE_ARCH_REFERENCE only) */
-  int32_t compute_dtype;  /* ANE_DTYPE_BF16 (tensor cores), ANE_DTYPE_F32 (SIMT parity mode) or ANE_DTYPE_BF16X3 */
+  int32_t compute_dtype;  /* ANE_DTYPE_BF16 (tensor cores), ANE_DTYPE_F32 (parity mode, see below) or ANE_DTYPE_BF16X3 */
   float rope_theta;       /* 0: 100000 (reference arch) / 10000 (llama arch) */
   int32_t accum_steps;    /* ane_step calls per optimizer update */
   float lr;
@@ -155,6 +155,9 @@ typedef struct ane_options {
   int32_t ce_chunk_cols;   /* vocabulary columns per gradient block of the logit-free training head (0: library chooses) */
   int32_t reserved[5];
 } ane_options;
+/* ANE_DTYPE_F32 engines hold, beside the buffers of every mode, room for their largest operands in three bf16 parts: about twice 6 bytes
+ * per element of the chunk of d logits [ce_chunk_rows, vocab], 0.8 GB at 2048 x 32000.  It is taken by ane_open where there is memory for
+ * it, given back when a later allocation of the engine finds none, and not needed: large products are slower without. */
 
 /* Mirrors ane.StepResult (ane/engine.go:55-69); durations in nanoseconds. */
 typedef struct ane_step_result {
