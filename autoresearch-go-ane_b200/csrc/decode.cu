@@ -23,6 +23,7 @@
 // lane reads 16 contiguous bytes of a weight row (k = 8 (lane % 4) ..) and uses them as the fragments of two MMAs: no
 // ldmatrix.
 #include <algorithm>
+#include <cmath>
 
 #include "decode_common.cuh"
 
@@ -231,7 +232,7 @@ struct RowShare {
 // conversion; rows wider than that go through in segments and are read twice.  gains: the norm's weights in shared memory.
 template <class Row>
 __device__ __forceinline__ void stage_norm(int K, int B, Row row, const uint2* words, uint32_t epoch, const float* gains, uint8_t* stage,
-                                           float* s_sq, const RowShare& sh, const Wait& wait) {
+                                           float* s_sq, const RowShare& sh, float inv_dim, const Wait& wait) {
   constexpr int V = 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = sh.row;
   const int stride = sh.per_row * 128, seg = stride * V, nseg = (K + seg - 1) / seg;
@@ -271,7 +272,7 @@ __device__ __forceinline__ void stage_norm(int K, int B, Row row, const uint2* w
       sq = 0.f;  // the row's other warps
 #pragma unroll 1
       for (int i = 0; i < sh.per_row; ++i) sq += s_sq[warp - sh.sub + i];
-      rms = 1.0f / sqrtf(sq / (float)K + 1e-5f);
+      rms = inverse_sqrt(fmaf(sq, inv_dim, 1e-5f));
     }
     if (it >= nseg || nseg == 1) {
 #pragma unroll
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_steps_kernel(const __grid_
         group_ready();
         const float* gains = reinterpret_cast<const float*>(smem + a.stage_bytes + (group % kSlots + 1) * a.slot_bytes - D * 4);
         stage_norm(D, a.B, [&](int r) { return a.p + a.off_embed_f32 + (size_t)(embed ? s_tok[r] : 0) * D; }, words,
-                       kind == kW13 ? epoch : epoch - 1, gains, stage, s_sq, share, wait);
+                       kind == kW13 ? epoch : epoch - 1, gains, stage, s_sq, share, a.inv_dim, wait);
         __syncthreads();
         src.stage = reinterpret_cast<const uint4*>(stage);
       }
@@ -527,7 +528,13 @@ int decode_steps(DecodeArgs a, void* words, int sms, cudaStream_t s) {
   const int qd = a.H * a.hd, qkv = (a.H + 2 * a.KV) * a.hd;
   const int rep = a.H / a.KV;
   a.group = rep <= 8 ? rep : 1;  // query heads per attention item: rows of one fragment
-  a.hd_magic = 0xffffffffu / (unsigned)a.hd + 1u;  // col / hd = umulhi(col, hd_magic) for col < 2^16
+  a.rep = rep;
+  a.items = a.H / a.group;
+  a.hd_magic = 0xffffffffu / (unsigned)a.hd + 1u;
+  a.rep_magic = 0xffffffffu / (unsigned)a.rep + 1u;
+  a.items_magic = 0xffffffffu / (unsigned)a.items + 1u;
+  a.score_scale = 1.4426950408889634f / sqrtf((float)a.hd);
+  a.inv_dim = 1.0f / (float)a.D;
   const size_t rows = word_rows(a.D, a.Hd, a.H, a.KV, a.hd, a.B, sms);
   uint2* p = reinterpret_cast<uint2*>(words);
   a.w_x0 = p; p += rows * a.D;

@@ -258,9 +258,9 @@ __global__ void __launch_bounds__(kLaunch, 1) decode_batch_kernel(const __grid_c
         if (warp == 1) {
           int group = a.group, hd = a.hd;
           asm volatile("" : "+r"(group), "+r"(hd));  // see attention_phase()
-          const int hgroups = a.H / group, box = min(256, a.S);
+          const int hgroups = a.items, box = min(256, a.S);
           for (int item = blockIdx.x; item < a.B * hgroups; item += gridDim.x) {
-            const int b = item / hgroups, kvh = (item - b * hgroups) * group / (a.H / a.KV);
+            const int b = quotient(item, hgroups, a.items_magic), kvh = quotient((item - b * hgroups) * group, a.rep, a.rep_magic);
             for (int j = lane * box; j < pos; j += 32 * box) {
               asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(&maps.keys)), "r"(kvh * hd),
                            "r"(b * a.S + j), "r"(l) : "memory");
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(kLaunch, 1) decode_batch_kernel(const __grid_c
                   wait_for(smem_u32(&s_squares), squares_parity);
                   squares_parity ^= 1u;
                   sq = (s_sq[0][r] + s_sq[1][r]) + (s_sq[2][r] + s_sq[3][r]);
-                  rms = 1.0f / sqrtf(sq / (float)p.K + 1e-5f);
+                  rms = inverse_sqrt(fmaf(sq, a.inv_dim, 1e-5f));
                 }
                 if ((it >= nseg || nseg == 1) && p.nu > 0) {
 #pragma unroll

@@ -32,6 +32,19 @@ __device__ __forceinline__ float4 ldf_l2_if(const float* p, bool take) {
   return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
 }
 
+// n / d for n below 2^16 with magic = 0xffffffff / d + 1 from the host.  A division, like an IEEE square root, is a long run of
+// dependent instructions, and where it is reached once in a phase they come from beyond the instruction cache: between the sum of
+// squares and the first normalised column, 1 / sqrt(x / dim) took 2000 cycles.
+__device__ __forceinline__ int quotient(int n, int d, unsigned magic) { return d == 1 ? n : (int)__umulhi((unsigned)n, magic); }
+// 1 / sqrt(x) and 1 / x to an ulp or two: the hardware's approximation and one step of Newton's method
+__device__ __forceinline__ float inverse_sqrt(float x) {
+  const float y = rsqrtf(x);
+  return y * fmaf(-0.5f * x * y, y, 1.5f);
+}
+__device__ __forceinline__ float inverse(float x) {
+  const float y = __fdividef(1.0f, x);
+  return y * fmaf(-x, y, 2.0f);
+}
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&v);
@@ -119,12 +132,12 @@ __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16*
   // opaque: what follows from the sizes is computed here, not kept in registers (or spilled) through the whole generation
   int hd = a.hd, G = a.group, H = a.H, KV = a.KV;
   asm volatile("" : "+r"(hd), "+r"(G), "+r"(H), "+r"(KV));
-  const int kvd = KV * hd, qd = H * hd, rep = H / KV, hgroups = H / G;
-  const float sc = 1.4426950408889634f / sqrtf((float)hd);  // scores in the log2 domain
+  const int kvd = KV * hd, qd = H * hd, hgroups = a.items;
+  const float sc = a.score_scale;  // scores in the log2 domain
   constexpr int kStep = NW * 16;                              // keys of one tile of every warp
 #pragma unroll 1
   for (int item = blockIdx.x; item < a.B * hgroups; item += gridDim.x) {
-    const int b = item / hgroups, h0 = (item - b * hgroups) * G, kvh = h0 / rep;
+    const int b = quotient(item, hgroups, a.items_magic), h0 = (item - b * hgroups) * G, kvh = quotient(h0, a.rep, a.rep_magic);
     const bf16* kb = kc + (size_t)b * a.S * kvd + (size_t)kvh * hd;
     const bf16* vb = vc + (size_t)b * a.S * kvd + (size_t)kvh * hd;
     const uint2* wk = nullptr;  // words of the new key
@@ -266,7 +279,7 @@ __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16*
     const int used = min(NW, pos / 16 + 1);  // warps that had keys
 #pragma unroll 1
     for (int i = threadIdx.x; i < G * hd / 2; i += NW * 32) {
-      const int h = (2 * i) / hd, d = 2 * i - h * hd;
+      const int h = quotient(2 * i, hd, a.hd_magic), d = 2 * i - h * hd;
       const float* from = sm + h * kPitch;
       float mx = -INFINITY;
 #pragma unroll 8
@@ -281,7 +294,8 @@ __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16*
         o0 += v.x * f;
         o1 += v.y * f;
       }
-      const uint32_t v = pack2(o0 / ls, o1 / ls);
+      const float inv = inverse(ls);
+      const uint32_t v = pack2(o0 * inv, o1 * inv);
       const size_t at = (size_t)b * (qd / 2) + (size_t)((h0 + h) * hd + d) / 2;
       put_word(a.w_att + at, v, epoch);
     }

@@ -124,7 +124,9 @@ struct DecodeArgs {
   float temperature;             // <= 1e-6: argmax
   int B, D, Hd, L, H, KV, hd, V, S, prompt, n_new, u_stride;
   int group, stage_bytes, slot_bytes, slots, units, units_w2;  // set by decode_steps
-  unsigned hd_magic;
+  unsigned hd_magic, rep_magic, items_magic;  // see quotient()
+  int rep, items;                             // query heads of a KV head; attention items of a sequence
+  float score_scale, inv_dim;
   uint2 *w_x0, *w_x1, *w_qkv, *w_att, *w_gate;
 };
 bool decode_steps_supported(int D, int Hd, int H, int KV, int hd, int V, int batch, int sms);
