@@ -319,6 +319,26 @@ class EngineT final : public EngineBase {
     if constexpr (kIsF32) return P_ + off;
     else return Sh_ + off;
   }
+  // Sums of shares of a contraction (GemmDesc::parts), from a product on the main stream to the norm behind it; a wave of tiles.
+  size_t dx_parts_floats() const {
+    const size_t wave = (size_t)gemm_num_sms() * 128 * 128, most = (size_t)kMostParts * parts_rows(M_) * D_;
+    return rmsnorm_backward_adds(D_) && (!kIsF32 || x3_) ? std::min(wave, most) : 0;
+  }
+  // The gradient of a norm's output, which only that norm's backward reads: the product, then what it left and in how many parts.
+  struct Parts {
+    const float* dy;
+    int n = 1;
+    size_t stride = 0;
+  };
+  int gemm_to_norm(GemmDesc& d, Parts& out) {
+    d.parts = dx_parts_;
+    d.parts_bytes = sizeof(float) * dx_parts_floats();
+    d.n_parts = &out.n;
+    const int rc = gemm(d);
+    out.dy = out.n > 1 ? dx_parts_ : (const float*)d.C;
+    out.stride = (size_t)parts_rows(d.M) * d.N;
+    return rc;
+  }
   int gemm(const GemmDesc& d, cudaStream_t on = nullptr) {
     int rc;
     cudaStream_t st = on ? on : stream_;
@@ -444,7 +464,7 @@ class EngineT final : public EngineBase {
   T *x0_t_ = nullptr, *dgp_t_ = nullptr;
   // Backward operands that the weight-gradient GEMMs read are double-buffered by layer parity, so those
   // GEMMs can trail the main chain on their own stream by up to two layers.
-  float *dcur_[2] = {nullptr, nullptr}, *dxn_ = nullptr, *dy_ = nullptr, *dx2_[2] = {nullptr, nullptr},
+  float *dcur_[2] = {nullptr, nullptr}, *dxn_ = nullptr, *dy_ = nullptr, *dx_parts_ = nullptr, *dx2_[2] = {nullptr, nullptr},
         *dqkv_f32_[2] = {nullptr, nullptr};
   T *dcur_t_[2] = {nullptr, nullptr}, *dx2_t_[2] = {nullptr, nullptr}, *dgate_ = nullptr, *dh13_[2] = {nullptr, nullptr},
     *datt_ = nullptr, *dqkv_[2] = {nullptr, nullptr}, *xnf_ = nullptr;
@@ -470,7 +490,7 @@ class EngineT final : public EngineBase {
   int head_cols_ = 0;
   float *ce_stats_ = nullptr, *ce_lse2_ = nullptr, *ce_coef_ = nullptr;
   bf16* dl_block_ = nullptr;
-  int fused_head(int B);
+  int fused_head(int B, Parts& dy);
   T* dlogits_ = nullptr;
   T* dlogits2_ = nullptr;                  // second chunk buffer: the classifier dW GEMM of chunk c runs on the
   cudaEvent_t ev_cls_ce_[2] = {nullptr, nullptr};  // side stream while chunk c+1 is computed
@@ -734,7 +754,7 @@ int EngineT<T>::alloc_buffers() {
     A(x0_, MD); A(xraw_, MD); A(gate_pre_, MD); A(gx0_, MD); A(gmid_, MD); A(dgp_, MD); A(dxs_, MD); A(dxs2_, MD);
     if (!kIsF32) { A(x0_t_, MD); A(dgp_t_, MD); }
   }
-  A(dcur_[0], MD); A(dcur_[1], MD); A(dxn_, MD); A(dy_, MD); A(dx2_[0], MD); A(dx2_[1], MD);
+  A(dcur_[0], MD); A(dcur_[1], MD); A(dxn_, MD); A(dy_, MD); A(dx_parts_, dx_parts_floats()); A(dx2_[0], MD); A(dx2_[1], MD);
   A(dqkv_f32_[0], (size_t)M_ * QKVD_); A(dqkv_f32_[1], (size_t)M_ * QKVD_);
   if (!kIsF32) {
     A(dcur_t_[0], MD); A(dcur_t_[1], MD); A(dx2_t_[0], MD); A(dx2_t_[1], MD);
@@ -1165,18 +1185,20 @@ int EngineT<T>::head_and_backward(int B) {
   count_launch();
   count_valid_targets(d_tgt_, inv_valid_, B, S_, V_, stream_);
   if (head_fused_) {
-    if ((rc = fused_head(B)) != 0) return rc;
+    Parts dy;
+    if ((rc = fused_head(B, dy)) != 0) return rc;
     count_launch();
     reduce_loss(loss_rows_, inv_valid_, d_loss_, B, S_, stream_);
     const float* w_fin = isN_ ? nullptr : P_ + s_rms_final_.off;
     count_launch();
-    rmsnorm_backward<T>(dy_, xs_[L_], w_fin, rstdf_, nullptr, nullptr, dcur_[0], tcopy_arg(dcur_t_[0]),
-                        isN_ ? nullptr : G_ + s_rms_final_.off, M, D_, stream_);
+    rmsnorm_backward<T>(dy.dy, xs_[L_], w_fin, rstdf_, nullptr, nullptr, dcur_[0], tcopy_arg(dcur_t_[0]),
+                        isN_ ? nullptr : G_ + s_rms_final_.off, M, D_, stream_, dy.n, dy.stride);
     return backward_layers(B);
   }
   // The dEmbed GEMM of a chunk runs on the side stream (it only feeds the optimizer); the two dlogits
   // buffers alternate so that the next chunk's cross-entropy does not overwrite its operand.
   cudaStream_t dws = (dw_overlap_ && !profiling_) ? dw_stream_ : stream_;
+  Parts dy;
   int chunk = 0;
   for (int r0 = 0; r0 < M; r0 += ce_rows_, ++chunk) {
     const int rows = std::min(ce_rows_, M - r0);
@@ -1211,7 +1233,8 @@ int EngineT<T>::head_and_backward(int B) {
     gx.A = dlogits; gx.B = wop(s_embed_.off); gx.C = dy_ + (size_t)r0 * D_;
     gx.M = rows; gx.N = D_; gx.K = V_; gx.lda = V_; gx.ldb = D_; gx.ldc = D_; gx.b_mn = true; gx.out = GEMM_OUT_F32;
     count_launch();
-    if ((rc = gemm(gx)) != 0) return rc;
+    dy.dy = dy_;
+    if ((rc = rows == M ? gemm_to_norm(gx, dy) : gemm(gx)) != 0) return rc;
     GemmDesc gw;  // gEmbed += dlogits^T * xn   (ane/stories/cpu.go:366-385)
     gw.A = dlogits; gw.B = xnf_ + (size_t)r0 * D_; gw.C = G_ + s_embed_.off;
     gw.M = V_; gw.N = D_; gw.K = rows; gw.lda = V_; gw.ldb = D_; gw.ldc = D_; gw.a_mn = true; gw.b_mn = true;
@@ -1224,8 +1247,8 @@ int EngineT<T>::head_and_backward(int B) {
   reduce_loss(loss_rows_, inv_valid_, d_loss_, B, S_, stream_);
   const float* w_final = isN_ ? nullptr : P_ + s_rms_final_.off;
   count_launch();
-  rmsnorm_backward<T>(dy_, xs_[L_], w_final, rstdf_, nullptr, nullptr, dcur_[0], tcopy_arg(dcur_t_[0]),
-                      isN_ ? nullptr : G_ + s_rms_final_.off, M, D_, stream_);
+  rmsnorm_backward<T>(dy.dy, xs_[L_], w_final, rstdf_, nullptr, nullptr, dcur_[0], tcopy_arg(dcur_t_[0]),
+                      isN_ ? nullptr : G_ + s_rms_final_.off, M, D_, stream_, dy.n, dy.stride);
   return backward_layers(B);
 }
 
@@ -1239,7 +1262,7 @@ int EngineT<T>::head_and_backward(int B) {
 // HBM traffic per step and no [tokens, vocab] buffer.
 // ------------------------------------------------------------------------------------------------
 template <typename T>
-int EngineT<T>::fused_head(int B) {
+int EngineT<T>::fused_head(int B, Parts& dy) {
   if constexpr (kIsF32) {
     return fail(ANE_ERR_STATE, "storiesane step: the logit-free head runs on bf16 engines");
   } else {
@@ -1271,7 +1294,8 @@ int EngineT<T>::fused_head(int B) {
       gx.M = M; gx.N = D_; gx.K = nc; gx.lda = head_cols_; gx.ldb = D_; gx.ldc = D_; gx.b_mn = true; gx.out = GEMM_OUT_F32;
       if (v0 > 0) { gx.res1 = dy_; gx.s1 = d_one_; gx.ldres = D_; }  // in place: every piece is read before it is written
       count_launch();
-      if ((rc = gemm(gx)) != 0) return rc;
+      dy.dy = dy_;
+      if ((rc = nc == V_ ? gemm_to_norm(gx, dy) : gemm(gx)) != 0) return rc;
       GemmDesc gw;  // gEmbed[v0 : v0 + nc] += block^T * xn   (ane/stories/cpu.go:366-385)
       gw.A = dl_block_; gw.B = xnf_; gw.C = G_ + s_embed_.off + (size_t)v0 * D_;
       gw.M = nc; gw.N = D_; gw.K = M; gw.lda = head_cols_; gw.ldb = D_; gw.ldc = D_; gw.a_mn = true; gw.b_mn = true;
@@ -1354,17 +1378,18 @@ int EngineT<T>::backward_layers(int B) {
       count_launch();
       to_f32_kernel<T><<<ew_grid((uint64_t)M * N13_), 256, 0, stream_>>>(dh13, a.t_dh13, (uint64_t)M * N13_);
     }
+    Parts dx;
     {
       GemmDesc g;  // dx2n = dh13 * W13
       g.A = dh13; g.B = wop(s_w13_[l].off); g.C = dxn_;
       g.M = M; g.N = D_; g.K = N13_; g.lda = N13_; g.ldb = D_; g.ldc = D_; g.b_mn = true; g.out = GEMM_OUT_F32;
       count_launch();
-      if ((rc = gemm(g)) != 0) return rc;
+      if ((rc = gemm_to_norm(g, dx)) != 0) return rc;
     }
     // dx2 = rl*dOut + rms_bwd(dx2n; x2)
     count_launch();
-    rmsnorm_backward<T>(dxn_, a.x2, w_ffn, a.rstd2, dcur, rl, dx2, tcopy_arg(dx2_t_[pb]),
-                        isN_ ? nullptr : G_ + s_rms_ffn_[l].off, M, D_, stream_);
+    rmsnorm_backward<T>(dx.dy, a.x2, w_ffn, a.rstd2, dcur, rl, dx2, tcopy_arg(dx2_t_[pb]),
+                        isN_ ? nullptr : G_ + s_rms_ffn_[l].off, M, D_, stream_, dx.n, dx.stride);
     if (o_.debug_taps) cudaMemcpyAsync(a.t_dx2, dx2, sizeof(float) * MD, cudaMemcpyDeviceToDevice, stream_);
     GemmDesc dw[4];  // this layer's weight-gradient products: dW2, dW13, dWo, dWqkv
     const bool grouped = group_dw_ && M == M_;
@@ -1460,15 +1485,15 @@ int EngineT<T>::backward_layers(int B) {
       g.A = dqkv; g.B = wop(s_qkv_[l].off); g.C = dxn_;
       g.M = M; g.N = D_; g.K = QKVD_; g.lda = QKVD_; g.ldb = D_; g.ldc = D_; g.b_mn = true; g.out = GEMM_OUT_F32;
       count_launch();
-      if ((rc = gemm(g)) != 0) return rc;
+      if ((rc = gemm_to_norm(g, dx)) != 0) return rc;
     }
     // dprev = rms_bwd(dxn; x) + rl*dx2  (+ value-embedding gate path, + mid-layer backout gradient)
     const bool post_fix = is_ve_layer(l) || (isN_ && l == L_ / 2);
     // dprev's buffers were read (as that layer's dOut) by the dW2 GEMM of layer l+1.
     if (dws != stream_ && l + 1 < L_) cudaStreamWaitEvent(stream_, ev_dw_done_[l + 1], 0);
     count_launch();
-    rmsnorm_backward<T>(dxn_, xs_[l], w_att, a.rstd1, dx2, rl, dprev, post_fix ? nullptr : tcopy_arg(dcur_t_[cur ^ 1]),
-                        isN_ ? nullptr : G_ + s_rms_att_[l].off, M, D_, stream_);
+    rmsnorm_backward<T>(dx.dy, xs_[l], w_att, a.rstd1, dx2, rl, dprev, post_fix ? nullptr : tcopy_arg(dcur_t_[cur ^ 1]),
+                        isN_ ? nullptr : G_ + s_rms_att_[l].off, M, D_, stream_, dx.n, dx.stride);
     if (is_ve_layer(l)) {
       count_launch();
       ve_backward<float>(dqkv_f32, xs_[l], d_in_, P_ + s_ve_embed_[l].off, P_ + s_ve_gate_[l].off, a.ve_act,

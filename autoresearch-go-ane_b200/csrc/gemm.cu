@@ -225,7 +225,7 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
                         int* d_status, cudaStream_t stream) {
   EpiParams epi{d.alpha, d.res1, d.s1, d.res2, d.s2, d.ldres, reinterpret_cast<bf16*>(d.aux), d.ldaux,
                 d.rope_cos, d.rope_sin, d.rope_seq, d.rope_pos0, d.rope_cols, d.tgt, d.tgt_out, d.tgt_row0,
-                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, d.seg_kb};
+                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, d.part_rows, d.seg_kb};
   constexpr int whole = 1;  // schedule of the epilogues that need whole tiles
   constexpr bool NARROW = GemmCfg<BN, MT>::NARROW;
   CUtensorMap tc;
@@ -319,8 +319,9 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
     }
   }
   }
-  if (!make_tmap(&tc, d.C, d.N, d.M, d.ldc, 32, 32, true)) return -2;
+  if (!make_tmap(&tc, d.C, d.N, d.part_rows > 0 ? (uint64_t)split_k * d.part_rows : d.M, d.ldc, 32, 32, true)) return -2;
   if (d.out == GEMM_OUT_F32) {
+    if (d.part_rows > 0) return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_F32>(ta, tb, tc, tc, epi, d, split_k, d_status, stream);
     // One residual, K-major operands and room for the residual buffers: let TMA fetch the residual pieces.
     if constexpr (!A_MN && !B_MN && MT != GEMM_MT_PAIR2 && GemmCfg<BN, MT>::fits(EPI_STORE_F32_TMARES)) {
       static const bool no_tma_res = getenv("ANE_B200_NO_TMA_RES") != nullptr;  // A/B measurements
@@ -542,7 +543,40 @@ static int narrow_width(const GemmDesc& d) {
   }
   return best_bn < 128 ? best_bn : 0;
 }
+// Shares of the contraction for a product of few tiles whose consumer adds them up, and the tiles' width; 1: none.  The chain of one
+// CTA is its k-blocks (see narrow_width); a share more costs the consumer about 300 cycles of reading.  us, whole -> shares: 256 x 768
+// x 2304 13.3 -> 9.4, 256 x 768 x 4096 18.3 -> 10.1, 256 x 768 x 32000 96 -> 23, 512 x 768 x 32000 in three passes 285 -> 69, 1000 x
+// 288 x 1536 11.2 -> 8.8, 1000 x 288 x 32000 98 -> 29; the norm behind them 5.3 -> 7.5 at six shares of 256 x 768, 4.0 -> 5.0 at
+// three of 1000 x 288.  (In a pass: one window 2469 -> 2297 us an update, three micro-steps of 5 x 200 3030 -> 2812, the split-precision
+// update of 2 x 256 6749 -> 6287.)
+static int plan_parts(const GemmDesc& d, int& best_bn) {
+  static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_PARTS"); return e && e[0] == '0'; }();  // A/B measurements
+  if (off || d.parts == nullptr || d.n_parts == nullptr || d.out != GEMM_OUT_F32 || d.res1 || d.res2 || d.split_k > 1 || d.N % 4 != 0 ||
+      (reinterpret_cast<uintptr_t>(d.parts) & 15) != 0)
+    return 1;
+  const int sms = gemm_num_sms();
+  const long tiles_m = (d.M + GEMM_BM - 1) / GEMM_BM, kblocks = (d.K + GEMM_BK - 1) / GEMM_BK;
+  const size_t part = sizeof(float) * (size_t)parts_rows(d.M) * d.N;
+  int best = 1;
+  long least = 0;
+  for (int bn : {64, 128}) {
+    const long tiles = tiles_m * ((d.N + bn - 1) / bn);
+    if (tiles > sms) continue;
+    for (int most = 1; most <= kMostParts && tiles * most <= sms && (most == 1 || part * most <= d.parts_bytes); ++most) {
+      const long share = (kblocks + most - 1) / most;
+      const int n = (int)((kblocks + share - 1) / share);  // (none is empty)
+      const long cost = share * (290 + 5 * bn / 8) + bn / 32 * 700 + (n > 1 ? 300 * n : 0);
+      if (least == 0 || cost < least) {
+        least = cost;
+        best = n;
+        best_bn = bn;
+      }
+    }
+  }
+  return best;
+}
 int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
+  if (d.n_parts) *d.n_parts = 1;
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return 0;
   if (d.out == GEMM_OUT_F32 && (d.res1 || d.res2) && (d.ldres % 4 != 0 ||
       (reinterpret_cast<uintptr_t>(d.res1) & 15) != 0 || (reinterpret_cast<uintptr_t>(d.res2) & 15) != 0)) {
@@ -595,6 +629,15 @@ int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
     static const bool no_pair = [] { const char* e = getenv("ANE_B200_GEMM_PAIR"); return e && atoi(e) == 0; }();
     if (!no_pair && d.M >= 256 && eff >= 0.8) return dispatch_layout<256, GEMM_MT_PAIR>(d, 1, d_status, stream);
     return dispatch_layout<256, 1>(d, 1, d_status, stream);
+  }
+  int parts_bn = 0;
+  if (const int n = plan_parts(d, parts_bn); n > 1) {
+    GemmDesc e = d;
+    e.C = d.parts;
+    e.ldc = d.N;
+    e.part_rows = parts_rows(d.M);
+    *d.n_parts = n;
+    return parts_bn == 64 ? dispatch_layout<64, 1>(e, n, d_status, stream) : dispatch_layout<128, 1>(e, n, d_status, stream);
   }
   if (const int bn = narrow_width(d))
     return bn == 64 ? dispatch_layout<64, 1>(d, 1, d_status, stream) : dispatch_layout<32, 1>(d, 1, d_status, stream);

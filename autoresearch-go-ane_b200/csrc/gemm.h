@@ -80,9 +80,17 @@ struct GemmDesc {
   int ce_rows = 0, ce_col0 = 0;
   bool ce_softcap = false;
   int split_k = 0;  // 0 => choose
+  // GEMM_OUT_F32 without residuals, into a consumer that can add: room for `parts` sums of a share of the contraction each, dense
+  // [part][parts_rows(M)][N], where few tiles would leave most SMs idle.  *n_parts = how many there are; 1: the product is in C.
+  float* parts = nullptr;
+  size_t parts_bytes = 0;
+  int* n_parts = nullptr;
+  int part_rows = 0;  // set by gemm_bf16
   int seg_kb = 0;   // > 0: operands hold bf16 (hi | lo) halves of seg_kb k-blocks of 64, K = 3 * 64 * seg_kb (see gemm_bf16x3)
 };
 
+constexpr int kMostParts = 8;
+inline int parts_rows(int M) { return (M + 127) / 128 * 128; }
 // bf16 operands, tcgen05 tensor cores.  Returns 0 or a negative error code.
 int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream);
 // fp32 operands at split precision on the tensor cores: A and B are each cut into a bf16 (hi, lo) pair

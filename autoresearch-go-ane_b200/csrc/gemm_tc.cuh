@@ -209,6 +209,7 @@ struct EpiParams {
   int ce_rows;           // row count of the statistics buffer
   int ce_col0;           // vocabulary column of this product's column 0
   int ce_softcap;        // z = 15 tanh(logit / 15) (ane/common.go:272-287)
+  int part_rows;         // EPI_STORE_F32: rows from one share's sums to the next's
   int seg_kb;            // > 0: operands are (hi | lo) halves of seg_kb k-blocks each, three passes hi*lo, lo*hi, hi*hi
 };
 
@@ -234,13 +235,14 @@ struct GemmSched {
   int bid, nblk;  // this CTA's (or CTA pair's) index and the number of them
   const GemmGroup* grp;  // grouped launch: tiles index the concatenated list
   int bm_tile, prob;     // prob = problem of the segment returned last
+  int part;              // its share of the contraction
   __device__ __forceinline__ void init(int M, int N, int K, int BM_TILE, int BN, int split, int bid_, int nblk_,
                                        const GemmGroup* g = nullptr) {
     bid = bid_;
     nblk = nblk_;
     grp = g;
     bm_tile = BM_TILE;
-    prob = 0;
+    prob = part = 0;
     tiles_m = (M + BM_TILE - 1) / BM_TILE;
     const int tiles_n = (N + BN - 1) / BN;
     tiles = g ? g->tile0[g->n] : tiles_m * tiles_n;
@@ -266,6 +268,7 @@ struct GemmSched {
         kb0 = split * kb_per_split;
         kb1 = min(kb0 + kb_per_split, kblocks);
         if (kb1 <= kb0) continue;
+        part = split;
         place(rem, tm, tn);
         return true;
       }
@@ -950,6 +953,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const uint32_t src = stage_base + (uint32_t)sbuf * 4096u;
           if constexpr (EPI == EPI_REDUCE_F32) tma_reduce_add_2d(pC, src, n0, m_warp);
           else if constexpr (EPI == EPI_DSWIGLU) tma_store_2d(&tmC, src, 2 * n0, m_warp);
+          else if constexpr (EPI == EPI_STORE_F32) tma_store_2d(&tmC, src, n0, m_warp + sched.part * epi.part_rows);
           else tma_store_2d(&tmC, src, n0, m_warp);
           tma_store_commit();
         }

@@ -38,9 +38,11 @@ void rmsnorm_forward(const float* x, const float* w, T* y, float* rstd, int M, i
 // dx = rms_bwd(dy; x, w) + res_scale * res   (ane/common.go:176-197; ane/stories/cpu.go:129-150)
 //   dy: fp32 [M,D];  res/res_scale optional;  dx_f32 and dx_t outputs (dx_t optional copy in T);
 //   dw (optional, weighted norm): dw[i] += sum_m dy*x*rstd.
+//   parts > 1: dy is the sum of that many matrices, part_stride elements apart (rmsnorm_backward_adds(D) only).
 template <typename T>
 void rmsnorm_backward(const float* dy, const float* x, const float* w, const float* rstd, const float* res,
-                      const float* res_scale, float* dx_f32, T* dx_t, float* dw, int M, int D, cudaStream_t s);
+                      const float* res_scale, float* dx_f32, T* dx_t, float* dw, int M, int D, cudaStream_t s, int parts = 1, size_t part_stride = 0);
+inline bool rmsnorm_backward_adds(int D) { return D % 4 == 0 && D <= 1024; }
 
 // In-place interleaved-pair RoPE (ane/train_util.go:204-224) on the q and k column blocks of a packed
 // [M, (H+2KV)*hd] buffer, followed (qk_norm) by the per-head 1.2*rms norm (ane/common.go:199-227);

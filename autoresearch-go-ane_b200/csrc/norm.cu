@@ -292,19 +292,20 @@ __global__ void rmsnorm_backward_kernel(const float* __restrict__ dy, const floa
 
 // Register-resident variant for D <= 128*NV, D % 4 == 0 (NV float4 per lane): each row is read once, and all three
 // inputs of a row (dy, x, residual) are requested before anything is computed, so a row costs one memory
-// round trip.  One block of twelve warps per SM, rows dealt round-robin.
+// round trip.  One block of up to twelve warps per SM (a row a warp where there are few), rows dealt round-robin.
 static constexpr int kRmsBwdWarps = 12;
-template <typename T, int NV>
+// PARTS: dy comes as the sums of shares of a contraction (GemmDesc::parts), added here in their order, two in flight.
+template <typename T, int NV, bool PARTS>
 __global__ void __launch_bounds__(kRmsBwdWarps * 32)
 rmsnorm_backward_reg_kernel(const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ w,
                             const float* __restrict__ rstd, const float* __restrict__ res,
                             const float* __restrict__ res_scale, float* __restrict__ dx_f32, T* __restrict__ dx_t,
-                            float* __restrict__ dw, int M, int D) {
+                            float* __restrict__ dw, int M, int D, int parts, size_t part_stride) {
   pdl_trigger();
   pdl_wait();
   __shared__ float s_dw[kRmsBwdWarps][128 * NV];
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const float rs = res ? (res_scale ? *res_scale : 1.f) : 0.f;
   const float inv_d = 1.0f / (float)D;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -316,7 +317,7 @@ rmsnorm_backward_reg_kernel(const float* __restrict__ dy, const float* __restric
   float4 dwacc[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) dwacc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int row = blockIdx.x * kRmsBwdWarps + warp; row < M; row += gridDim.x * kRmsBwdWarps) {
+  for (int row = blockIdx.x * warps + warp; row < M; row += gridDim.x * warps) {
     const float4* dyr = reinterpret_cast<const float4*>(dy + (size_t)row * D);
     const float4* xr = reinterpret_cast<const float4*>(x + (size_t)row * D);
     const float4* rr = res ? reinterpret_cast<const float4*>(res + (size_t)row * D) : nullptr;
@@ -326,6 +327,26 @@ rmsnorm_backward_reg_kernel(const float* __restrict__ dy, const float* __restric
       g[k] = in(k) ? dyr[lane + 32 * k] : zero;
       v[k] = in(k) ? xr[lane + 32 * k] : zero;
       q[k] = rr && in(k) ? rr[lane + 32 * k] : zero;
+    }
+    if constexpr (PARTS) {
+#pragma unroll 1
+      for (int p = 1; p < parts; p += 2) {
+        const float4* more = reinterpret_cast<const float4*>(dy + p * part_stride + (size_t)row * D);
+        const float4* last = reinterpret_cast<const float4*>(dy + (p + 1) * part_stride + (size_t)row * D);
+        float4 a[NV], b[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+          a[k] = in(k) ? more[lane + 32 * k] : zero;
+          b[k] = in(k) && p + 1 < parts ? last[lane + 32 * k] : zero;
+        }
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+          g[k].x = (g[k].x + a[k].x) + b[k].x;
+          g[k].y = (g[k].y + a[k].y) + b[k].y;
+          g[k].z = (g[k].z + a[k].z) + b[k].z;
+          g[k].w = (g[k].w + a[k].w) + b[k].w;
+        }
+      }
     }
     float r;
     if (rstd) {
@@ -374,7 +395,8 @@ rmsnorm_backward_reg_kernel(const float* __restrict__ dy, const float* __restric
     for (int i = threadIdx.x; i < D; i += blockDim.x) {
       float t = 0.f;
 #pragma unroll
-      for (int wq = 0; wq < kRmsBwdWarps; ++wq) t += s_dw[wq][i];
+      for (int wq = 0; wq < kRmsBwdWarps; ++wq)
+        if (wq < warps) t += s_dw[wq][i];
       atomicAdd(dw + i, t);
     }
   }
@@ -382,15 +404,16 @@ rmsnorm_backward_reg_kernel(const float* __restrict__ dy, const float* __restric
 
 template <typename T>
 void rmsnorm_backward(const float* dy, const float* x, const float* w, const float* rstd, const float* res,
-                      const float* res_scale, float* dx_f32, T* dx_t, float* dw, int M, int D, cudaStream_t s) {
+                      const float* res_scale, float* dx_f32, T* dx_t, float* dw, int M, int D, cudaStream_t s, int parts,
+                      size_t part_stride) {
   if (M <= 0) return;
   int blocks = (M + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  if (D % 4 == 0 && D <= 1024) {
-    const int rb = std::min((M + kRmsBwdWarps - 1) / kRmsBwdWarps, 148);
+  if (rmsnorm_backward_adds(D)) {
+    const int warps = std::min(std::max((M + 147) / 148, 4), kRmsBwdWarps), rb = std::min((M + warps - 1) / warps, 148);
 #define ANE_RMS_BWD_CASE(NV)                                                                                      \
   case NV:                                                                                                         \
-    launch_pdl(rmsnorm_backward_reg_kernel<T, NV>, dim3(rb), dim3(kRmsBwdWarps * 32), 0, s, dy, x, w, rstd, res,    \
-               res_scale, dx_f32, dx_t, dw, M, D);                                                                 \
+    launch_pdl(parts > 1 ? rmsnorm_backward_reg_kernel<T, NV, true> : rmsnorm_backward_reg_kernel<T, NV, false>, dim3(rb),    \
+               dim3(warps * 32), 0, s, dy, x, w, rstd, res, res_scale, dx_f32, dx_t, dw, M, D, parts, part_stride);   \
     return;
     switch ((D + 127) / 128) {
       ANE_RMS_BWD_CASE(1)
@@ -411,8 +434,8 @@ void rmsnorm_backward(const float* dy, const float* x, const float* w, const flo
                                                                          dw, M, D);
 }
 template void rmsnorm_backward<float>(const float*, const float*, const float*, const float*, const float*,
-                                      const float*, float*, float*, float*, int, int, cudaStream_t);
+                                      const float*, float*, float*, float*, int, int, cudaStream_t, int, size_t);
 template void rmsnorm_backward<bf16>(const float*, const float*, const float*, const float*, const float*,
-                                     const float*, float*, bf16*, float*, int, int, cudaStream_t);
+                                     const float*, float*, bf16*, float*, int, int, cudaStream_t, int, size_t);
 
 }  // namespace ane

@@ -521,3 +521,68 @@ def test_gemm_rejects_misaligned_pitch():
     assert b"16-byte" in lib.ane_ops_last_error()
     for p in (dA, dB, dC):
         lib.ane_dev_free(p)
+
+
+def _gradients_in_a_child(env, cases):
+    """Gradients of one micro-step by tensor for each case, from a process with `env`."""
+    import os
+    import subprocess
+    import sys
+    import tempfile
+    code = """
+import sys
+import numpy as np
+import ane
+out = {}
+for i, (dim, hidden, heads, layers, vocab, seq, batch, arch, dtype) in enumerate(%r):
+    rng = np.random.default_rng(7)
+    e = ane.open(ane.Options(dim=dim, hidden=hidden, n_layers=layers, n_heads=heads, n_kv_heads=heads, vocab=vocab, seq=seq, batch=batch, seed=3,
+                             arch=arch, quirks=0, compute_dtype=dtype, accum_steps=1000))
+    for tid in (ane.T_WQ, ane.T_WK, ane.T_WV, ane.T_WO, ane.T_W1, ane.T_W2, ane.T_W3):
+        for l in range(layers):
+            n = e.tensor_size(tid, l)
+            if n > 0:
+                e.import_tensor(tid, l, (0.05 * rng.standard_normal(n)).astype(np.float32))
+    e.import_tensor(ane.T_EMBED, 0, (0.05 * rng.standard_normal(e.tensor_size(ane.T_EMBED, 0))).astype(np.float32))
+    tokens = rng.integers(0, vocab, (batch, seq + 1)).astype(np.uint16)
+    assert e.step_tokens(tokens[:, :-1].copy(), tokens[:, 1:].copy()).device_status == 0
+    for tid in (ane.T_EMBED, ane.T_WQ, ane.T_WO, ane.T_W1, ane.T_W2):
+        out["%%d %%d" %% (i, tid)] = e.export_tensor(tid, 0, ane.engine.G)
+    e.close()
+np.savez(sys.argv[1], **out)
+""" % (cases,)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.path.join(root, "autoresearch-go-ane_b200"), **env)
+    with tempfile.TemporaryDirectory() as where:
+        path = os.path.join(where, "g.npz")
+        done = subprocess.run([sys.executable, "-c", code, path], env=env, capture_output=True, text=True, timeout=300)
+        assert done.returncode == 0, done.stderr[-2000:]
+        return dict(np.load(path))
+
+
+def test_products_in_shares_behind_a_norm():
+    """Gradients with the dX products of few tiles shared out along the contraction (their sums added by the norm's backward)
+    against whole ones.  At split precision what differs is the order of fp32 sums: K / 16 additions, each off by up to 2^-24 of
+    the sum, 9e-6 at K = 2304; 2e-5 for what three layers of it amount to.  In bf16 a difference d of a value moves its rounding
+    (steps of u = 2^-8) with a probability of d / u, by u: sqrt(d u) in the mean, which three or four roundings on is the roundings' own
+    size.  So both are two chains of independent roundings, some 18 of 1.6e-3 in three layers: sqrt(2 * 18) * 1.6e-3 = 1e-2; a share
+    that is left out or added twice is off by tenths.  Rows that end inside a tile, fewer rows than a tile, a contraction with a
+    remainder, no weights of the norm (reference architecture)."""
+    cases = [
+        (288, 768, 6, 3, 1000, 100, 1, ane.ARCH_LLAMA, ane.DTYPE_BF16),
+        (768, 2048, 12, 2, 4096, 256, 1, ane.ARCH_LLAMA, ane.DTYPE_BF16),
+        (200, 544, 5, 3, 504, 67, 3, ane.ARCH_LLAMA, ane.DTYPE_BF16),
+        (128, 512, 2, 3, 2000, 128, 3, ane.ARCH_REFERENCE, ane.DTYPE_BF16),
+        (320, 768, 5, 3, 1000, 300, 1, ane.ARCH_REFERENCE, ane.DTYPE_BF16X3),
+    ]
+    whole, shares = _gradients_in_a_child({"ANE_B200_GEMM_PARTS": "0"}, cases), _gradients_in_a_child({}, cases)
+    assert whole.keys() == shares.keys()
+    for i, case in enumerate(cases):
+        differ = 0
+        for key in [k for k in whole if k.startswith(f"{i} ")]:
+            a, b = whole[key].astype(np.float64), shares[key].astype(np.float64)
+            assert np.isfinite(b).all() and np.linalg.norm(a) > 0
+            off = np.linalg.norm(a - b) / np.linalg.norm(a)
+            differ += off > 0
+            assert off < (2e-5 if case[-1] == ane.DTYPE_BF16X3 else 1e-2), (case, key, off)
+        assert differ > 0, case  # the sums were formed in another order
