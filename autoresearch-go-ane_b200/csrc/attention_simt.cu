@@ -19,21 +19,30 @@ static constexpr int kMaxHdPerLane = 4;  // head_dim <= 128
 // floats, so score operands are read as float4 along the head dimension without bank conflicts, 64 FMAs for eight
 // 16-byte reads; probabilities pass through shared memory transposed, [streamed row][resident row], one float4 per
 // streamed row.  32 resident rows (not 64 or 128) because the fp32 modes run with few sequences: 2 x 12 heads x 256
-// make 192 blocks.  One warp per query with scalar loads and global atomics, which this replaces, took 709 us for
+// make 192 blocks.  The next tile is on its way (cp.async, two buffers) while one is worked on: a block has its SM almost to
+// itself, and waiting for a tile took a third of the time its products do.  us, forward / dQ / dK and dV: 2 x 12 heads of 64, seq 256,
+// 24.8 / 43.7 / 59.4 -> 21.1 / 43.1 / 45.6; 8 x 6 heads of 48 32.1 / 77.1 / 47.4 -> 23.9 / 49.9 / 44.5.  One warp per query with scalar loads and global atomics, which this replaces, took 709 us for
 // the backward of 2 x 12 heads x 256 x 64.
 // ------------------------------------------------------------------------------------------------
 namespace {
 
 constexpr int kRes = 32, kStr = 64, kSimtThreads = 128;
+constexpr int kShortTiles = 4;  // tiles of keys that attention_dq_short_simt_kernel keeps
 constexpr int kPPitch = kRes + 4;  // floats of one streamed row of the probability tile
 
 template <int HDP>
 struct Simt {
   static constexpr int kPitch = HDP + 4;
   static constexpr int kResFloats = kRes * kPitch, kStrFloats = kStr * kPitch, kProbFloats = kStr * kPPitch;
-  static constexpr size_t kFwdSmem = sizeof(float) * (kResFloats + 2 * kStrFloats + kProbFloats);
+  // Buffers of streamed tiles: two where the next tile can be on its way and two or three blocks still fit an SM
+  template <typename T>
+  __host__ __device__ static constexpr int bufs() { return sizeof(T) == 4 && HDP <= 64 ? 2 : 1; }
+  template <typename T>
+  static constexpr size_t fwd_smem() { return sizeof(float) * (kResFloats + 2 * bufs<T>() * kStrFloats + kProbFloats); }
   static constexpr size_t kDqSmem = sizeof(float) * (2 * kResFloats + 2 * kStrFloats + kProbFloats);
-  static constexpr size_t kDkvSmem = sizeof(float) * (2 * kResFloats + 2 * kStrFloats + 2 * kProbFloats + 3 * kStr);
+  static constexpr size_t dq_short_smem() { return sizeof(float) * (2 * kResFloats + (kShortTiles + 2) * kStrFloats + kProbFloats); }
+  template <typename T>
+  static constexpr size_t dkv_smem() { return sizeof(float) * (2 * kResFloats + bufs<T>() * (2 * kStrFloats + 3 * kStr) + 2 * kProbFloats); }
 };
 
 template <typename T>
@@ -63,6 +72,28 @@ __device__ __forceinline__ void load_rows(float* dst, const T* src, int ld, int 
     const int e = threadIdx.x + i * kSimtThreads, r = e / (HDP / 4), c = (e - r * (HDP / 4)) * 4;
     *reinterpret_cast<float4*>(dst + r * Simt<HDP>::kPitch + c) = v[i];
   }
+}
+
+// The same without waiting, for fp32 (others arrive at once): to be waited for with tile_wait().
+template <int HDP, int ROWS, typename T>
+__device__ __forceinline__ void request_rows(float* dst, const T* src, int ld, int valid, int hd) {
+  if constexpr (sizeof(T) != 4) {
+    load_rows<HDP, ROWS>(dst, src, ld, valid, hd);
+  } else {
+#pragma unroll
+    for (int i = 0; i < ROWS * (HDP / 4) / kSimtThreads; ++i) {
+      const int e = threadIdx.x + i * kSimtThreads, r = e / (HDP / 4), c = (e - r * (HDP / 4)) * 4;
+      const bool in = r < valid && c < hd;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + r * Simt<HDP>::kPitch + c)), "l"(in ? src + (size_t)r * ld + c : src), "r"(in ? 16 : 0)
+                   : "memory");
+    }
+  }
+}
+__device__ __forceinline__ void tile_requested() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void tile_wait() {  // all but the LEFT newest, of every thread
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+  __syncthreads();
 }
 
 // s[i][j] = <resident row 4 ty + i, streamed row tx + 16 j>
@@ -164,9 +195,9 @@ attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, f
   pdl_wait();
   extern __shared__ __align__(16) float simt_smem[];
   float* Qs = simt_smem;
-  float* Ks = Qs + Simt<HDP>::kResFloats;
-  float* Vs = Ks + Simt<HDP>::kStrFloats;
-  float* Ps = Vs + Simt<HDP>::kStrFloats;
+  constexpr int kBufs = Simt<HDP>::template bufs<T>();
+  float* Kb = Qs + Simt<HDP>::kResFloats;  // buffers of a tile's keys and values
+  float* Ps = Kb + 2 * kBufs * Simt<HDP>::kStrFloats;
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const int b = blockIdx.x / H, h = blockIdx.x - b * H, kvh = h / (H / KV);
   const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRes;
@@ -174,7 +205,14 @@ attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, f
   const size_t row0 = (size_t)b * seq;
   const T* kb = qkv + row0 * ld + (size_t)(H + kvh) * hd;
   const T* vb = qkv + row0 * ld + (size_t)(H + KV + kvh) * hd;
-  load_rows<HDP, kRes>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
+  auto request = [&](int k0) {
+    float* to = Kb + (k0 / kStr & (kBufs - 1)) * 2 * Simt<HDP>::kStrFloats;
+    request_rows<HDP, kStr>(to, kb + (size_t)k0 * ld, ld, seq - k0, hd);
+    request_rows<HDP, kStr>(to + Simt<HDP>::kStrFloats, vb + (size_t)k0 * ld, ld, seq - k0, hd);
+    tile_requested();
+  };
+  request_rows<HDP, kRes>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
+  if (kBufs == 2) request(0);
   float m[4], l[4], acc[4][HDP / 16];
   zero<HDP>(acc);
 #pragma unroll
@@ -184,10 +222,14 @@ attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, f
   }
   const int last = min(q0 + kRes, seq) - 1;
   for (int k0 = 0; k0 <= last; k0 += kStr) {
-    __syncthreads();
-    load_rows<HDP, kStr>(Ks, kb + (size_t)k0 * ld, ld, seq - k0, hd);
-    load_rows<HDP, kStr>(Vs, vb + (size_t)k0 * ld, ld, seq - k0, hd);
-    __syncthreads();
+    if (kBufs == 1) {
+      __syncthreads();
+      request(k0);
+    }
+    tile_wait<0>();  // (and everybody has left the buffer that is filled next)
+    const float* Ks = Kb + (k0 / kStr & (kBufs - 1)) * 2 * Simt<HDP>::kStrFloats;
+    const float* Vs = Ks + Simt<HDP>::kStrFloats;
+    if (kBufs == 2 && k0 + kStr <= last) request(k0 + kStr);
     float s[4][4];
     scores<HDP>(s, Qs, Ks, ty, tx);
 #pragma unroll
@@ -342,6 +384,117 @@ attention_dq_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_out
   }
 }
 
+// The first kernel for up to kShortTiles tiles of keys in fp32: scores and dP of the first sweep stay in registers and the keys in
+// shared memory, so that the second sweep is one product instead of three.  (One buffer of values and two blocks an SM instead: 1 %
+// slower in a whole update.)
+template <int HDP>
+__global__ void __launch_bounds__(kSimtThreads)
+attention_dq_short_simt_kernel(const float* __restrict__ qkv, const float* __restrict__ d_out, float* __restrict__ dqkv, float* __restrict__ stats, int rows,
+                               int seq, int H, int KV, int hd, float scale) {
+  pdl_trigger();
+  pdl_wait();
+  extern __shared__ __align__(16) float simt_smem[];
+  float* Qs = simt_smem;
+  float* dOs = Qs + Simt<HDP>::kResFloats;
+  float* Kb = dOs + Simt<HDP>::kResFloats;                // all tiles' keys
+  float* Vb = Kb + kShortTiles * Simt<HDP>::kStrFloats;  // two buffers of values
+  float* Ps = Vb + 2 * Simt<HDP>::kStrFloats;
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int b = blockIdx.x / H, h = blockIdx.x - b * H, kvh = h / (H / KV);
+  const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRes;
+  const int ld = (H + 2 * KV) * hd;
+  const size_t row0 = (size_t)b * seq;
+  const float* kb = qkv + row0 * ld + (size_t)(H + kvh) * hd;
+  const float* vb = qkv + row0 * ld + (size_t)(H + KV + kvh) * hd;
+  const int last = min(q0 + kRes, seq) - 1, tiles = last / kStr + 1;
+  auto request = [&](int t) {  // (an empty group past the last tile, so that the groups of all threads count alike)
+    if (t < tiles) {
+      request_rows<HDP, kStr>(Kb + t * Simt<HDP>::kStrFloats, kb + (size_t)t * kStr * ld, ld, seq - t * kStr, hd);
+      request_rows<HDP, kStr>(Vb + (t & 1) * Simt<HDP>::kStrFloats, vb + (size_t)t * kStr * ld, ld, seq - t * kStr, hd);
+    }
+    tile_requested();
+  };
+  request_rows<HDP, kRes>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
+  request_rows<HDP, kRes>(dOs, d_out + (row0 + q0) * (size_t)(H * hd) + (size_t)h * hd, H * hd, seq - q0, hd);
+  request(0);
+  float m[4], l[4], dl[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = dl[i] = 0.f;
+  }
+  float s[kShortTiles][4][4], dp[kShortTiles][4][4];
+#pragma unroll
+  for (int t = 0; t < kShortTiles; ++t) {
+    if (t >= tiles) continue;
+    tile_wait<0>();
+    request(t + 1);
+    scores<HDP>(s[t], Qs, Kb + t * Simt<HDP>::kStrFloats, ty, tx);
+    scores<HDP>(dp[t], dOs, Vb + (t & 1) * Simt<HDP>::kStrFloats, ty, tx);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = q0 + 4 * ty + i;
+      float mx = m[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[t][i][j] = t * kStr + tx + 16 * j <= row ? s[t][i][j] * scale : -INFINITY;
+        mx = fmaxf(mx, s[t][i][j]);
+      }
+      mx = row_max(mx);
+      const float corr = expf(m[i] - mx);
+      m[i] = mx;
+      l[i] *= corr;
+      dl[i] *= corr;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = expf(s[t][i][j] - mx);
+        l[i] += p;
+        dl[i] += p * dp[t][i][j];
+      }
+    }
+  }
+  float acc[4][HDP / 16];
+  zero<HDP>(acc);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    l[i] = 1.0f / row_sum(l[i]);
+    dl[i] = row_sum(dl[i]) * l[i];
+    const int row = q0 + 4 * ty + i;
+    if (tx == 0 && row < seq) {
+      float* st = stats + ((size_t)b * H + h) * seq + row;
+      st[0] = m[i];
+      st[(size_t)rows] = l[i];
+      st[(size_t)2 * rows] = dl[i];
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < kShortTiles; ++t) {
+    if (t >= tiles) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = expf(s[t][i][j] - m[i]) * l[i];
+        s[t][i][j] = p * (dp[t][i][j] - dl[i]) * scale;
+      }
+    if (t > 0) __syncthreads();  // the tile before has been read
+    put_probs(Ps, s[t], ty, tx);
+    __syncthreads();
+    accumulate<HDP>(acc, Ps, Kb + t * Simt<HDP>::kStrFloats, ty, tx);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = q0 + 4 * ty + i;
+    if (row >= seq) continue;
+    float* op = dqkv + (row0 + row) * ld + (size_t)h * hd;
+#pragma unroll
+    for (int c = 0; c < HDP / 16; ++c) {
+      const int d = col_of<HDP>(tx, c);
+      if (d < hd) op[d] = acc[i][c];
+    }
+  }
+}
+
 // Backward, second kernel: dK and dV of 32 keys over the queries of every head that shares them; no atomics.
 template <int HDP, typename T, typename TD>
 __global__ void __launch_bounds__(kSimtThreads)
@@ -352,31 +505,48 @@ attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_ou
   extern __shared__ __align__(16) float simt_smem[];
   float* Ks = simt_smem;
   float* Vs = Ks + Simt<HDP>::kResFloats;
-  float* Qs = Vs + Simt<HDP>::kResFloats;
-  float* dOs = Qs + Simt<HDP>::kStrFloats;
-  float* Ps = dOs + Simt<HDP>::kStrFloats;
+  constexpr int kBufs = Simt<HDP>::template bufs<T>();
+  float* Qb = Vs + Simt<HDP>::kResFloats;  // buffers of a tile's queries and output gradients
+  float* Ps = Qb + 2 * kBufs * Simt<HDP>::kStrFloats;
   float* Ds = Ps + Simt<HDP>::kProbFloats;
-  float* st = Ds + Simt<HDP>::kProbFloats;  // maximum, 1 / sum, delta of the 64 queries
+  float* sb = Ds + Simt<HDP>::kProbFloats;  // and of maximum, 1 / sum, delta of the 64 queries
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const int b = blockIdx.x / KV, kvh = blockIdx.x - b * KV, group = H / KV;
   const int k0 = (int)blockIdx.y * kRes;
   const int ld = (H + 2 * KV) * hd;
   const size_t row0 = (size_t)b * seq;
-  load_rows<HDP, kRes>(Ks, qkv + (row0 + k0) * ld + (size_t)(H + kvh) * hd, ld, seq - k0, hd);
-  load_rows<HDP, kRes>(Vs, qkv + (row0 + k0) * ld + (size_t)(H + KV + kvh) * hd, ld, seq - k0, hd);
+  request_rows<HDP, kRes>(Ks, qkv + (row0 + k0) * ld + (size_t)(H + kvh) * hd, ld, seq - k0, hd);
+  request_rows<HDP, kRes>(Vs, qkv + (row0 + k0) * ld + (size_t)(H + KV + kvh) * hd, ld, seq - k0, hd);
+  auto request = [&](int h, int q0, int buf) {
+    float* to = Qb + buf * 2 * Simt<HDP>::kStrFloats;
+    request_rows<HDP, kStr>(to, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
+    request_rows<HDP, kStr>(to + Simt<HDP>::kStrFloats, d_out + (row0 + q0) * (size_t)(H * hd) + (size_t)h * hd, H * hd, seq - q0, hd);
+    tile_requested();
+    for (int i = threadIdx.x; i < 3 * kStr; i += kSimtThreads) {
+      const int q = q0 + (i & (kStr - 1));
+      sb[buf * 3 * kStr + i] = q < seq ? stats[(size_t)(i / kStr) * rows + ((size_t)b * H + h) * seq + q] : 0.f;
+    }
+  };
+  const int first = k0 / kStr * kStr;
+  int buf = 0;
+  if (kBufs == 2) request(kvh * group, first, 0);
   float dk[4][HDP / 16], dv[4][HDP / 16];
   zero<HDP>(dk);
   zero<HDP>(dv);
   for (int h = kvh * group; h < (kvh + 1) * group; ++h) {
-    for (int q0 = k0 / kStr * kStr; q0 < seq; q0 += kStr) {
-      __syncthreads();
-      load_rows<HDP, kStr>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
-      load_rows<HDP, kStr>(dOs, d_out + (row0 + q0) * (size_t)(H * hd) + (size_t)h * hd, H * hd, seq - q0, hd);
-      for (int i = threadIdx.x; i < 3 * kStr; i += kSimtThreads) {
-        const int q = q0 + (i & (kStr - 1));
-        st[i] = q < seq ? stats[(size_t)(i / kStr) * rows + ((size_t)b * H + h) * seq + q] : 0.f;
+    for (int q0 = first; q0 < seq; q0 += kStr, buf ^= kBufs - 1) {
+      if (kBufs == 1) {
+        __syncthreads();
+        request(h, q0, 0);
       }
-      __syncthreads();
+      tile_wait<0>();
+      const float* Qs = Qb + buf * 2 * Simt<HDP>::kStrFloats;
+      const float* dOs = Qs + Simt<HDP>::kStrFloats;
+      const float* st = sb + buf * 3 * kStr;
+      if (kBufs == 2) {
+        if (q0 + kStr < seq) request(h, q0 + kStr, buf ^ 1);
+        else if (h + 1 < (kvh + 1) * group) request(h + 1, first, buf ^ 1);
+      }
       float s[4][4], dp[4][4];
       scores<HDP>(s, Ks, Qs, ty, tx);
       scores<HDP>(dp, Vs, dOs, ty, tx);
@@ -420,8 +590,8 @@ template <int HDP, typename T, typename TO>
 void forward_hdp(const T* qkv, TO* out, float* lse, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
   auto kern = attention_forward_simt_kernel<HDP, T, TO>;
   static unsigned long long done = 0;
-  smem_opt_in(kern, Simt<HDP>::kFwdSmem, done);
-  launch_pdl(kern, dim3(B * H, (seq + kRes - 1) / kRes), dim3(kSimtThreads), Simt<HDP>::kFwdSmem, s, qkv, out, lse, seq, H, KV, hd, scale);
+  smem_opt_in(kern, Simt<HDP>::template fwd_smem<T>(), done);
+  launch_pdl(kern, dim3(B * H, (seq + kRes - 1) / kRes), dim3(kSimtThreads), Simt<HDP>::template fwd_smem<T>(), s, qkv, out, lse, seq, H, KV, hd, scale);
 }
 template <int HDP, typename T, typename TD>
 void backward_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
@@ -429,10 +599,21 @@ void backward_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int 
   auto dkv = attention_dkv_simt_kernel<HDP, T, TD>;
   static unsigned long long done_q = 0, done_k = 0;
   smem_opt_in(dq, Simt<HDP>::kDqSmem, done_q);
-  smem_opt_in(dkv, Simt<HDP>::kDkvSmem, done_k);
+  smem_opt_in(dkv, Simt<HDP>::template dkv_smem<T>(), done_k);
   const int tiles = (seq + kRes - 1) / kRes, rows = B * H * seq;
+  // up to 256 positions, heads whose keys fit: everything of the first sweep is kept for the second
+  if constexpr (HDP <= 64 && sizeof(T) == 4 && sizeof(TD) == 4) {
+    if (seq <= kShortTiles * kStr) {
+      auto dq_short = attention_dq_short_simt_kernel<HDP>;
+      static unsigned long long done_s = 0;
+      smem_opt_in(dq_short, Simt<HDP>::dq_short_smem(), done_s);
+      launch_pdl(dq_short, dim3(B * H, tiles), dim3(kSimtThreads), Simt<HDP>::dq_short_smem(), s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
+      launch_pdl(dkv, dim3(B * KV, tiles), dim3(kSimtThreads), Simt<HDP>::template dkv_smem<T>(), s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
+      return;
+    }
+  }
   launch_pdl(dq, dim3(B * H, tiles), dim3(kSimtThreads), Simt<HDP>::kDqSmem, s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
-  launch_pdl(dkv, dim3(B * KV, tiles), dim3(kSimtThreads), Simt<HDP>::kDkvSmem, s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
+  launch_pdl(dkv, dim3(B * KV, tiles), dim3(kSimtThreads), Simt<HDP>::template dkv_smem<T>(), s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
 }
 
 }  // namespace

@@ -34,6 +34,13 @@ def test_fp32_tiles(arch, hd, heads, kv, seq):
     e.close()
 
 
+@pytest.mark.parametrize("arch,hd,heads,kv,seq", [
+    (O.ARCH_L, 32, 2, 1, 256), (O.ARCH_L, 40, 2, 2, 193), (O.ARCH_L, 48, 4, 2, 255), (O.ARCH_L, 64, 2, 1, 257), (O.ARCH_N, 64, 2, 2, 256)])
+def test_fp32_tiles_of_several_sweeps(arch, hd, heads, kv, seq):
+    """Up to 256 positions the dQ kernel keeps the scores of all its tiles; from 257 on it forms them twice."""
+    test_fp32_tiles(arch, hd, heads, kv, seq)
+
+
 @pytest.mark.parametrize("hd,heads,kv,seq,batch", [(32, 2, 1, 63, 2), (48, 2, 2, 65, 2), (48, 4, 2, 200, 2), (48, 2, 2, 257, 50),
                                                    (64, 2, 1, 100, 2), (64, 4, 4, 129, 40)])
 def test_bf16_tiles(hd, heads, kv, seq, batch):
