@@ -665,8 +665,9 @@ adam_kernel(float* __restrict__ w, float* __restrict__ g, float* __restrict__ m,
 void adam_update(float* w, float* g, float* m, float* v, bf16* shadow, uint64_t n, AdamHyper h, const float* gscale,
                  cudaStream_t s) {
   if (!n) return;
+  // One float4 a thread: the blocks go over memory in order.  110 M parameters took 602 us in 148 * 8 blocks that strode over
+  // all of it (two thirds of them resident, each at its own pace) and 541 like this, 6.9 TB/s; 2 float4 a thread: 565.
   uint64_t grid = ((n >> 2) + 255) / 256;
-  if (grid > 148ull * 8) grid = 148ull * 8;
   if (grid < 1) grid = 1;
   auto al = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
   const int vec_ok = al(w, 16) && al(g, 16) && al(m, 16) && al(v, 16) && (!shadow || al(shadow, 8));
