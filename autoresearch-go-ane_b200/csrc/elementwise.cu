@@ -861,7 +861,8 @@ __global__ void ve_backward_kernel(const T* __restrict__ dqkv, const float* __re
                                    const uint16_t* __restrict__ tok, const float* __restrict__ ve_embed,
                                    const float* __restrict__ ve_gate, const float* __restrict__ gate_act,
                                    float* __restrict__ g_ve_embed, float* __restrict__ g_ve_gate,
-                                   float* __restrict__ d_prev, int M, int D, int H, int KV, int hd, int vocab) {
+                                   float* __restrict__ d_prev, unsigned* __restrict__ rows_at, unsigned epoch, int M,
+                                   int D, int H, int KV, int hd, int vocab) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ float s_gate[];  // [H][kVEGateChannels]
@@ -874,6 +875,7 @@ __global__ void ve_backward_kernel(const T* __restrict__ dqkv, const float* __re
     const int m = (int)(wid / H), h = (int)(wid - (long long)m * H);
     const int t = tok[m];
     if (t >= vocab) continue;
+    if (rows_at && h == 0 && lane == 0) rows_at[t] = epoch;
     const float act = gate_act[(size_t)m * H + h];
     const float gate = 3.0f * act;
     const int ld = (H + 2 * KV) * hd;
@@ -899,19 +901,19 @@ __global__ void ve_backward_kernel(const T* __restrict__ dqkv, const float* __re
 }
 template <typename T>
 void ve_backward(const T* dqkv, const float* x, const uint16_t* tok, const float* ve_embed, const float* ve_gate,
-                 const float* gate_act, float* g_ve_embed, float* g_ve_gate, float* d_prev, int M, int D, int H,
-                 int KV, int hd, int vocab, cudaStream_t s) {
+                 const float* gate_act, float* g_ve_embed, float* g_ve_gate, float* d_prev, unsigned* rows_at,
+                 unsigned epoch, int M, int D, int H, int KV, int hd, int vocab, cudaStream_t s) {
   const long long warps = (long long)M * H;
   if (warps <= 0) return;
   long long blocks = (warps + 7) / 8;
   if (blocks > 148 * 4) blocks = 148 * 4;
   launch_pdl(ve_backward_kernel<T>, dim3((unsigned)blocks), dim3(256), sizeof(float) * H * kVEGateChannels, s, 
-      dqkv, x, tok, ve_embed, ve_gate, gate_act, g_ve_embed, g_ve_gate, d_prev, M, D, H, KV, hd, vocab);
+      dqkv, x, tok, ve_embed, ve_gate, gate_act, g_ve_embed, g_ve_gate, d_prev, rows_at, epoch, M, D, H, KV, hd, vocab);
 }
 template void ve_backward<float>(const float*, const float*, const uint16_t*, const float*, const float*,
-                                 const float*, float*, float*, float*, int, int, int, int, int, int, cudaStream_t);
+                                 const float*, float*, float*, float*, unsigned*, unsigned, int, int, int, int, int, int, cudaStream_t);
 template void ve_backward<bf16>(const bf16*, const float*, const uint16_t*, const float*, const float*, const float*,
-                                float*, float*, float*, int, int, int, int, int, int, cudaStream_t);
+                                float*, float*, float*, unsigned*, unsigned, int, int, int, int, int, int, cudaStream_t);
 
 // ------------------------------------------------------------------------------------------
 // Transpose and argmax

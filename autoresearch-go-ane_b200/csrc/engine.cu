@@ -546,6 +546,14 @@ class EngineT final : public EngineBase {
   int reduce_bucket(int b);
   int gather_moments();
   bool overlap_reduce_ = false;           // this micro-step is the last before the optimizer update
+  // The tables of value embeddings lie one after another, without gaps, in [r_ve0_, r_ve1_).  Their rows have a gradient only where
+  // the tokens of the pending micro-steps named them: ve_rows_[row] == ve_epoch_ then.  Sums over ranks and gradients set from
+  // outside have any row.
+  unsigned* ve_rows_ = nullptr;
+  unsigned ve_epoch_ = 1;
+  bool ve_any_row_ = false;
+  unsigned* ve_rows_of(int l) const { return ve_rows_ + (s_ve_embed_[l].off - r_ve0_) / D_; }
+  bool ve_by_row() const { return ve_rows_ && !dp_.active() && !ve_any_row_; }
   size_t reduced_lo_ = 0;                 // G_[reduced_lo_, r_mat1_) has already been handed to the all-reduce
   std::vector<void*> allocs_;
   bool profiling_ = false;
@@ -723,6 +731,7 @@ int EngineT<T>::alloc_buffers() {
   } while (0)
   A(P_, n_params_); A(G_, n_params_); A(Mo_, n_params_); A(Vo_, n_params_);
   if (!kIsF32) A(Sh_, shadow_n_);
+  if (r_ve1_ > r_ve0_ && D_ % 4 == 0 && (size_t)V_ * D_ % 128 == 0) A(ve_rows_, (r_ve1_ - r_ve0_) / D_);
   A(d_one_, 1); A(d_zero_, 1);
   xs_.assign(L_ + 1, nullptr);
   for (int l = 0; l <= L_; ++l) A(xs_[l], MD);
@@ -897,6 +906,7 @@ int EngineT<T>::open(const ane_options& opts, const uint16_t* tokens, uint64_t n
   if ((rc = cuda_check(cudaMallocHost(&h_logits_, sizeof(float) * (size_t)V_ * S_), "cudaMallocHost")) != 0) return rc;
   for (float* p : {P_, G_, Mo_, Vo_})
     if ((rc = cuda_check(cudaMemsetAsync(p, 0, sizeof(float) * n_params_, stream_), "memset")) != 0) return rc;
+  if (ve_rows_) cudaMemsetAsync(ve_rows_, 0, sizeof(unsigned) * ((r_ve1_ - r_ve0_) / D_), stream_);
   cudaMemsetAsync(d_status_, 0, sizeof(int), stream_);
   const float one = 1.f, zero = 0.f;
   cudaMemcpyAsync(d_one_, &one, sizeof(float), cudaMemcpyHostToDevice, stream_);
@@ -1497,7 +1507,8 @@ int EngineT<T>::backward_layers(int B) {
     if (is_ve_layer(l)) {
       count_launch();
       ve_backward<float>(dqkv_f32, xs_[l], d_in_, P_ + s_ve_embed_[l].off, P_ + s_ve_gate_[l].off, a.ve_act,
-                         G_ + s_ve_embed_[l].off, G_ + s_ve_gate_[l].off, dprev, M, D_, H_, KV_, hd_, V_, stream_);
+                         G_ + s_ve_embed_[l].off, G_ + s_ve_gate_[l].off, dprev,
+                         ve_rows_ ? ve_rows_of(l) : nullptr, ve_epoch_, M, D_, H_, KV_, hd_, V_, stream_);
     }
     {
       GemmDesc& g = dw[2];  // dWo += dx2^T * att
@@ -1663,8 +1674,15 @@ int EngineT<T>::do_flush() {
       count_launch();
       sumsq_accumulate(G_ + r_mat0_, r_mat1_ - r_mat0_, pre_scale, d_acc_, stream_);
     }
-    count_launch();
-    sumsq_accumulate(G_ + s_embed_.off, r_veg1_ - s_embed_.off, pre_scale, d_acc_, stream_);
+    if (ve_by_row()) {
+      count_launch(3);
+      sumsq_accumulate(G_ + s_embed_.off, r_ve0_ - s_embed_.off, pre_scale, d_acc_, stream_);
+      sumsq_rows_accumulate(G_ + r_ve0_, (int)((r_ve1_ - r_ve0_) / D_), D_, ve_rows_, ve_epoch_, pre_scale, d_acc_, stream_);
+      sumsq_accumulate(G_ + r_veg0_, r_veg1_ - r_veg0_, pre_scale, d_acc_, stream_);
+    } else {
+      count_launch();
+      sumsq_accumulate(G_ + s_embed_.off, r_veg1_ - s_embed_.off, pre_scale, d_acc_, stream_);
+    }
     if (!isN_) {
       count_launch();
       sumsq_accumulate(G_ + r_rms0_, r_rms1_ - r_rms0_, pre_scale, d_acc_, stream_);
@@ -1699,7 +1717,15 @@ int EngineT<T>::do_flush() {
   }
   if (isN_) run(s_smear_gate_.off, s_embed_.off - s_smear_gate_.off, hyper(lr_, b1, b2, o_.weight_decay), pre_s, true);
   run(s_embed_.off, r_ve0_ - s_embed_.off, hyper(embed_lr_, b1, b2, 0.f), clip_s, true);
-  run(r_ve0_, r_ve1_ - r_ve0_, hyper(embed_lr_, b1, b2, 0.f), clip_s, false);
+  if (ve_by_row()) {
+    count_launch();
+    adam_update_rows(P_ + r_ve0_, G_ + r_ve0_, Mo_ + r_ve0_, Vo_ + r_ve0_, (int)((r_ve1_ - r_ve0_) / D_), D_, ve_rows_, ve_epoch_,
+                     hyper(embed_lr_, b1, b2, 0.f), clip_s, stream_);
+  } else {
+    run(r_ve0_, r_ve1_ - r_ve0_, hyper(embed_lr_, b1, b2, 0.f), clip_s, false);
+  }
+  ve_epoch_++;
+  ve_any_row_ = false;
   run(r_veg0_, r_veg1_ - r_veg0_, hyper(scalar_lr_, b1, b2, 0.f), clip_s, false);
   run(r_rms0_, r_rms1_ - r_rms0_, hyper(lr_, b1, b2, 0.f), clip_s, false);
   if (isN_) {
@@ -2166,6 +2192,7 @@ int EngineT<T>::import_tensor(uint32_t id, uint32_t layer, uint32_t which, const
   float* base = which == 0 ? P_ : which == 1 ? G_ : which == 2 ? Mo_ : Vo_;
   int rc;
   wait_all_buckets();
+  if (which == 1) ve_any_row_ = true;
   if (!isN_ && (id == ANE_T_W1 || id == ANE_T_W3)) {
     // W1 and W3 share the fused W13 matrix in blocks of 32 rows: [W1 rows 0..31 | W3 rows 0..31 | W1 rows 32..63 | ...]
     const size_t blk = (size_t)32 * D_ * sizeof(float);

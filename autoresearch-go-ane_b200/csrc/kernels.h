@@ -197,6 +197,9 @@ void reduce_loss(const float* loss_rows, const float* inv_valid, float* loss_out
 // Gradient norm and optimizer -------------------------------------------------------------------
 // acc[0] += sum (g*pre_scale)^2 in double (ane/train_full.go:167-196, ane/accel_stub.go:88-95).
 void sumsq_accumulate(const float* g, uint64_t n, float pre_scale, double* acc, cudaStream_t s);
+// The same of a [rows, D] table whose gradient is zero outside the rows with rows_at[row] == epoch: only those are read.  D % 4 == 0.
+void sumsq_rows_accumulate(const float* g, int rows, int D, const unsigned* rows_at, unsigned epoch, float pre_scale,
+                           double* acc, cudaStream_t s);
 // scales[0] = pre_scale; scales[1] = pre_scale * (clip>0 && norm>clip ? clip/norm : 1)
 void finalize_clip(const double* acc, float pre_scale, float clip, float* scales, float* norm_out, cudaStream_t s);
 struct AdamHyper {
@@ -205,6 +208,9 @@ struct AdamHyper {
 // ane/train_full.go:1113-1150.  g_eff = g * (*gscale);  writes w, m, v, optional bf16 shadow, zeroes g.
 void adam_update(float* w, float* g, float* m, float* v, bf16* shadow, uint64_t n, AdamHyper h, const float* gscale,
                  cudaStream_t s);
+// The same of such a table, every row of it updated: the zeros of the other rows are neither read nor written.
+void adam_update_rows(float* w, float* g, float* m, float* v, int rows, int D, const unsigned* rows_at, unsigned epoch,
+                      AdamHyper h, const float* gscale, cudaStream_t s);
 
 // Reference-architecture extras ---------------------------------------------------------------------
 // Smear: x[m,:] = x_pre[m,:] + lambda * sigmoid(gate_pre[m,:]) * x_pre[m-1,:] (0 at t=0), ane/common.go:324-339.
@@ -228,8 +234,8 @@ void ve_forward(T* qkv, const float* x, const uint16_t* tok, const float* ve_emb
                 float* gate_act, int M, int D, int H, int KV, int hd, int vocab, cudaStream_t s);
 template <typename T>
 void ve_backward(const T* dqkv, const float* x, const uint16_t* tok, const float* ve_embed, const float* ve_gate,
-                 const float* gate_act, float* g_ve_embed, float* g_ve_gate, float* d_prev, int M, int D, int H,
-                 int KV, int hd, int vocab, cudaStream_t s);
+                 const float* gate_act, float* g_ve_embed, float* g_ve_gate, float* d_prev, unsigned* rows_at,
+                 unsigned epoch, int M, int D, int H, int KV, int hd, int vocab, cudaStream_t s);
 
 // [rows, cols] fp32 -> [cols, rows] fp32 (tap export in the reference's channel-first layout).
 void transpose_f32(const float* in, float* out, int rows, int cols, cudaStream_t s);

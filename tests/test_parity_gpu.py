@@ -577,6 +577,49 @@ def test_split_precision_head_with_a_token_outside_the_vocabulary_reference_arch
     e.close()
 
 
+@pytest.mark.parametrize("dim,vocab", [(64, 256), (192, 304), (320, 1016)])
+def test_update_of_value_embeddings_by_row(dim, vocab):
+    """Rows of the value embeddings that no token named are updated without a look at their gradient.  Against an engine
+    whose gradients are set from outside, which reads every row: one sum of squares differs in its order, so the clip scale by
+    2^-23 or two, m by as much, v by twice that, w by the step lr * that.  Then a gradient set in a row that no token named."""
+    cfg = dict(dim=dim, hidden=96, heads=4, layers=3, vocab=vocab, seq=8)
+    pair = [make_pair(ane, cfg, arch=O.ARCH_N, quirks=0, dtype=ane.DTYPE_F32, batch=2, hyper=dict(lr=1e-2, accum_steps=1000, grad_clip=0.1))[1]
+            for _ in range(2)]
+    names = [(t, l) for t, n in O.TENSOR_NAMES.items() for l in range(cfg["layers"]) if pair[0].tensor_size(t, l) > 0]
+    ve = [(t, l) for t, l in names if O.TENSOR_NAMES[t] == "ve_embed"]
+    assert len(ve) == 2
+    rng = np.random.default_rng(3)
+    for named in ([0, vocab - 1, 5, 5], [vocab - 1, 17], [1]):
+        for _ in range(2):
+            inp = rng.choice(named, (2, 8)).astype(np.uint16)
+            tgt = rng.integers(0, vocab, (2, 8)).astype(np.uint16)
+            for e in pair:
+                e.step_tokens(inp, tgt)
+        for t, l in names:
+            pair[1].import_tensor(t, l, pair[0].export_tensor(t, l, O.G), O.G)
+        g = pair[0].export_tensor(*ve[0], O.G).reshape(vocab, dim)
+        assert set(np.flatnonzero(np.abs(g).sum(1))) <= set(named) and np.any(g)
+        for e in pair:
+            e.flush()
+        for t, l in names:
+            a, b = ([e.export_tensor(t, l, w) for w in (O.W, O.G, O.M, O.V)] for e in pair)
+            assert not a[1].any() and not b[1].any()
+            np.testing.assert_allclose(a[2], b[2], rtol=2e-6, atol=1e-12)
+            np.testing.assert_allclose(a[3], b[3], rtol=4e-6, atol=1e-20)
+            np.testing.assert_allclose(a[0], b[0], rtol=1e-6, atol=1e-2 * 1e-5)
+    e, (t, l) = pair[0], ve[1]
+    e.step_tokens(np.full((2, 8), 9, np.uint16), tgt)
+    g = e.export_tensor(t, l, O.G).reshape(vocab, dim)
+    g[vocab - 2] = 1e-3
+    before = e.export_tensor(t, l, O.M).reshape(vocab, dim)[vocab - 2]
+    e.import_tensor(t, l, g, O.G)
+    e.flush()
+    after = e.export_tensor(t, l, O.M).reshape(vocab, dim)[vocab - 2]
+    assert not before.any() and after.all() and not e.export_tensor(t, l, O.G).any()
+    for e in pair:
+        e.close()
+
+
 def test_eval_logits_layout_and_eval_loss():
     cfg = dict(MID)
     m, e = make_pair(ane, cfg, arch=O.ARCH_N, quirks=1, dtype=ane.DTYPE_BF16, batch=2, debug_taps=False)
