@@ -337,6 +337,7 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
     g_gemm_err = "pair tiles and 32-column tiles are built for the non-accumulating epilogues";
     return -2;
   } else {
+    if (d.first) return launch_tc<BN, MT, A_MN, B_MN, EPI_STORE_F32>(ta, tb, tc, tc, epi, d, whole, d_status, stream);
     return launch_tc<BN, MT, A_MN, B_MN, EPI_REDUCE_F32>(ta, tb, tc, tc, epi, d, split_k, d_status, stream);
   }
 }
@@ -575,8 +576,15 @@ static int plan_parts(const GemmDesc& d, int& best_bn) {
   }
   return best;
 }
+bool gemm_whole_tiles(const GemmDesc& d) {
+  return d.out == GEMM_OUT_ACCUM && (narrow_width(d) != 0 || plan_gemm(d, gemm_num_sms()).sched == 1);
+}
 int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream) {
   if (d.n_parts) *d.n_parts = 1;
+  if (d.first && !gemm_whole_tiles(d)) {
+    g_gemm_err = "a product in shares of the contraction adds to C and cannot overwrite it";
+    return -2;
+  }
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return 0;
   if (d.out == GEMM_OUT_F32 && (d.res1 || d.res2) && (d.ldres % 4 != 0 ||
       (reinterpret_cast<uintptr_t>(d.res1) & 15) != 0 || (reinterpret_cast<uintptr_t>(d.res2) & 15) != 0)) {

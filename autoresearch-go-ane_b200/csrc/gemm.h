@@ -80,6 +80,7 @@ struct GemmDesc {
   int ce_rows = 0, ce_col0 = 0;
   bool ce_softcap = false;
   int split_k = 0;  // 0 => choose
+  bool first = false;  // GEMM_OUT_ACCUM: C counts as zero, whatever it holds; where gemm_whole_tiles
   // GEMM_OUT_F32 without residuals, into a consumer that can add: room for `parts` sums of a share of the contraction each, dense
   // [part][parts_rows(M)][N], where few tiles would leave most SMs idle.  *n_parts = how many there are; 1: the product is in C.
   float* parts = nullptr;
@@ -93,6 +94,8 @@ constexpr int kMostParts = 8;
 inline int parts_rows(int M) { return (M + 127) / 128 * 128; }
 // bf16 operands, tcgen05 tensor cores.  Returns 0 or a negative error code.
 int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream);
+// An accumulated product of which gemm_bf16 hands each tile to one CTA as a whole: it can overwrite C instead of adding to it.
+bool gemm_whole_tiles(const GemmDesc& d);
 // fp32 operands at split precision on the tensor cores: A and B are each cut into a bf16 (hi, lo) pair
 // (hi = bf16(x), lo = bf16(x - hi): together ~16 significand bits) and the product is formed as Ah*Bh + Ah*Bl + Al*Bh
 // with fp32 accumulation, one GEMM over a contraction of three passes (the dropped Al*Bl term is ~2^-18 relative).

@@ -206,8 +206,9 @@ struct AdamHyper {
   float lr, b1, b2, eps, wd, inv_bc1, inv_bc2;
 };
 // ane/train_full.go:1113-1150.  g_eff = g * (*gscale);  writes w, m, v, optional bf16 shadow, zeroes g.
+// clear: g is zero afterwards, else it stays.
 void adam_update(float* w, float* g, float* m, float* v, bf16* shadow, uint64_t n, AdamHyper h, const float* gscale,
-                 cudaStream_t s);
+                 bool clear, cudaStream_t s);
 // The same of such a table, every row of it updated: the zeros of the other rows are neither read nor written.
 void adam_update_rows(float* w, float* g, float* m, float* v, int rows, int D, const unsigned* rows_at, unsigned epoch,
                       AdamHyper h, const float* gscale, cudaStream_t s);

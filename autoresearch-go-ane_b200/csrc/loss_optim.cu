@@ -656,7 +656,8 @@ __device__ __forceinline__ void adam_one(float& w, float g, float& m, float& v, 
 
 __global__ void __launch_bounds__(256)
 adam_kernel(float* __restrict__ w, float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-            bf16* __restrict__ shadow, uint64_t n, AdamHyper h, const float* __restrict__ gscale, int vec_ok) {
+            bf16* __restrict__ shadow, uint64_t n, AdamHyper h, const float* __restrict__ gscale, int vec_ok,
+            int clear) {
   pdl_trigger();
   pdl_wait();
   const float gs = gscale ? *gscale : 1.f;
@@ -676,7 +677,7 @@ adam_kernel(float* __restrict__ w, float* __restrict__ g, float* __restrict__ m,
     w4[k] = ww;
     m4[k] = mm;
     v4[k] = vv;
-    g4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (clear) g4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (shadow) {
       __nv_bfloat162 lo = __floats2bfloat162_rn(ww.x, ww.y), hi = __floats2bfloat162_rn(ww.z, ww.w);
       uint2 u;
@@ -691,7 +692,7 @@ adam_kernel(float* __restrict__ w, float* __restrict__ g, float* __restrict__ m,
     w[k] = ww;
     m[k] = mm;
     v[k] = vv;
-    g[k] = 0.f;
+    if (clear) g[k] = 0.f;
     if (shadow) shadow[k] = __float2bfloat16_rn(ww);
   }
 }
@@ -746,7 +747,7 @@ void adam_update_rows(float* w, float* g, float* m, float* v, int rows, int D, c
 }
 
 void adam_update(float* w, float* g, float* m, float* v, bf16* shadow, uint64_t n, AdamHyper h, const float* gscale,
-                 cudaStream_t s) {
+                 bool clear, cudaStream_t s) {
   if (!n) return;
   // One float4 a thread: the blocks go over memory in order.  110 M parameters took 602 us in 148 * 8 blocks that strode over
   // all of it (two thirds of them resident, each at its own pace) and 541 like this, 6.9 TB/s; 2 float4 a thread: 565.
@@ -754,7 +755,7 @@ void adam_update(float* w, float* g, float* m, float* v, bf16* shadow, uint64_t 
   if (grid < 1) grid = 1;
   auto al = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
   const int vec_ok = al(w, 16) && al(g, 16) && al(m, 16) && al(v, 16) && (!shadow || al(shadow, 8));
-  launch_pdl(adam_kernel, dim3((unsigned)grid), dim3(256), 0, s, w, g, m, v, shadow, n, h, gscale, vec_ok);
+  launch_pdl(adam_kernel, dim3((unsigned)grid), dim3(256), 0, s, w, g, m, v, shadow, n, h, gscale, vec_ok, clear ? 1 : 0);
 }
 
 }  // namespace ane

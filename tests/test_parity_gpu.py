@@ -620,6 +620,44 @@ def test_update_of_value_embeddings_by_row(dim, vocab):
         e.close()
 
 
+@pytest.mark.parametrize("dim,hidden,batch,seq", [(64, 96, 1, 8), (256, 512, 4, 64), (192, 320, 3, 149), (256, 512, 8, 128)])
+def test_gradients_that_the_next_pass_overwrites(dim, hidden, batch, seq):
+    """Few tokens: an update leaves the gradients and the next pass's products overwrite them.  Against an engine whose gradients
+    are read before every micro-step, which makes them zeros to add to: the same sums but for the order of the atomic ones (norm
+    weights and embedding, up to 1024 terms: 2^-24 * 32 relative at random signs)."""
+    cfg = dict(dim=dim, hidden=hidden, heads=4, layers=2, vocab=512, seq=seq)
+    a, b = (make_pair(ane, cfg, arch=O.ARCH_L, quirks=0, dtype=ane.DTYPE_BF16, batch=batch, hyper=dict(lr=1e-2, accum_steps=1000))[1]
+            for _ in range(2))
+    names = [(t, l) for t, n in O.TENSOR_NAMES.items() for l in range(1 if n in ("embed", "rms_final") else 2) if a.tensor_size(t, l) > 0]
+    for micro_steps in (1, 2, 1):
+        for k in range(micro_steps):
+            inp, tgt = batch_tokens(cfg, batch, 31 + k, invalid=False)
+            b.export_tensor(*names[0], O.G)
+            a.step_tokens(inp, tgt)
+            b.step_tokens(inp, tgt)
+        for t, l in names:
+            assert rel_l2(a.export_tensor(t, l, O.G), b.export_tensor(t, l, O.G)) < 2e-6, (O.TENSOR_NAMES[t], l)
+        a.flush()
+        b.flush()
+        for t, l in names:
+            for w in (O.W, O.M, O.V):
+                b.import_tensor(t, l, a.export_tensor(t, l, w), w)
+    assert not any(a.export_tensor(t, l, O.G).any() for t, l in names)
+    a.step_tokens(inp, tgt)
+    a.flush()
+    t, l = O.T_WQ, 1
+    g = np.full(a.tensor_size(t, l), 0.5, np.float32)  # set from outside where old values lie: one tensor, the others are zero
+    a.import_tensor(t, l, g, O.G)
+    assert all(np.array_equal(a.export_tensor(*n, O.G), g) if n == (t, l) else not a.export_tensor(*n, O.G).any() for n in names)
+    a.step_tokens(inp, tgt)
+    for n in names:
+        b.import_tensor(*n, a.export_tensor(*n, O.W))
+    b.step_tokens(inp, tgt)
+    assert rel_l2(a.export_tensor(t, l, O.G), b.export_tensor(t, l, O.G) + g) < 2e-6
+    a.close()
+    b.close()
+
+
 def test_eval_logits_layout_and_eval_loss():
     cfg = dict(MID)
     m, e = make_pair(ane, cfg, arch=O.ARCH_N, quirks=1, dtype=ane.DTYPE_BF16, batch=2, debug_taps=False)
