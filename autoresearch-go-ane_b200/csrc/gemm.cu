@@ -225,7 +225,7 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
                         int* d_status, cudaStream_t stream) {
   EpiParams epi{d.alpha, d.res1, d.s1, d.res2, d.s2, d.ldres, reinterpret_cast<bf16*>(d.aux), d.ldaux,
                 d.rope_cos, d.rope_sin, d.rope_seq, d.rope_pos0, d.rope_cols, d.tgt, d.tgt_out, d.tgt_row0,
-                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, d.part_rows, d.seg_kb};
+                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, d.part_rows, d.seg_kb, d.lda / 2, d.ldb / 2};
   constexpr int whole = 1;  // schedule of the epilogues that need whole tiles
   constexpr bool NARROW = GemmCfg<BN, MT>::NARROW;
   CUtensorMap tc;
@@ -346,13 +346,15 @@ template <int BN, int MT>
 static int dispatch_layout(const GemmDesc& d, int split_k, int* d_status, cudaStream_t stream) {
   CUtensorMap ta, tb;
   bool ok;
-  const int k_extent = d.seg_kb > 0 ? 2 * d.seg_kb * GEMM_BK : d.K;  // (hi | lo) operands: both halves
+  // (hi | lo) operands: both halves of a row, and as many rows as there are
+  const bool seg = d.seg_kb > 0;
+  const int k_extent = seg ? 2 * d.seg_kb * GEMM_BK : d.K;
   if (!d.a_mn) ok = make_tmap(&ta, d.A, k_extent, d.M, d.lda, GEMM_BK, GEMM_BM);
-  else         ok = make_tmap(&ta, d.A, d.M, k_extent, d.lda, 64, GEMM_BK);
+  else         ok = make_tmap(&ta, d.A, seg ? d.lda : d.M, seg ? d.seg_k : d.K, d.lda, 64, GEMM_BK);
   if (!ok) return -2;
   // K-major B: one box per CTA and stage (a CTA of a pair loads half of the tile's rows)
   if (!d.b_mn) ok = make_tmap(&tb, d.B, k_extent, d.N, d.ldb, GEMM_BK, GemmCfg<BN, MT>::PAIR ? BN / 2 : BN);
-  else         ok = make_tmap(&tb, d.B, d.N, k_extent, d.ldb, 64, GEMM_BK);
+  else         ok = make_tmap(&tb, d.B, seg ? d.ldb : d.N, seg ? d.seg_k : d.K, d.ldb, 64, GEMM_BK);
   if (!ok) return -2;
   if constexpr (BN == 32) {
     if (!d.a_mn && !d.b_mn) return dispatch_epi<BN, MT, false, false>(ta, tb, d, split_k, d_status, stream);
@@ -787,9 +789,10 @@ size_t gemm_group_slot_bytes() { return sizeof(GemmGroup); }
 // Split-precision GEMM: fp32 operands as bf16 (hi, lo) pairs, three tensor-core products.
 // ------------------------------------------------------------------------------------------
 // Both operands of a product in one launch (blockIdx.y), four values per thread and step.  Operand [rows, cols] fp32
-// with row pitch ld; its parts (hi, lo or hi, mid, lo) lie behind one another along the contraction: for a K-major operand (k = cols)
-// [rows][hi (kp) | lo (kp)], for an MN-major one (k = rows) [hi (kp rows) | lo (kp rows)][cols rounded up to 8].  kp =
-// k rounded up to a whole k-block; what lies past k is zero.  Three parts are exactly F32TC_SCALE times the fp32 value; where that is not
+// with row pitch ld.  Two parts (hi, lo) lie beside one another in each row, [rows][hi (kp) | lo (kp)], kp = cols rounded up to 64,
+// whichever way a product contracts: what has been cut for one serves the others.  Three (hi, mid, lo) lie behind one another along
+// the contraction: for a K-major operand (k = cols) [rows][hi (kp) | mid | lo], for an MN-major one (k = rows) [hi (kp rows) | mid |
+// lo][cols rounded up to 8], kp = k rounded up to a whole k-block.  What lies past cols, or k, is zero.  Three parts are exactly F32TC_SCALE times the fp32 value; where that is not
 // finite, or its first part is not, the others are not either.
 struct SplitOperand {
   const float* src;
@@ -855,6 +858,26 @@ bool SplitScratch::reserve(const size_t (&bytes)[2]) {
   }
   return true;
 }
+static constexpr int kNoScratch = -3;
+int SplitScratch::grow(int i, size_t need, cudaStream_t stream) {
+  if (cap[i] >= need) return 0;
+  ++generation;
+  // the previous, smaller buffer may still be read by GEMMs in flight on this stream
+  if (buf[i]) {
+    cudaStreamSynchronize(stream);
+    cudaFree(buf[i]);
+    buf[i] = nullptr;
+    cap[i] = 0;
+  }
+  const size_t bytes = need + need / 4 + 256;
+  if (cudaMalloc(&buf[i], bytes) != cudaSuccess) {
+    cudaGetLastError();
+    g_gemm_err = "split-precision GEMM: out of memory for the operands' parts";
+    return kNoScratch;
+  }
+  cap[i] = bytes;
+  return 0;
+}
 void SplitScratch::release() {
   if (buf[0] || buf[1]) ++generation;
   for (int i = 0; i < 2; ++i) {
@@ -864,16 +887,16 @@ void SplitScratch::release() {
   }
 }
 
-static constexpr int kNoScratch = -3;
-// Bytes of operand `i` of `d` in `parts` bf16 parts, and their pitch.
-static size_t parts_bytes(const GemmDesc& d, int parts, int i, int* pitch) {
+// Bytes of operand `i` of `d` in three bf16 parts, and their pitch.
+static size_t parts_bytes(const GemmDesc& d, int i, int* pitch) {
+  constexpr int parts = 3;
   const bool mn = i == 0 ? d.a_mn : d.b_mn;
   const int outer = i == 0 ? d.M : d.N, kp = (d.K + GEMM_BK - 1) / GEMM_BK * GEMM_BK;
   *pitch = mn ? (outer + 7) / 8 * 8 : parts * kp;
   return sizeof(bf16) * (size_t)(mn ? parts * kp : outer) * *pitch;
 }
-// The operands of `d` in `parts` bf16 parts each, in the scratch.
-static int split_operands(const GemmDesc& d, int parts, SplitScratch* sc, SplitOperand (&o)[2], cudaStream_t stream) {
+// The operands of `d` in three bf16 parts each, in the scratch.
+static int split_operands(const GemmDesc& d, SplitScratch* sc, SplitOperand (&o)[2], cudaStream_t stream) {
   const int kp = (d.K + GEMM_BK - 1) / GEMM_BK * GEMM_BK;
   size_t used = 0;  // of an arena
   for (int i = 0; i < 2; ++i) {
@@ -885,7 +908,7 @@ static int split_operands(const GemmDesc& d, int parts, SplitScratch* sc, SplitO
     o[i].cols = mn ? outer : d.K;
     o[i].kp = kp;
     o[i].k_major = mn ? 0 : 1;
-    const size_t need = parts_bytes(d, parts, i, &o[i].pitch);
+    const size_t need = parts_bytes(d, i, &o[i].pitch);
     o[i].vec = o[i].ld % 4 == 0 && (reinterpret_cast<uintptr_t>(o[i].src) & 15) == 0;
     if (sc->arena != nullptr) {
       o[i].dst = reinterpret_cast<bf16*>(static_cast<char*>(sc->arena) + used);
@@ -896,31 +919,13 @@ static int split_operands(const GemmDesc& d, int parts, SplitScratch* sc, SplitO
       }
       continue;
     }
-    if (sc->cap[i] < need && parts == 3) return kNoScratch;
-    if (sc->cap[i] < need) {
-      ++sc->generation;
-      // the previous, smaller buffer may still be read by GEMMs in flight on this stream
-      if (sc->buf[i]) {
-        cudaStreamSynchronize(stream);
-        cudaFree(sc->buf[i]);
-        sc->buf[i] = nullptr;
-        sc->cap[i] = 0;
-      }
-      const size_t bytes = need + need / 4 + 256;
-      if (cudaMalloc(&sc->buf[i], bytes) != cudaSuccess) {
-        cudaGetLastError();
-        g_gemm_err = "split-precision GEMM: out of memory for the operands' parts";
-        return kNoScratch;
-      }
-      sc->cap[i] = bytes;
-    }
+    if (sc->cap[i] < need) return kNoScratch;
     o[i].dst = reinterpret_cast<bf16*>(sc->buf[i]);
   }
   const long long most = std::max((long long)(o[0].k_major ? o[0].rows : kp) * (o[0].k_major ? kp : o[0].pitch),
                                   (long long)(o[1].k_major ? o[1].rows : kp) * (o[1].k_major ? kp : o[1].pitch));
   const unsigned blocks = (unsigned)std::min<long long>(148 * 8, (most / 4 + 255) / 256);
-  const cudaError_t e = parts == 2 ? launch_pdl(split_operands_kernel<2>, dim3(blocks, 2), dim3(256), 0, stream, o[0], o[1])
-                                   : launch_pdl(split_operands_kernel<3>, dim3(blocks, 2), dim3(256), 0, stream, o[0], o[1]);
+  const cudaError_t e = launch_pdl(split_operands_kernel<3>, dim3(blocks, 2), dim3(256), 0, stream, o[0], o[1]);
   if (e != cudaSuccess) {
     g_gemm_err = "split-precision GEMM: operand split launch failed";
     return -4;
@@ -937,14 +942,44 @@ int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t
     g_gemm_err = "split-precision GEMM writes fp32 (store or accumulate) only";
     return -2;
   }
-  SplitOperand o[2];
-  const int rc = split_operands(d, 2, sc, o, stream);
-  if (rc != 0) return rc;
-  const int kp = o[0].kp;
+  SplitOperand cut[2];
+  bf16* halves[2] = {static_cast<bf16*>(d.a_halves), static_cast<bf16*>(d.b_halves)};
+  int pitch[2], cuts = 0;
+  long long most = 0;
+  for (int i = 0; i < 2; ++i) {
+    const bool mn = i == 0 ? d.a_mn : d.b_mn;
+    const int outer = i == 0 ? d.M : d.N, rows = mn ? d.K : outer, cols = mn ? outer : d.K;
+    pitch[i] = halves_pitch(cols);
+    if (halves[i] != nullptr && (i == 0 ? d.a_cut : d.b_cut)) continue;
+    if (halves[i] == nullptr) {
+      if (const int rc = sc->grow(i, sizeof(bf16) * (size_t)rows * pitch[i], stream); rc != 0) return rc;
+      halves[i] = reinterpret_cast<bf16*>(sc->buf[i]);
+    }
+    SplitOperand& o = cut[cuts++];
+    o.src = reinterpret_cast<const float*>(i == 0 ? d.A : d.B);
+    o.dst = halves[i];
+    o.ld = i == 0 ? d.lda : d.ldb;
+    o.rows = rows;
+    o.cols = cols;
+    o.kp = pitch[i] / 2;
+    o.pitch = pitch[i];
+    o.k_major = 1;
+    o.vec = o.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(o.src) & 15) == 0;
+    most = std::max(most, (long long)rows * o.kp);
+  }
+  if (cuts > 0) {
+    const unsigned blocks = (unsigned)std::min<long long>(148 * 8, (most / 4 + 255) / 256);
+    if (launch_pdl(split_operands_kernel<2>, dim3(blocks, cuts), dim3(256), 0, stream, cut[0], cut[cuts - 1]) != cudaSuccess) {
+      g_gemm_err = "split-precision GEMM: operand split launch failed";
+      return -4;
+    }
+  }
+  const int kp = (d.K + GEMM_BK - 1) / GEMM_BK * GEMM_BK;
   GemmDesc g = d;
-  g.A = o[0].dst; g.B = o[1].dst; g.lda = o[0].pitch; g.ldb = o[1].pitch;
+  g.A = halves[0]; g.B = halves[1]; g.lda = pitch[0]; g.ldb = pitch[1];
   g.K = 3 * kp;
   g.seg_kb = kp / GEMM_BK;
+  g.seg_k = d.K;
   return gemm_bf16(g, d_status, stream);
 }
 
@@ -1304,7 +1339,7 @@ static cudaError_t launch_f32_tc_layout(const GemmDesc& d, const CUtensorMap& ta
 }
 static int gemm_f32_tc(const GemmDesc& d, int parts, SplitScratch* sc, int* d_status, cudaStream_t stream) {
   SplitOperand o[2];
-  const int rc = split_operands(d, 3, sc, o, stream);
+  const int rc = split_operands(d, sc, o, stream);
   if (rc != 0) return rc;
   const int kp = o[0].kp;
   CUtensorMap ta, tb, tc;
@@ -1327,7 +1362,7 @@ bool gemm_f32_parts(const GemmDesc& d, size_t (&bytes)[2]) {
   const int parts = d.M > 0 && d.N > 0 && d.K > 0 ? f32_on_tensor_cores(d) : 0;
   if (parts == 0) return false;
   int pitch;
-  for (int i = 0; i < 2; ++i) bytes[i] = parts_bytes(d, 3, i, &pitch);
+  for (int i = 0; i < 2; ++i) bytes[i] = parts_bytes(d, i, &pitch);
   cudaFuncAttributes attr;
   cudaFuncGetAttributes(&attr, split_operands_kernel<3>);
   if (parts > 1) d.a_mn ? (d.b_mn ? load_f32_tc<true, true, true>() : load_f32_tc<true, false, true>())

@@ -87,7 +87,12 @@ struct GemmDesc {
   size_t parts_bytes = 0;
   int* n_parts = nullptr;
   int part_rows = 0;  // set by gemm_bf16
-  int seg_kb = 0;   // > 0: operands hold bf16 (hi | lo) halves of seg_kb k-blocks of 64, K = 3 * 64 * seg_kb (see gemm_bf16x3)
+  // gemm_bf16x3: where an operand's halves lie (halves_pitch x its rows in memory), or go unless they lie there already.
+  // nullptr: in the scratch.
+  void *a_halves = nullptr, *b_halves = nullptr;
+  bool a_cut = false, b_cut = false;
+  int seg_kb = 0;   // > 0: operands hold bf16 (hi | lo) halves, K = 3 * 64 * seg_kb, seg_k of 64 * seg_kb filled (see gemm_bf16x3)
+  int seg_k = 0;
 };
 
 constexpr int kMostParts = 8;
@@ -96,6 +101,7 @@ inline int parts_rows(int M) { return (M + 127) / 128 * 128; }
 int gemm_bf16(const GemmDesc& d, int* d_status, cudaStream_t stream);
 // An accumulated product of which gemm_bf16 hands each tile to one CTA as a whole: it can overwrite C instead of adding to it.
 bool gemm_whole_tiles(const GemmDesc& d);
+inline int halves_pitch(int cols) { return 2 * ((cols + 63) / 64 * 64); }
 // fp32 operands at split precision on the tensor cores: A and B are each cut into a bf16 (hi, lo) pair
 // (hi = bf16(x), lo = bf16(x - hi): together ~16 significand bits) and the product is formed as Ah*Bh + Ah*Bl + Al*Bh
 // with fp32 accumulation, one GEMM over a contraction of three passes (the dropped Al*Bl term is ~2^-18 relative).
@@ -109,6 +115,7 @@ struct SplitScratch {
   size_t cap[2] = {0, 0};             // bytes
   uint64_t generation = 0;            // counts the times that a buffer moved: what was captured before holds old addresses
   bool reserve(const size_t (&bytes)[2]);  // both buffers or none
+  int grow(int i, size_t need, cudaStream_t stream);
   void release();
 };
 int gemm_bf16x3(const GemmDesc& d, SplitScratch* scratch, int* d_status, cudaStream_t stream);

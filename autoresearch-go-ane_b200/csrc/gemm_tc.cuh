@@ -211,6 +211,7 @@ struct EpiParams {
   int ce_softcap;        // z = 15 tanh(logit / 15) (ane/common.go:272-287)
   int part_rows;         // EPI_STORE_F32: rows from one share's sums to the next's
   int seg_kb;            // > 0: operands are (hi | lo) halves of seg_kb k-blocks each, three passes hi*lo, lo*hi, hi*hi
+  int lo_a, lo_b;        // columns from an MN-major operand's hi half to its lo half (K-major: seg_kb k-blocks)
 };
 
 // Several accumulating products with one contraction length, run by one launch (the four weight gradients of a
@@ -402,11 +403,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const uint32_t sa = smem_a0 + stage * Cfg::A_BYTES;
           const uint32_t sb = smem_b0 + stage * Cfg::B_BYTES;
           int ka = kb * BK, kb_ = ka;  // first k of this block in A and B
+          int ma = 0, nb = 0;          // MN-major operands: columns to its half
           if (epi.seg_kb > 0) {
             // (two compares; the other products only test seg_kb)
             const int pass = (kb >= epi.seg_kb) + (kb >= 2 * epi.seg_kb), in_pass = kb - pass * epi.seg_kb;
-            ka = (in_pass + (pass == 1 ? epi.seg_kb : 0)) * BK;
-            kb_ = (in_pass + (pass == 0 ? epi.seg_kb : 0)) * BK;
+            ka = (in_pass + (!A_MN && pass == 1 ? epi.seg_kb : 0)) * BK;
+            kb_ = (in_pass + (!B_MN && pass == 0 ? epi.seg_kb : 0)) * BK;
+            if (A_MN && pass == 1) ma = epi.lo_a;
+            if (B_MN && pass == 0) nb = epi.lo_b;
           }
           if constexpr (PAIR) {
             // both CTAs' bytes complete on the leader's barrier, which expects the sum
@@ -422,7 +426,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               } else {
 #pragma unroll
                 for (int j = 0; j < GEMM_BM / 64; ++j)
-                  tma_load_2d_pair(sai + j * (64 * BK * 2), &tmA, full, m0 + j * 64, ka);
+                  tma_load_2d_pair(sai + j * (64 * BK * 2), &tmA, full, m0 + j * 64 + ma, ka);
               }
             }
             if constexpr (!B_MN) {
@@ -430,7 +434,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             } else {
 #pragma unroll
               for (int j = 0; j < Cfg::B_ROWS / 64; ++j)  // the last chunk may reach past this CTA's half: unused columns
-                tma_load_2d_pair(sb + j * (64 * BK * 2), &tmB, full, n0 + j * 64, kb_);
+                tma_load_2d_pair(sb + j * (64 * BK * 2), &tmB, full, n0 + j * 64 + nb, kb_);
             }
           } else {
           const uint32_t full = smem_u32(&bar_full[stage]);
@@ -442,14 +446,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           } else {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
-              tma_load_2d(sa + j * (64 * BK * 2), pA, full, tm * BM + j * 64, ka);
+              tma_load_2d(sa + j * (64 * BK * 2), pA, full, tm * BM + j * 64 + ma, ka);
           }
           if constexpr (!B_MN) {
             tma_load_2d(sb, pB, full, kb_, tn * BN);
           } else {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(sb + j * (64 * BK * 2), pB, full, tn * BN + j * 64, kb_);
+              tma_load_2d(sb + j * (64 * BK * 2), pB, full, tn * BN + j * 64 + nb, kb_);
           }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }

@@ -562,6 +562,22 @@ def test_grouped_weight_gradient_launch_matches_the_separate_launches(monkeypatc
         assert rel_l2(grads[1][k], grads[0][k]) < 1e-5, k
 
 
+@pytest.mark.parametrize("arch,quirks", [(O.ARCH_L, 0), (O.ARCH_N, 1)])
+def test_split_precision_operands_of_odd_widths_cut_once(arch, quirks):
+    """Widths that are no multiple of a k-block (80, 104, 520), the head in chunks of rows, two micro-steps: the stated tolerance
+    above, which one operand read with the wrong half (2^-9 relative in every product) or from another chunk exceeds."""
+    cfg = dict(dim=80, hidden=128 if arch == O.ARCH_L else 104, heads=2, layers=3, vocab=520, seq=37)
+    m, e = make_pair(ane, cfg, arch=arch, quirks=quirks, dtype=ane.DTYPE_BF16X3, batch=3, hyper=dict(lr=3e-4, accum_steps=1000, ce_chunk_rows=40))
+    for seed in (5, 6):
+        inp, tgt = batch_tokens(cfg, 3, seed)
+        oracle_batch_accumulate(m, inp, tgt, cfg["seq"])
+        e.step_tokens(inp, tgt)
+    rep = []
+    worst = compare_grads(m, e, rep)
+    assert worst < 1e-3, sorted(rep, key=lambda x: -x[2])[:5]
+    e.close()
+
+
 def test_split_precision_head_with_a_token_outside_the_vocabulary_reference_arch():
     """The case that plain bf16 fails (xfail above) in the split-precision mode: inside the stated tolerance."""
     cfg = dict(dim=128, hidden=256, heads=2, layers=2, vocab=512, seq=128)
