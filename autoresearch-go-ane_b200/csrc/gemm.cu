@@ -225,7 +225,11 @@ static int dispatch_epi(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
                         int* d_status, cudaStream_t stream) {
   EpiParams epi{d.alpha, d.res1, d.s1, d.res2, d.s2, d.ldres, reinterpret_cast<bf16*>(d.aux), d.ldaux,
                 d.rope_cos, d.rope_sin, d.rope_seq, d.rope_pos0, d.rope_cols, d.tgt, d.tgt_out, d.tgt_row0,
-                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, d.part_rows, d.seg_kb, d.lda / 2, d.ldb / 2};
+                d.ce_stats, d.ce_lse2, d.ce_coef, d.ce_rows, d.ce_col0, d.ce_softcap ? 1 : 0, d.part_rows, d.seg_kb};
+  if (d.seg_kb > 0) {
+    epi.lo_a = d.lda / 2;
+    epi.lo_b = d.ldb / 2;
+  }
   constexpr int whole = 1;  // schedule of the epilogues that need whole tiles
   constexpr bool NARROW = GemmCfg<BN, MT>::NARROW;
   CUtensorMap tc;
