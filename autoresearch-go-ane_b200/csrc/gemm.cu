@@ -555,7 +555,8 @@ static int narrow_width(const GemmDesc& d) {
 // x 2304 13.3 -> 9.4, 256 x 768 x 4096 18.3 -> 10.1, 256 x 768 x 32000 96 -> 23, 512 x 768 x 32000 in three passes 285 -> 69, 1000 x
 // 288 x 1536 11.2 -> 8.8, 1000 x 288 x 32000 98 -> 29; the norm behind them 5.3 -> 7.5 at six shares of 256 x 768, 4.0 -> 5.0 at
 // three of 1000 x 288.  (In a pass: one window 2469 -> 2297 us an update, three micro-steps of 5 x 200 3030 -> 2812, the split-precision
-// update of 2 x 256 6749 -> 6287.)
+// update of 2 x 256 6749 -> 6287.)  Against the fp32 engine the split-precision gradients are half as far off in shares, shorter chains
+// of sums (2.1 to 3.6e-5 for 6.2 to 6.9e-5), and the bf16 ones as far (4.7 to 11.3e-3).
 static int plan_parts(const GemmDesc& d, int& best_bn) {
   static const bool off = [] { const char* e = getenv("ANE_B200_GEMM_PARTS"); return e && e[0] == '0'; }();  // A/B measurements
   if (off || d.parts == nullptr || d.n_parts == nullptr || d.out != GEMM_OUT_F32 || d.res1 || d.res2 || d.split_k > 1 || d.N % 4 != 0 ||
