@@ -36,10 +36,11 @@ __device__ __forceinline__ float4 ldf_l2_if(const float* p, bool take) {
 // dependent instructions, and where it is reached once in a phase they come from beyond the instruction cache: between the sum of
 // squares and the first normalised column, 1 / sqrt(x / dim) took 2000 cycles.
 __device__ __forceinline__ int quotient(int n, int d, unsigned magic) { return d == 1 ? n : (int)__umulhi((unsigned)n, magic); }
-// 1 / sqrt(x) and 1 / x to an ulp or two: the hardware's approximation and one step of Newton's method
+// 1 / sqrt(x) and 1 / x to an ulp or two: the hardware's approximation and one step of Newton's method.  1 / sqrt(inf) is 0, as in
+// the norms of the forward pass (the step alone would make it 0 * inf).
 __device__ __forceinline__ float inverse_sqrt(float x) {
   const float y = rsqrtf(x);
-  return y * fmaf(-0.5f * x * y, y, 1.5f);
+  return y == 0.f ? y : y * fmaf(-0.5f * x * y, y, 1.5f);
 }
 __device__ __forceinline__ float inverse(float x) {
   const float y = __fdividef(1.0f, x);

@@ -320,3 +320,24 @@ def test_decode_where_the_persistent_kernel_does_not_fit():
     for (tokens, launches), (same, more) in zip(whole, two):
         assert same == tokens
         assert more > 2 * launches
+
+
+@pytest.mark.parametrize("batch", [2, 9])
+def test_norm_of_a_row_whose_squares_overflow(batch):
+    """A row with a sum of squares beyond fp32 is normalised to zeros (1 / sqrt(inf)), in the persistent kernels as in prefill and
+    step by step.  All weights but the embedding are zero, so the stream is the token's embedding: after BIG all logits are 0
+    (index 0), after 0 the largest is NEXT's, after NEXT it is BIG's."""
+    dim, vocab, prompt, new = 128, 96, 3, 9
+    big, nxt = 5, 7
+    embed = np.full((vocab, dim), 1.0 / 64, np.float32)
+    embed[:, 0] = 0
+    embed[0], embed[nxt], embed[big] = 0, 0, 0
+    embed[0, 0], embed[0, 1] = -1, 8
+    embed[nxt, 0], embed[nxt, 1] = 1, 16
+    embed[big, 0] = 1e20
+    e = ane.open(ane.Options(dim=dim, hidden=256, n_layers=2, n_heads=2, n_kv_heads=2, vocab=vocab, seq=64, batch=batch,
+                             arch=ane.ARCH_LLAMA, quirks=0, compute_dtype=ane.DTYPE_BF16))
+    e.import_tensor(ane.T_EMBED, 0, embed)
+    got = e.decode_greedy(np.full((batch, prompt), nxt, np.uint16), new)
+    e.close()
+    np.testing.assert_array_equal(got, np.tile(np.array([big, 0, nxt], np.uint16), (batch, 3)))
