@@ -530,9 +530,9 @@ int decode_steps(DecodeArgs a, void* words, int sms, cudaStream_t s) {
   a.group = rep <= 8 ? rep : 1;  // query heads per attention item: rows of one fragment
   a.rep = rep;
   a.items = a.H / a.group;
-  a.hd_magic = 0xffffffffu / (unsigned)a.hd + 1u;
-  a.rep_magic = 0xffffffffu / (unsigned)a.rep + 1u;
-  a.items_magic = 0xffffffffu / (unsigned)a.items + 1u;
+  a.hd_magic = quotient_magic((unsigned)a.hd);
+  a.rep_magic = quotient_magic((unsigned)a.rep);
+  a.items_magic = quotient_magic((unsigned)a.items);
   a.score_scale = 1.4426950408889634f / sqrtf((float)a.hd);
   a.inv_dim = 1.0f / (float)a.D;
   const size_t rows = word_rows(a.D, a.Hd, a.H, a.KV, a.hd, a.B, sms);

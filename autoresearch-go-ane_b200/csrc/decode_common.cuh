@@ -2,6 +2,7 @@
 // and decode_batch.cu (9 to 32, clusters that split every contraction).
 #pragma once
 #include "common.cuh"
+#include "decode_math.h"
 #include "kernels.h"
 
 namespace ane {
@@ -32,20 +33,9 @@ __device__ __forceinline__ float4 ldf_l2_if(const float* p, bool take) {
   return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
 }
 
-// n / d for n below 2^16 with magic = 0xffffffff / d + 1 from the host.  A division, like an IEEE square root, is a long run of
-// dependent instructions, and where it is reached once in a phase they come from beyond the instruction cache: between the sum of
-// squares and the first normalised column, 1 / sqrt(x / dim) took 2000 cycles.
-__device__ __forceinline__ int quotient(int n, int d, unsigned magic) { return d == 1 ? n : (int)__umulhi((unsigned)n, magic); }
-// 1 / sqrt(x) and 1 / x to an ulp or two: the hardware's approximation and one step of Newton's method.  1 / sqrt(inf) is 0, as in
-// the norms of the forward pass (the step alone would make it 0 * inf).
-__device__ __forceinline__ float inverse_sqrt(float x) {
-  const float y = rsqrtf(x);
-  return y == 0.f ? y : y * fmaf(-0.5f * x * y, y, 1.5f);
-}
-__device__ __forceinline__ float inverse(float x) {
-  const float y = __fdividef(1.0f, x);
-  return y * fmaf(-x, y, 2.0f);
-}
+// 1 / x for divide(), |x| up to 2^126.  1 / sqrt(x).
+__device__ __forceinline__ float inverse(float x) { return newton_inverse(x, __fdividef(1.0f, x)); }
+__device__ __forceinline__ float inverse_sqrt(float x) { return newton_inverse_sqrt(x, rsqrtf(x)); }
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&v);
@@ -296,7 +286,7 @@ __device__ __forceinline__ void attention_phase(const DecodeArgs& a, const bf16*
         o1 += v.y * f;
       }
       const float inv = inverse(ls);
-      const uint32_t v = pack2(o0 * inv, o1 * inv);
+      const uint32_t v = pack2(divide(o0, ls, inv), divide(o1, ls, inv));
       const size_t at = (size_t)b * (qd / 2) + (size_t)((h0 + h) * hd + d) / 2;
       put_word(a.w_att + at, v, epoch);
     }
