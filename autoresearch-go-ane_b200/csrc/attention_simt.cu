@@ -19,30 +19,29 @@ static constexpr int kMaxHdPerLane = 4;  // head_dim <= 128
 // floats, so score operands are read as float4 along the head dimension without bank conflicts, 64 FMAs for eight
 // 16-byte reads; probabilities pass through shared memory transposed, [streamed row][resident row], one float4 per
 // streamed row.  32 resident rows (not 64 or 128) because the fp32 modes run with few sequences: 2 x 12 heads x 256
-// make 192 blocks.  The next tile is on its way (cp.async, two buffers) while one is worked on: a block has its SM almost to
-// itself, and waiting for a tile took a third of the time its products do.  us, forward / dQ / dK and dV: 2 x 12 heads of 64, seq 256,
-// 24.8 / 43.7 / 59.4 -> 21.1 / 43.1 / 45.6; 8 x 6 heads of 48 32.1 / 77.1 / 47.4 -> 23.9 / 49.9 / 44.5.  One warp per query with scalar loads and global atomics, which this replaces, took 709 us for
-// the backward of 2 x 12 heads x 256 x 64.
+// make 192 blocks.  With few blocks an SM the next tile is on its way (cp.async, two buffers) while one is worked on: a block has its SM
+// almost to itself then, and waiting for a tile took a third of the time its products do.  us, forward / dQ / dK and dV: 2 x 12 heads of
+// 64, seq 256, 34.7 / 83.2 / 125.2 -> 24.4 / 48.6 / 55.2 (a step of one layer); 8 x 6 heads of 48 32.6 / 54.5 / 70.1 -> 24.8 / 39.4 /
+// 45.0.  One warp per query with scalar loads and global atomics, which this replaces, took 709 us for the backward of 2 x 12 heads x 256 x 64.
 // ------------------------------------------------------------------------------------------------
 namespace {
 
 constexpr int kRes = 32, kStr = 64, kSimtThreads = 128;
 constexpr int kShortTiles = 4;  // tiles of keys that attention_dq_short_simt_kernel keeps
+constexpr size_t kSmemOfSm = 228 * 1024;  // 1 KB of it goes to each block
 constexpr int kPPitch = kRes + 4;  // floats of one streamed row of the probability tile
 
 template <int HDP>
 struct Simt {
   static constexpr int kPitch = HDP + 4;
   static constexpr int kResFloats = kRes * kPitch, kStrFloats = kStr * kPitch, kProbFloats = kStr * kPPitch;
-  // Buffers of streamed tiles: two where the next tile can be on its way and two or three blocks still fit an SM
-  template <typename T>
-  __host__ __device__ static constexpr int bufs() { return sizeof(T) == 4 && HDP <= 64 ? 2 : 1; }
-  template <typename T>
-  static constexpr size_t fwd_smem() { return sizeof(float) * (kResFloats + 2 * bufs<T>() * kStrFloats + kProbFloats); }
+  static constexpr bool kTwoBuffers = HDP <= 64;  // of streamed tiles, for fp32: two blocks or more fit an SM
+  static constexpr size_t fwd_smem(int bufs) { return sizeof(float) * (kResFloats + 2 * bufs * kStrFloats + kProbFloats); }
   static constexpr size_t kDqSmem = sizeof(float) * (2 * kResFloats + 2 * kStrFloats + kProbFloats);
-  static constexpr size_t dq_short_smem() { return sizeof(float) * (2 * kResFloats + (kShortTiles + 2) * kStrFloats + kProbFloats); }
-  template <typename T>
-  static constexpr size_t dkv_smem() { return sizeof(float) * (2 * kResFloats + bufs<T>() * (2 * kStrFloats + 3 * kStr) + 2 * kProbFloats); }
+  static constexpr size_t dq_short_smem(int tiles) {  // two buffers of values
+    return sizeof(float) * (2 * kResFloats + (tiles + (tiles < 2 ? tiles : 2)) * kStrFloats + kProbFloats);
+  }
+  static constexpr size_t dkv_smem(int bufs) { return sizeof(float) * (2 * kResFloats + bufs * (2 * kStrFloats + 3 * kStr) + 2 * kProbFloats); }
 };
 
 template <typename T>
@@ -188,16 +187,15 @@ __device__ __forceinline__ void zero(float (&a)[4][HDP / 16]) {
 }
 
 // Forward: grid (B * H, query tiles), the longest rows first.
-template <int HDP, typename T, typename TO>
+template <int HDP, int BUFS, typename T, typename TO>
 __global__ void __launch_bounds__(kSimtThreads)
 attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, float* __restrict__ lse, int seq, int H, int KV, int hd, float scale) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ __align__(16) float simt_smem[];
   float* Qs = simt_smem;
-  constexpr int kBufs = Simt<HDP>::template bufs<T>();
   float* Kb = Qs + Simt<HDP>::kResFloats;  // buffers of a tile's keys and values
-  float* Ps = Kb + 2 * kBufs * Simt<HDP>::kStrFloats;
+  float* Ps = Kb + 2 * BUFS * Simt<HDP>::kStrFloats;
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const int b = blockIdx.x / H, h = blockIdx.x - b * H, kvh = h / (H / KV);
   const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRes;
@@ -206,13 +204,13 @@ attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, f
   const T* kb = qkv + row0 * ld + (size_t)(H + kvh) * hd;
   const T* vb = qkv + row0 * ld + (size_t)(H + KV + kvh) * hd;
   auto request = [&](int k0) {
-    float* to = Kb + (k0 / kStr & (kBufs - 1)) * 2 * Simt<HDP>::kStrFloats;
+    float* to = Kb + (k0 / kStr & (BUFS - 1)) * 2 * Simt<HDP>::kStrFloats;
     request_rows<HDP, kStr>(to, kb + (size_t)k0 * ld, ld, seq - k0, hd);
     request_rows<HDP, kStr>(to + Simt<HDP>::kStrFloats, vb + (size_t)k0 * ld, ld, seq - k0, hd);
     tile_requested();
   };
   request_rows<HDP, kRes>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
-  if (kBufs == 2) request(0);
+  if (BUFS == 2) request(0);
   float m[4], l[4], acc[4][HDP / 16];
   zero<HDP>(acc);
 #pragma unroll
@@ -222,14 +220,14 @@ attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, f
   }
   const int last = min(q0 + kRes, seq) - 1;
   for (int k0 = 0; k0 <= last; k0 += kStr) {
-    if (kBufs == 1) {
+    if (BUFS == 1) {
       __syncthreads();
       request(k0);
     }
     tile_wait<0>();  // (and everybody has left the buffer that is filled next)
-    const float* Ks = Kb + (k0 / kStr & (kBufs - 1)) * 2 * Simt<HDP>::kStrFloats;
+    const float* Ks = Kb + (k0 / kStr & (BUFS - 1)) * 2 * Simt<HDP>::kStrFloats;
     const float* Vs = Ks + Simt<HDP>::kStrFloats;
-    if (kBufs == 2 && k0 + kStr <= last) request(k0 + kStr);
+    if (BUFS == 2 && k0 + kStr <= last) request(k0 + kStr);
     float s[4][4];
     scores<HDP>(s, Qs, Ks, ty, tx);
 #pragma unroll
@@ -384,9 +382,9 @@ attention_dq_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_out
   }
 }
 
-// The first kernel for up to kShortTiles tiles of keys in fp32: scores and dP of the first sweep stay in registers and the keys in
-// shared memory, so that the second sweep is one product instead of three.  (One buffer of values and two blocks an SM instead: 1 %
-// slower in a whole update.)
+// The first kernel for two to kShortTiles tiles of keys in fp32: scores and dP of the first sweep stay in registers and the keys in
+// shared memory, so that the second sweep is one product instead of three.  (Four tiles with one buffer of values and two blocks an SM: 1 %
+// slower in a whole update of 2 x 256 tokens.)
 template <int HDP>
 __global__ void __launch_bounds__(kSimtThreads)
 attention_dq_short_simt_kernel(const float* __restrict__ qkv, const float* __restrict__ d_out, float* __restrict__ dqkv, float* __restrict__ stats, int rows,
@@ -397,8 +395,9 @@ attention_dq_short_simt_kernel(const float* __restrict__ qkv, const float* __res
   float* Qs = simt_smem;
   float* dOs = Qs + Simt<HDP>::kResFloats;
   float* Kb = dOs + Simt<HDP>::kResFloats;                // all tiles' keys
-  float* Vb = Kb + kShortTiles * Simt<HDP>::kStrFloats;  // two buffers of values
-  float* Ps = Vb + 2 * Simt<HDP>::kStrFloats;
+  const int held = (seq + kStr - 1) / kStr;                // (shared memory for as many: dq_short_smem())
+  float* Vb = Kb + held * Simt<HDP>::kStrFloats;          // buffers of values, two where there are tiles for them
+  float* Ps = Vb + min(held, 2) * Simt<HDP>::kStrFloats;
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const int b = blockIdx.x / H, h = blockIdx.x - b * H, kvh = h / (H / KV);
   const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRes;
@@ -496,7 +495,7 @@ attention_dq_short_simt_kernel(const float* __restrict__ qkv, const float* __res
 }
 
 // Backward, second kernel: dK and dV of 32 keys over the queries of every head that shares them; no atomics.
-template <int HDP, typename T, typename TD>
+template <int HDP, int BUFS, typename T, typename TD>
 __global__ void __launch_bounds__(kSimtThreads)
 attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_out, float* __restrict__ dqkv, const float* __restrict__ stats, int rows,
                           int seq, int H, int KV, int hd, float scale) {
@@ -505,9 +504,8 @@ attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_ou
   extern __shared__ __align__(16) float simt_smem[];
   float* Ks = simt_smem;
   float* Vs = Ks + Simt<HDP>::kResFloats;
-  constexpr int kBufs = Simt<HDP>::template bufs<T>();
   float* Qb = Vs + Simt<HDP>::kResFloats;  // buffers of a tile's queries and output gradients
-  float* Ps = Qb + 2 * kBufs * Simt<HDP>::kStrFloats;
+  float* Ps = Qb + 2 * BUFS * Simt<HDP>::kStrFloats;
   float* Ds = Ps + Simt<HDP>::kProbFloats;
   float* sb = Ds + Simt<HDP>::kProbFloats;  // and of maximum, 1 / sum, delta of the 64 queries
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
@@ -529,13 +527,13 @@ attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_ou
   };
   const int first = k0 / kStr * kStr;
   int buf = 0;
-  if (kBufs == 2) request(kvh * group, first, 0);
+  if (BUFS == 2) request(kvh * group, first, 0);
   float dk[4][HDP / 16], dv[4][HDP / 16];
   zero<HDP>(dk);
   zero<HDP>(dv);
   for (int h = kvh * group; h < (kvh + 1) * group; ++h) {
-    for (int q0 = first; q0 < seq; q0 += kStr, buf ^= kBufs - 1) {
-      if (kBufs == 1) {
+    for (int q0 = first; q0 < seq; q0 += kStr, buf ^= BUFS - 1) {
+      if (BUFS == 1) {
         __syncthreads();
         request(h, q0, 0);
       }
@@ -543,7 +541,7 @@ attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_ou
       const float* Qs = Qb + buf * 2 * Simt<HDP>::kStrFloats;
       const float* dOs = Qs + Simt<HDP>::kStrFloats;
       const float* st = sb + buf * 3 * kStr;
-      if (kBufs == 2) {
+      if (BUFS == 2) {
         if (q0 + kStr < seq) request(h, q0 + kStr, buf ^ 1);
         else if (h + 1 < (kvh + 1) * group) request(h + 1, first, buf ^ 1);
       }
@@ -586,34 +584,73 @@ attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_ou
   }
 }
 
+template <int HDP, int BUFS, typename T, typename TO>
+void launch_forward(const T* qkv, TO* out, float* lse, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
+  auto kern = attention_forward_simt_kernel<HDP, BUFS, T, TO>;
+  static unsigned long long done = 0;
+  smem_opt_in(kern, Simt<HDP>::fwd_smem(BUFS), done);
+  launch_pdl(kern, dim3(B * H, (seq + kRes - 1) / kRes), dim3(kSimtThreads), Simt<HDP>::fwd_smem(BUFS), s, qkv, out, lse, seq, H, KV, hd, scale);
+}
+// Two buffers where they leave (nearly) all blocks resident, else one, so that more blocks hide one another's loads.  us, one / two:
+// 240 blocks of head size 64, seq 128, 21.7 / 15.5, 384 blocks, seq 256, 26.7 / 23.2, 576 blocks, seq 192, 24.7 / 29.3, 2400 blocks, seq 256,
+// 99.6 / 130.1; head size 48, seq 256: 384 blocks 30.0 / 24.8, 1200 blocks 46.1 / 47.9.  With one tile there is nothing to request
+// early: 384 blocks of head size 64, seq 64, 11.2 / 19.9, but 216 blocks 14.1 / 10.3 (they spread over the SMs).
 template <int HDP, typename T, typename TO>
 void forward_hdp(const T* qkv, TO* out, float* lse, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
-  auto kern = attention_forward_simt_kernel<HDP, T, TO>;
-  static unsigned long long done = 0;
-  smem_opt_in(kern, Simt<HDP>::template fwd_smem<T>(), done);
-  launch_pdl(kern, dim3(B * H, (seq + kRes - 1) / kRes), dim3(kSimtThreads), Simt<HDP>::template fwd_smem<T>(), s, qkv, out, lse, seq, H, KV, hd, scale);
+  if constexpr (Simt<HDP>::kTwoBuffers && sizeof(T) == 4) {
+    constexpr long long resident = 148 * (kSmemOfSm / (Simt<HDP>::fwd_smem(2) + 1024));
+    const long long blocks = (long long)B * H * ((seq + kRes - 1) / kRes);
+    if (blocks <= (seq > kStr ? resident * 4 / 3 : resident)) return launch_forward<HDP, 2>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
+  }
+  launch_forward<HDP, 1>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
 }
+template <int HDP, int BUFS, typename T, typename TD>
+void launch_dkv(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
+  auto kern = attention_dkv_simt_kernel<HDP, BUFS, T, TD>;
+  static unsigned long long done = 0;
+  smem_opt_in(kern, Simt<HDP>::dkv_smem(BUFS), done);
+  launch_pdl(kern, dim3(B * KV, (seq + kRes - 1) / kRes), dim3(kSimtThreads), Simt<HDP>::dkv_smem(BUFS), s, qkv, d_out, dqkv, stats, B * H * seq, seq, H,
+             KV, hd, scale);
+}
+// As in the forward pass, but up to four blocks an SM (two or three are resident).  us, one / two: 192 blocks of head size 64, seq 256, 118.9 / 55.2, 576 blocks 72.8 / 64.6, 1152 blocks 110.1 /
+// 119.0; head size 48, seq 256: 576 blocks 54.5 / 47.5, 1200 blocks 85.5 / 97.1; one tile of 64, head size 64: 216 blocks 27.8 / 25.2, 384
+// blocks 29.5 / 37.6; head size 32: 384 blocks 22.5 / 18.2, 592 blocks, seq 48, 23.6 / 30.9.
+template <int HDP, typename T, typename TD>
+void dkv_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
+  if constexpr (Simt<HDP>::kTwoBuffers && sizeof(T) == 4) {
+    constexpr long long resident = 148 * (kSmemOfSm / (Simt<HDP>::dkv_smem(2) + 1024));
+    const long long blocks = (long long)B * KV * ((seq + kRes - 1) / kRes);
+    if (blocks <= (seq > kStr || H > KV ? 148 * 4 : resident)) return launch_dkv<HDP, 2>(qkv, d_out, dqkv, stats, B, seq, H, KV, hd, scale, s);
+  }
+  launch_dkv<HDP, 1>(qkv, d_out, dqkv, stats, B, seq, H, KV, hd, scale, s);
+}
+// dQ of two to four tiles of keys, in fp32: the kernel that keeps everything of its first sweep, with shared memory for the tiles that
+// there are.  us, two sweeps / kept: head size 64, 1200 blocks, seq 100, 102.8 / 95.9, 1152 blocks, seq 192, 111.3 / 95.4, 192 blocks, seq
+// 256, 80.5 / 48.6; head size 48, 1176 blocks, seq 100, 81.5 / 70.8.  One tile is swept once by the other kernel as well, in less shared
+// memory: 1176 blocks of head size 64, seq 48, 70.2 / 77.3.  Four tiles of head size 64 leave one block an SM, which pays up to three
+// rounds of blocks: seq 256, 384 blocks 84.5 / 69.5, 576 blocks 82.4 / 88.9, 2400 blocks 267 / 269.
 template <int HDP, typename T, typename TD>
 void backward_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
-  auto dq = attention_dq_simt_kernel<HDP, T, TD>;
-  auto dkv = attention_dkv_simt_kernel<HDP, T, TD>;
-  static unsigned long long done_q = 0, done_k = 0;
-  smem_opt_in(dq, Simt<HDP>::kDqSmem, done_q);
-  smem_opt_in(dkv, Simt<HDP>::template dkv_smem<T>(), done_k);
-  const int tiles = (seq + kRes - 1) / kRes, rows = B * H * seq;
-  // up to 256 positions, heads whose keys fit: everything of the first sweep is kept for the second
-  if constexpr (HDP <= 64 && sizeof(T) == 4 && sizeof(TD) == 4) {
-    if (seq <= kShortTiles * kStr) {
-      auto dq_short = attention_dq_short_simt_kernel<HDP>;
-      static unsigned long long done_s = 0;
-      smem_opt_in(dq_short, Simt<HDP>::dq_short_smem(), done_s);
-      launch_pdl(dq_short, dim3(B * H, tiles), dim3(kSimtThreads), Simt<HDP>::dq_short_smem(), s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
-      launch_pdl(dkv, dim3(B * KV, tiles), dim3(kSimtThreads), Simt<HDP>::template dkv_smem<T>(), s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
-      return;
+  const int tiles = (seq + kStr - 1) / kStr, rows = B * H * seq;
+  const dim3 grid(B * H, (seq + kRes - 1) / kRes);
+  bool kept = false;
+  if constexpr (Simt<HDP>::kTwoBuffers && sizeof(T) == 4 && sizeof(TD) == 4) {
+    kept = tiles > 1 && tiles <= kShortTiles &&
+           (2 * (Simt<HDP>::dq_short_smem(tiles) + 1024) <= kSmemOfSm || (long long)grid.x * grid.y <= 148 * 3);
+    if (kept) {
+      auto kern = attention_dq_short_simt_kernel<HDP>;
+      static unsigned long long done = 0;
+      smem_opt_in(kern, Simt<HDP>::dq_short_smem(kShortTiles), done);
+      launch_pdl(kern, grid, dim3(kSimtThreads), Simt<HDP>::dq_short_smem(tiles), s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
     }
   }
-  launch_pdl(dq, dim3(B * H, tiles), dim3(kSimtThreads), Simt<HDP>::kDqSmem, s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
-  launch_pdl(dkv, dim3(B * KV, tiles), dim3(kSimtThreads), Simt<HDP>::template dkv_smem<T>(), s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
+  if (!kept) {
+    auto kern = attention_dq_simt_kernel<HDP, T, TD>;
+    static unsigned long long done = 0;
+    smem_opt_in(kern, Simt<HDP>::kDqSmem, done);
+    launch_pdl(kern, grid, dim3(kSimtThreads), Simt<HDP>::kDqSmem, s, qkv, d_out, dqkv, stats, rows, seq, H, KV, hd, scale);
+  }
+  dkv_hdp<HDP>(qkv, d_out, dqkv, stats, B, seq, H, KV, hd, scale, s);
 }
 
 }  // namespace

@@ -41,6 +41,17 @@ def test_fp32_tiles_of_several_sweeps(arch, hd, heads, kv, seq):
     test_fp32_tiles(arch, hd, heads, kv, seq)
 
 
+@pytest.mark.parametrize("hd,heads,kv,seq,batch", [
+    (32, 4, 4, 65, 70), (40, 2, 2, 193, 50), (64, 2, 2, 64, 150), (64, 2, 1, 129, 80), (64, 2, 2, 256, 28), (64, 2, 2, 256, 38)])
+def test_fp32_tiles_of_many_blocks(hd, heads, kv, seq, batch):
+    """More blocks than the SMs hold with two buffers take one, more than three an SM with four tiles of head size 64 two sweeps for dQ."""
+    cfg, m, e, inp, tgt = _step(ane.DTYPE_F32, O.ARCH_L, 0, hd, heads, kv, seq, batch, 0.1)
+    oracle_batch_accumulate(m, inp, tgt, seq)
+    rep = []
+    assert compare_grads(m, e, rep) < F32_TOL, rep
+    e.close()
+
+
 @pytest.mark.parametrize("hd,heads,kv,seq,batch", [(32, 2, 1, 63, 2), (48, 2, 2, 65, 2), (48, 4, 2, 200, 2), (48, 2, 2, 257, 50),
                                                    (64, 2, 1, 100, 2), (64, 4, 4, 129, 40)])
 def test_bf16_tiles(hd, heads, kv, seq, batch):
