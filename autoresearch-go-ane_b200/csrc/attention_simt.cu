@@ -88,10 +88,8 @@ __device__ __forceinline__ void request_rows(float* dst, const T* src, int ld, i
     }
   }
 }
-__device__ __forceinline__ void tile_requested() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int LEFT>
-__device__ __forceinline__ void tile_wait() {  // all but the LEFT newest, of every thread
-  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+__device__ __forceinline__ void tile_wait() {  // everything that any thread has requested
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
 }
 
@@ -207,7 +205,6 @@ attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, f
     float* to = Kb + (k0 / kStr & (BUFS - 1)) * 2 * Simt<HDP>::kStrFloats;
     request_rows<HDP, kStr>(to, kb + (size_t)k0 * ld, ld, seq - k0, hd);
     request_rows<HDP, kStr>(to + Simt<HDP>::kStrFloats, vb + (size_t)k0 * ld, ld, seq - k0, hd);
-    tile_requested();
   };
   request_rows<HDP, kRes>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
   if (BUFS == 2) request(0);
@@ -224,7 +221,7 @@ attention_forward_simt_kernel(const T* __restrict__ qkv, TO* __restrict__ out, f
       __syncthreads();
       request(k0);
     }
-    tile_wait<0>();  // (and everybody has left the buffer that is filled next)
+    tile_wait();  // (and everybody has left the buffer that is filled next)
     const float* Ks = Kb + (k0 / kStr & (BUFS - 1)) * 2 * Simt<HDP>::kStrFloats;
     const float* Vs = Ks + Simt<HDP>::kStrFloats;
     if (BUFS == 2 && k0 + kStr <= last) request(k0 + kStr);
@@ -406,12 +403,10 @@ attention_dq_short_simt_kernel(const float* __restrict__ qkv, const float* __res
   const float* kb = qkv + row0 * ld + (size_t)(H + kvh) * hd;
   const float* vb = qkv + row0 * ld + (size_t)(H + KV + kvh) * hd;
   const int last = min(q0 + kRes, seq) - 1, tiles = last / kStr + 1;
-  auto request = [&](int t) {  // (an empty group past the last tile, so that the groups of all threads count alike)
-    if (t < tiles) {
-      request_rows<HDP, kStr>(Kb + t * Simt<HDP>::kStrFloats, kb + (size_t)t * kStr * ld, ld, seq - t * kStr, hd);
-      request_rows<HDP, kStr>(Vb + (t & 1) * Simt<HDP>::kStrFloats, vb + (size_t)t * kStr * ld, ld, seq - t * kStr, hd);
-    }
-    tile_requested();
+  auto request = [&](int t) {
+    if (t >= tiles) return;
+    request_rows<HDP, kStr>(Kb + t * Simt<HDP>::kStrFloats, kb + (size_t)t * kStr * ld, ld, seq - t * kStr, hd);
+    request_rows<HDP, kStr>(Vb + (t & 1) * Simt<HDP>::kStrFloats, vb + (size_t)t * kStr * ld, ld, seq - t * kStr, hd);
   };
   request_rows<HDP, kRes>(Qs, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
   request_rows<HDP, kRes>(dOs, d_out + (row0 + q0) * (size_t)(H * hd) + (size_t)h * hd, H * hd, seq - q0, hd);
@@ -426,7 +421,7 @@ attention_dq_short_simt_kernel(const float* __restrict__ qkv, const float* __res
 #pragma unroll
   for (int t = 0; t < kShortTiles; ++t) {
     if (t >= tiles) continue;
-    tile_wait<0>();
+    tile_wait();
     request(t + 1);
     scores<HDP>(s[t], Qs, Kb + t * Simt<HDP>::kStrFloats, ty, tx);
     scores<HDP>(dp[t], dOs, Vb + (t & 1) * Simt<HDP>::kStrFloats, ty, tx);
@@ -519,7 +514,6 @@ attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_ou
     float* to = Qb + buf * 2 * Simt<HDP>::kStrFloats;
     request_rows<HDP, kStr>(to, qkv + (row0 + q0) * ld + (size_t)h * hd, ld, seq - q0, hd);
     request_rows<HDP, kStr>(to + Simt<HDP>::kStrFloats, d_out + (row0 + q0) * (size_t)(H * hd) + (size_t)h * hd, H * hd, seq - q0, hd);
-    tile_requested();
     for (int i = threadIdx.x; i < 3 * kStr; i += kSimtThreads) {
       const int q = q0 + (i & (kStr - 1));
       sb[buf * 3 * kStr + i] = q < seq ? stats[(size_t)(i / kStr) * rows + ((size_t)b * H + h) * seq + q] : 0.f;
@@ -537,7 +531,7 @@ attention_dkv_simt_kernel(const T* __restrict__ qkv, const TD* __restrict__ d_ou
         __syncthreads();
         request(h, q0, 0);
       }
-      tile_wait<0>();
+      tile_wait();
       const float* Qs = Qb + buf * 2 * Simt<HDP>::kStrFloats;
       const float* dOs = Qs + Simt<HDP>::kStrFloats;
       const float* st = sb + buf * 3 * kStr;
