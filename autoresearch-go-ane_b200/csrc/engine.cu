@@ -299,19 +299,34 @@ class EngineT final : public EngineBase {
   int dalloc(U** p, size_t count) {
     void* q = nullptr;
     cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(U));
-    if (e == cudaErrorMemoryAllocation && kIsF32 && !x3_ && (split_.buf[0] || split_.buf[1])) {
-      // The fp32 mode can do without the room for its operands' parts, what is asked for here it cannot.
+    if (e == cudaErrorMemoryAllocation && give_back()) {
       cudaGetLastError();
-      cudaStreamSynchronize(stream_);
-      cudaStreamSynchronize(dw_stream_);
-      split_.release();
-      dw_split_.release();
       e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(U));
     }
     if (e != cudaSuccess) return cuda_check(e, "cudaMalloc");
     allocs_.push_back(q);
     *p = reinterpret_cast<U*>(q);
     return 0;
+  }
+  // Memory that the engine can do without goes to an allocation that it cannot do without: the room for operands' parts of the fp32
+  // mode, the kept halves of split precision, of which a pass under way may have cut some (see gemm_x3).  False: there is none.
+  bool give_back() {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (!kIsF32 || !stream_ || cudaStreamIsCapturing(stream_, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
+    if (x3_ ? halves_block_ == nullptr : !split_.buf[0] && !split_.buf[1]) return false;
+    cudaStreamSynchronize(stream_);
+    cudaStreamSynchronize(dw_stream_);
+    if (x3_) {
+      cudaFree(halves_block_);
+      halves_block_ = nullptr;
+      halves_.assign(L_, Halves());
+      halves_of_ = HeadHalves();
+      drop_loss_graphs();  // the next pass of each takes what scratch it needs
+    } else {
+      split_.release();
+      dw_split_.release();
+    }
+    return true;
   }
   void destroy();
   bool is_ve_layer(int i) const { return isN_ && (i % 2 == (L_ - 1) % 2); }  // ane/stories/weights.go:22
@@ -339,6 +354,15 @@ class EngineT final : public EngineBase {
     out.stride = (size_t)parts_rows(d.M) * d.N;
     return rc;
   }
+  // Without the block of halves (none taken, or given back since the pass cut some of them) operands are cut into the scratch.
+  int gemm_x3(const GemmDesc& d, cudaStream_t st) {
+    GemmDesc e = d;
+    for (;;) {
+      if (!halves_block_) e.a_halves = e.b_halves = nullptr;
+      const int rc = gemm_bf16x3(e, &split_, d_status_, st);
+      if (rc != GEMM_NO_SCRATCH || !give_back()) return rc;
+    }
+  }
   int gemm(const GemmDesc& d, cudaStream_t on = nullptr) {
     int rc;
     cudaStream_t st = on ? on : stream_;
@@ -348,7 +372,7 @@ class EngineT final : public EngineBase {
       cudaEventCreate(&e1);
       cudaEventRecord(e0, st);
     }
-    if constexpr (kIsF32) rc = x3_ ? gemm_bf16x3(d, &split_, d_status_, st) : gemm_f32(d, st == stream_ ? &split_ : &dw_split_, d_status_, st);
+    if constexpr (kIsF32) rc = x3_ ? gemm_x3(d, st) : gemm_f32(d, st == stream_ ? &split_ : &dw_split_, d_status_, st);
     else rc = gemm_bf16(d, d_status_, st);
     if (profiling_) {
       cudaEventRecord(e1, st);
@@ -433,9 +457,10 @@ class EngineT final : public EngineBase {
     bf16 *xn = nullptr, *att = nullptr, *x2n = nullptr, *gate = nullptr, *wqkv = nullptr, *wo = nullptr, *w13 = nullptr, *w2 = nullptr;
   };
   std::vector<Halves> halves_;  // by layer; nullptrs: no memory for them
-  struct {
+  struct HeadHalves {
     bf16 *dout = nullptr, *dh13 = nullptr, *dx2 = nullptr, *dqkv = nullptr, *xnf = nullptr, *embed = nullptr, *dlogits = nullptr;
   } halves_of_;
+  bf16* halves_block_ = nullptr;  // all of them
   void alloc_halves();
   bool decoding_ = false;  // forward() runs one KV-cached decode step
   std::vector<T*> kcache_, vcache_;  // [B, S_, KV*hd] per layer (one block each for all layers), allocated by the first decode
@@ -526,6 +551,11 @@ class EngineT final : public EngineBase {
     uint64_t scratch = 0;  // split_.generation at its capture: the pass reads and writes that scratch
   };
   std::vector<LossGraph> loss_graphs_;  // by number of windows
+  void drop_loss_graphs() {
+    for (auto& g : loss_graphs_)
+      if (g.exec) cudaGraphExecDestroy(g.exec);
+    loss_graphs_.clear();
+  }
   uint64_t n_tokens_ = 0, rng_ = 0;
   // ---- state
   ane_state st_{};
@@ -601,6 +631,8 @@ void EngineT<T>::destroy() {
   if (dw_stream_) cudaStreamSynchronize(dw_stream_);
   split_.release();
   dw_split_.release();
+  if (halves_block_) cudaFree(halves_block_);
+  halves_block_ = nullptr;
   for (void* p : allocs_) cudaFree(p);
   allocs_.clear();
   if (h_in_) cudaFreeHost(h_in_);
@@ -609,9 +641,7 @@ void EngineT<T>::destroy() {
   if (h_loss_) cudaFreeHost(h_loss_);
   if (h_rows_) cudaFreeHost(h_rows_);
   h_rows_ = nullptr;
-  for (auto& g : loss_graphs_)
-    if (g.exec) cudaGraphExecDestroy(g.exec);
-  loss_graphs_.clear();
+  drop_loss_graphs();
   if (h_logits_) cudaFreeHost(h_logits_);
   h_logits_ = nullptr;
   h_in_ = h_tgt_ = nullptr;
@@ -1029,7 +1059,7 @@ void EngineT<T>::reserve_parts() {
 }
 
 // What is left must do for the scratch of the other products and for whatever else the program does: an eighth of the free memory
-// at most, else every product cuts its operands into the scratch.
+// at most, else every product cuts its operands into the scratch.  They go back when the engine needs memory later: give_back().
 template <typename T>
 void EngineT<T>::alloc_halves() {
   halves_.assign(L_, Halves());
@@ -1058,7 +1088,7 @@ void EngineT<T>::alloc_halves() {
         cudaGetLastError();
         return;
       }
-      allocs_.push_back(base);
+      halves_block_ = base;
     }
   }
 }

@@ -863,7 +863,6 @@ bool SplitScratch::reserve(const size_t (&bytes)[2]) {
   }
   return true;
 }
-static constexpr int kNoScratch = -3;
 int SplitScratch::grow(int i, size_t need, cudaStream_t stream) {
   if (cap[i] >= need) return 0;
   ++generation;
@@ -878,7 +877,7 @@ int SplitScratch::grow(int i, size_t need, cudaStream_t stream) {
   if (cudaMalloc(&buf[i], bytes) != cudaSuccess) {
     cudaGetLastError();
     g_gemm_err = "split-precision GEMM: out of memory for the operands' parts";
-    return kNoScratch;
+    return GEMM_NO_SCRATCH;
   }
   cap[i] = bytes;
   return 0;
@@ -920,11 +919,11 @@ static int split_operands(const GemmDesc& d, SplitScratch* sc, SplitOperand (&o)
       used += (need + 255) / 256 * 256;
       if (used > sc->arena_bytes) {
         g_gemm_err = "split-precision GEMM: the operands' parts do not fit the arena";
-        return kNoScratch;
+        return GEMM_NO_SCRATCH;
       }
       continue;
     }
-    if (sc->cap[i] < need) return kNoScratch;
+    if (sc->cap[i] < need) return GEMM_NO_SCRATCH;
     o[i].dst = reinterpret_cast<bf16*>(sc->buf[i]);
   }
   const long long most = std::max((long long)(o[0].k_major ? o[0].rows : kp) * (o[0].k_major ? kp : o[0].pitch),
@@ -1385,7 +1384,7 @@ int gemm_f32(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t st
   }
   if (const int parts = sc != nullptr ? f32_on_tensor_cores(d) : 0) {
     const int rc = gemm_f32_tc(d, parts, sc, d_status, stream);
-    if (rc != kNoScratch) return rc;  // no memory for the parts: the FMA kernels need none
+    if (rc != GEMM_NO_SCRATCH) return rc;  // no memory for the parts: the FMA kernels need none
   }
   if (f32_aligned(d)) {
     const cudaError_t e = launch_f32(d, stream);

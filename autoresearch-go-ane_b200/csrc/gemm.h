@@ -118,6 +118,7 @@ struct SplitScratch {
   int grow(int i, size_t need, cudaStream_t stream);
   void release();
 };
+constexpr int GEMM_NO_SCRATCH = -16;  // returned by gemm_bf16x3 where the scratch could not grow
 int gemm_bf16x3(const GemmDesc& d, SplitScratch* scratch, int* d_status, cudaStream_t stream);
 // fp32 operands with the error of fp32 sums (the fp32 parity mode): on the FMA units or, for products that are large enough, as six
 // products of bf16 parts (hi, mid, lo) on the tensor cores: none without a scratch for the parts (nullptr, or no memory for it).

@@ -328,3 +328,35 @@ def test_fp32_engine_gives_the_parts_of_its_operands_back_for_a_decode():
         e.close()
     finally:
         ane._ffi.lib.ane_dev_free(filler)
+
+
+@pytest.mark.parametrize("first", ["logits", "decode"])
+def test_split_precision_engine_gives_its_halves_back(first):
+    """What fits only without the kept halves of the operands gets their place: a larger scratch for the classifier product of EvalLogits,
+    the caches of the first decode.  Whoever cuts them, the halves are the same: equal losses (a graph of the former halves by then),
+    logits and tokens, and gradients but for the order of their atomic sums."""
+    toks = O.zipf_tokens(1 << 14, F32_CFG["vocab"], 31)
+    cfg = dict(F32_CFG, seq=1024)
+    windows, prompts = toks[:3 * cfg["seq"]].reshape(3, -1), np.ascontiguousarray(toks[:64]).reshape(4, 16)
+    results = []
+    for left in (None, 48):  # MiB: the scratch takes 51, the caches 151, the halves 500
+        e = ane.open(_options(cfg, tokens=toks, batch=16, arch=ane.ARCH_LLAMA, quirks=0, compute_dtype=ane.DTYPE_BF16X3, accum_steps=1000, ce_chunk_rows=256))
+        C.random_init(e, 6)
+        out = [e.step().loss] + [e.eval_loss(windows)[0] for _ in range(3)]
+        filler = ane._ffi.lib.ane_dev_malloc(int((_free_mib() - left) * 2**20)) if left else None
+        assert filler or not left
+        try:
+            use = {"logits": lambda: e.eval_logits(windows[0]), "decode": lambda: e.decode_greedy(prompts, 5)}
+            for name in sorted(use, key=lambda name: name != first):
+                out.append(use[name]())
+            out += [e.eval_loss(windows)[0] for _ in range(3)] + [e.step().loss]
+            grads = [e.export_tensor(t, 0, O.G) for t in (ane.T_EMBED, ane.T_WQ, ane.T_W2)]
+            e.close()
+        finally:
+            if filler:
+                ane._ffi.lib.ane_dev_free(filler)
+        results.append((out, grads))
+    for a, b in zip(results[0][0], results[1][0]):
+        np.testing.assert_array_equal(a, b)
+    for a, b in zip(results[0][1], results[1][1]):
+        assert rel_l2(b, a) < 2e-6
