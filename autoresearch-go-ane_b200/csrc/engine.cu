@@ -258,6 +258,16 @@ struct Slot {
   size_t off = 0, n = 0;
 };
 
+// Engines that hold memory which they can do without.
+struct SpareMemory {
+  std::mutex mutex;
+  std::vector<EngineBase*> engines;
+};
+SpareMemory& spare_memory() {
+  static SpareMemory* s = new SpareMemory;  // outlives engines that are closed when the process ends
+  return *s;
+}
+
 template <typename T>
 class EngineT final : public EngineBase {
  public:
@@ -299,7 +309,7 @@ class EngineT final : public EngineBase {
   int dalloc(U** p, size_t count) {
     void* q = nullptr;
     cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(U));
-    if (e == cudaErrorMemoryAllocation && give_back()) {
+    while (e == cudaErrorMemoryAllocation && make_room()) {
       cudaGetLastError();
       e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(U));
     }
@@ -310,9 +320,8 @@ class EngineT final : public EngineBase {
   }
   // Memory that the engine can do without goes to an allocation that it cannot do without: the room for operands' parts of the fp32
   // mode, the kept halves of split precision, of which a pass under way may have cut some (see gemm_x3).  False: there is none.
-  bool give_back() {
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (!kIsF32 || !stream_ || cudaStreamIsCapturing(stream_, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
+  bool give_back() override {
+    if (!kIsF32) return false;
     if (x3_ ? halves_block_ == nullptr : !split_.buf[0] && !split_.buf[1]) return false;
     cudaStreamSynchronize(stream_);
     cudaStreamSynchronize(dw_stream_);
@@ -354,13 +363,19 @@ class EngineT final : public EngineBase {
     out.stride = (size_t)parts_rows(d.M) * d.N;
     return rc;
   }
+  // Memory for an allocation that failed: this engine's, then other engines'.
+  bool make_room() {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (!stream_ || cudaStreamIsCapturing(stream_, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
+    return give_back() || engines_give_back(device_, this);
+  }
   // Without the block of halves (none taken, or given back since the pass cut some of them) operands are cut into the scratch.
   int gemm_x3(const GemmDesc& d, cudaStream_t st) {
     GemmDesc e = d;
     for (;;) {
       if (!halves_block_) e.a_halves = e.b_halves = nullptr;
       const int rc = gemm_bf16x3(e, &split_, d_status_, st);
-      if (rc != GEMM_NO_SCRATCH || !give_back()) return rc;
+      if (rc != GEMM_NO_SCRATCH || !make_room()) return rc;
     }
   }
   int gemm(const GemmDesc& d, cudaStream_t on = nullptr) {
@@ -625,6 +640,11 @@ class EngineT final : public EngineBase {
 
 template <typename T>
 void EngineT<T>::destroy() {
+  {
+    SpareMemory& spare = spare_memory();
+    std::lock_guard<std::mutex> lock(spare.mutex);
+    spare.engines.erase(std::remove(spare.engines.begin(), spare.engines.end(), this), spare.engines.end());
+  }
   if (stream_) cudaStreamSynchronize(stream_);
   if (comm_stream_) cudaStreamSynchronize(comm_stream_);  // weight gathers of the last update may still run
   dp_.shutdown();
@@ -860,6 +880,7 @@ int EngineT<T>::alloc_buffers() {
 template <typename T>
 int EngineT<T>::open(const ane_options& opts, const uint16_t* tokens, uint64_t n_tokens, const uint8_t* dp_id) {
   o_ = opts;
+  device_ = o_.device;
   // ---- defaults (ane/engine.go:188-239, ane/stories/config.go:3-18)
   if (o_.dim <= 0) o_.dim = 768;
   if (o_.hidden <= 0) o_.hidden = 2048;
@@ -1089,6 +1110,9 @@ void EngineT<T>::alloc_halves() {
         return;
       }
       halves_block_ = base;
+      SpareMemory& spare = spare_memory();
+      std::lock_guard<std::mutex> lock(spare.mutex);
+      spare.engines.push_back(this);
     }
   }
 }
@@ -1928,6 +1952,7 @@ int EngineT<T>::check_device_status(int* out_status) {
 template <typename T>
 int EngineT<T>::step(const uint16_t* input, const uint16_t* target, uint32_t n_seq, ane_step_result* out) {
   const int64_t t0 = now_ns();
+  std::lock_guard<std::mutex> call(in_call_);
   int rc;
   if ((rc = cuda_check(cudaSetDevice(o_.device), "cudaSetDevice")) != 0) return rc;
   cudaEventRecord(ev0_, stream_);
@@ -1996,6 +2021,7 @@ int EngineT<T>::step(const uint16_t* input, const uint16_t* target, uint32_t n_s
 // ------------------------------------------------------------------------------------------------
 template <typename T>
 int EngineT<T>::eval_logits(const uint16_t* tokens, uint32_t n_seq, float* out, uint64_t cap, uint32_t layout) {
+  std::lock_guard<std::mutex> call(in_call_);
   int rc;
   if ((rc = cuda_check(cudaSetDevice(o_.device), "cudaSetDevice")) != 0) return rc;
   const uint64_t per_seq = (uint64_t)V_ * S_;
@@ -2044,6 +2070,7 @@ int EngineT<T>::eval_logits(const uint16_t* tokens, uint32_t n_seq, float* out, 
 // Fused evaluation loss: classifier chunk + cross-entropy on the device, only the scalar comes back.
 template <typename T>
 int EngineT<T>::eval_loss(const uint16_t* tokens, uint32_t n_seq, double* loss_sum, uint64_t* n_pos) {
+  std::lock_guard<std::mutex> call(in_call_);
   int rc;
   if ((rc = cuda_check(cudaSetDevice(o_.device), "cudaSetDevice")) != 0) return rc;
   double total = 0.0;
@@ -2201,6 +2228,7 @@ int EngineT<T>::alloc_decode() {
 template <typename T>
 int EngineT<T>::decode(const uint16_t* prompts, uint32_t n_seq, uint32_t prompt_len, uint32_t n_new,
                        float temperature, const double* uniforms, uint16_t* out) {
+  std::lock_guard<std::mutex> call(in_call_);
   int rc;
   const bool sampling = temperature > 1e-6f;  // ane/train_full.go:319
   if (sampling && !uniforms) return fail(ANE_ERR_ARG, "storiesane decode: sampling needs one uniform draw per token");
@@ -2529,6 +2557,15 @@ int EngineT<T>::timer_end(float* ms) {
 }
 
 }  // namespace
+
+bool engines_give_back(int device, const EngineBase* asking) {
+  SpareMemory& spare = spare_memory();
+  std::lock_guard<std::mutex> lock(spare.mutex);
+  bool any = false;
+  for (EngineBase* e : spare.engines)
+    if (e != asking && e->give_back_idle(device)) any = true;
+  return any;
+}
 
 EngineBase* create_engine(int compute_dtype) {
   if (compute_dtype == ANE_DTYPE_F32 || compute_dtype == ANE_DTYPE_BF16X3) return new EngineT<float>();

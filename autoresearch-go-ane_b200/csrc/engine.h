@@ -3,6 +3,7 @@
 
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -37,16 +38,28 @@ class EngineBase {
   virtual int timer_begin() = 0;
   virtual int timer_end(float* ms) = 0;
 
+  // give_back() for an allocation outside the engine: not while a call of the engine is under way.
+  bool give_back_idle(int device) {
+    std::unique_lock<std::mutex> idle(in_call_, std::try_to_lock);
+    return idle && device == device_ && give_back();
+  }
+
   const std::string& last_error() const { return err_; }
   uint64_t launches() const { return launches_; }
 
  protected:
+  // Frees memory that the engine can do without; false: there is none.
+  virtual bool give_back() { return false; }
+  std::mutex in_call_;  // held by the calls that use such memory
+  int device_ = 0;
   void count_launch(int n = 1) { launches_ += (uint64_t)n; }
   std::string err_;
   uint64_t launches_ = 0;
 };
 
 EngineBase* create_engine(int compute_dtype);
+// Memory for an allocation that failed, from the engines of this process on `device`, idle ones other than `asking`: false if none had any.
+bool engines_give_back(int device, const EngineBase* asking);
 
 void sample_windows(uint64_t* rng, uint64_t n_tokens, uint32_t seq, uint32_t batch, uint32_t rank, uint32_t world,
                     uint64_t* out_pos);

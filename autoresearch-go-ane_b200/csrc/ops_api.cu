@@ -12,6 +12,7 @@
 
 #include "../../include/ane_b200.h"
 #include "common.cuh"
+#include "engine.h"
 #include "gemm.h"
 #include "kernels.h"
 
@@ -97,6 +98,10 @@ void* ane_dev_malloc(uint64_t bytes) {
       g_parts_dev[dev] = {nullptr, true};
       e = cudaMalloc(&p, bytes ? bytes : 1);
     }
+  }
+  if (e == cudaErrorMemoryAllocation && engines_give_back(dev, nullptr)) {
+    cudaGetLastError();
+    e = cudaMalloc(&p, bytes ? bytes : 1);
   }
   if (e != cudaSuccess) {
     cuda_fail(e, "cudaMalloc");

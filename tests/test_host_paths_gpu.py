@@ -360,3 +360,54 @@ def test_split_precision_engine_gives_its_halves_back(first):
         np.testing.assert_array_equal(a, b)
     for a, b in zip(results[0][1], results[1][1]):
         assert rel_l2(b, a) < 2e-6
+
+
+@pytest.mark.parametrize("busy", [False, True])
+def test_split_precision_engine_gives_its_halves_back_to_another_engine(busy):
+    """An engine that fits only without the halves that another one holds opens, as soon as the other one is in no call (busy: a thread
+    steps it all the while), and the other one goes on with the same losses."""
+    import threading
+    toks = O.zipf_tokens(1 << 14, F32_CFG["vocab"], 31)
+    cfg = dict(F32_CFG, seq=1024)
+
+    def holder():
+        e = ane.open(_options(cfg, tokens=toks, batch=16, arch=ane.ARCH_LLAMA, quirks=0, compute_dtype=ane.DTYPE_BF16X3, accum_steps=1000, ce_chunk_rows=256))
+        C.random_init(e, 6)
+        return e
+
+    def other():
+        e = ane.open(_options(F32_CFG, tokens=toks, batch=4, arch=ane.ARCH_LLAMA, quirks=0, compute_dtype=ane.DTYPE_BF16))
+        C.random_init(e, 7)
+        return e
+
+    e = holder()
+    free = _free_mib()
+    second = other()
+    takes = free - _free_mib()
+    want = [e.step().loss for _ in range(12)], second.step().loss
+    second.close()
+    e.close()
+    assert 100 < takes < 900  # (the halves are 500)
+    e = holder()
+    filler = ane._ffi.lib.ane_dev_malloc(int((_free_mib() - takes / 2) * 2**20))
+    assert filler
+    losses = []
+    try:
+        turns = threading.Thread(target=lambda: losses.extend(e.step().loss for _ in range(12)))
+        if busy:
+            turns.start()
+        second = None
+        while second is None:
+            idle = not turns.is_alive()
+            try:
+                second = other()
+            except ane.EngineError:
+                assert not idle
+        if not busy:
+            turns.start()
+        turns.join()
+        assert losses == want[0] and second.step().loss == want[1]
+        second.close()
+        e.close()
+    finally:
+        ane._ffi.lib.ane_dev_free(filler)
