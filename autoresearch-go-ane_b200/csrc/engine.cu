@@ -1084,7 +1084,8 @@ void EngineT<T>::reserve_parts() {
 template <typename T>
 void EngineT<T>::alloc_halves() {
   halves_.assign(L_, Halves());
-  if (!x3_) return;
+  const char* env = getenv("ANE_B200_HALVES");  // 0: none, as without memory for them
+  if (!x3_ || (env && env[0] == '0')) return;
   size_t free_bytes = 0, total = 0;
   if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
     cudaGetLastError();

@@ -578,6 +578,13 @@ def test_split_precision_operands_of_odd_widths_cut_once(arch, quirks):
     e.close()
 
 
+@pytest.mark.parametrize("arch,quirks", [(O.ARCH_L, 0), (O.ARCH_N, 1)])
+def test_split_precision_operands_of_odd_widths_cut_for_each_product(arch, quirks, monkeypatch):
+    """Where there is no memory for the halves of a whole pass."""
+    monkeypatch.setenv("ANE_B200_HALVES", "0")
+    test_split_precision_operands_of_odd_widths_cut_once(arch, quirks)
+
+
 def test_split_precision_head_with_a_token_outside_the_vocabulary_reference_arch():
     """The case that plain bf16 fails (xfail above) in the split-precision mode: inside the stated tolerance."""
     cfg = dict(dim=128, hidden=256, heads=2, layers=2, vocab=512, seq=128)
@@ -670,6 +677,46 @@ def test_gradients_that_the_next_pass_overwrites(dim, hidden, batch, seq):
         b.import_tensor(*n, a.export_tensor(*n, O.W))
     b.step_tokens(inp, tgt)
     assert rel_l2(a.export_tensor(t, l, O.G), b.export_tensor(t, l, O.G) + g) < 2e-6
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("arch,dim,hidden,heads,batch,seq,vocab,hyper,unfused", [
+    (O.ARCH_N, 128, 256, 4, 3, 37, 512, {}, False),                        # the smear gate lies between matrices and embedding
+    (O.ARCH_L, 128, 256, 4, 4, 64, 520, dict(ce_chunk_cols=256), False),   # blocks of the vocabulary store rows of their own, the last 8
+    (O.ARCH_L, 128, 256, 4, 5, 40, 512, dict(ce_chunk_rows=72), True),     # the first chunk of rows stores, the others add
+    (O.ARCH_L, 1296, 2592, 18, 3, 152, 512, {}, False)])                   # the embedding's product adds in shares: cleared before it
+def test_gradients_that_other_heads_overwrite(arch, dim, hidden, heads, batch, seq, vocab, hyper, unfused, monkeypatch):
+    """As above, for the forms that the first product into the embedding's gradient takes; the first micro-step behind an update is
+    seen to store weight gradients (EPI_STORE_F32 with both operands MN-major, which nothing else takes) where the other engine adds."""
+    import re
+    import torch
+    if unfused:
+        monkeypatch.setenv("ANE_B200_HEAD_UNFUSED", "1")
+    cfg = dict(dim=dim, hidden=hidden, heads=heads, layers=2, vocab=vocab, seq=seq)
+    a, b = (make_pair(ane, cfg, arch=arch, quirks=0, dtype=ane.DTYPE_BF16, batch=batch, hyper=dict(lr=1e-3, accum_steps=1000, **hyper))[1]
+            for _ in range(2))
+    names = [(t, l) for t in O.TENSOR_NAMES for l in range(2) if a.tensor_size(t, l) > 0]
+    for update in range(2):
+        inp, tgt = batch_tokens(cfg, batch, 31 + update, invalid=False)
+        b.export_tensor(*names[0], O.G)
+        for e, stores in ((a, update > 0), (b, False)):
+            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+                e.step_tokens(inp, tgt)
+                torch.cuda.synchronize()
+            products = [re.findall(r"gemm_tc_kernel<(.*?)>", ev.key) for ev in prof.key_averages()]
+            products = [re.sub(r"\(\w+\)|\s", "", found[0]).replace("true", "1").split(",") for found in products if found]
+            if products:  # (nothing was recorded where the profiler has no access to the device)
+                assert stores == any(p[2:] == ["1", "1", "1"] for p in products), products
+        a.step_tokens(inp, tgt)
+        b.step_tokens(inp, tgt)
+        for t, l in names:
+            assert rel_l2(a.export_tensor(t, l, O.G), b.export_tensor(t, l, O.G)) < 2e-6, (O.TENSOR_NAMES[t], l)
+        a.flush()
+        b.flush()
+        for t, l in names:
+            for w in (O.W, O.M, O.V):
+                b.import_tensor(t, l, a.export_tensor(t, l, w), w)
     a.close()
     b.close()
 
