@@ -409,6 +409,8 @@ void rmsnorm_backward(const float* dy, const float* x, const float* w, const flo
   if (M <= 0) return;
   int blocks = (M + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (rmsnorm_backward_adds(D)) {
+    // Few rows go to more SMs, at least four warps a block (1000 rows of 768 9.8 -> 9.4 us, 48 rows 6.4 -> 5.5, 256 rows 10.7 -> 11.0; three
+    // micro-steps of 5 x 200 tokens 2829 -> 2800 us an update, one window of 256 the same).
     const int warps = std::min(std::max((M + 147) / 148, 4), kRmsBwdWarps), rb = std::min((M + warps - 1) / warps, 148);
 #define ANE_RMS_BWD_CASE(NV)                                                                                      \
   case NV:                                                                                                         \
