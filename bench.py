@@ -71,10 +71,9 @@ TRAIN_FLOPS_PER_TOKEN = train_flops_per_token(WORKLOAD, "llama")
 
 # DRAM bytes (read + write) of all gemm_tc_kernel launches of one 110M step, from an ncu capture of this
 # command; bench.py cannot run ncu itself, so the figure is tagged with the commit it was taken at.
-GEMM_TRAFFIC = {"dram_bytes_per_step": 12312445952,
+GEMM_TRAFFIC = {"dram_bytes_per_step": 12340527104,
                 "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum over the 169 gemm_tc_kernel launches of one step "
-                          "(--cache-control none, one pass per launch), captured at commit 883cf8c; 14.42 GB with the "
-                          "stored-logits head"}
+                          "(--cache-control none, one pass per launch), captured at commit 973e595"}
 
 
 def zipf_tokens(n, vocab, seed, s=1.1):
