@@ -701,7 +701,7 @@ def test_gradients_that_other_heads_overwrite(arch, dim, hidden, heads, batch, s
         inp, tgt = batch_tokens(cfg, batch, 31 + update, invalid=False)
         b.export_tensor(*names[0], O.G)
         for e, stores in ((a, update > 0), (b, False)):
-            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
                 e.step_tokens(inp, tgt)
                 torch.cuda.synchronize()
             products = [re.findall(r"gemm_tc_kernel<(.*?)>", ev.key) for ev in prof.key_averages()]
