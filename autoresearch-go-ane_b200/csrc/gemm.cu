@@ -795,7 +795,8 @@ size_t gemm_group_slot_bytes() { return sizeof(GemmGroup); }
 // ------------------------------------------------------------------------------------------
 // Both operands of a product in one launch (blockIdx.y), four values per thread and step.  Operand [rows, cols] fp32
 // with row pitch ld.  Two parts (hi, lo) lie beside one another in each row, [rows][hi (kp) | lo (kp)], kp = cols rounded up to 64,
-// whichever way a product contracts: what has been cut for one serves the others.  Three (hi, mid, lo) lie behind one another along
+// whichever way a product contracts: what has been cut for one serves the others (up to 8 where it is cut for one that contracts over
+// rows alone).  Three (hi, mid, lo) lie behind one another along
 // the contraction: for a K-major operand (k = cols) [rows][hi (kp) | mid | lo], for an MN-major one (k = rows) [hi (kp rows) | mid |
 // lo][cols rounded up to 8], kp = k rounded up to a whole k-block.  What lies past cols, or k, is zero.  Three parts are exactly F32TC_SCALE times the fp32 value; where that is not
 // finite, or its first part is not, the others are not either.
@@ -953,7 +954,8 @@ int gemm_bf16x3(const GemmDesc& d, SplitScratch* sc, int* d_status, cudaStream_t
   for (int i = 0; i < 2; ++i) {
     const bool mn = i == 0 ? d.a_mn : d.b_mn;
     const int outer = i == 0 ? d.M : d.N, rows = mn ? d.K : outer, cols = mn ? outer : d.K;
-    pitch[i] = halves_pitch(cols);
+    // (an operand of few columns that contracts over its rows would be up to eight times as wide in whole k-blocks)
+    pitch[i] = mn && halves[i] == nullptr ? (cols + 7) / 8 * 16 : halves_pitch(cols);
     if (halves[i] != nullptr && (i == 0 ? d.a_cut : d.b_cut)) continue;
     if (halves[i] == nullptr) {
       if (const int rc = sc->grow(i, sizeof(bf16) * (size_t)rows * pitch[i], stream); rc != 0) return rc;

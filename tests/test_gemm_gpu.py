@@ -509,6 +509,33 @@ t.lib.ane_dev_free(filler)
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("M,N,K", [(8, 8, 200), (40, 136, 72), (72, 24, 1000), (200, 8, 64), (264, 328, 130)])
+def test_split_precision_of_thin_operands(M, N, K):
+    """MN-major operands of widths that are no multiple of a k-block, hi beside lo: the tolerance of the other layouts above."""
+    rng = np.random.default_rng(M + N)
+    A, B, C0 = (rng.standard_normal(s).astype(np.float32) for s in ((K, M), (K, N), (M, N)))
+    want = A.astype(np.float64).T @ B
+    got = _gemm(ane.DTYPE_BF16X3, A, B, np.zeros((M, N), np.float32), M, N, K, 1, 1, 1)
+    assert rel_l2(got, want) < 2e-5
+    got = _gemm(ane.DTYPE_BF16X3, A, B, C0, M, N, K, 1, 1, 2)
+    assert rel_l2(got, want + C0) < 2e-5
+
+
+def test_split_precision_of_thin_operands_takes_little_memory():
+    """A million rows of eight columns, twice: 64 MiB of halves and not 512.  Whole numbers: exact in any order of addition."""
+    import torch
+    rng = np.random.default_rng(7)
+    K = 1 << 20
+    A, B = (rng.integers(-1, 2, (K, 8)).astype(np.float32) for _ in range(2))
+    filler = lib.ane_dev_malloc(torch.cuda.mem_get_info()[0] - (300 << 20))
+    assert filler
+    try:
+        got = _gemm(ane.DTYPE_BF16X3, A, B, np.zeros((8, 8), np.float32), 8, 8, K, 1, 1, 1)
+    finally:
+        lib.ane_dev_free(filler)
+    np.testing.assert_array_equal(got, A.T @ B)
+
+
 def test_gemm_rejects_misaligned_pitch():
     A = np.zeros((16, 20), np.float32)  # 20 bf16 = 40 bytes per row: not a 16-byte multiple
     dA, dB, dC = _up_bf16(A), _up_bf16(A), _up(np.zeros((16, 16), np.float32))
