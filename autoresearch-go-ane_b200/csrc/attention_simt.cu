@@ -585,16 +585,20 @@ void launch_forward(const T* qkv, TO* out, float* lse, int B, int seq, int H, in
   smem_opt_in(kern, Simt<HDP>::fwd_smem(BUFS), done);
   launch_pdl(kern, dim3(B * H, (seq + kRes - 1) / kRes), dim3(kSimtThreads), Simt<HDP>::fwd_smem(BUFS), s, qkv, out, lse, seq, H, KV, hd, scale);
 }
-// Two buffers where they leave (nearly) all blocks resident, else one, so that more blocks hide one another's loads.  us, one / two:
-// 240 blocks of head size 64, seq 128, 21.7 / 15.5, 384 blocks, seq 256, 26.7 / 23.2, 576 blocks, seq 192, 24.7 / 29.3, 2400 blocks, seq 256,
-// 99.6 / 130.1; head size 48, seq 256: 384 blocks 30.0 / 24.8, 1200 blocks 46.1 / 47.9.  With one tile there is nothing to request
-// early: 384 blocks of head size 64, seq 64, 11.2 / 19.9, but 216 blocks 14.1 / 10.3 (they spread over the SMs).
+// Two buffers of streamed tiles, or one and more blocks an SM, which hide one another's loads?  `turns` tiles pass through the longest
+// block; `resident` blocks fit the SMs with two buffers.  Step of split precision, six layers of eight heads of 64, us, one / two buffers
+// in the forward kernel, and in the one for dK and dV beside two in the forward: seq 256, 384 blocks 2127 / 2093 / 2027, 576 blocks 2511 /
+// 2505, 2501 / 2505, 768 blocks 3029 / 3076, 3090 with two for dK and dV alone; seq 128, 384 blocks 1773 / 1760 / 1740, 576 blocks 2062 / 2082,
+// 2093.  With one tile there is nothing to request early, but few blocks spread over more SMs: 192 blocks of fp32, four layers,
+// 969 / 953 / 936, 512 blocks 1393 / 1421 / 1441.
+bool two_buffers(long long blocks, int turns, long long resident) { return blocks <= (turns == 1 ? resident : 148 * (turns < 4 ? 3 : 4)); }
+
 template <int HDP, typename T, typename TO>
 void forward_hdp(const T* qkv, TO* out, float* lse, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
   if constexpr (Simt<HDP>::kTwoBuffers && sizeof(T) == 4) {
     constexpr long long resident = 148 * (kSmemOfSm / (Simt<HDP>::fwd_smem(2) + 1024));
     const long long blocks = (long long)B * H * ((seq + kRes - 1) / kRes);
-    if (blocks <= (seq > kStr ? resident * 4 / 3 : resident)) return launch_forward<HDP, 2>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
+    if (two_buffers(blocks, (seq + kStr - 1) / kStr, resident)) return launch_forward<HDP, 2>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
   }
   launch_forward<HDP, 1>(qkv, out, lse, B, seq, H, KV, hd, scale, s);
 }
@@ -606,23 +610,20 @@ void launch_dkv(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B,
   launch_pdl(kern, dim3(B * KV, (seq + kRes - 1) / kRes), dim3(kSimtThreads), Simt<HDP>::dkv_smem(BUFS), s, qkv, d_out, dqkv, stats, B * H * seq, seq, H,
              KV, hd, scale);
 }
-// As in the forward pass, but up to four blocks an SM (two or three are resident).  us, one / two: 192 blocks of head size 64, seq 256, 118.9 / 55.2, 576 blocks 72.8 / 64.6, 1152 blocks 110.1 /
-// 119.0; head size 48, seq 256: 576 blocks 54.5 / 47.5, 1200 blocks 85.5 / 97.1; one tile of 64, head size 64: 216 blocks 27.8 / 25.2, 384
-// blocks 29.5 / 37.6; head size 32: 384 blocks 22.5 / 18.2, 592 blocks, seq 48, 23.6 / 30.9.
 template <int HDP, typename T, typename TD>
 void dkv_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
   if constexpr (Simt<HDP>::kTwoBuffers && sizeof(T) == 4) {
     constexpr long long resident = 148 * (kSmemOfSm / (Simt<HDP>::dkv_smem(2) + 1024));
     const long long blocks = (long long)B * KV * ((seq + kRes - 1) / kRes);
-    if (blocks <= (seq > kStr || H > KV ? 148 * 4 : resident)) return launch_dkv<HDP, 2>(qkv, d_out, dqkv, stats, B, seq, H, KV, hd, scale, s);
+    if (two_buffers(blocks, (seq + kStr - 1) / kStr * (H / KV), resident)) return launch_dkv<HDP, 2>(qkv, d_out, dqkv, stats, B, seq, H, KV, hd, scale, s);
   }
   launch_dkv<HDP, 1>(qkv, d_out, dqkv, stats, B, seq, H, KV, hd, scale, s);
 }
 // dQ of two to four tiles of keys, in fp32: the kernel that keeps everything of its first sweep, with shared memory for the tiles that
-// there are.  us, two sweeps / kept: head size 64, 1200 blocks, seq 100, 102.8 / 95.9, 1152 blocks, seq 192, 111.3 / 95.4, 192 blocks, seq
-// 256, 80.5 / 48.6; head size 48, 1176 blocks, seq 100, 81.5 / 70.8.  One tile is swept once by the other kernel as well, in less shared
-// memory: 1176 blocks of head size 64, seq 48, 70.2 / 77.3.  Four tiles of head size 64 leave one block an SM, which pays up to three
-// rounds of blocks: seq 256, 384 blocks 84.5 / 69.5, 576 blocks 82.4 / 88.9, 2400 blocks 267 / 269.
+// there are.  The same steps, two sweeps / kept: seq 192, 384 blocks 2007 / 1847, 720 blocks 2766 / 2690; head size 48, seq 128, 1176 blocks
+// of fp32, 2256 / 2217.  One tile is swept once by the other kernel as well, in less shared memory: 1776 blocks of fp32, 3113 / 3152.  Four
+// tiles of head size 64 leave one block an SM, which pays up to four rounds of blocks: seq 256, 384 blocks 2162 / 2027, 448 blocks
+// 2303 / 2197, 576 blocks 2556 / 2501, 768 blocks 3029 / 3091.
 template <int HDP, typename T, typename TD>
 void backward_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
   const int tiles = (seq + kStr - 1) / kStr, rows = B * H * seq;
@@ -630,7 +631,7 @@ void backward_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int 
   bool kept = false;
   if constexpr (Simt<HDP>::kTwoBuffers && sizeof(T) == 4 && sizeof(TD) == 4) {
     kept = tiles > 1 && tiles <= kShortTiles &&
-           (2 * (Simt<HDP>::dq_short_smem(tiles) + 1024) <= kSmemOfSm || (long long)grid.x * grid.y <= 148 * 3);
+           (2 * (Simt<HDP>::dq_short_smem(tiles) + 1024) <= kSmemOfSm || (long long)grid.x * grid.y <= 148 * 4);
     if (kept) {
       auto kern = attention_dq_short_simt_kernel<HDP>;
       static unsigned long long done = 0;
