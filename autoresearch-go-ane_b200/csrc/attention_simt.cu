@@ -623,15 +623,16 @@ void dkv_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, in
 // there are.  The same steps, two sweeps / kept: seq 192, 384 blocks 2007 / 1847, 720 blocks 2766 / 2690; head size 48, seq 128, 1176 blocks
 // of fp32, 2256 / 2217.  One tile is swept once by the other kernel as well, in less shared memory: 1776 blocks of fp32, 3113 / 3152.  Four
 // tiles of head size 64 leave one block an SM, which pays up to four rounds of blocks: seq 256, 384 blocks 2162 / 2027, 448 blocks
-// 2303 / 2197, 576 blocks 2556 / 2501, 768 blocks 3029 / 3091.
+// 2303 / 2197, 576 blocks 2556 / 2501, 768 blocks 3029 / 3091.  Two tiles of head size 32 have little to sweep again: 192 blocks of
+// fp32, four layers, seq 100, 805 / 792, but seq 128, 960 blocks 1451 / 1496, 1184 blocks 1679 / 1740.
 template <int HDP, typename T, typename TD>
 void backward_hdp(const T* qkv, const TD* d_out, float* dqkv, float* stats, int B, int seq, int H, int KV, int hd, float scale, cudaStream_t s) {
   const int tiles = (seq + kStr - 1) / kStr, rows = B * H * seq;
   const dim3 grid(B * H, (seq + kRes - 1) / kRes);
   bool kept = false;
   if constexpr (Simt<HDP>::kTwoBuffers && sizeof(T) == 4 && sizeof(TD) == 4) {
-    kept = tiles > 1 && tiles <= kShortTiles &&
-           (2 * (Simt<HDP>::dq_short_smem(tiles) + 1024) <= kSmemOfSm || (long long)grid.x * grid.y <= 148 * 4);
+    const bool few = (long long)grid.x * grid.y <= 148 * 4;
+    kept = tiles > (HDP > 32 || few ? 1 : 2) && tiles <= kShortTiles && (few || 2 * (Simt<HDP>::dq_short_smem(tiles) + 1024) <= kSmemOfSm);
     if (kept) {
       auto kern = attention_dq_short_simt_kernel<HDP>;
       static unsigned long long done = 0;
